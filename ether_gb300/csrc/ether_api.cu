@@ -207,7 +207,7 @@ void free_ctx(Ctx &c) {
                     c.t.mweight, c.t.site_of_storage, c.spins, c.spins4, c.beta_slot,
                     c.beta_slot_f, c.slot_of_rep, c.rep_of_slot, c.thr, c.stream_id,
                     c.step, c.ovrr_step, c.fresh_call, c.acc_count, c.E, c.M, c.sums,
-                    c.partials, c.pt_accepts, c.swap_dev, c.copy_from, c.err, c.spiral_ptr,
+                    c.partials, c.pt_accepts, c.swap_dev, c.copy_from, c.spiral_ptr,
                     c.spiral_nbr, c.acc_before, c.acc_ratio, c.spiral_part, c.spiral_sums,
                     c.acc_slot, c.acc_mark, c.t.sia_cls, c.t.sia_ax, c.t.mweight_f, c.t.storage};
     for (void *p : ptrs)
@@ -553,6 +553,7 @@ extern "C" int ether_create(const ether_desc *d, ether_ctx **out) {
     TRY(dev_alloc(c, &c.M, 3 * (size_t)c.R));
     TRY(dev_alloc(c, &c.sums, 7 * (size_t)c.R));
     c.partial_blocks = energy_blocks(c);
+    if (c.fast && c.model == ETHER_MODEL_ISING) c.ising_vpt = ising_default_vpt(c);
     {
         // small simple-cubic Ising lattices: ether_mcs keeps each replica in shared memory for
         // the sweeps between two PT or measurement steps, when the replicas alone fill the GPU
@@ -567,13 +568,11 @@ extern "C" int ether_create(const ether_desc *d, ether_ctx **out) {
     TRY(dev_alloc(c, &c.partials, (size_t)c.R * c.partial_blocks * 5));
     TRY(dev_alloc(c, &c.pt_accepts, 1));
     TRY(dev_alloc(c, &c.swap_dev, 1));
-    TRY(dev_alloc(c, &c.err, 1));
     TRY(dev_alloc(c, &c.acc_before, c.R));
     TRY(dev_alloc(c, &c.acc_ratio, c.R));
     TRY(dev_alloc(c, &c.acc_slot, c.R));
     TRY(dev_alloc(c, &c.acc_mark, c.R));
     CUDA_TRY(cudaMallocHost((void **)&c.acc_host, sizeof(double) * c.R));
-    CUDA_TRY(cudaMemset(c.err, 0, sizeof(int)));
     TRY(dev_alloc(c, &c.copy_from, c.R));
 #undef TRY
     std::vector<uint32_t> sid(c.R);
@@ -1619,12 +1618,6 @@ extern "C" int ether_get_colouring(ether_ctx *h, int32_t *colour, int32_t *rank_
 extern "C" int ether_sync(ether_ctx *h) {
     if (!h) return fail(ETHER_ERR_ARG, "null context");
     CUDA_TRY(cudaStreamSynchronize(h->c.stream));
-    int e = 0;
-    CUDA_TRY(cudaMemcpy(&e, h->c.err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (e) {
-        CUDA_TRY(cudaMemset(h->c.err, 0, sizeof(int)));
-        return fail(ETHER_ERR_TIMEOUT, "a staged sweep kernel's bounded wait ran out (code " + std::to_string(e) + ")");
-    }
     return ETHER_OK;
 }
 
@@ -1663,60 +1656,44 @@ std::map<std::vector<long>, int> g_tune_cache;  // variant per (model, L, R)
 
 static int variant_of(const Ctx &c) {
     if (c.model == ETHER_MODEL_XYZ) return 5000 + c.xyz_variant;
-    if (c.ising_stream) return 4000 + 10 * c.ising_vpt + (c.ising_cap ? 4 : 1);
-    if (c.ising_cap5) return 6000 + c.vec_bytes * 10 + c.ising_vpt;
-    return (c.ising_persist ? 1000 : 0) + (c.ising_cap ? 2000 : 0) + c.vec_bytes * 10 + c.ising_vpt;
+    return c.ising_code ? c.ising_code : c.vec_bytes * 10 + c.ising_vpt;
 }
 
 namespace ether {
 int ctx_variant(const Ctx &c) { return variant_of(c); }
 }  // namespace ether
 
-// variant = 1000 (persistent kernel) + 2000 (register cap: four 256-thread blocks per SM)
-//           + 10 * bytes per vector + vectors per thread
-//           or 6162: the phase kernel capped at five blocks per SM (two 16-byte vectors
-//           per thread in 48 registers)
-//           or 4000 + 10 * vectors per thread and step + 1 / 4 (register cap): the
-//           shared-memory staged kernel (4011, 4014, 4021, 4041)
-//           or 5000 + 10 * sites per thread + register cap (blocks per SM) for the
-//           simple-cubic XYZ kernel (5011 .. 5015, 5021 .. 5024, 5041, 5042; with two or
-//           more sites per thread a warp draws the second Philox block of its sites together)
+// Ising: variant = 10 * bytes per vector + vectors per thread (1, 2, 4); + 1000 doubles the
+// vectors per thread (of 2 and 4).  + 2000 and 6162 named register caps, which the 16-byte
+// kernels now always have, 4011, 4014, 4021, 4041 a staged kernel (k_ising.cu): still accepted,
+// they run the kernel of their vector size and count.
+// XYZ: 5000 + 10 * sites per thread + register cap (blocks per SM) for the simple-cubic XYZ
+// kernel (5011 .. 5015, 5021, 5022).
 static bool apply_variant(Ctx &c, int variant) {
     if (c.model == ETHER_MODEL_XYZ) {
         if (!xyz_variant_valid(variant - 5000)) return false;
         c.xyz_variant = variant - 5000;
         return true;
     }
+    int w = 16, v;
     if (variant == 4011 || variant == 4014 || variant == 4021 || variant == 4041) {
-        const int vs = (variant / 10) % 10;
-        if (!ising_stream_supported(c, vs)) return false;
-        c.ising_stream = true;
-        c.ising_cap5 = false;
-        c.ising_cap = variant % 10 == 4;
-        c.vec_bytes = 16;
-        c.ising_vpt = vs;
-        return true;
-    }
-    if (variant == 6162) {
+        v = (variant / 10) % 10;
+        if (!ising_staged_shape(c, v)) return false;
+    } else if (variant == 6162) {
+        v = 2;
         if ((c.L[0] / 2) % 16) return false;
-        c.ising_stream = false;
-        c.ising_persist = false;
-        c.ising_cap = false;
-        c.ising_cap5 = true;
-        c.vec_bytes = 16;
-        c.ising_vpt = 2;
-        return true;
+    } else {
+        if (variant < 0 || variant >= 4000) return false;
+        const bool twice = (variant / 1000) & 1, cap = (variant / 1000) >= 2;
+        const int rest = variant % 1000;
+        w = rest / 10;
+        v = rest % 10;
+        if ((w != 4 && w != 8 && w != 16) || (c.L[0] / 2) % w) return false;
+        if (twice ? (v != 2 && v != 4) : (v != 1 && v != 2 && v != 4)) return false;
+        if (cap && (w != 16 || v == 1)) return false;
+        if (twice) v *= 2;
     }
-    if (variant < 0 || variant >= 4000) return false;
-    c.ising_stream = false;
-    c.ising_cap5 = false;
-    const bool p = (variant / 1000) & 1, cap = (variant / 1000) >= 2;
-    const int rest = variant % 1000, w = rest / 10, v = rest % 10;
-    if ((w != 4 && w != 8 && w != 16) || (c.L[0] / 2) % w) return false;
-    if (p ? (v != 2 && v != 4) : (v != 1 && v != 2 && v != 4)) return false;
-    if (cap && (w != 16 || v == 1)) return false;
-    c.ising_persist = p;
-    c.ising_cap = cap;
+    c.ising_code = variant;
     c.vec_bytes = w;
     c.ising_vpt = v;
     return true;
@@ -1809,13 +1786,12 @@ extern "C" int ether_autotune(ether_ctx *h, int32_t *variant, float *best_ms) {
     CUDA_TRY(cudaMemcpyAsync(backup, c.spins, bytes, cudaMemcpyDeviceToDevice, c.stream));
     CUDA_TRY(cudaMemcpyAsync(acc_backup, c.acc_count, sizeof(unsigned long long) * c.R,
                              cudaMemcpyDeviceToDevice, c.stream));
-    int best_var = variant_of(c);
+    int best_var = c.vec_bytes * 10 + (c.ising_vpt == 8 ? 1004 : c.ising_vpt);
     float best = 1e30f;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    for (int cand : {161, 162, 164, 81, 82, 84, 41, 42, 44, 2162, 2164, 6162, 1162, 1164, 1082, 1084, 1042,
-                     1044, 3162, 3164, 4011, 4014, 4021, 4041}) {
+    for (int cand : {161, 162, 164, 1164, 81, 82, 84, 1084, 41, 42, 44, 1044}) {
         if (!apply_variant(c, cand)) continue;
         CUDA_TRY(launch_ising_sweep(c, 0));  // warm-up
         CUDA_TRY(cudaEventRecord(e0, c.stream));

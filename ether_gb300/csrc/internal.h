@@ -118,13 +118,9 @@ struct Ctx {
     int32_t *rep_of_slot = nullptr;  // R (group*n_slots + slot -> replica)
     uint32_t *thr = nullptr;     // n_slots * table_entries: flip iff u32 <= thr
     int ising_vpt = 1;           // vectors per thread of the simple-cubic Ising kernel
-    bool ising_persist = false;  // persistent simple-cubic Ising kernel
-    bool ising_cap = false;      // register-capped (four blocks per SM) instantiation
-    bool ising_cap5 = false;     // register-capped to five blocks per SM (48 registers)
-    bool ising_stream = false;   // shared-memory staged simple-cubic Ising kernel
+    int ising_code = 0;          // the variant that was asked for (0: the default choice)
     int xyz_variant = 11;        // simple-cubic XYZ kernel: 10 * sites per thread + blocks per SM cap
     bool resident = false;       // ether_mcs runs runs of sweeps with ising_sc_resident
-    int *err = nullptr;          // device: first bounded-wait failure of a kernel (0 = none)
     unsigned long long *acc_before = nullptr;  // R: acceptance counts at the start of a call
     double *acc_ratio = nullptr;               // R: device acceptance ratios of a call
     double *acc_host = nullptr;                // R: pinned host copy
@@ -239,7 +235,8 @@ cudaError_t launch_ising_sweep(Ctx &c, int colour);
 bool ising_resident_possible(const Ctx &c, size_t smem_max);
 cudaError_t prepare_ising_resident(const Ctx &c);
 cudaError_t launch_ising_resident(Ctx &c, int nsweeps);
-bool ising_stream_supported(const Ctx &c, int vectors_per_step);
+bool ising_staged_shape(const Ctx &c, int vectors_per_step);
+int ising_default_vpt(const Ctx &c);
 cudaError_t launch_xyz_sweep(Ctx &c, int colour);
 bool xyz_variant_valid(int variant);
 cudaError_t launch_overrelax(Ctx &c, int colour, int pass, float part);

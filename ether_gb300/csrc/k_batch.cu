@@ -70,7 +70,7 @@ struct BatchSeg {
 // One segment of a member of each class.  m lives in shared memory.
 template <int W>
 __device__ __forceinline__ unsigned batch_ising_sc(const BatchMember &m, uint32_t r, int first, int end,
-                                                   uint32_t colour, const uint32_t *s_th, const uint32_t *s_tl,
+                                                   uint32_t colour, const ScTab &tab,
                                                    uint32_t t, uint32_t stream, int upt) {
     const uint32_t c3 = kMetro | (colour << 8);
     const int half = m.H * m.L2 * m.L3;
@@ -80,7 +80,7 @@ __device__ __forceinline__ unsigned batch_ising_sc(const BatchMember &m, uint32_
     unsigned acc = 0;
     for (int j = 0; j < upt; ++j) {
         const int v = first + (int)threadIdx.x + j * (int)blockDim.x;
-        acc += byte_sum(ising_sc_vectors<W, 1>(A, v, 0, end, s_th, s_tl, t, stream, c3, m.seed, m.K));
+        acc += byte_sum(ising_sc_vectors<W, 1>(A, v, 0, end, tab, t, stream, c3, m.seed, m.K));
     }
     return acc;
 }
@@ -150,7 +150,7 @@ batch_phase_kernel(const BatchMember *__restrict__ members, const BatchSeg *__re
     // parameters cost no registers.
     constexpr bool kIsingSc = CLS == kCIsing16 || CLS == kCIsing8 || CLS == kCIsing4;
     __shared__ BatchMember s_m[8];
-    __shared__ uint32_t s_th[8][kIsingSc ? 16 : 1], s_tl[8][kIsingSc ? 16 : 1];
+    __shared__ uint32_t s_tab[8][kIsingSc ? kScTabWords : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     BatchMember &m = s_m[warp];
     uint32_t cur_member = 0xFFFFFFFFu, cur_rep = 0xFFFFFFFFu;
@@ -169,11 +169,8 @@ batch_phase_kernel(const BatchMember *__restrict__ members, const BatchSeg *__re
         }
         if constexpr (kIsingSc) {
             if (S.member != cur_member || r != cur_rep) {
-                if (lane < 14) {
-                    const uint32_t T = m.thr[(size_t)m.slot_of_rep[r] * m.table_entries + lane];
-                    s_th[warp][lane] = T >> 16;
-                    s_tl[warp][lane] = T & 0xFFFFu;
-                }
+                __syncwarp();
+                fill_sc_table(m.thr + (size_t)m.slot_of_rep[r] * m.table_entries, s_tab[warp], lane, 32);
                 __syncwarp();
             }
         }
@@ -183,11 +180,11 @@ batch_phase_kernel(const BatchMember *__restrict__ members, const BatchSeg *__re
         const int first = (int)S.first, end = (int)(S.first + S.count);
         unsigned acc;
         if constexpr (CLS == kCIsing16)
-            acc = batch_ising_sc<16>(m, r, first, end, colour, s_th[warp], s_tl[warp], t, stream, upt);
+            acc = batch_ising_sc<16>(m, r, first, end, colour, sc_tab(s_tab[warp]), t, stream, upt);
         else if constexpr (CLS == kCIsing8)
-            acc = batch_ising_sc<8>(m, r, first, end, colour, s_th[warp], s_tl[warp], t, stream, upt);
+            acc = batch_ising_sc<8>(m, r, first, end, colour, sc_tab(s_tab[warp]), t, stream, upt);
         else if constexpr (CLS == kCIsing4)
-            acc = batch_ising_sc<4>(m, r, first, end, colour, s_th[warp], s_tl[warp], t, stream, upt);
+            acc = batch_ising_sc<4>(m, r, first, end, colour, sc_tab(s_tab[warp]), t, stream, upt);
         else if constexpr (CLS == kCIsingEll)
             acc = batch_ising_ell(m, r, first, end, colour, t, stream);
         else if constexpr (CLS == kCXyzScX)

@@ -96,8 +96,7 @@ __device__ __forceinline__ bool ising_ell_site(const IsingEll &A, int rho, uint3
 // All six neighbours live in the other colour's array: same xh in rows (y±1,z), (y,z±1),
 // and xh, xh∓1 in row (y,z).  A thread takes W (4, 8 or 16) consecutive bytes of one row
 // (W | H): half of a random-number group, one or two.  Byte sums of 0/1 spins never carry
-// (max 6); e = n + 7 s (<= 13) is formed for four sites at once; flips are one predicated
-// XOR per site and are counted with popc.
+// (max 6); the table indices e = n + 7 s (<= 13) are formed for four sites at once.
 template <int W>
 struct Vec {
     uint32_t w[W / 4];
@@ -128,27 +127,52 @@ __device__ __forceinline__ void stv(uint8_t *p, const Vec<W> &v) {
     }
 }
 
-// Sites of word q (odd: words 1, 3 of the group's blocks) whose high random halves tie with
-// their threshold's high half: decided by the low halves (block 1 of the group).  Returns
-// the XOR mask of the extra flips.  Kept out of line: it runs for about one vector in 4000
-// and must not cost the hot loop registers.
-__device__ __noinline__ inline uint32_t resolve_ties(uint32_t grp, uint32_t t, uint32_t stream,
-                                                     uint32_t c3, uint32_t seed, int odd,
-                                                     uint32_t e4s, const uint32_t *s_th,
-                                                     const uint32_t *s_tl) {
+// Thresholds of a replica, in shared memory.  The decision is taken for two sites at once: one
+// 32-bit load, indexed by the two sites' e = n + 7 s (n up neighbours, s the own spin;
+// e <= 13), gives both thresholds' high halves, packed as the random halves are:
+// pair[14 e0 + e1] = (T[e1] >> 16) << 16 | T[e0] >> 16 (e0: the site in the low halfword);
+// thr[e] = the whole T (for the rare ties).  At T_c the 32 lanes' loads take 2.5 wavefronts on
+// average with the row length 14, 3.4 with 16 (bank = index mod 32; counted on a 64^3
+// configuration).
+struct ScTab {
+    const uint32_t *pair;  // kPairEntries words
+    const uint32_t *thr;   // 14 words
+};
+constexpr int kPairEntries = 14 * 14;
+constexpr int kScTabWords = kPairEntries + 14;
+
+// Fills a replica's table (kScTabWords words at tab) from its 14 thresholds in global memory;
+// the caller synchronises the n threads.
+__device__ __forceinline__ void fill_sc_table(const uint32_t *__restrict__ thr, uint32_t *tab, int tid, int n) {
+    for (int i = tid; i < kScTabWords; i += n) {
+        const int e0 = i / 14, e1 = i - 14 * e0;
+        tab[i] = e0 < 14 ? (thr[e0] >> 16) | (thr[e1] & 0xFFFF0000u) : thr[e1];
+    }
+}
+__device__ __forceinline__ ScTab sc_tab(const uint32_t *tab) { return ScTab{tab, tab + kPairEntries}; }
+
+// The eight sites of a random-number group whose high random halves tie with their
+// threshold's high half: decided by the low halves (block 1 of the group).  E0, E1: bytewise
+// table indices of the group's two words.  Returns the XOR masks of the extra flips (word 0 in
+// the low half of the result).  Kept out of line: it runs for about one vector in 2000 and
+// must not cost the hot loop registers.
+__device__ __noinline__ inline uint64_t resolve_ties(uint32_t grp, uint32_t t, uint32_t stream, uint32_t c3,
+                                                     uint32_t seed, uint32_t E0, uint32_t E1, const uint32_t *thr) {
     const U4 rh = draw(grp, t, stream, c3, seed);
-    const uint32_t ha = odd ? rh.z : rh.x, hb = odd ? rh.w : rh.y;
-    const uint32_t h[4] = {ha & 0xFFFFu, ha >> 16, hb & 0xFFFFu, hb >> 16};
     uint32_t tie = 0;
-    for (int k = 0; k < 4; ++k)
-        if (h[k] == s_th[((e4s >> (8 * k)) & 0xFFu) >> 2]) tie |= 1u << k;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t T = thr[((k < 4 ? E0 : E1) >> (8 * (k & 3))) & 15u];
+        if (half_of(rh, k) == T >> 16) tie |= 1u << k;
+    }
     if (!tie) return 0;
     const U4 rl = draw(grp, t, stream, c3 | (1u << 16), seed);
-    const uint32_t la = odd ? rl.z : rl.x, lb = odd ? rl.w : rl.y;
-    const uint32_t l[4] = {la & 0xFFFFu, la >> 16, lb & 0xFFFFu, lb >> 16};
-    uint32_t m = 0;
-    for (int k = 0; k < 4; ++k)
-        if (((tie >> k) & 1u) && l[k] <= s_tl[((e4s >> (8 * k)) & 0xFFu) >> 2]) m |= 1u << (8 * k);
+    uint64_t m = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t T = thr[((k < 4 ? E0 : E1) >> (8 * (k & 3))) & 15u];
+        if (((tie >> k) & 1u) && half_of(rl, k) <= (T & 0xFFFFu)) m |= 1ull << (8 * k);
+    }
     return m;
 }
 
@@ -160,86 +184,116 @@ struct IsingSc {
     uint32_t colour;
 };
 
-// Word q of a vector: the four sites' threshold byte offsets (4 (n + 7 s)), given the own
-// spins s0 and the six neighbour words.
-template <int W>
-__device__ __forceinline__ uint32_t sc_e4s(const Vec<W> &o0, uint32_t edge, int par, const Vec<W> &a,
-                                           const Vec<W> &b, const Vec<W> &c, const Vec<W> &d, int q,
-                                           uint32_t s0) {
-    constexpr int NW = W / 4;
-    uint32_t sh;
-    if (par == 0) {  // neighbour x-1 -> xh-1: window shifted up by one byte
-        const uint32_t lo = (q == 0) ? (edge << 24) : o0.w[q > 0 ? q - 1 : 0];
-        sh = __funnelshift_l(lo, o0.w[q], 8);
-    } else {         // neighbour x+1 -> xh+1: window shifted down by one byte
-        const uint32_t hi = (q == NW - 1) ? edge : o0.w[q < NW - 1 ? q + 1 : q];
-        sh = __funnelshift_r(o0.w[q], hi, 8);
-    }
-    const uint32_t n = o0.w[q] + sh + a.w[q] + b.w[q] + c.w[q] + d.w[q];
-    // bytewise 4*(n + 7 s) <= 52: the byte offsets of the thresholds in s_th
-    return (n + (s0 << 3) - s0) << 2;
+// Halfword-wise floor((t + ~u) / 2): (t & ~u) + ((t ^ ~u) >> 1), no carry crosses the halves.
+// The logic operations are explicit: the compiler complements u on its own otherwise (five
+// instructions instead of three).
+__device__ __forceinline__ uint32_t havg2_not(uint32_t t, uint32_t u) {
+    uint32_t a, b;
+    asm("lop3.b32 %0, %1, %2, 0, 0x30;" : "=r"(a) : "r"(t), "r"(u));
+    asm("lop3.b32 %0, %1, %2, %3, 0x82;" : "=r"(b) : "r"(t), "r"(u), "r"(0xFFFEFFFEu));
+    return a + (b >> 1);
+}
+// prmt with sign replication: byte i of the result is 0xFF if bit 7 of the selected byte is set.
+__device__ __forceinline__ uint32_t sign_bytes(uint32_t a, uint32_t b) {
+    uint32_t r;  // bytes 1, 3 of a, then 1, 3 of b
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(0xFDB9u));
+    return r;
 }
 
-// The update of one W-byte vector (sites rho0 .. rho0+W-1 of the updated colour) from its own
-// spins `me` and the six neighbour words of the other colour; returns the new spins and adds
-// the flips to the bytewise counts.  A site whose high random half ties with its threshold's
-// high half (probability 2^-16) is decided by the low halves: whether any site of the vector
-// ties is checked once, and the rare vector with a tie is finished by resolve_ties.
+// The decisions of one W-byte vector (sites rho0 .. rho0+W-1 of the updated colour) from its
+// own spins `me` and the bytewise up-neighbour counts n; returns the new spins and adds the
+// flips to cnt as -1 per flip and byte lane (flip_bytes turns the sum into bytewise counts).
+// Two sites per step: with t their thresholds' high halves and u their random halves, bit 15
+// of each half of d = floor((t + ~u) / 2) is u < t, and t == u gives d = 0x7FFF (so does
+// t == u - 1): the minimum over the vector of d + 0x8001 mod 2^16 is zero iff some site may
+// tie (probability 2^-15 each), and only then the words are looked at again by resolve_ties.
+// Bound: ALU and FMA-heavy pipes.  Against one site at a time (a threshold load, an extracted
+// half, two compares and a predicated OR per site: 22.7 instructions per update) this takes
+// about half the instructions; 64^3 x 1024 replicas: see ising_sc_kernel.
 template <int W>
-__device__ __forceinline__ Vec<W> ising_sc_update(const Vec<W> &me, const Vec<W> &o0, const Vec<W> &a,
-                                                  const Vec<W> &b, const Vec<W> &c, const Vec<W> &d,
-                                                  uint32_t edge, int par, int rho0, const uint32_t *s_th,
-                                                  const uint32_t *s_tl, uint32_t t, uint32_t stream,
-                                                  uint32_t c3, uint32_t seed, const RoundKeys &K,
-                                                  uint32_t &cnt) {
+__device__ __forceinline__ Vec<W> ising_sc_decide(const Vec<W> &me, const Vec<W> &n, int rho0, const ScTab &tab,
+                                                  uint32_t t, uint32_t stream, uint32_t c3, uint32_t seed,
+                                                  const RoundKeys &K, uint32_t &cnt) {
     constexpr int NW = W / 4;
-    const char *th_bytes = reinterpret_cast<const char *>(s_th);
     Vec<W> out;
-    uint32_t e4[NW];
-    bool tie = false;
+    uint32_t E[NW];
+    const char *pair = reinterpret_cast<const char *>(tab.pair);
+    uint32_t near = 0xFFFFFFFFu;
     U4 rh{0, 0, 0, 0};
 #pragma unroll
     for (int q = 0; q < NW; ++q) {
         // word q's half of its group's block: q & 1, or for W = 4 the vector's own half
         const int odd = W == 4 ? (rho0 >> 2) & 1 : q & 1;
         if (W == 4 || (q & 1) == 0) rh = draw_rk((uint32_t)((rho0 >> 3) + (q >> 1)), t, stream, c3, K);
-        const uint32_t s0 = me.w[q];
-        const uint32_t e4s = sc_e4s<W>(o0, edge, par, a, b, c, d, q, s0);
-        e4[q] = e4s;
-        const uint32_t t0 = *reinterpret_cast<const uint32_t *>(th_bytes + (e4s & 0xFFu));
-        const uint32_t t1 = *reinterpret_cast<const uint32_t *>(th_bytes + __byte_perm(e4s, 0, 0x4441));
-        const uint32_t t2 = *reinterpret_cast<const uint32_t *>(th_bytes + __byte_perm(e4s, 0, 0x4442));
-        const uint32_t t3 = *reinterpret_cast<const uint32_t *>(th_bytes + (e4s >> 24));
-        const uint32_t wa = odd ? rh.z : rh.x, wb = odd ? rh.w : rh.y;
-        const uint32_t u0 = wa & 0xFFFFu, u1 = wa >> 16, u2 = wb & 0xFFFFu, u3 = wb >> 16;
-        uint32_t m = 0;
-        if (u0 < t0) m |= 0x00000001u;
-        if (u1 < t1) m |= 0x00000100u;
-        if (u2 < t2) m |= 0x00010000u;
-        if (u3 < t3) m |= 0x01000000u;
-        tie |= (u0 == t0) | (u1 == t1) | (u2 == t2) | (u3 == t3);
-        out.w[q] = s0 ^ m;
+        // byte offsets 56 e0 + 4 e1 of the pairs (0, 1) and (2, 3) by one byte dot product each
+        E[q] = me.w[q] * 7u + n.w[q];
+        const uint32_t t01 = *reinterpret_cast<const uint32_t *>(pair + __dp4a(E[q], 0x00000438u, 0u));
+        const uint32_t t23 = *reinterpret_cast<const uint32_t *>(pair + __dp4a(E[q], 0x04380000u, 0u));
+        const uint32_t d01 = havg2_not(t01, odd ? rh.z : rh.x), d23 = havg2_not(t23, odd ? rh.w : rh.y);
+        near = __viaddmin_u16x2(d01, 0x80018001u, near);
+        near = __viaddmin_u16x2(d23, 0x80018001u, near);
+        const uint32_t m = sign_bytes(d01, d23);
+        out.w[q] = me.w[q] ^ (m & 0x01010101u);
         cnt += m;
     }
-    if (tie) {
+    if ((near & 0xFFFFu) == 0 || near < 0x10000u) {
+        if constexpr (W == 4) {  // the vector is one half of its group; the other is not ours
+            const int odd = (rho0 >> 2) & 1;
+            const uint64_t m2 = resolve_ties((uint32_t)(rho0 >> 3), t, stream, c3, seed, E[0], E[0], tab.thr);
+            const uint32_t m = odd ? (uint32_t)(m2 >> 32) : (uint32_t)m2;
+            out.w[0] ^= m;
+            cnt += 255u * m;
+        } else {
 #pragma unroll
-        for (int q = 0; q < NW; ++q) {
-            const uint32_t m = resolve_ties((uint32_t)((rho0 >> 3) + (q >> 1)), t, stream, c3, seed,
-                                            W == 4 ? (rho0 >> 2) & 1 : q & 1, e4[q], s_th, s_tl);
-            out.w[q] ^= m;
-            cnt += m;
+            for (int q = 0; q < NW; q += 2) {
+                const uint64_t m2 = resolve_ties((uint32_t)((rho0 >> 3) + (q >> 1)), t, stream, c3, seed, E[q],
+                                                 E[q + 1], tab.thr);
+                out.w[q] ^= (uint32_t)m2;
+                out.w[q + 1] ^= (uint32_t)(m2 >> 32);
+                cnt += 255u * ((uint32_t)m2 + (uint32_t)(m2 >> 32));
+            }
         }
     }
     return out;
 }
 
+// Bytewise flip counts from ising_sc_decide's sum: that sum is 255 times the counts' word
+// modulo 2^32, and 255 * 0x01010101 = -1 there.
+__device__ __forceinline__ uint32_t flip_bytes(uint32_t cnt) { return 0u - cnt * 0x01010101u; }
+
+// Window of the x neighbours of a vector of the other colour's same row: parity 0 takes the
+// byte before each site (x-1 -> xh-1), parity 1 the byte after it.
+template <int W>
+__device__ __forceinline__ uint32_t sc_side(const Vec<W> &o, uint32_t edge, int par, int q) {
+    constexpr int NW = W / 4;
+    if (par == 0) {
+        const uint32_t lo = (q == 0) ? (edge << 24) : o.w[q > 0 ? q - 1 : 0];
+        return __funnelshift_l(lo, o.w[q], 8);
+    }
+    const uint32_t hi = (q == NW - 1) ? edge : o.w[q < NW - 1 ? q + 1 : q];
+    return __funnelshift_r(o.w[q], hi, 8);
+}
+
+// The update of one W-byte vector from the six neighbour words of the other colour.
+template <int W>
+__device__ __forceinline__ Vec<W> ising_sc_update(const Vec<W> &me, const Vec<W> &o0, const Vec<W> &a,
+                                                  const Vec<W> &b, const Vec<W> &c, const Vec<W> &d,
+                                                  uint32_t edge, int par, int rho0, const ScTab &tab,
+                                                  uint32_t t, uint32_t stream, uint32_t c3, uint32_t seed,
+                                                  const RoundKeys &K, uint32_t &cnt) {
+    Vec<W> n;
+#pragma unroll
+    for (int q = 0; q < W / 4; ++q)
+        n.w[q] = o0.w[q] + sc_side<W>(o0, edge, par, q) + a.w[q] + b.w[q] + c.w[q] + d.w[q];
+    return ising_sc_decide<W>(me, n, rho0, tab, t, stream, c3, seed, K, cnt);
+}
+
 // VPT vectors of W bytes per thread, vector indices vfirst + j*vstride (j < VPT, < nvec),
-// one after another, loaded from global memory.  s_th / s_tl: the 14 thresholds' high / low
-// halves in shared memory.  Returns the flips as bytewise counts (each byte <= NW VPT).
+// one after another, loaded from global memory.  Returns the flips as bytewise counts (each
+// byte <= NW VPT).
 template <int W, int VPT>
 __device__ __forceinline__ uint32_t ising_sc_vectors(const IsingSc &A, int vfirst, int vstride,
-                                                     int nvec, const uint32_t *s_th,
-                                                     const uint32_t *s_tl, uint32_t t,
+                                                     int nvec, const ScTab &tab, uint32_t t,
                                                      uint32_t stream, uint32_t c3, uint32_t seed,
                                                      const RoundKeys &K) {
     static_assert(W == 4 || W == 8 || W == 16, "vector of half, one or two random-number groups");
@@ -265,27 +319,80 @@ __device__ __forceinline__ uint32_t ising_sc_vectors(const IsingSc &A, int vfirs
         const Vec<W> d = ldv<W>(A.opp + (zp * L2 + y) * H + xh0);
         const uint32_t edge = par == 0 ? A.opp[row * H + (xh0 == 0 ? H - 1 : xh0 - 1)]
                                        : A.opp[row * H + (xh0 + W == H ? 0 : xh0 + W)];
-        const Vec<W> out = ising_sc_update<W>(me, o0, a, b, c, d, edge, par, rho0, s_th, s_tl, t, stream,
+        const Vec<W> out = ising_sc_update<W>(me, o0, a, b, c, d, edge, par, rho0, tab, t, stream,
                                               c3, seed, K, cnt);
         stv<W>(A.own_a + rho0, out);
     }
-    return cnt;
+    return flip_bytes(cnt);
+}
+
+// A pair of vectors: the same (y, xh) in the planes z0 and z0 + 1 (z0 even; every extent of
+// these lattices is even).  Of the two vectors the one whose sites have their x neighbours at
+// xh-1 (parity y + z + colour even) comes first on every lane, so the window shift is the
+// same for the whole warp, each of the two serves the other as one z neighbour (ten vector
+// loads for two vectors instead of twelve), and the index arithmetic is done once for 2 W
+// sites.  Offsets are unsigned, so that the loads take them beside the replica's uniform base
+// address.  The loads are a step of their own, so that a kernel can issue them before it has
+// its thresholds.
+template <int W>
+struct ScPair {
+    Vec<W> meA, meB, o0A, o0B, aA, aB, bA, bB, uA, uB;
+    uint32_t eA, eB, oA, oB;
+};
+template <int W>
+__device__ __forceinline__ ScPair<W> sc_pair_load(const IsingSc &A, int p) {
+    const uint32_t H = A.H, L2 = A.L2, L3 = A.L3;
+    const uint32_t plane = L2 * H;
+    const uint8_t *const own = A.own_a;
+    const uint8_t *const opp = A.opp;
+    const uint32_t pos = (uint32_t)p * W;
+    const uint32_t row = fdiv(pos, A.fH);
+    const uint32_t xh0 = pos - row * H;
+    const uint32_t zp = fdiv(row, A.fL2);
+    const uint32_t y = row - zp * L2;
+    const bool pz = (y + A.colour) & 1u;  // parity of plane z0 = 2 zp: the first vector lies in z0 + pz
+    const uint32_t base = pos + zp * plane;  // (2 zp L2 + y) H + xh0
+    const uint32_t oA = base + (pz ? plane : 0u), oB = base + (pz ? 0u : plane);
+    const uint32_t below = base + (zp == 0 ? (L3 - 1) * plane : 0u - plane);
+    const uint32_t above = base + (2 * zp + 2 == L3 ? (2 - L3) * plane : 2 * plane);
+    const uint32_t dym = y == 0 ? plane - H : 0u - H, dyp = y == L2 - 1 ? H - plane : H;
+    ScPair<W> I;
+    I.oA = oA;
+    I.oB = oB;
+    I.o0A = ldv<W>(opp + oA);
+    I.o0B = ldv<W>(opp + oB);
+    I.aA = ldv<W>(opp + (oA + dym));
+    I.aB = ldv<W>(opp + (oB + dym));
+    I.bA = ldv<W>(opp + (oA + dyp));
+    I.bB = ldv<W>(opp + (oB + dyp));
+    I.uA = ldv<W>(opp + (pz ? above : below));
+    I.uB = ldv<W>(opp + (pz ? below : above));
+    I.eA = opp[oA + (xh0 == 0 ? H - 1 : ~0u)];
+    I.eB = opp[oB + (xh0 + W == H ? W - H : (uint32_t)W)];
+    I.meA = ldv<W>(own + oA);
+    I.meB = ldv<W>(own + oB);
+    return I;
+}
+// Decides and stores both vectors; adds the flips to cnt as ising_sc_decide does.
+template <int W>
+__device__ __forceinline__ void sc_pair_update(const IsingSc &A, const ScPair<W> &I, const ScTab &tab, uint32_t t,
+                                               uint32_t stream, uint32_t c3, uint32_t seed, const RoundKeys &K,
+                                               uint32_t &cnt) {
+    Vec<W> nA, nB;
+#pragma unroll
+    for (int q = 0; q < W / 4; ++q) {
+        const uint32_t both = I.o0A.w[q] + I.o0B.w[q];
+        nA.w[q] = both + sc_side<W>(I.o0A, I.eA, 0, q) + I.aA.w[q] + I.bA.w[q] + I.uA.w[q];
+        nB.w[q] = both + sc_side<W>(I.o0B, I.eB, 1, q) + I.aB.w[q] + I.bB.w[q] + I.uB.w[q];
+    }
+    stv<W>(A.own_a + I.oA, ising_sc_decide<W>(I.meA, nA, (int)I.oA, tab, t, stream, c3, seed, K, cnt));
+    stv<W>(A.own_a + I.oB, ising_sc_decide<W>(I.meB, nB, (int)I.oB, tab, t, stream, c3, seed, K, cnt));
 }
 
 // Sum of the four byte lanes (each <= 255).
 __device__ __forceinline__ unsigned byte_sum(uint32_t cnt) {
     const uint32_t x = (cnt & 0x00FF00FFu) + ((cnt >> 8) & 0x00FF00FFu);
     return (x & 0xFFFFu) + (x >> 16);
-}
-
-// Loads a replica's 14 simple-cubic thresholds into shared memory (all threads call it).
-__device__ __forceinline__ void load_sc_thresholds(const uint32_t *thr, uint32_t *s_th,
-                                                   uint32_t *s_tl) {
-    if (threadIdx.x < 14) {
-        const uint32_t T = thr[threadIdx.x];
-        s_th[threadIdx.x] = T >> 16;
-        s_tl[threadIdx.x] = T & 0xFFFFu;
-    }
 }
 
 }  // namespace ether

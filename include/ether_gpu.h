@@ -259,10 +259,11 @@ int ether_end_sweep(ether_ctx *ctx);
 
 /* Autotuner: times the kernel variants of this context's fast path on its own data
  * (spins and counters are restored) and keeps the fastest; the choice is cached per size
- * class for the process.  Ising simple cubic: variant = 1000 (persistent) + 2000 (register
- * cap) + bytes per vector (4, 8, 16) * 10 + vectors per thread, or 4000 + 10 * vectors per step + 1 / 4
- * (shared-memory staged kernel).  XYZ simple cubic: variant = 5000 + 10 * sites per thread +
- * blocks per SM of the register cap (5011 .. 5015, 5021 .. 5024, 5041, 5042).  best_ms = one colour
+ * class for the process.  Ising simple cubic: variant = 10 * bytes per vector (4, 8, 16) +
+ * vectors per thread (1, 2, 4), + 1000 for twice the vectors per thread; + 2000, 6162 and 4000 +
+ * 10 * vectors + 1 / 4 name forms that now run as the kernel of their vector size and count.
+ * XYZ simple cubic: variant = 5000 + 10 * sites per thread +
+ * blocks per SM of the register cap (5011 .. 5015, 5021, 5022).  best_ms = one colour
  * phase.  Either
  * output may be NULL. */
 int ether_autotune(ether_ctx *ctx, int32_t *variant, float *best_ms);
