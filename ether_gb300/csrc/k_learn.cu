@@ -19,7 +19,7 @@
 //     sweep bit for bit given the logits).
 // Training: maximum likelihood of the A-sites given the boundary on configurations the plain
 // sweep produced (any temperature of the context's ladder), Adam, straight-through BF16
-// rounding; hand-written FP32 GEMM, activation and optimiser kernels.
+// rounding (train.cuh).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -31,6 +31,7 @@
 #include "learn_common.cuh"
 #include "rng_math.cuh"
 #include "tc_util.cuh"
+#include "train.cuh"
 
 namespace ether {
 namespace learn {
@@ -542,135 +543,6 @@ __global__ void collect_kernel(const uint8_t *__restrict__ spins, int L1, int L2
     }
 }
 
-// --------------------------------------------------------------- training kernels ----
-// C (M x N, ldc) = beta C + sum_k A(m, k) B(k, n), A(m, k) = ta ? A[k lda + m] : A[m lda + k],
-// B(k, n) = tb ? B[n ldb + k] : B[k ldb + n].  64 x 64 tiles, 16 x 16 threads of 4 x 4, K in
-// steps of 16; fixed summation order.
-__global__ void __launch_bounds__(256)
-gemm_kernel(int M, int N, int K, const float *__restrict__ A, int lda, int ta, const float *__restrict__ B,
-            int ldb, int tb, float *__restrict__ C, int ldc, float beta) {
-    __shared__ float As[16][68], Bs[16][68];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-            const int kk = e >> 6, mm = e & 63;
-            const int m = m0 + mm, k = k0 + kk;
-            float va = 0.f;
-            if (m < M && k < K) va = ta ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k];
-            As[kk][mm] = va;
-            const int n = n0 + mm;
-            float vb = 0.f;
-            if (n < N && k < K) vb = tb ? B[(size_t)n * ldb + k] : B[(size_t)k * ldb + n];
-            Bs[kk][mm] = vb;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-            if (m < M && n < N) {
-                float *c = C + (size_t)m * ldc + n;
-                *c = beta == 0.f ? acc[i][j] : fmaf(beta, *c, acc[i][j]);
-            }
-        }
-}
-
-__device__ __forceinline__ float bf16r(float f) { return __bfloat162float(__float2bfloat16_rn(f)); }
-
-// minibatch: rows of the data set chosen by Philox, BF16 -> FP32, targets as 0/1
-__global__ void batch_kernel(const __nv_bfloat16 *__restrict__ X, const uint32_t *__restrict__ Y,
-                             long long n, int B, uint32_t seed, uint32_t step, float *__restrict__ Xb,
-                             float *__restrict__ Yb) {
-    const int b = blockIdx.x;
-    if (b >= B) return;
-    __shared__ long long row;
-    if (threadIdx.x == 0) {
-        const U4 d = draw((uint32_t)b, step, 0x4C524E00u, kLearn | (0xFDu << 8), seed);
-        row = (long long)((((unsigned long long)d.y << 32) | d.x) % (unsigned long long)n);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < NI; i += blockDim.x) Xb[(size_t)b * NI + i] = __bfloat162float(X[(size_t)row * NI + i]);
-    for (int i = threadIdx.x; i < NO; i += blockDim.x) Yb[(size_t)b * NO + i] = (float)((Y[row] >> i) & 1u);
-}
-
-__global__ void quantise_kernel(const float *__restrict__ p, float *__restrict__ q, int n) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const bool is_bias = (i >= OFF_B1 && i < OFF_W2) || (i >= OFF_B2 && i < OFF_W3) || i >= OFF_B3;
-        q[i] = is_bias ? p[i] : bf16r(p[i]);
-    }
-}
-
-__global__ void bias_relu_kernel(float *__restrict__ Hm, const float *__restrict__ b, int rows, int cols) {
-    const long long n = (long long)rows * cols;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        Hm[i] = bf16r(fmaxf(Hm[i] + b[i % cols], 0.0f));
-}
-
-// logits += b3; dZ = (sigmoid - y) / B; loss += softplus(z) - y z (block sums, one atomic each)
-__global__ void bce_kernel(float *__restrict__ Zm, const float *__restrict__ b3, const float *__restrict__ Yb,
-                           float *__restrict__ dZ, int B, double *__restrict__ loss) {
-    __shared__ double red[256];
-    double s = 0.0;
-    const int n = B * NO;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float zz = Zm[i] + b3[i % NO];
-        const float y = Yb[i];
-        const float p = 1.0f / (1.0f + expf(-zz));
-        dZ[i] = (p - y) / (float)B;
-        const float sp = zz > 0.0f ? zz + log1pf(expf(-zz)) : log1pf(expf(zz));
-        s += (double)(sp - y * zz);
-    }
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) atomicAdd(loss, red[0] / B);
-}
-
-__global__ void colsum_kernel(const float *__restrict__ D, int rows, int cols, float *__restrict__ out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float s = 0.f;
-    for (int r = 0; r < rows; ++r) s += D[(size_t)r * cols + c];
-    out[c] = s;
-}
-
-__global__ void relu_mask_kernel(float *__restrict__ dH, const float *__restrict__ Hm, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        if (!(Hm[i] > 0.0f)) dH[i] = 0.0f;
-}
-
-__global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
-                            float *__restrict__ v, int n, float lr, float c1, float c2) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = 0.9f * m[i] + 0.1f * gi;
-        const float vi = 0.999f * v[i] + 0.001f * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + 1e-8f);
-    }
-}
-
 // inference image: quantised weights as BF16 in the swizzled K-major tiles, biases FP32
 __global__ void pack_kernel(const float *__restrict__ q, uint8_t *__restrict__ img) {
     const int total = NH * NI + NH * NH + NO * NH;
@@ -730,10 +602,8 @@ struct ether_learn {
     uint32_t *Y = nullptr;
     long long cap = 0, n = 0, write = 0;
     uint32_t collect_calls = 0;
-    // training scratch (max batch)
-    int maxB = 0;
-    float *Xb = nullptr, *Yb = nullptr, *H1 = nullptr, *H2 = nullptr, *Z = nullptr, *dZ = nullptr,
-          *dH1 = nullptr, *dH2 = nullptr;
+    TrainBuffers tb;               // training scratch
+    uint32_t *wp = nullptr;        // packed weights of the training kernels
     double *loss = nullptr;
     // sweeps
     uint32_t *lstep = nullptr;
@@ -826,55 +696,23 @@ int refresh_tables(ether_learn &l) {
     return ETHER_OK;
 }
 
-int quantise_and_pack(ether_learn &l, cudaStream_t st) {
-    quantise_kernel<<<64, 256, 0, st>>>(l.p, l.pq, NPARAM);
+using Net = TrainNet<NI, NO>;
+static_assert(Net::N == NPARAM && Net::W2 == OFF_W2 && Net::W3 == OFF_W3, "parameter layout");
+
+TrainParams train_params(ether_learn &l) { return TrainParams{l.p, l.g, l.m, l.v, l.pq, l.wp, l.loss}; }
+
+// The inference image of the rounded parameters.
+int pack_image(ether_learn &l, cudaStream_t st) {
     pack_kernel<<<64, 256, 0, st>>>(l.pq, l.img);
-    l.launches += 2;
+    l.launches++;
     LCUDA(cudaGetLastError());
     return ETHER_OK;
 }
 
-int ensure_batch(ether_learn &l, int B) {
-    if (B <= l.maxB) return ETHER_OK;
-    float **bufs[] = {&l.Xb, &l.Yb, &l.H1, &l.H2, &l.Z, &l.dZ, &l.dH1, &l.dH2};
-    const size_t cols[] = {NI, NO, NH, NH, NO, NO, NH, NH};
-    for (int i = 0; i < 8; ++i) {
-        cudaFree(*bufs[i]);
-        *bufs[i] = nullptr;
-        LCUDA(cudaMalloc((void **)bufs[i], (size_t)B * cols[i] * sizeof(float)));
-    }
-    l.maxB = B;
-    return ETHER_OK;
-}
-
-void gemm(cudaStream_t st, int M, int N, int K, const float *A, int lda, int ta, const float *B, int ldb,
-          int tb, float *C, int ldc) {
-    dim3 grid((N + 63) / 64, (M + 63) / 64);
-    gemm_kernel<<<grid, 256, 0, st>>>(M, N, K, A, lda, ta, B, ldb, tb, C, ldc, 0.f);
-}
-
-// Forward and backward of a batch already in Xb / Yb; gradients into l.g, mean loss added to *l.loss.
-int forward_backward(ether_learn &l, int B, cudaStream_t st) {
-    const float *W1 = l.pq + OFF_W1, *W2 = l.pq + OFF_W2, *W3 = l.pq + OFF_W3;
-    gemm(st, B, NH, NI, l.Xb, NI, 0, W1, NI, 1, l.H1, NH);
-    bias_relu_kernel<<<256, 256, 0, st>>>(l.H1, l.pq + OFF_B1, B, NH);
-    gemm(st, B, NH, NH, l.H1, NH, 0, W2, NH, 1, l.H2, NH);
-    bias_relu_kernel<<<256, 256, 0, st>>>(l.H2, l.pq + OFF_B2, B, NH);
-    gemm(st, B, NO, NH, l.H2, NH, 0, W3, NH, 1, l.Z, NO);
-    bce_kernel<<<64, 256, 0, st>>>(l.Z, l.pq + OFF_B3, l.Yb, l.dZ, B, l.loss);
-    gemm(st, NO, NH, B, l.dZ, NO, 1, l.H2, NH, 0, l.g + OFF_W3, NH);
-    colsum_kernel<<<1, 128, 0, st>>>(l.dZ, B, NO, l.g + OFF_B3);
-    gemm(st, B, NH, NO, l.dZ, NO, 0, W3, NH, 0, l.dH2, NH);
-    relu_mask_kernel<<<256, 256, 0, st>>>(l.dH2, l.H2, (long long)B * NH);
-    gemm(st, NH, NH, B, l.dH2, NH, 1, l.H1, NH, 0, l.g + OFF_W2, NH);
-    colsum_kernel<<<1, 128, 0, st>>>(l.dH2, B, NH, l.g + OFF_B2);
-    gemm(st, B, NH, NH, l.dH2, NH, 0, W2, NH, 0, l.dH1, NH);
-    relu_mask_kernel<<<256, 256, 0, st>>>(l.dH1, l.H1, (long long)B * NH);
-    gemm(st, NH, NI, B, l.dH1, NH, 1, l.Xb, NI, 0, l.g + OFF_W1, NI);
-    colsum_kernel<<<1, 128, 0, st>>>(l.dH1, B, NH, l.g + OFF_B1);
-    l.launches += 17;
-    LCUDA(cudaGetLastError());
-    return ETHER_OK;
+int quantise_and_pack(ether_learn &l, cudaStream_t st) {
+    LCUDA((train_pack<NI, NO>(train_params(l), st)));
+    l.launches++;
+    return pack_image(l, st);
 }
 
 int read_err(ether_learn &l) {
@@ -969,6 +807,7 @@ extern "C" int ether_learn_create(ether_ctx *h, const ether_learn_desc *d, ether
     for (float **b : pb)
         if (e == cudaSuccess) e = cudaMalloc((void **)b, NPARAM * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&l->img, IMG_BYTES);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&l->wp, Net::WORDS * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc((void **)&l->X, (size_t)l->cap * NI * sizeof(__nv_bfloat16));
     if (e == cudaSuccess) e = cudaMalloc((void **)&l->Y, (size_t)l->cap * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc((void **)&l->loss, sizeof(double));
@@ -1013,8 +852,8 @@ extern "C" int ether_learn_destroy(ether_learn *l) {
         return ETHER_OK;
     }
     if (l->ctx) cudaStreamSynchronize(l->ctx->c.stream);
-    void *ptrs[] = {l->p, l->pq, l->g, l->m, l->v, l->img, l->X, l->Y, l->Xb, l->Yb, l->H1, l->H2,
-                    l->Z, l->dZ, l->dH1, l->dH2, l->loss, l->lstep, l->k4, l->betaJf, l->TB,
+    l->tb.release();
+    void *ptrs[] = {l->p, l->pq, l->g, l->m, l->v, l->img, l->X, l->Y, l->wp, l->loss, l->lstep, l->k4, l->betaJf, l->TB,
                     l->LBup, l->LBdn, l->acc, l->dump, l->err};
     for (void *q : ptrs)
         if (q) cudaFree(q);
@@ -1050,23 +889,16 @@ extern "C" int ether_learn_train(ether_learn *l, int32_t steps, int32_t batch, f
     if (steps < 0 || batch < 1 || batch > 65536 || !(lr > 0.f)) return lfail(ETHER_ERR_ARG, "bad training arguments");
     if (l->xyz) return learn::xyz_train(l->xyz, steps, batch, lr, loss_out);
     if (l->n == 0) return lfail(ETHER_ERR_STATE, "no training samples (ether_learn_collect)");
-    int rc = ensure_batch(*l, batch);
-    if (rc) return rc;
+    LCUDA((l->tb.ensure<NI, NO>(batch)));
     cudaStream_t st = l->ctx->c.stream;
     LCUDA(cudaEventRecord(l->e0, st));
     for (int s = 0; s < steps; ++s) {
-        LCUDA(cudaMemsetAsync(l->loss, 0, sizeof(double), st));
-        batch_kernel<<<batch, 128, 0, st>>>(l->X, l->Y, l->n, batch, l->seed, (uint32_t)(l->adam_t + 1), l->Xb, l->Yb);
-        l->launches++;
-        rc = forward_backward(*l, batch, st);
-        if (rc) return rc;
+        TrainIo T{l->X, l->Y, l->n, batch, l->seed, (uint32_t)(l->adam_t + 1), 0x4C524E00u};
         ++l->adam_t;
         const float c1 = 1.0f - std::pow(0.9f, (float)l->adam_t), c2 = 1.0f - std::pow(0.999f, (float)l->adam_t);
-        adam_kernel<<<64, 256, 0, st>>>(l->p, l->g, l->m, l->v, NPARAM, lr, c1, c2);
-        quantise_kernel<<<64, 256, 0, st>>>(l->p, l->pq, NPARAM);
-        l->launches += 2;
+        LCUDA((train_step<NI, NO>(train_params(*l), T, l->tb, AdamStep{lr, c1, c2}, s == steps - 1, st, &l->launches)));
     }
-    rc = quantise_and_pack(*l, st);
+    const int rc = pack_image(*l, st);
     if (rc) return rc;
     LCUDA(cudaEventRecord(l->e1, st));
     if (loss_out) {
@@ -1222,17 +1054,16 @@ extern "C" int ether_learn_loss_grad(ether_learn *l, const float *x, const uint3
     if (!l || !x || !y || !grad) return lfail(ETHER_ERR_ARG, "null argument");
     if (B < 1 || B > 65536) return lfail(ETHER_ERR_ARG, "batch out of range");
     if (l->xyz) return lfail(ETHER_ERR_UNSUPPORTED, "XYZ learner: targets are spin components (ether_learn_loss_grad_f)");
-    int rc = ensure_batch(*l, B);
-    if (rc) return rc;
+    LCUDA((l->tb.ensure<NI, NO>(B)));
     cudaStream_t st = l->ctx->c.stream;
     std::vector<float> yf((size_t)B * NO);
     for (int b = 0; b < B; ++b)
         for (int o = 0; o < NO; ++o) yf[(size_t)b * NO + o] = (float)((y[b] >> o) & 1u);
-    LCUDA(cudaMemcpyAsync(l->Xb, x, (size_t)B * NI * sizeof(float), cudaMemcpyHostToDevice, st));
-    LCUDA(cudaMemcpyAsync(l->Yb, yf.data(), (size_t)B * NO * sizeof(float), cudaMemcpyHostToDevice, st));
-    LCUDA(cudaMemsetAsync(l->loss, 0, sizeof(double), st));
-    rc = forward_backward(*l, B, st);
-    if (rc) return rc;
+    LCUDA(cudaMemcpyAsync(l->tb.Xb, x, (size_t)B * NI * sizeof(float), cudaMemcpyHostToDevice, st));
+    LCUDA(cudaMemcpyAsync(l->tb.Yb, yf.data(), (size_t)B * NO * sizeof(float), cudaMemcpyHostToDevice, st));
+    TrainIo T{};
+    T.B = B;
+    LCUDA((train_step<NI, NO>(train_params(*l), T, l->tb, AdamStep{0.f, 1.f, 1.f}, true, st, &l->launches)));
     double lv = 0.0;
     LCUDA(cudaMemcpyAsync(&lv, l->loss, sizeof(double), cudaMemcpyDeviceToHost, st));
     LCUDA(cudaMemcpyAsync(grad, l->g, NPARAM * sizeof(float), cudaMemcpyDeviceToHost, st));

@@ -10,8 +10,7 @@
 //     outputs 3k .. 3k+2 (+ bias) are the von Mises-Fisher parameter m_k of A-site k;
 //     inference: xmlp_kernel, the three layers on the tensor cores (tcgen05, TMA-loaded
 //     inputs, weights resident in shared memory, FP32 accumulators in tensor memory; the
-//     hidden layers' bias (BF16) + ReLU + BF16 rounding in the epilogue); training on the FP32
-//     GEMM of k_learn.cu;
+//     hidden layers' bias (BF16) + ReLU + BF16 rounding in the epilogue); training: train.cuh;
 //   * proposal: A-site k ~ vMF(m_k) (Wood's exact sampler on the sphere, own log / exp /
 //     sincos); then every B-site from its exact heat-bath conditional vMF(-beta g), g = J o
 //     (sum of its six neighbours: new A-sites and the boundary); a vMF with |m| < 1e-3 is
@@ -36,6 +35,7 @@
 #include "learn_common.cuh"
 #include "rng_math.cuh"
 #include "tc_util.cuh"
+#include "train.cuh"
 
 namespace ether {
 namespace learn {
@@ -262,69 +262,8 @@ __global__ void __launch_bounds__(256) xcollect_kernel(XPatchParams P, int per_r
     }
 }
 
-// minibatch: rows of the data set chosen by Philox, BF16 -> FP32
-__global__ void xbatch_kernel(const __nv_bfloat16 *__restrict__ X, const float *__restrict__ Y, long long n, int B,
-                              uint32_t seed, uint32_t step, float *__restrict__ Xb, float *__restrict__ Yb) {
-    const int b = blockIdx.x;
-    if (b >= B) return;
-    __shared__ long long row;
-    if (threadIdx.x == 0) {
-        const U4 d = draw((uint32_t)b, step, 0x4C524E01u, kLearn | (0xFDu << 8), seed);
-        row = (long long)((((unsigned long long)d.y << 32) | d.x) % (unsigned long long)n);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < XNI; i += blockDim.x) Xb[(size_t)b * XNI + i] = __bfloat162float(X[(size_t)row * XNI + i]);
-    for (int i = threadIdx.x; i < XNO; i += blockDim.x) Yb[(size_t)b * XNO + i] = Y[(size_t)row * XNO + i];
-}
-
 __global__ void to_bf16_kernel(const float *__restrict__ q, __nv_bfloat16 *__restrict__ o, int n) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) o[i] = __float2bfloat16_rn(q[i]);
-}
-
-// weights BF16-rounded, biases kept
-__global__ void xquantise_kernel(const float *__restrict__ p, float *__restrict__ q, int n) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const bool is_bias = (i >= XOFF_B1 && i < XOFF_W2) || (i >= XOFF_B2 && i < XOFF_W3) || i >= XOFF_B3;
-        q[i] = is_bias ? p[i] : xbf16r(p[i]);
-    }
-}
-
-// m = z + b3 per A-site; loss += -(log C(kappa) + m . y) / B, C(kappa) = kappa / (4 pi sinh kappa);
-// dZ = -(y + A(kappa) m) / B with A = (1/kappa - coth kappa) / kappa (series below 1e-2).
-__global__ void vmf_loss_kernel(float *__restrict__ Zm, const float *__restrict__ b3, const float *__restrict__ Yb,
-                                float *__restrict__ dZ, int B, double *__restrict__ loss) {
-    __shared__ double red[256];
-    double s = 0.0;
-    const int n = B * 32;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int b = i >> 5, k = i & 31;
-        const float *z = Zm + (size_t)b * XNO + 3 * k;
-        const float *y = Yb + (size_t)b * XNO + 3 * k;
-        const float mx = z[0] + b3[3 * k], my = z[1] + b3[3 * k + 1], mz = z[2] + b3[3 * k + 2];
-        const float kap = sqrtf(mx * mx + my * my + mz * mz);
-        float logc, A;
-        if (kap < 1e-2f) {
-            const float k2 = kap * kap;
-            logc = -kLog4Pi - k2 * (1.0f / 6.0f) + k2 * k2 * (1.0f / 180.0f);
-            A = -1.0f / 3.0f + k2 * (1.0f / 45.0f);
-        } else {
-            logc = logf(kap) - kap - logf(-expm1f(-2.0f * kap)) - kLog2Pi;
-            A = (1.0f / kap - 1.0f / tanhf(kap)) / kap;
-        }
-        const float my_dot = mx * y[0] + my * y[1] + mz * y[2];
-        s += -(double)(logc + my_dot);
-        float *g = dZ + (size_t)b * XNO + 3 * k;
-        g[0] = -(y[0] + A * mx) / (float)B;
-        g[1] = -(y[1] + A * my) / (float)B;
-        g[2] = -(y[2] + A * mz) / (float)B;
-    }
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) atomicAdd(loss, red[0] / B);
 }
 
 // The Metropolis-Hastings step of the patches of one pass (one warp per patch; lane k owns
@@ -648,10 +587,8 @@ struct XyzLearn {
     float *Y = nullptr;
     long long cap = 0, n = 0, write = 0;
     uint32_t collect_calls = 0;
-    // training scratch (max batch)
-    int maxB = 0;
-    float *Xb = nullptr, *Yb = nullptr, *H1 = nullptr, *H2 = nullptr, *Z = nullptr, *dZ = nullptr,
-          *dH1 = nullptr, *dH2 = nullptr;
+    TrainBuffers tb;               // training scratch
+    uint32_t *wp = nullptr;        // packed weights of the training kernels
     double *loss = nullptr;
     // inference: BF16 weights and their swizzled image, one pass of up to `rows` patches
     __nv_bfloat16 *W16 = nullptr;  // W1, W2, W3 (and b1, b2) at their parameter offsets
@@ -714,19 +651,24 @@ int warp_grid(const XyzLearn &x, long long warps) {
     return (int)std::max<long long>(1, std::min<long long>((warps + 7) / 8, 8LL * x.sm_count));
 }
 
-void xgemm(cudaStream_t st, int M, int N, int K, const float *A, int lda, int ta, const float *B, int ldb, int tb,
-           float *C, int ldc) {
-    dim3 grid((N + 63) / 64, (M + 63) / 64);
-    gemm_kernel<<<grid, 256, 0, st>>>(M, N, K, A, lda, ta, B, ldb, tb, C, ldc, 0.f);
+using Net = TrainNet<XNI, XNO>;
+static_assert(Net::N == XNPARAM && Net::W2 == XOFF_W2 && Net::W3 == XOFF_W3, "parameter layout");
+
+TrainParams train_params(XyzLearn &x) { return TrainParams{x.p, x.g, x.m, x.v, x.pq, x.wp, x.loss}; }
+
+// xmlp_kernel's image of the rounded parameters.
+int pack_image(XyzLearn &x, cudaStream_t st) {
+    to_bf16_kernel<<<64, 256, 0, st>>>(x.pq, x.W16, XNPARAM);
+    xpack_kernel<<<64, 256, 0, st>>>(x.W16, x.ximg);
+    x.launches += 2;
+    XCUDA(cudaGetLastError());
+    return ETHER_OK;
 }
 
 int quantise(XyzLearn &x, cudaStream_t st) {
-    xquantise_kernel<<<64, 256, 0, st>>>(x.p, x.pq, XNPARAM);
-    to_bf16_kernel<<<64, 256, 0, st>>>(x.pq, x.W16, XNPARAM);
-    xpack_kernel<<<64, 256, 0, st>>>(x.W16, x.ximg);
-    x.launches += 3;
-    XCUDA(cudaGetLastError());
-    return ETHER_OK;
+    XCUDA((train_pack<XNI, XNO>(train_params(x), st)));
+    x.launches++;
+    return pack_image(x, st);
 }
 
 // The inference network on M rows of Xh (BF16, M <= rows): Zi (no output bias), by
@@ -762,49 +704,6 @@ int xread_err(XyzLearn &x) {
         return xfail(ETHER_ERR_TIMEOUT, "learned proposal: an inference pipeline wait timed out (stage " +
                                             std::to_string(e) + ")");
     }
-    return ETHER_OK;
-}
-
-// The network on M rows of X (FP32, BF16 values): H1, H2 (ReLU, BF16) and Z (no output bias).
-void forward_rows(XyzLearn &x, cudaStream_t st, int M, const float *X, float *H1, float *H2, float *Z) {
-    xgemm(st, M, NH, XNI, X, XNI, 0, x.pq + XOFF_W1, XNI, 1, H1, NH);
-    bias_relu_kernel<<<256, 256, 0, st>>>(H1, x.pq + XOFF_B1, M, NH);
-    xgemm(st, M, NH, NH, H1, NH, 0, x.pq + XOFF_W2, NH, 1, H2, NH);
-    bias_relu_kernel<<<256, 256, 0, st>>>(H2, x.pq + XOFF_B2, M, NH);
-    xgemm(st, M, XNO, NH, H2, NH, 0, x.pq + XOFF_W3, NH, 1, Z, XNO);
-    x.launches += 5;
-}
-
-int ensure_batch(XyzLearn &x, int B) {
-    if (B <= x.maxB) return ETHER_OK;
-    float **bufs[] = {&x.Xb, &x.Yb, &x.H1, &x.H2, &x.Z, &x.dZ, &x.dH1, &x.dH2};
-    const size_t cols[] = {XNI, XNO, NH, NH, XNO, XNO, NH, NH};
-    for (int i = 0; i < 8; ++i) {
-        cudaFree(*bufs[i]);
-        *bufs[i] = nullptr;
-        XCUDA(cudaMalloc((void **)bufs[i], (size_t)B * cols[i] * sizeof(float)));
-    }
-    x.maxB = B;
-    return ETHER_OK;
-}
-
-// Forward and backward of a batch already in Xb / Yb; gradients into x.g, mean loss added to *x.loss.
-int forward_backward(XyzLearn &x, int B, cudaStream_t st) {
-    const float *W2 = x.pq + XOFF_W2, *W3 = x.pq + XOFF_W3;
-    forward_rows(x, st, B, x.Xb, x.H1, x.H2, x.Z);
-    vmf_loss_kernel<<<64, 256, 0, st>>>(x.Z, x.pq + XOFF_B3, x.Yb, x.dZ, B, x.loss);
-    xgemm(st, XNO, NH, B, x.dZ, XNO, 1, x.H2, NH, 0, x.g + XOFF_W3, NH);
-    colsum_kernel<<<1, 128, 0, st>>>(x.dZ, B, XNO, x.g + XOFF_B3);
-    xgemm(st, B, NH, XNO, x.dZ, XNO, 0, W3, NH, 0, x.dH2, NH);
-    relu_mask_kernel<<<256, 256, 0, st>>>(x.dH2, x.H2, (long long)B * NH);
-    xgemm(st, NH, NH, B, x.dH2, NH, 1, x.H1, NH, 0, x.g + XOFF_W2, NH);
-    colsum_kernel<<<1, 128, 0, st>>>(x.dH2, B, NH, x.g + XOFF_B2);
-    xgemm(st, B, NH, NH, x.dH2, NH, 0, W2, NH, 0, x.dH1, NH);
-    relu_mask_kernel<<<256, 256, 0, st>>>(x.dH1, x.H1, (long long)B * NH);
-    xgemm(st, NH, XNI, B, x.dH1, NH, 1, x.Xb, XNI, 0, x.g + XOFF_W1, XNI);
-    colsum_kernel<<<1, 128, 0, st>>>(x.dH1, B, NH, x.g + XOFF_B1);
-    x.launches += 12;
-    XCUDA(cudaGetLastError());
     return ETHER_OK;
 }
 
@@ -881,6 +780,7 @@ int xyz_create(ether_ctx *h, const ether_learn_desc *d, XyzLearn **out) {
     if (e == cudaSuccess) e = cudaMalloc((void **)&x->W16, XNPARAM * sizeof(__nv_bfloat16));
     if (e == cudaSuccess) e = cudaMalloc((void **)&x->Xh, (size_t)x->rows * XNI * sizeof(__nv_bfloat16));
     if (e == cudaSuccess) e = cudaMalloc((void **)&x->ximg, XIMG_BYTES);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&x->wp, Net::WORDS * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(x->ximg, 0, XIMG_BYTES);  // W1's K padding stays zero
     if (e == cudaSuccess) e = cudaMalloc((void **)&x->err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(x->err, 0, sizeof(int));
@@ -945,8 +845,8 @@ int xyz_create(ether_ctx *h, const ether_learn_desc *d, XyzLearn **out) {
 void xyz_destroy(XyzLearn *x) {
     if (!x) return;
     if (x->ctx) cudaStreamSynchronize(x->ctx->c.stream);
-    void *ptrs[] = {x->p, x->pq, x->g, x->m, x->v, x->X, x->Y, x->Xb, x->Yb, x->H1, x->H2, x->Z, x->dZ, x->dH1,
-                    x->dH2, x->loss, x->W16, x->ximg, x->err, x->Xh, x->Zi, x->lstep, x->acc, x->dump};
+    x->tb.release();
+    void *ptrs[] = {x->p, x->pq, x->g, x->m, x->v, x->X, x->Y, x->wp, x->loss, x->W16, x->ximg, x->err, x->Xh, x->Zi, x->lstep, x->acc, x->dump};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (x->e0) cudaEventDestroy(x->e0);
@@ -970,21 +870,17 @@ int xyz_collect(XyzLearn *x, int per_replica) {
 
 int xyz_train(XyzLearn *x, int steps, int batch, float lr, double *loss_out) {
     if (x->n == 0) return xfail(ETHER_ERR_STATE, "no training samples (ether_learn_collect)");
-    int rc = ensure_batch(*x, batch);
-    if (rc) return rc;
+    XCUDA((x->tb.ensure<XNI, XNO>(batch)));
     cudaStream_t st = x->ctx->c.stream;
     XCUDA(cudaEventRecord(x->e0, st));
     for (int s = 0; s < steps; ++s) {
-        XCUDA(cudaMemsetAsync(x->loss, 0, sizeof(double), st));
-        xbatch_kernel<<<batch, 128, 0, st>>>(x->X, x->Y, x->n, batch, x->seed, (uint32_t)(x->adam_t + 1), x->Xb, x->Yb);
-        x->launches++;
-        rc = forward_backward(*x, batch, st);
-        if (rc) return rc;
+        TrainIo T{x->X, x->Y, x->n, batch, x->seed, (uint32_t)(x->adam_t + 1), 0x4C524E01u};
         ++x->adam_t;
         const float c1 = 1.0f - std::pow(0.9f, (float)x->adam_t), c2 = 1.0f - std::pow(0.999f, (float)x->adam_t);
-        adam_kernel<<<64, 256, 0, st>>>(x->p, x->g, x->m, x->v, XNPARAM, lr, c1, c2);
-        x->launches++;
-        rc = quantise(*x, st);
+        XCUDA((train_step<XNI, XNO>(train_params(*x), T, x->tb, AdamStep{lr, c1, c2}, s == steps - 1, st, &x->launches)));
+    }
+    if (steps > 0) {
+        const int rc = pack_image(*x, st);
         if (rc) return rc;
     }
     XCUDA(cudaEventRecord(x->e1, st));
@@ -1074,14 +970,13 @@ int xyz_set_params(XyzLearn *x, const float *params) {
 }
 
 int xyz_loss_grad(XyzLearn *x, const float *xin, const float *y, int B, double *loss, float *grad) {
-    int rc = ensure_batch(*x, B);
-    if (rc) return rc;
+    XCUDA((x->tb.ensure<XNI, XNO>(B)));
     cudaStream_t st = x->ctx->c.stream;
-    XCUDA(cudaMemcpyAsync(x->Xb, xin, (size_t)B * XNI * sizeof(float), cudaMemcpyHostToDevice, st));
-    XCUDA(cudaMemcpyAsync(x->Yb, y, (size_t)B * XNO * sizeof(float), cudaMemcpyHostToDevice, st));
-    XCUDA(cudaMemsetAsync(x->loss, 0, sizeof(double), st));
-    rc = forward_backward(*x, B, st);
-    if (rc) return rc;
+    XCUDA(cudaMemcpyAsync(x->tb.Xb, xin, (size_t)B * XNI * sizeof(float), cudaMemcpyHostToDevice, st));
+    XCUDA(cudaMemcpyAsync(x->tb.Yb, y, (size_t)B * XNO * sizeof(float), cudaMemcpyHostToDevice, st));
+    TrainIo T{};
+    T.B = B;
+    XCUDA((train_step<XNI, XNO>(train_params(*x), T, x->tb, AdamStep{0.f, 1.f, 1.f}, true, st, &x->launches)));
     double lv = 0.0;
     XCUDA(cudaMemcpyAsync(&lv, x->loss, sizeof(double), cudaMemcpyDeviceToHost, st));
     XCUDA(cudaMemcpyAsync(grad, x->g, XNPARAM * sizeof(float), cudaMemcpyDeviceToHost, st));

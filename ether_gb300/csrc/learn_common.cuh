@@ -1,5 +1,5 @@
 // learn_common.cuh -- what the two learned patch proposals share: the 4^3 patch geometry in
-// closed form, the FP32 training kernels (defined in k_learn.cu), and the entry points of
+// closed form, the sweep counter's kernel (k_learn.cu), and the entry points of
 // the Heisenberg learner (k_learn_xyz.cu) that the ether_learn_* functions hand an XYZ
 // context over to.
 #pragma once
@@ -51,18 +51,6 @@ __host__ __device__ inline void geo_bnd(int i, int &a, int &b, int &c) {
     else { a = u; b = v; c = e; }
 }
 
-// --------------------------------------------------- FP32 training kernels (k_learn.cu) ----
-// C (M x N, ldc) = beta C + sum_k A(m, k) B(k, n), A(m, k) = ta ? A[k lda + m] : A[m lda + k],
-// B(k, n) = tb ? B[n ldb + k] : B[k ldb + n]; fixed summation order.
-__global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, const float *__restrict__ A, int lda, int ta,
-                            const float *__restrict__ B, int ldb, int tb, float *__restrict__ C, int ldc,
-                            float beta);
-// H = bf16(max(H + b, 0)) row-wise
-__global__ void bias_relu_kernel(float *__restrict__ Hm, const float *__restrict__ b, int rows, int cols);
-__global__ void colsum_kernel(const float *__restrict__ D, int rows, int cols, float *__restrict__ out);
-__global__ void relu_mask_kernel(float *__restrict__ dH, const float *__restrict__ Hm, long long n);
-__global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
-                            float *__restrict__ v, int n, float lr, float c1, float c2);
 __global__ void advance_lstep_kernel(uint32_t *c, int R);
 
 // ------------------------------------------------ the Heisenberg learner (k_learn_xyz.cu) ----
