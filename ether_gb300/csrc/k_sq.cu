@@ -19,7 +19,7 @@
 //     16-byte chunk of every row), lane l the site 8w + l/4 and the q-points h1_0 + 4a + l%4
 //     (a = 0..15): phase factors
 //       exp(i q.r) = E1[h1_0 + l%4][i] * E2[h2][i] * E3[h3][i] * b4_i^a,  b4_i = exp(2 pi i 4 dq_1 u_i)
-//     (complex FP32 from FP64-built tables, 15 steps of the recurrence), split into hi/lo
+//     (complex FP32 from FP64-built tables, sq_tables, 15 steps of the recurrence), split into hi/lo
 //     BF16 pairs (cos, sin) and written four 8x8 blocks at a time with stmatrix.trans into the
 //     K-major 128-byte-swizzled layout the MMA descriptors describe;
 //   * one thread of warp 8 loads the B_hi / B_lo tiles with TMA (same swizzle) and issues the
@@ -337,6 +337,34 @@ __global__ void sq_prep_b(const uint8_t *__restrict__ spins, const float4 *__res
     }
 }
 
+// The phase tables in FP64, rounded to FP32: rows 0 .. M1/16 - 1 are E1 (row 4t + p: the phase at
+// h1 = 64t + p, the first q-point of q-phase p of tile t), then M2 rows of E2, M3 of E3 and one
+// of b4; frac: fractional coordinates (3 per site).  3.7e6 FP64 sincos for 27648 sites on a 64^3
+// grid: 0.3 ms here, 40 ms on one of the host's cores, where they were three quarters of the
+// whole call.  blockIdx.y strides over the rows.
+__global__ void __launch_bounds__(256)
+sq_tables(const double *__restrict__ frac, int N, int Kpad, int M1, int M2, int M3, double q01, double q02,
+          double q03, double dq1, double dq2, double dq3, float2 *__restrict__ tab) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= Kpad) return;
+    const double tp = 2.0 * 3.14159265358979323846;
+    const int r1 = M1 / 16, r2 = r1 + M2, r3 = r2 + M3;
+    for (int row = blockIdx.y; row <= r3; row += gridDim.y) {
+        float2 e = make_float2(row < r3 ? 0.f : 1.f, 0.f);  // padding sites
+        if (i < N) {
+            double ph;
+            if (row < r1) ph = tp * (q01 + (64.0 * (row >> 2) + (row & 3)) * dq1) * frac[3 * i];
+            else if (row < r2) ph = tp * (q02 + (row - r1) * dq2) * frac[3 * i + 1];
+            else if (row < r3) ph = tp * (q03 + (row - r2) * dq3) * frac[3 * i + 2];
+            else ph = tp * 4.0 * dq1 * frac[3 * i];
+            double s, c;
+            sincos(ph, &s, &c);
+            e = make_float2((float)c, (float)s);
+        }
+        tab[(size_t)row * Kpad + i] = e;
+    }
+}
+
 }  // namespace sq
 }  // namespace ether
 
@@ -378,33 +406,12 @@ int structure_factor_launch(Ctx &c, const double *frac /*3N, storage order*/, co
     if (Q * 2 > 0x7FFFFFFFL) { msg = "q-grid too large"; return ETHER_ERR_ARG; }
     PFN_cuTensorMapEncodeTiled_v12000 encode = get_encode();
     if (!encode) { msg = "cuTensorMapEncodeTiled not available"; return ETHER_ERR_CUDA; }
-    // phase tables in FP64 on the host
-    const double tp = 2.0 * M_PI;
-    // E1 row 4t + p: the phase at h1 = 64t + p (the first q-point of q-phase p of tile t)
-    std::vector<float2> E1((size_t)(M1 / 16) * Kpad, make_float2(0.f, 0.f));
-    std::vector<float2> E2((size_t)M2 * Kpad, make_float2(0.f, 0.f)), E3((size_t)M3 * Kpad, make_float2(0.f, 0.f));
-    std::vector<float2> bb(Kpad, make_float2(1.f, 0.f));
-    for (int i = 0; i < N; ++i) {
-        const double u = frac[3 * i], v = frac[3 * i + 1], w = frac[3 * i + 2];
-        for (int m = 0; m < M1 / 16; ++m) {
-            const double ph = tp * (q0[0] + (64.0 * (m >> 2) + (m & 3)) * dq[0]) * u;
-            E1[(size_t)m * Kpad + i] = make_float2((float)cos(ph), (float)sin(ph));
-        }
-        for (int h = 0; h < M2; ++h) {
-            const double ph = tp * (q0[1] + h * dq[1]) * v;
-            E2[(size_t)h * Kpad + i] = make_float2((float)cos(ph), (float)sin(ph));
-        }
-        for (int h = 0; h < M3; ++h) {
-            const double ph = tp * (q0[2] + h * dq[2]) * w;
-            E3[(size_t)h * Kpad + i] = make_float2((float)cos(ph), (float)sin(ph));
-        }
-        const double ph = tp * 4.0 * dq[0] * u;
-        bb[i] = make_float2((float)cos(ph), (float)sin(ph));
-    }
     const bool ising = c.model == ETHER_MODEL_ISING;
     const int cols = ising ? 1 : 3;            // TMEM columns per replica
     const int rmax = ising ? 256 : 85;         // 3 * 85 = 255 <= 256 columns of TMEM per pass
-    float2 *dE1 = nullptr, *dE2 = nullptr, *dE3 = nullptr, *dbb = nullptr;
+    float2 *dtab = nullptr;  // E1, E2, E3, b4 (sq_tables)
+    double *dfrac = nullptr;
+    const size_t rows1 = M1 / 16, tab_rows = rows1 + M2 + M3 + 1;
     __nv_bfloat16 *bhi = nullptr, *blo = nullptr;
     float *dsq = nullptr, *dcomp = nullptr;
     int *derr = nullptr;
@@ -412,23 +419,22 @@ int structure_factor_launch(Ctx &c, const double *frac /*3N, storage order*/, co
     const int rpass = std::min(c.R, rmax);
     const int BNmax = (cols * rpass + 15) / 16 * 16;
     auto cleanup = [&]() {
-        cudaFree(dE1); cudaFree(dE2); cudaFree(dE3); cudaFree(dbb); cudaFree(bhi); cudaFree(blo);
+        cudaFree(dtab); cudaFree(dfrac); cudaFree(bhi); cudaFree(blo);
         cudaFree(dsq); cudaFree(dcomp); cudaFree(derr);
     };
 #define SQ_TRY(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) { msg = std::string(#x) + ": " + cudaGetErrorString(e_); cleanup(); return ETHER_ERR_CUDA; } } while (0)
-    SQ_TRY(cudaMalloc(&dE1, E1.size() * sizeof(float2)));
-    SQ_TRY(cudaMalloc(&dE2, E2.size() * sizeof(float2)));
-    SQ_TRY(cudaMalloc(&dE3, E3.size() * sizeof(float2)));
-    SQ_TRY(cudaMalloc(&dbb, bb.size() * sizeof(float2)));
+    SQ_TRY(cudaMalloc(&dtab, tab_rows * Kpad * sizeof(float2)));
+    SQ_TRY(cudaMalloc(&dfrac, 3 * (size_t)N * sizeof(double)));
     SQ_TRY(cudaMalloc(&bhi, (size_t)BNmax * Kpad * 2));
     SQ_TRY(cudaMalloc(&blo, (size_t)BNmax * Kpad * 2));
     SQ_TRY(cudaMalloc(&dsq, (size_t)rpass * Q * sizeof(float)));
     SQ_TRY(cudaMalloc(&dcomp, (size_t)rpass * Q * 3 * sizeof(float)));
     SQ_TRY(cudaMalloc(&derr, sizeof(int)));
-    SQ_TRY(cudaMemcpyAsync(dE1, E1.data(), E1.size() * sizeof(float2), cudaMemcpyHostToDevice, c.stream));
-    SQ_TRY(cudaMemcpyAsync(dE2, E2.data(), E2.size() * sizeof(float2), cudaMemcpyHostToDevice, c.stream));
-    SQ_TRY(cudaMemcpyAsync(dE3, E3.data(), E3.size() * sizeof(float2), cudaMemcpyHostToDevice, c.stream));
-    SQ_TRY(cudaMemcpyAsync(dbb, bb.data(), bb.size() * sizeof(float2), cudaMemcpyHostToDevice, c.stream));
+    SQ_TRY(cudaMemcpyAsync(dfrac, frac, 3 * (size_t)N * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+    sq_tables<<<dim3((Kpad + 255) / 256, (unsigned)std::min<size_t>(tab_rows, 65535)), 256, 0, c.stream>>>(
+        dfrac, N, Kpad, M1, M2, M3, q0[0], q0[1], q0[2], dq[0], dq[1], dq[2], dtab);
+    SQ_TRY(cudaGetLastError());
+    c.launches++;
     for (int r0 = 0; r0 < c.R && rc == ETHER_OK; r0 += rpass) {
         const int R = std::min(rpass, c.R - r0);
         const int BN = (cols * R + 15) / 16 * 16;
@@ -453,7 +459,7 @@ int structure_factor_launch(Ctx &c, const double *frac /*3N, storage order*/, co
         P.nk = Kpad / kBK;
         P.M1 = M1; P.M2 = M2; P.M3 = M3;
         P.N = N; P.Kpad = Kpad; P.R = R; P.BN = BN;
-        P.E1 = dE1; P.E2 = dE2; P.E3 = dE3; P.bb = dbb;
+        P.E1 = dtab; P.E2 = dtab + rows1 * Kpad; P.E3 = P.E2 + (size_t)M2 * Kpad; P.bb = P.E3 + (size_t)M3 * Kpad;
         P.sq = dsq; P.comp = dcomp; P.err = derr;
         const int stage_bytes = 2 * Smem::a_bytes + (ising ? 1 : 2) * BN * kBK * 2;
         const int smem = 1024 + kStages * stage_bytes + 64;
