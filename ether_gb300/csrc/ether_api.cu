@@ -1667,8 +1667,9 @@ int ctx_variant(const Ctx &c) { return variant_of(c); }
 // vectors per thread (of 2 and 4).  + 2000 and 6162 named register caps, which the 16-byte
 // kernels now always have, 4011, 4014, 4021, 4041 a staged kernel (k_ising.cu): still accepted,
 // they run the kernel of their vector size and count.
-// XYZ: 5000 + 10 * sites per thread + register cap (blocks per SM) for the simple-cubic XYZ
-// kernel (5011 .. 5015, 5021, 5022).
+// XYZ: 5011 the planes per thread that xyz_planes chooses (k_xyz.cu), 5012 half and 5013 twice as
+// many; 5014, 5015, 5021, 5022 named register caps and sites per thread of a former kernel and
+// run as 5011.
 static bool apply_variant(Ctx &c, int variant) {
     if (c.model == ETHER_MODEL_XYZ) {
         if (!xyz_variant_valid(variant - 5000)) return false;
@@ -1725,7 +1726,7 @@ static int autotune_xyz(Ctx &c, int32_t *variant, float *best_ms) {
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    for (int cand : {5011, 5012, 5013, 5014, 5015, 5021, 5022, 5023, 5024, 5041, 5042}) {
+    for (int cand : {5011, 5012, 5013}) {
         if (!apply_variant(c, cand)) continue;
         CUDA_TRY(launch_xyz_sweep(c, 0));  // warm-up
         CUDA_TRY(cudaEventRecord(e0, c.stream));

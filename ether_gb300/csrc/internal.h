@@ -119,7 +119,7 @@ struct Ctx {
     uint32_t *thr = nullptr;     // n_slots * table_entries: flip iff u32 <= thr
     int ising_vpt = 1;           // vectors per thread of the simple-cubic Ising kernel
     int ising_code = 0;          // the variant that was asked for (0: the default choice)
-    int xyz_variant = 11;        // simple-cubic XYZ kernel: 10 * sites per thread + blocks per SM cap
+    int xyz_variant = 11;        // simple-cubic XYZ kernel: planes per thread (xyz_planes, k_xyz.cu)
     bool resident = false;       // ether_mcs runs runs of sweeps with ising_sc_resident
     unsigned long long *acc_before = nullptr;  // R: acceptance counts at the start of a call
     double *acc_ratio = nullptr;               // R: device acceptance ratios of a call

@@ -205,7 +205,7 @@ __device__ __forceinline__ void energy_block(const ObsMember &a, int r, int b) {
                 const int xh = rho - row * H;
                 const int z = (int)fdiv((uint32_t)row, a.sc_fL2), y = row - z * a.sc_L2;
                 const int p = (y + z + colour) & 1;
-                const Acc3 h = sc_field(sp + (size_t)(colour ^ 1) * half, a.sc_L1, a.sc_L2, a.sc_L3, H, xh, y, z, p,
+                const Acc3 h = sc_field(sp + (size_t)(colour ^ 1) * half + rho, a.sc_L2, a.sc_L3, H, xh, y, z, p,
                                         a.sc_jx, a.sc_jy, a.sc_jz);
                 hx = h.x;
                 hy = h.y;

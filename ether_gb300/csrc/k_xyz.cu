@@ -30,29 +30,34 @@ xyz_ell_kernel(float4 *__restrict__ spins4, int N, int col_off, int n_c, uint32_
     warp_add_count_x(acc_count + r, acc);
 }
 
-// Simple cubic, colour-split arrays.  A block takes VPT * 256 consecutive ranks per step,
-// thread i the ranks i, i + 256, ... (coalesced), processed side by side (xyz_sc_sites);
-// MINB is the register cap (blocks per SM).
-template <int OPT, int VPT, int MINB>
-__global__ void __launch_bounds__(256, MINB)
-xyz_sc_kernel(float4 *__restrict__ spins4, int L1, int L2, int L3, FastDiv fH, FastDiv fL2, uint32_t colour, float jx,
-              float jy, float jz, XyzParams P, const float *__restrict__ beta_slot_f,
-              const int32_t *__restrict__ slot_of_rep, const uint32_t *__restrict__ stream_id,
-              const uint32_t *__restrict__ step, const RoundKeys K,
-              unsigned long long *__restrict__ acc_count) {
+// Simple cubic, a thread per column and chunk of ZC planes (xyz_sc_column).  64 registers, four
+// blocks per SM.  Bound: issue (65%) and the latency of the neighbour loads between ALU and
+// FMA-heavy phases (53% each); 285 instructions per update, 400 when every site looked up its
+// six neighbours and its indices itself.  Updates/ns at T_c, before and now: 64^3 x 64 66 and
+// 83.8 (0.60 of the measured copy rate at 48 bytes per update), 32^3 x 290 58 and 74.8.
+// Measured and not kept: three blocks per SM without the register cap (81.2), five with spills
+// (54), the neighbour offsets' cases in a branch before the loads (75.9; 60.3 on 32^3).
+template <int OPT>
+__global__ void __launch_bounds__(256, 4)
+xyz_col_kernel(float4 *__restrict__ spins4, int L1, int L2, int L3, FastDiv fH, FastDiv fP, int ZC, int items,
+               uint32_t colour, float jx, float jy, float jz, XyzParams P, const float *__restrict__ beta_slot_f,
+               const int32_t *__restrict__ slot_of_rep, const uint32_t *__restrict__ stream_id,
+               const uint32_t *__restrict__ step, const RoundKeys K, unsigned long long *__restrict__ acc_count) {
     const int r = blockIdx.y;
     const int H = L1 >> 1;
     const int half = H * L2 * L3;
     float4 *base = spins4 + (size_t)r * 2 * half;
     const XyzSc A{base + (size_t)colour * half, base + (size_t)(colour ^ 1u) * half, L1, L2, L3, H,
-                  fH, fL2, colour, jx, jy, jz};
+                  fH, fP, colour, jx, jy, jz};
     const float beta_f = beta_slot_f[slot_of_rep[r]];
     const uint32_t k1 = stream_id[r], t = step[r];
-    const uint32_t c3 = kMetro | (colour << 8);
     unsigned acc = 0;
-    const int tile = VPT * (int)blockDim.x;
-    for (int rho0 = blockIdx.x * tile + threadIdx.x; rho0 < half; rho0 += gridDim.x * tile)
-        acc += xyz_sc_sites<OPT, VPT>(A, P, rho0, (int)blockDim.x, half, beta_f, t, c3, K, k1);
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < items) {
+        const int chunk = (int)fdiv((uint32_t)i, fP), col = i - chunk * (int)fP.d;
+        acc = xyz_sc_column<OPT>(A, P, col, chunk * ZC, min(chunk * ZC + ZC, L3), beta_f, t, kMetro | (colour << 8), K,
+                                 k1);
+    }
     warp_add_count_x(acc_count + r, acc);
 }
 
@@ -120,7 +125,7 @@ ovrr_sc_kernel(float4 *__restrict__ spins4, int L1, int L2, int L3, FastDiv fH, 
         const int xh = rho - row * H;
         const int z = (int)fdiv((uint32_t)row, fL2), y = row - z * L2;
         const int p = (y + z + (int)colour) & 1;
-        const Acc3 h = sc_field(opp, L1, L2, L3, H, xh, y, z, p, jx, jy, jz);
+        const Acc3 h = sc_field(opp + rho, L2, L3, H, xh, y, z, p, jx, jy, jz);
         ovrr_reflect(own + rho, h.x, h.y, h.z);
     }
 }
@@ -209,32 +214,31 @@ static XyzParams xyz_params(const Ctx &c) {
     return P;
 }
 
-template <int OPT, int VPT, int MINB>
-static void launch_xyz_sc(Ctx &c, int colour, const XyzParams &P, const RoundKeys &K) {
-    const int bs = 256;
-    const int half = c.N / 2;
-    dim3 grid(blocks_for_x(c, (half + VPT - 1) / VPT, bs), c.R);
-    // single shell, single species: J(1,1,1,:)
-    const float jx = c.h_Jf[0], jy = c.h_Jf[1], jz = c.h_Jf[2];
-    XyzParams Pc = P;  // the kernel indexes sites by rank in the colour array
-    if (Pc.sia_cls) Pc.sia_cls += (size_t)colour * half;
-    xyz_sc_kernel<OPT, VPT, MINB><<<grid, bs, 0, c.stream>>>(
-        c.spins4, c.L[0], c.L[1], c.L[2], make_fastdiv((uint32_t)(c.L[0] / 2)), make_fastdiv((uint32_t)c.L[1]),
-        (uint32_t)colour, jx, jy, jz, Pc, c.beta_slot_f, c.slot_of_rep, c.stream_id, c.step, K, c.acc_count);
+// Planes per thread: the most of 8, 4, 2 that still gives six blocks per SM (64^3 x 64: 83.8
+// updates/ns with 8, 80.5 with 4, 73.3 with 2; 48^3 x 32, where 8 leaves 864 blocks: 65.5 and
+// 66.9; 16^3 x 512, where it leaves 512: 51.5 and 56.7).  Variants 12 and 13 halve and double it.
+static int xyz_planes(const Ctx &c) {
+    const long plane = (long)(c.L[0] / 2) * c.L[1];
+    int zc = 1;
+    for (int v = 8; v > 1 && zc == 1; v /= 2)
+        if (c.R * ((plane * ((c.L[2] + v - 1) / v) + 255) / 256) >= 6L * c.sm_count) zc = v;
+    if (c.xyz_variant == 12) zc = std::max(1, zc / 2);
+    if (c.xyz_variant == 13) zc *= 2;
+    return zc;
 }
 
-// xyz_variant = 10 * VPT + MINB (11 = one site per thread, no register cap)
 template <int OPT>
-static void launch_xyz_sc_opt(Ctx &c, int colour, const XyzParams &P, const RoundKeys &K) {
-    switch (c.xyz_variant) {
-        case 12: launch_xyz_sc<OPT, 1, 2>(c, colour, P, K); break;
-        case 13: launch_xyz_sc<OPT, 1, 3>(c, colour, P, K); break;
-        case 14: launch_xyz_sc<OPT, 1, 4>(c, colour, P, K); break;
-        case 15: launch_xyz_sc<OPT, 1, 5>(c, colour, P, K); break;
-        case 21: launch_xyz_sc<OPT, 2, 1>(c, colour, P, K); break;
-        case 22: launch_xyz_sc<OPT, 2, 2>(c, colour, P, K); break;
-        default: launch_xyz_sc<OPT, 1, 1>(c, colour, P, K); break;
-    }
+static void launch_xyz_col(Ctx &c, int colour, const XyzParams &P, const RoundKeys &K) {
+    const int half = c.N / 2, plane = c.L[0] / 2 * c.L[1], ZC = xyz_planes(c);
+    const int items = plane * ((c.L[2] + ZC - 1) / ZC);
+    dim3 grid((items + 255) / 256, c.R);
+    XyzParams Pc = P;  // the kernel indexes sites by rank in the colour array
+    if (Pc.sia_cls) Pc.sia_cls += (size_t)colour * half;
+    // single shell, single species: J(1,1,1,:)
+    xyz_col_kernel<OPT><<<grid, 256, 0, c.stream>>>(
+        c.spins4, c.L[0], c.L[1], c.L[2], make_fastdiv((uint32_t)(c.L[0] / 2)), make_fastdiv((uint32_t)plane), ZC, items,
+        (uint32_t)colour, c.h_Jf[0], c.h_Jf[1], c.h_Jf[2], Pc, c.beta_slot_f, c.slot_of_rep, c.stream_id, c.step, K,
+        c.acc_count);
 }
 
 // The general-lattice kernel for a class's ELL width: common widths at compile time.
@@ -260,8 +264,8 @@ cudaError_t launch_xyz_sweep(Ctx &c, int colour) {
     const RoundKeys K = round_keys(c.seed);
     const bool exchange_only = !P.zeeman && !P.sia && !P.angle && !P.sia_local;
     if (c.fast) {
-        if (exchange_only) launch_xyz_sc_opt<kXyzExchange>(c, colour, P, K);
-        else launch_xyz_sc_opt<kXyzGeneral>(c, colour, P, K);
+        if (exchange_only) launch_xyz_col<kXyzExchange>(c, colour, P, K);
+        else launch_xyz_col<kXyzGeneral>(c, colour, P, K);
     } else {
         const int n_c = c.col_off[colour + 1] - c.col_off[colour];
         if (n_c == 0) return cudaSuccess;

@@ -37,7 +37,10 @@ ETHER_HD uint32_t mulhi32(uint32_t a, uint32_t b) {
 
 // a ^ b ^ c.  On the GPU one explicit three-input instruction: left to itself the compiler
 // regroups the round's XORs with the keys into two-input ones (51 instead of 42 instructions
-// per block, and as many more on the ALU pipe that bounds the Ising sweep).
+// per block, and as many more on the ALU pipe that bounds the Ising sweep).  draw_rk uses it
+// from the third round on (before that most words are the same for the whole launch, and the
+// compiler moves them out); draw, which serves kernels that wait on memory and draw once per
+// thread, does not (8% slower there: the keys then cost a register copy each).
 ETHER_HD uint32_t xor3(uint32_t a, uint32_t b, uint32_t c) {
 #if defined(__CUDA_ARCH__)
     uint32_t r;
@@ -55,8 +58,8 @@ ETHER_HD U4 philox(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t 
         // one 32x32->64 multiply each (a single wide multiply on the GPU)
         const uint64_t p0 = (uint64_t)0xD2511F53u * c0;
         const uint64_t p1 = (uint64_t)0xCD9E8D57u * c2;
-        const uint32_t n0 = xor3((uint32_t)(p1 >> 32), c1, k0);
-        const uint32_t n2 = xor3((uint32_t)(p0 >> 32), c3, k1);
+        const uint32_t n0 = (uint32_t)(p1 >> 32) ^ c1 ^ k0;
+        const uint32_t n2 = (uint32_t)(p0 >> 32) ^ c3 ^ k1;
         c0 = n0; c1 = (uint32_t)p1; c2 = n2; c3 = (uint32_t)p0;
         k0 += 0x9E3779B9u; k1 += 0xBB67AE85u;
     }
@@ -84,16 +87,18 @@ ETHER_HD U4 draw_rk(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, const Ro
     for (int r = 0; r < 10; ++r) {
         const uint64_t p0 = (uint64_t)0xD2511F53u * c0;
         const uint64_t p1 = (uint64_t)0xCD9E8D57u * c2;
-        const uint32_t n0 = xor3((uint32_t)(p1 >> 32), c1, K.k[r]);
-        const uint32_t n2 = xor3((uint32_t)(p0 >> 32), c3, kKey1 + (uint32_t)r * 0xBB67AE85u);
+        const uint32_t h1 = (uint32_t)(p1 >> 32), h0 = (uint32_t)(p0 >> 32), k1 = kKey1 + (uint32_t)r * 0xBB67AE85u;
+        const uint32_t n0 = r < 2 ? h1 ^ c1 ^ K.k[r] : xor3(h1, c1, K.k[r]);
+        const uint32_t n2 = r < 2 ? h0 ^ c3 ^ k1 : xor3(h0, c3, k1);
         c0 = n0; c1 = (uint32_t)p1; c2 = n2; c3 = (uint32_t)p0;
     }
     return U4{c0, c1, c2, c3};
 }
 
 // u32 -> [0,1) with 24 bits, and u32 -> [-1,1) with 24 bits (both exact in FP32).
-ETHER_HD float u01(uint32_t u) { return (float)(u >> 8) * 0x1p-24f; }
-ETHER_HD float upm1(uint32_t u) { return (float)(u >> 8) * 0x1p-23f - 1.0f; }
+ETHER_HD float u01(uint32_t u) { return (float)(u & 0xFFFFFF00u) * 0x1p-32f; }
+// The second by one fmaf, exact like the product and the difference it stands for.
+ETHER_HD float upm1(uint32_t u) { return fmaf((float)(u & 0xFFFFFF00u), 0x1p-31f, -1.0f); }
 
 ETHER_HD float bits_f(uint32_t b) {
 #if defined(__CUDA_ARCH__)

@@ -116,10 +116,7 @@ __device__ __forceinline__ bool metro_site(const XyzParams &P, float4 *sp, int s
 }
 
 // ------------------------------------------------------- simple cubic, colour-split ----
-// Neighbours are summed in increasing site-number order, which is the reference's nn
-// order: below-plane z neighbours, below-row y neighbours, the x pair, above-row y,
-// above-plane z.  At a periodic boundary a pair changes side (u=0: both above, in
-// order u+1, u-1; u=L-1: both below, in order u+1, u-1).
+// Neighbours are summed in increasing site-number order, which is the reference's nn order.
 struct Acc3 {
     float x, y, z;
 };
@@ -129,40 +126,58 @@ __device__ __forceinline__ void fma3(Acc3 &h, float jx, float jy, float jz, cons
     h.z = fmaf(jz, S.z, h.z);
 }
 
-__device__ __forceinline__ Acc3 sc_field(const float4 *__restrict__ opp, int L1, int L2, int L3,
-                                         int H, int xh, int y, int z, int p, float jx, float jy,
-                                         float jz) {
-    const int row = z * L2 + y;
-    const int x = 2 * xh + p;
-    const int ym = (y == 0 ? L2 - 1 : y - 1), yp = (y == L2 - 1 ? 0 : y + 1);
-    const int zm = (z == 0 ? L3 - 1 : z - 1), zp = (z == L3 - 1 ? 0 : z + 1);
-    int xh_m, xh_p;
-    if (p == 0) { xh_m = (xh == 0 ? H - 1 : xh - 1); xh_p = xh; }
-    else { xh_m = xh; xh_p = (xh == H - 1 ? 0 : xh + 1); }
-    const float4 Sxm = opp[row * H + xh_m];
-    const float4 Sxp = opp[row * H + xh_p];
-    const float4 Sym = opp[(z * L2 + ym) * H + xh];
-    const float4 Syp = opp[(z * L2 + yp) * H + xh];
-    const float4 Szm = opp[(zm * L2 + y) * H + xh];
-    const float4 Szp = opp[(zp * L2 + y) * H + xh];
+// The six neighbours of rank rho of a colour array; o points at that rank in the other
+// colour's array, where they sit at six offsets (one of the x pair at 0), and increasing site
+// number is increasing offset.  Away from the y and z faces that is z, y, x, x, y, z; at a face
+// a pair's offsets have one sign.  Loads and sum are separate steps, so that the sweep draws
+// its random numbers while the loads are in flight.
+struct ScNbr {
+    float4 za, zb, ya, yb, xa, xb;  // a: the lower site number of the pair
+    int nz, ny;                     // neighbours of the pair below the site (1 inside)
+};
+__device__ __forceinline__ ScNbr sc_neighbours(const float4 *__restrict__ o, int L2, int L3, int H, int xh, int y,
+                                               int z, int p) {
+    ScNbr n;
+    const int plane = L2 * H;
+    const int d = p == 0 ? (xh == 0 ? H - 1 : -1) : (xh == H - 1 ? 1 - H : 1);
+    const bool y0 = y == 0, y1 = y == L2 - 1, z0 = z == 0, z1 = z == L3 - 1;
+    const int far = (L3 - 1) * plane;
+    n.za = o[z0 ? plane : z1 ? -far : -plane];
+    n.ya = o[y0 ? H : y1 ? H - plane : -H];
+    n.xa = o[min(d, 0)];
+    n.xb = o[max(d, 0)];
+    n.yb = o[y0 ? plane - H : y1 ? -H : H];
+    n.zb = o[z0 ? far : z1 ? -plane : plane];
+    n.ny = y0 ? 0 : y1 ? 2 : 1;
+    n.nz = z0 ? 0 : z1 ? 2 : 1;
+    return n;
+}
+__device__ __forceinline__ Acc3 sc_sum(const ScNbr &n, float jx, float jy, float jz) {
     Acc3 h{0.f, 0.f, 0.f};
-    // below
-    if (z == L3 - 1) { fma3(h, jx, jy, jz, Szp); fma3(h, jx, jy, jz, Szm); }
-    else if (z != 0) fma3(h, jx, jy, jz, Szm);
-    if (y == L2 - 1) { fma3(h, jx, jy, jz, Syp); fma3(h, jx, jy, jz, Sym); }
-    else if (y != 0) fma3(h, jx, jy, jz, Sym);
-    // x pair in index order
-    const bool interior = (x != 0) && (x != L1 - 1);
-    const float4 xa = interior ? Sxm : Sxp;
-    const float4 xb = interior ? Sxp : Sxm;
-    fma3(h, jx, jy, jz, xa);
-    fma3(h, jx, jy, jz, xb);
-    // above
-    if (y == 0) { fma3(h, jx, jy, jz, Syp); fma3(h, jx, jy, jz, Sym); }
-    else if (y != L2 - 1) fma3(h, jx, jy, jz, Syp);
-    if (z == 0) { fma3(h, jx, jy, jz, Szp); fma3(h, jx, jy, jz, Szm); }
-    else if (z != L3 - 1) fma3(h, jx, jy, jz, Szp);
+    if ((n.ny & n.nz) == 1) {  // whole rows take this path: 94% of a 64^3 lattice's
+        fma3(h, jx, jy, jz, n.za);
+        fma3(h, jx, jy, jz, n.ya);
+        fma3(h, jx, jy, jz, n.xa);
+        fma3(h, jx, jy, jz, n.xb);
+        fma3(h, jx, jy, jz, n.yb);
+        fma3(h, jx, jy, jz, n.zb);
+        return h;
+    }
+    if (n.nz > 0) fma3(h, jx, jy, jz, n.za);
+    if (n.nz > 1) fma3(h, jx, jy, jz, n.zb);
+    if (n.ny > 0) fma3(h, jx, jy, jz, n.ya);
+    if (n.ny > 1) fma3(h, jx, jy, jz, n.yb);
+    fma3(h, jx, jy, jz, n.xa);
+    fma3(h, jx, jy, jz, n.xb);
+    if (n.ny == 0) fma3(h, jx, jy, jz, n.ya);
+    if (n.ny < 2) fma3(h, jx, jy, jz, n.yb);
+    if (n.nz == 0) fma3(h, jx, jy, jz, n.za);
+    if (n.nz < 2) fma3(h, jx, jy, jz, n.zb);
     return h;
+}
+__device__ __forceinline__ Acc3 sc_field(const float4 *__restrict__ o, int L2, int L3, int H, int xh, int y, int z,
+                                         int p, float jx, float jy, float jz) {
+    return sc_sum(sc_neighbours(o, L2, L3, H, xh, y, z, p), jx, jy, jz);
 }
 
 // Exchange field of rank rho of a colour class from its ELL block (ell: entries k * n_c + rho,
@@ -241,43 +256,77 @@ __device__ __forceinline__ bool xyz_sc_site(const XyzSc &A, const XyzParams &P, 
     const int xh = rho - row * A.H;
     const int z = (int)fdiv((uint32_t)row, A.fL2), y = row - z * A.L2;
     const int p = (y + z + (int)A.colour) & 1;
-    Acc3 h = sc_field(A.opp, A.L1, A.L2, A.L3, A.H, xh, y, z, p, A.jx, A.jy, A.jz);
-    return metro_site<OPT>(P, A.own, rho, (uint32_t)rho, h.x, h.y, h.z, beta_f, t, c3, K, stream);
+    const ScNbr nb = sc_neighbours(A.opp + rho, A.L2, A.L3, A.H, xh, y, z, p);
+    const float4 S = A.own[rho];
+    U4 b0, b1;
+    site_draws<OPT>(P, (uint32_t)rho, t, c3, K, stream, b0, b1);
+    const Acc3 h = sc_sum(nb, A.jx, A.jy, A.jz);
+    float4 nv;
+    const bool acc = metro_decide<OPT>(P, rho, S, b0, b1, h.x, h.y, h.z, beta_f, (uint32_t)rho, t, c3, K, stream, nv);
+    if (acc) A.own[rho] = nv;
+    return acc;
 }
 
-// VPT sites rho0 + j * step (j < VPT, all < n) in three passes -- loads and exchange fields,
-// the Philox blocks, then decisions and stores -- so that the independent chains of the
-// sites interleave.  Returns the number of accepted updates.
-template <int OPT, int VPT>
-__device__ __forceinline__ unsigned xyz_sc_sites(const XyzSc &A, const XyzParams &P, int rho0, int step,
-                                                 int n, float beta_f, uint32_t t, uint32_t c3,
-                                                 const RoundKeys &K, uint32_t stream) {
-    float4 S[VPT];
-    Acc3 h[VPT];
-#pragma unroll
-    for (int j = 0; j < VPT; ++j) {
-        const int rho = min(rho0 + j * step, n - 1);  // a clamped duplicate is never stored
-        const int row = (int)fdiv((uint32_t)rho, A.fH);
-        const int xh = rho - row * A.H;
-        const int z = (int)fdiv((uint32_t)row, A.fL2), y = row - z * A.L2;
-        const int p = (y + z + (int)A.colour) & 1;
-        h[j] = sc_field(A.opp, A.L1, A.L2, A.L3, A.H, xh, y, z, p, A.jx, A.jy, A.jz);
-        S[j] = A.own[rho];
-    }
-    U4 b0[VPT], b1[VPT];
-#pragma unroll
-    for (int j = 0; j < VPT; ++j) site_draws<OPT>(P, (uint32_t)(rho0 + j * step), t, c3, K, stream, b0[j], b1[j]);
+// The sites (col, z), z0 <= z < z1, of one column (col = y H + xh) up the z axis.  Of a site's
+// neighbours two are known from the site below it -- its z - 1 neighbour was that site's x
+// neighbour at offset 0, and its own one at offset 0 was that site's z + 1 neighbour -- and
+// the column fixes all indices but z: four neighbour loads a site instead of six, and a fifth
+// fewer instructions.  The random numbers are drawn while the loads are in flight.
+template <int OPT>
+__device__ __forceinline__ unsigned xyz_sc_column(const XyzSc &A, const XyzParams &P, int col, int z0, int z1,
+                                                  float beta_f, uint32_t t, uint32_t c3, const RoundKeys &K,
+                                                  uint32_t stream) {
+    const int H = A.H, L2 = A.L2, L3 = A.L3, plane = L2 * H;
+    const int y = (int)fdiv((uint32_t)col, A.fH), xh = col - y * H;
+    const int d0 = xh == 0 ? H - 1 : -1, d1 = xh == H - 1 ? 1 - H : 1;
+    const bool y0 = y == 0, y1 = y == L2 - 1;
+    const int dym = y0 ? plane - H : -H, dyp = y1 ? H - plane : H;
+    int rho = z0 * plane + col;
+    int p = (y + z0 + (int)A.colour) & 1;
+    const float4 *o = A.opp + rho;
+    float4 *w = A.own + rho;
+    float4 zm = o[z0 == 0 ? (L3 - 1) * plane : -plane], x0 = o[0];
     unsigned acc = 0;
-#pragma unroll
-    for (int j = 0; j < VPT; ++j) {
-        const int rho = rho0 + j * step;
+#pragma unroll 1
+    for (int z = z0; z < z1; ++z) {
+        const int d = p ? d1 : d0;
+        const float4 ym = o[dym], yp = o[dyp], xd = o[d], zp = o[z == L3 - 1 ? plane - L3 * plane : plane];
+        const float4 S = *w;
+        U4 b0, b1;
+        site_draws<OPT>(P, (uint32_t)rho, t, c3, K, stream, b0, b1);
+        // increasing site number; at a face the wrapped neighbour changes side
+        Acc3 h{0.f, 0.f, 0.f};
+        const float4 xa = d < 0 ? xd : x0, xb = d < 0 ? x0 : xd;
+        if (!y0 && !y1 && z != 0 && z != L3 - 1) {
+            fma3(h, A.jx, A.jy, A.jz, zm);
+            fma3(h, A.jx, A.jy, A.jz, ym);
+            fma3(h, A.jx, A.jy, A.jz, xa);
+            fma3(h, A.jx, A.jy, A.jz, xb);
+            fma3(h, A.jx, A.jy, A.jz, yp);
+            fma3(h, A.jx, A.jy, A.jz, zp);
+        } else {
+            if (z == L3 - 1) fma3(h, A.jx, A.jy, A.jz, zp);
+            if (z != 0) fma3(h, A.jx, A.jy, A.jz, zm);
+            if (y1) fma3(h, A.jx, A.jy, A.jz, yp);
+            if (!y0) fma3(h, A.jx, A.jy, A.jz, ym);
+            fma3(h, A.jx, A.jy, A.jz, xa);
+            fma3(h, A.jx, A.jy, A.jz, xb);
+            if (!y1) fma3(h, A.jx, A.jy, A.jz, yp);
+            if (y0) fma3(h, A.jx, A.jy, A.jz, ym);
+            if (z != L3 - 1) fma3(h, A.jx, A.jy, A.jz, zp);
+            if (z == 0) fma3(h, A.jx, A.jy, A.jz, zm);
+        }
         float4 nv;
-        const bool a = metro_decide<OPT>(P, min(rho, n - 1), S[j], b0[j], b1[j], h[j].x, h[j].y, h[j].z,
-                                         beta_f, (uint32_t)rho, t, c3, K, stream, nv);
-        if (a && rho < n) {
-            A.own[rho] = nv;
+        if (metro_decide<OPT>(P, rho, S, b0, b1, h.x, h.y, h.z, beta_f, (uint32_t)rho, t, c3, K, stream, nv)) {
+            *w = nv;
             ++acc;
         }
+        zm = x0;
+        x0 = zp;
+        o += plane;
+        w += plane;
+        rho += plane;
+        p ^= 1;
     }
     return acc;
 }

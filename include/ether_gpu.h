@@ -262,9 +262,8 @@ int ether_end_sweep(ether_ctx *ctx);
  * class for the process.  Ising simple cubic: variant = 10 * bytes per vector (4, 8, 16) +
  * vectors per thread (1, 2, 4), + 1000 for twice the vectors per thread; + 2000, 6162 and 4000 +
  * 10 * vectors + 1 / 4 name forms that now run as the kernel of their vector size and count.
- * XYZ simple cubic: variant = 5000 + 10 * sites per thread +
- * blocks per SM of the register cap (5011 .. 5015, 5021, 5022).  best_ms = one colour
- * phase.  Either
+ * XYZ simple cubic: 5011, 5012, 5013 (planes per thread: chosen by size, half, twice); 5014,
+ * 5015, 5021, 5022 run as 5011.  best_ms = one colour phase.  Either
  * output may be NULL. */
 int ether_autotune(ether_ctx *ctx, int32_t *variant, float *best_ms);
 /* Force a kernel variant (same encoding as ether_autotune). */
