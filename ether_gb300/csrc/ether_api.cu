@@ -202,7 +202,7 @@ int upload_ladder(Ctx &c) {
 
 void free_ctx(Ctx &c) {
     void *ptrs[] = {c.t.row_ptr, c.t.nbr, c.t.jidx, c.t.wstride, c.t.species, c.t.itype,
-                    c.t.ell_nbr, c.t.ell_j, c.t.ell_deg, c.t.J4, c.t.ell_ws, c.t.ell_desc,
+                    c.t.ell_nbr, c.t.ell_j, c.t.ell_deg, c.t.res_ent, c.t.J4, c.t.ell_ws, c.t.ell_desc,
                     c.t.type_base, c.t.type_half, c.t.J, c.t.Jd, c.t.zee, c.t.zeed, c.t.D,
                     c.t.mweight, c.t.site_of_storage, c.spins, c.spins4, c.beta_slot,
                     c.beta_slot_f, c.slot_of_rep, c.rep_of_slot, c.thr, c.stream_id,
@@ -532,6 +532,18 @@ extern "C" int ether_create(const ether_desc *d, ether_ctx **out) {
             TRY(dev_upload(c, &c.t.J4, j4));
         } else {
             TRY(dev_upload(c, &c.t.ell_ws, ews));
+        }
+        // general lattices whose replicas fit in shared memory: runs of sweeps without a launch
+        // per colour phase
+        if (!(c.flags & ETHER_FLAG_NO_RESIDENT)) {
+            int optin = 0;
+            cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+            std::vector<uint4> ent;
+            plan_general_resident(c, optin, row_ptr, nbr, jidx, wstr, ent);
+            if (c.gen_resident) {
+                TRY(dev_upload(c, &c.t.res_ent, ent));
+                CUDA_TRY(prepare_general_resident(c));
+            }
         }
     }
     const size_t RN = (size_t)c.R * N;
@@ -1109,7 +1121,7 @@ int ether::plain_sweep(Ctx &c) { return sweep_once(c); }
 // How many replica parts ether_mcs splits this context's sweeps into (general lattices:
 // their colour phases are small, dependent, latency-bound launches): 1 (no split), 2 or 4.
 static int sweep_parts(const Ctx &c) {
-    if (c.fast || c.resident) return 1;
+    if (c.fast || c.resident || c.gen_resident) return 1;
     return c.R >= 32 ? 4 : c.R >= 16 ? 2 : 1;
 }
 
@@ -1199,7 +1211,10 @@ extern "C" int ether_metropolis(ether_ctx *h, int32_t nsweeps, double *accept) {
         const int rc = ensure_parts(c);
         if (rc) return rc;
     }
-    if (nsweeps > 1 && c.n_parts > 1) {  // general lattices: replica parts side by side, same bits
+    if (nsweeps > 1 && c.gen_resident) {
+        for (int k = 0; k < nsweeps; k += 256)  // bounded launches
+            CUDA_TRY(launch_general_resident(c, std::min(256, nsweeps - k)));
+    } else if (nsweeps > 1 && c.n_parts > 1) {  // general lattices: replica parts side by side, same bits
         const int rc = sweeps_in_parts(c, nsweeps);
         if (rc) return rc;
     } else {
@@ -1434,7 +1449,7 @@ static int issue_step(Ctx &c, const ether_schedule *sch, int gates) {
 static int variant_of(const Ctx &c);
 
 // Steps sig[0 .. n): with a resident context the sweeps that no OVRR, PT or measurement
-// separates run as one ising_sc_resident launch; otherwise step by step.
+// separates run as one launch (ising_sc_resident, k_resident.cu); otherwise step by step.
 static int issue_steps(Ctx &c, const ether_schedule *sch, const int8_t *sig, int n) {
     if (c.n_parts > 1) {
         // runs of sweeps that no OVRR, PT or measurement separates, in replica parts
@@ -1451,36 +1466,25 @@ static int issue_steps(Ctx &c, const ether_schedule *sch, const int8_t *sig, int
         }
         return ETHER_OK;
     }
-    if (!c.resident) {
+    if (!c.resident && !c.gen_resident) {
         for (int k = 0; k < n; ++k) {
             int rc = issue_step(c, sch, sig[k]);
             if (rc) return rc;
         }
         return ETHER_OK;
     }
-    int pending = 0;
-    for (int k = 0; k < n; ++k) {
-        if (sig[k] & 1) {  // not reached for Ising (no OVRR), kept for the order of operations
-            if (pending) CUDA_TRY(launch_ising_resident(c, pending));
-            pending = 0;
-            int rc = overrelax_once(c, sch->ovrr_para);
-            if (rc) return rc;
-        }
-        ++pending;
-        if (sig[k] & 6) {
-            CUDA_TRY(launch_ising_resident(c, pending));
-            pending = 0;
-            if (sig[k] & 2) {
-                CUDA_TRY(launch_energy_mag(c, true));
-                CUDA_TRY(launch_pt(c, -1));
-            }
-            if (sig[k] & 4) {
-                CUDA_TRY(launch_energy_mag(c, true));
-                CUDA_TRY(launch_measure(c));
-            }
-        }
+    // runs of sweeps that no OVRR, PT or measurement separates: one resident launch each
+    auto run = [&](int m) { return c.resident ? launch_ising_resident(c, m) : launch_general_resident(c, m); };
+    for (int k = 0; k < n;) {
+        int rc = mcs_before_sweep(c, sch, sig[k]);
+        if (rc) return rc;
+        int j = k + 1;
+        while (j < n && !(sig[j - 1] & 6) && !(sig[j] & 1)) ++j;
+        CUDA_TRY(run(j - k));
+        rc = mcs_after_sweep(c, sig[j - 1]);
+        if (rc) return rc;
+        k = j;
     }
-    if (pending) CUDA_TRY(launch_ising_resident(c, pending));
     return ETHER_OK;
 }
 
@@ -1511,7 +1515,7 @@ extern "C" int ether_mcs(ether_ctx *h, const ether_schedule *sch, int32_t step0,
     int chunk = mcs_chunk(period);
     // resident contexts: the longest multiple of the period up to 256 steps, so that the
     // eventless stretches (equilibration) run as few long resident launches
-    if (c.resident && period <= 256) chunk = (int)(256 / period * period);
+    if ((c.resident || c.gen_resident) && period <= 256) chunk = (int)(256 / period * period);
     const bool use_graphs = !(c.flags & ETHER_FLAG_NO_GRAPHS);
     int step = step0 + 1;
     const int last = step0 + nsteps;

@@ -69,6 +69,7 @@ struct DevTables {
     int32_t *ell_ws = nullptr;    // Ising: stride of the threshold-table index
     uint16_t *ell_deg = nullptr;  // N: neighbours of a storage index
     int2 *ell_desc = nullptr;     // per colour: (offset of its ELL block, entries per rank)
+    uint4 *res_ent = nullptr;     // the lists packed for the resident sweep (k_resident.cu), or null
     float4 *J4 = nullptr;         // nJ: (Jxx, Jyy, Jzz, 0) in FP32
     uint8_t *sia_cls = nullptr;   // N: local-axis anisotropy class of a storage index
     float4 *sia_ax = nullptr;     // classes: (a_x, a_y, a_z, D) in FP32
@@ -120,6 +121,8 @@ struct Ctx {
     int ising_vpt = 1;           // vectors per thread of the simple-cubic Ising kernel
     int ising_code = 0;          // the variant that was asked for (0: the default choice)
     int xyz_variant = 11;        // simple-cubic XYZ kernel: planes per thread (xyz_planes, k_xyz.cu)
+    int gen_resident = 0;        // general lattices: blocks per replica of the resident sweep, 0 none
+    int res_q = 0, res_slots = 0, res_shell_end[8] = {0}, res_stride[8] = {0};  // its entries
     bool resident = false;       // ether_mcs runs runs of sweeps with ising_sc_resident
     unsigned long long *acc_before = nullptr;  // R: acceptance counts at the start of a call
     double *acc_ratio = nullptr;               // R: device acceptance ratios of a call
@@ -235,6 +238,12 @@ cudaError_t launch_ising_sweep(Ctx &c, int colour);
 bool ising_resident_possible(const Ctx &c, size_t smem_max);
 cudaError_t prepare_ising_resident(const Ctx &c);
 cudaError_t launch_ising_resident(Ctx &c, int nsweeps);
+// k_resident.cu
+void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &row_ptr, const std::vector<int32_t> &nbr,
+                           const std::vector<uint16_t> &jidx, const std::vector<int32_t> &wstride,
+                           std::vector<uint4> &ent);
+cudaError_t prepare_general_resident(const Ctx &c);
+cudaError_t launch_general_resident(Ctx &c, int nsweeps);
 bool ising_staged_shape(const Ctx &c, int vectors_per_step);
 int ising_default_vpt(const Ctx &c);
 cudaError_t launch_xyz_sweep(Ctx &c, int colour);

@@ -198,7 +198,7 @@ static int blocks_for_x(const Ctx &c, long work, int bs) {
     return (int)need;
 }
 
-static XyzParams xyz_params(const Ctx &c) {
+XyzParams xyz_params(const Ctx &c) {
     XyzParams P;
     P.zeeman = c.zeeman;
     P.sia = c.sia;

@@ -31,6 +31,8 @@ struct XyzParams {
     const float4 *sia_ax;     // class -> (a_x, a_y, a_z, D)
 };
 
+XyzParams xyz_params(const Ctx &c);  // k_xyz.cu
+
 // Option sets of the XYZ kernels: kXyzExchange folds the Zeeman, SIA and ANGLE branches away
 // at compile time (exchange only, Marsaglia proposals); kXyzGeneral reads them from P.
 enum : int { kXyzExchange = 0, kXyzGeneral = 1 };
