@@ -717,6 +717,7 @@ extern "C" int ether_get_spins(ether_ctx *h, int32_t replica, double *ion) {
 namespace {
 constexpr size_t kStageMax = size_t(512) << 20;  // pinned staging, per context
 constexpr size_t kChunkBytes = size_t(4) << 20;  // a copy per ~4 MB of spins
+constexpr size_t kKernelOnlyBytes = size_t(128) << 20;  // records of a call that no host thread helps with
 
 int host_threads() {
     const unsigned t = std::thread::hardware_concurrency();
@@ -951,6 +952,19 @@ static int spins_batch(Ctx &c, int32_t r0, int32_t n, double *ion, bool to_devic
         return fail(ETHER_ERR_ARG, std::string(to_device ? "ether_set_spins_batch" : "ether_get_spins_batch") +
                                        ": ion is not host memory mapped for n replicas' records");
     const size_t per_rep = c.model == ETHER_MODEL_ISING ? (size_t)c.N : sizeof(float4) * c.N;
+    // a small call goes through the kernel alone: its threads and staging cost the shared form
+    // about 1.2 ms whatever the size
+    if (sizeof(double) * 9 * (size_t)c.N * n <= kKernelOnlyBytes) {
+        const cudaError_t e = launch_ion_copy(c, r0, n, ion, to_device);
+        const cudaError_t e2 = e == cudaSuccess ? cudaStreamSynchronize(c.stream) : e;
+        if (e2 != cudaSuccess) {
+            cudaGetLastError();
+            return fail(ETHER_ERR_CUDA, std::string(to_device ? "ether_set_spins_batch: " : "ether_get_spins_batch: ") +
+                                            cudaGetErrorString(e2));
+        }
+        c.ion_last_kernel[to_device ? 1 : 0] = n;
+        return ETHER_OK;
+    }
     if (n >= 2 && host_threads() >= 2 && per_rep * (size_t)n <= kStageMax) {
         int nk = 0;
         const int rc = spins_shared(c, r0, n, ion, to_device, &nk);
