@@ -7,7 +7,7 @@
 // specialised for that class) and L2-sized group of members: a grid of blocks walks a table
 // of segments (member, replica, first unit, units), each segment a block-sized tile of one
 // replica's colour class.  A unit is what one thread updates at a time: a W-byte vector
-// (simple-cubic Ising) or one site (general Ising, XYZ; general lattices from the colour
+// (simple-cubic Ising), a column of planes (simple-cubic XYZ) or one site (general lattices, from the colour
 // classes' ELL neighbour blocks).  The per-site arithmetic is the member kernels' own
 // (sweep_ising.cuh, sweep_xyz.cuh) with the same random-number counters, so a batch sweep
 // reproduces the members' own sweeps bit for bit.  One sweep (the phases and the sweep
@@ -42,7 +42,8 @@ enum BatchClass : int {
 // to another member.  Plain data (no initialisers): it lives in __shared__.
 struct BatchMember {
     int32_t kind, N, L1, L2, L3, H;
-    FastDiv fH, fL2;
+    FastDiv fH, fL2, fP;  // fP: columns (H L2) of a simple-cubic XYZ member
+    int32_t planes, pad1; // its planes per unit
     uint8_t *spins;
     float4 *spins4;
     const uint32_t *thr;
@@ -106,15 +107,17 @@ __device__ __forceinline__ unsigned batch_xyz_sc(const BatchMember &m, uint32_t 
     const int half = m.H * m.L2 * m.L3;
     float4 *base = m.spins4 + (size_t)r * 2 * half;
     const XyzSc A{base + (size_t)colour * half, base + (size_t)(colour ^ 1u) * half,
-                  m.L1, m.L2, m.L3, m.H, m.fH, m.fL2, colour, m.jx, m.jy, m.jz};
+                  m.L1, m.L2, m.L3, m.H, m.fH, m.fP, colour, m.jx, m.jy, m.jz};
     const float beta_f = m.beta_slot_f[m.slot_of_rep[r]];
     const RoundKeys &K = m.K;  // read in place from shared memory: no registers held
     // exchange only, Marsaglia proposals: the options fold away at compile time
     XyzParams P = OPT == kXyzExchange ? XyzParams{0, 0, 0, 0.f, nullptr, nullptr, nullptr, 1} : m.P;
     if (P.sia_cls) P.sia_cls += (size_t)colour * half;  // sites are ranks in the colour array
     unsigned acc = 0;
-    for (int rho = first + (int)threadIdx.x; rho < end; rho += blockDim.x)
-        acc += xyz_sc_site<OPT>(A, P, rho, beta_f, t, c3, K, stream) ? 1u : 0u;
+    for (int u = first + (int)threadIdx.x; u < end; u += blockDim.x) {
+        const int chunk = (int)fdiv((uint32_t)u, m.fP), z0 = chunk * m.planes;
+        acc += xyz_sc_column<OPT>(A, P, u - chunk * (int)m.fP.d, z0, min(z0 + m.planes, m.L3), beta_f, t, c3, K, stream);
+    }
     return acc;
 }
 
@@ -139,18 +142,18 @@ __device__ __forceinline__ unsigned batch_xyz_ell(const BatchMember &m, uint32_t
 // b, b + gridDim.x, ...; the resident blocks sweep through memory together, so the
 // neighbour planes one tile reads are the planes its neighbours' tiles read at the same time
 // (L2 hits).  Contiguous: block b takes [block_first[b], block_first[b+1]), runs balanced by
-// an estimated cost per unit, so member and replica change rarely.  No block barriers: the
-// Ising thresholds live in a per-warp slot of shared memory.
+// an estimated cost per unit, so member and replica change rarely.  Block barriers only where a
+// simple-cubic Ising class moves to another replica (its thresholds' table).
 template <int CLS, int MINB>
 __global__ void __launch_bounds__(256, MINB)
 batch_phase_kernel(const BatchMember *__restrict__ members, const BatchSeg *__restrict__ segs,
                    const int32_t *__restrict__ block_first, int n_seg, uint32_t colour, int upt) {
-    // Per-warp copies of the current member's parameters and Ising thresholds: a warp moves
-    // to another member or replica without waiting for the rest of the block, and the
-    // parameters cost no registers.
+    // Per-warp copies of the current member's parameters: a warp moves to another member
+    // without waiting for the rest of the block, and the parameters cost no registers.  The
+    // thresholds' table (210 words) is the block's: every warp is on the same segment.
     constexpr bool kIsingSc = CLS == kCIsing16 || CLS == kCIsing8 || CLS == kCIsing4;
     __shared__ BatchMember s_m[8];
-    __shared__ uint32_t s_tab[8][kIsingSc ? kScTabWords : 1];
+    __shared__ uint32_t s_tab[kIsingSc ? kScTabWords : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     BatchMember &m = s_m[warp];
     uint32_t cur_member = 0xFFFFFFFFu, cur_rep = 0xFFFFFFFFu;
@@ -169,9 +172,9 @@ batch_phase_kernel(const BatchMember *__restrict__ members, const BatchSeg *__re
         }
         if constexpr (kIsingSc) {
             if (S.member != cur_member || r != cur_rep) {
-                __syncwarp();
-                fill_sc_table(m.thr + (size_t)m.slot_of_rep[r] * m.table_entries, s_tab[warp], lane, 32);
-                __syncwarp();
+                __syncthreads();  // the segment before is done
+                fill_sc_table(m.thr + (size_t)m.slot_of_rep[r] * m.table_entries, s_tab, threadIdx.x, blockDim.x);
+                __syncthreads();
             }
         }
         cur_member = S.member;
@@ -180,11 +183,11 @@ batch_phase_kernel(const BatchMember *__restrict__ members, const BatchSeg *__re
         const int first = (int)S.first, end = (int)(S.first + S.count);
         unsigned acc;
         if constexpr (CLS == kCIsing16)
-            acc = batch_ising_sc<16>(m, r, first, end, colour, sc_tab(s_tab[warp]), t, stream, upt);
+            acc = batch_ising_sc<16>(m, r, first, end, colour, sc_tab(s_tab), t, stream, upt);
         else if constexpr (CLS == kCIsing8)
-            acc = batch_ising_sc<8>(m, r, first, end, colour, sc_tab(s_tab[warp]), t, stream, upt);
+            acc = batch_ising_sc<8>(m, r, first, end, colour, sc_tab(s_tab), t, stream, upt);
         else if constexpr (CLS == kCIsing4)
-            acc = batch_ising_sc<4>(m, r, first, end, colour, sc_tab(s_tab[warp]), t, stream, upt);
+            acc = batch_ising_sc<4>(m, r, first, end, colour, sc_tab(s_tab), t, stream, upt);
         else if constexpr (CLS == kCIsingEll)
             acc = batch_ising_ell(m, r, first, end, colour, t, stream);
         else if constexpr (CLS == kCXyzScX)
@@ -280,17 +283,19 @@ struct ether_batch {
     int n_groups = 1;
     long long group_bytes = 0;          // spin bytes per group; 0: half the L2; 1: every member
                                         // alone, on its own phase kernels
+    bool by_size = true;                // large XYZ members alone on their own kernels (off once a tile
+                                        // shape was set or tuned)
     bool xyz_solo = false;              // every XYZ member alone on its own kernels, Ising members
                                         // in the class kernels
     long long l2_bytes = 0;
-    int n_branch = 2;
+    int n_branch = 4;
     std::vector<cudaStream_t> branch;
     std::vector<cudaEvent_t> ev_join;
     cudaEvent_t ev_fork = nullptr;
     int32_t *d_block_first = nullptr;
     size_t bf_capacity = 0;
     float xyz_cost = 20.f;              // estimated cost of an XYZ site, Ising site = 1
-    int minb = 1;                       // register cap: 1 = none, 3 or 4 = that many 256-thread blocks
+    int minb = 3;                       // register cap: 1 = none, 3 or 4 = that many 256-thread blocks
     int walk = 0;                       // 0 strided, 1 contiguous (see batch_phase_kernel), 2 one block per segment
     uint32_t **d_step_of = nullptr;
     int total_R = 0, max_col = 0;
@@ -315,6 +320,12 @@ struct ether_batch {
 };
 
 namespace {
+
+// XYZ members of at least this many sites (all replicas) run on their own kernels, side by side on
+// four branches of the graph, unless a tile shape was set: 32 mixed chains of 8^3 .. 48^3 with
+// 32 temperatures, MCS step with swaps every 5: 0.49 ms (2^18 sites: 0.50, 2^20: 0.50, none:
+// 0.53).
+constexpr long long kSoloSites = 65536;
 
 int bfail(int code, const std::string &msg) {
     set_error(msg);
@@ -346,6 +357,8 @@ BatchMember describe(const Ctx &c) {
     if (c.fast) {
         m.fH = make_fastdiv((uint32_t)m.H);
         m.fL2 = make_fastdiv((uint32_t)m.L2);
+        m.fP = make_fastdiv((uint32_t)(m.H * m.L2));
+        m.planes = 1;  // set_planes
     }
     m.spins = c.spins;
     m.spins4 = c.spins4;
@@ -387,6 +400,27 @@ BatchMember describe(const Ctx &c) {
     return m;
 }
 
+// Planes per unit of the simple-cubic XYZ members: the most of 8, 4, 2 with which the batch's units
+// still fill the GPU (six blocks of 256 per SM; 6 chains of 4 temperatures, where they do not:
+// MCS step 0.107 ms with 8, 0.093 with 1) and a replica has 512 of them, two per thread of a
+// block.
+void set_planes(std::vector<BatchMember> &hm, const std::vector<ether_ctx *> &members, int sm_count) {
+    auto units = [](const BatchMember &m, int v) { return (long)m.H * m.L2 * ((m.L3 + v - 1) / v); };
+    int most = 1;
+    for (int v = 8; v > 1 && most == 1; v /= 2) {
+        long n = 0;
+        for (size_t k = 0; k < hm.size(); ++k)
+            if (hm[k].kind == kBXyzSc) n += units(hm[k], v) * members[k]->c.R;
+        if (n >= 6L * 256 * sm_count) most = v;
+    }
+    for (BatchMember &m : hm)
+        if (m.kind == kBXyzSc) {
+            m.planes = 1;
+            for (int v = most; v > 1 && m.planes == 1; v /= 2)
+                if (units(m, v) >= 512) m.planes = v;
+        }
+}
+
 // Units of one replica's colour class: vectors (simple-cubic Ising) or sites.
 long units_of(const BatchMember &m, const Ctx &c, int colour) {
     if (colour >= c.ncol) return 0;
@@ -395,6 +429,7 @@ long units_of(const BatchMember &m, const Ctx &c, int colour) {
         case kBIsing16: return n_c / 16;
         case kBIsing8: return n_c / 8;
         case kBIsing4: return n_c / 4;
+        case kBXyzSc: return (long)m.H * m.L2 * ((m.L3 + m.planes - 1) / m.planes);
         default: return n_c;
     }
 }
@@ -422,6 +457,7 @@ int rebuild(ether_batch &b) {
         if (!h->c.beta_set) return bfail(ETHER_ERR_STATE, "batch member without beta (ether_set_beta / ether_set_ladder)");
         hm.push_back(describe(h->c));
     }
+    set_planes(hm, b.members, b.sm_count);
     // a member that runs its own phase kernels is captured with its variant of the moment:
     // a later ether_set_variant / ether_autotune of that member rebuilds the graph
     std::vector<int> hv;
@@ -445,28 +481,34 @@ int rebuild(ether_batch &b) {
     const long long budget = b.group_bytes > 0 ? b.group_bytes : std::max(1LL, b.l2_bytes / 2);
     b.group_of.assign(b.members.size(), 0);
     b.solo.clear();
+    // members that run their own phase kernels are a group each, after the others' groups: those
+    // above the budget; every XYZ member (xyz_solo); and unless a tile shape was asked for, the XYZ
+    // members that fill the GPU themselves (kSoloSites)
+    auto alone = [&](size_t k) {
+        const Ctx &c = b.members[k]->c;
+        const bool xyz = c.model == ETHER_MODEL_XYZ;
+        const long long sites = (long long)c.R * c.N;
+        return sites * (xyz ? (long long)sizeof(float4) : 1) > budget || (xyz && (b.xyz_solo || (b.by_size && sites >= kSoloSites)));
+    };
     {
-        int g = 0;
         long long used = 0;
-        b.solo.push_back(-1);
         for (size_t k = 0; k < b.members.size(); ++k) {
+            if (alone(k)) continue;
             const Ctx &c = b.members[k]->c;
             const long long bytes = (long long)c.R * c.N * (c.model == ETHER_MODEL_ISING ? 1 : (long long)sizeof(float4));
-            // a large member, or (xyz_solo) an XYZ member: a group of its own, its own kernels
-            const bool alone = bytes > budget || (b.xyz_solo && c.model == ETHER_MODEL_XYZ);
-            if (used > 0 && (used + bytes > budget || alone)) {
-                ++g;
-                used = 0;
+            if (b.solo.empty() || (used > 0 && used + bytes > budget)) {
                 b.solo.push_back(-1);
+                used = 0;
             }
-            b.group_of[k] = g;
+            b.group_of[k] = (int)b.solo.size() - 1;
             used += bytes;
-            if (alone) {
-                b.solo[g] = (int)k;  // no segments
-                used = budget + 1;   // the next member starts a new group
-            }
         }
-        b.n_groups = g + 1;
+        for (size_t k = 0; k < b.members.size(); ++k)
+            if (alone(k)) {
+                b.group_of[k] = (int)b.solo.size();
+                b.solo.push_back((int)k);
+            }
+        b.n_groups = (int)b.solo.size();
     }
     // segments: group, phase, class, member, replica, tile
     std::vector<BatchSeg> segs;
@@ -522,7 +564,7 @@ int rebuild(ether_batch &b) {
             case kBIsing8: unit_cost[k] = 9.0; break;
             case kBIsing4: unit_cost[k] = 5.5; break;
             case kBIsingEll: unit_cost[k] = 3.0 * deg; break;
-            case kBXyzSc: unit_cost[k] = b.xyz_cost; break;
+            case kBXyzSc: unit_cost[k] = b.xyz_cost * hm[k].planes; break;
             default: unit_cost[k] = 1.3 * b.xyz_cost * deg; break;
         }
     }
@@ -979,6 +1021,7 @@ extern "C" int ether_batch_set_config(ether_batch *b, int32_t threads, int32_t u
     b->bps = blocks_per_sm;
     b->group_bytes = 0;  // the class kernels over L2-sized groups, with this tile shape
     b->xyz_solo = false;
+    b->by_size = false;
     b->dirty = true;
     return ETHER_OK;
 }
@@ -1010,9 +1053,10 @@ extern "C" int ether_batch_autotune(ether_batch *b, int32_t *config, float *best
     for (const Saved &s : sv) BCUDA(cudaMemcpyAsync(backup + s.off, s.src, s.bytes, cudaMemcpyDeviceToDevice, b->stream));
     const int old_t = b->threads, old_u = b->upt, old_b = b->bps;
     const long long old_gb = b->group_bytes;
-    const bool old_xs = b->xyz_solo;
+    const bool old_xs = b->xyz_solo, old_bs = b->by_size;
     b->group_bytes = 0;  // the class-kernel stages below use L2-sized groups
     b->xyz_solo = false;
+    b->by_size = false;
     b->timed_sweeps = 0;
     int occ_max = 1;
     float best = 1e30f;
@@ -1159,6 +1203,7 @@ extern "C" int ether_batch_autotune(ether_batch *b, int32_t *config, float *best
     }
     b->group_bytes = rc ? old_gb : bgb;
     b->xyz_solo = rc ? old_xs : bxs;
+    b->by_size = rc ? old_bs : false;
     b->n_branch = rc ? old_nb : bnb;
     for (const Saved &s : sv) cudaMemcpyAsync(s.src, backup + s.off, s.bytes, cudaMemcpyDeviceToDevice, b->stream);
     cudaStreamSynchronize(b->stream);

@@ -240,8 +240,7 @@ __device__ __forceinline__ bool xyz_ell_site(const XyzParams &P, float4 *sp, int
     return metro_site<OPT>(P, sp, s, (uint32_t)rho, h.x, h.y, h.z, beta_f, t, c3, K, stream);
 }
 
-// One Metropolis update of rank rho of the simple-cubic colour array `own` (the other
-// colour's array is `opp`).
+// A replica's simple-cubic colour arrays: the updated colour's (own) and the other's (opp).
 struct XyzSc {
     float4 *own;
     const float4 *opp;
@@ -250,25 +249,6 @@ struct XyzSc {
     uint32_t colour;
     float jx, jy, jz;
 };
-template <int OPT>
-__device__ __forceinline__ bool xyz_sc_site(const XyzSc &A, const XyzParams &P, int rho,
-                                            float beta_f, uint32_t t, uint32_t c3, const RoundKeys &K,
-                                            uint32_t stream) {
-    const int row = (int)fdiv((uint32_t)rho, A.fH);
-    const int xh = rho - row * A.H;
-    const int z = (int)fdiv((uint32_t)row, A.fL2), y = row - z * A.L2;
-    const int p = (y + z + (int)A.colour) & 1;
-    const ScNbr nb = sc_neighbours(A.opp + rho, A.L2, A.L3, A.H, xh, y, z, p);
-    const float4 S = A.own[rho];
-    U4 b0, b1;
-    site_draws<OPT>(P, (uint32_t)rho, t, c3, K, stream, b0, b1);
-    const Acc3 h = sc_sum(nb, A.jx, A.jy, A.jz);
-    float4 nv;
-    const bool acc = metro_decide<OPT>(P, rho, S, b0, b1, h.x, h.y, h.z, beta_f, (uint32_t)rho, t, c3, K, stream, nv);
-    if (acc) A.own[rho] = nv;
-    return acc;
-}
-
 // The sites (col, z), z0 <= z < z1, of one column (col = y H + xh) up the z axis.  Of a site's
 // neighbours two are known from the site below it -- its z - 1 neighbour was that site's x
 // neighbour at offset 0, and its own one at offset 0 was that site's z + 1 neighbour -- and
