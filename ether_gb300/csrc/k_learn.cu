@@ -10,13 +10,17 @@
 //     A-sites are always colour 0 and the 32 B-sites colour 1;
 //   * network: input = the 96 boundary spins and 4 beta J; 128 -> 128 -> 128 -> 32 MLP, BF16
 //     weights and activations, FP32 accumulation, on the tensor cores (tcgen05, accumulators in
-//     TMEM): one CTA takes 128 patches, thread p owns patch p = TMEM lane p through all three
-//     layers and then performs the patch's Metropolis-Hastings step;
+//     TMEM): a group of 128 threads takes 128 patches, thread p owns patch p = TMEM lane p through all three
+//     layers;
 //   * proposal: A-site k up with probability T_k / 2^32 from the logit; every B-site then from
 //     its exact heat-bath conditional given the new A-sites and the boundary;
 //   * acceptance: log alpha = log q(old) - log q(new) - beta J (bond change), FP32 in a fixed
 //     order with an own exp (the same operations as oracle/learn_oracle.c, which replays a
 //     sweep bit for bit given the logits).
+// A class is three launches (gather_kernel, patch_kernel, mh_kernel): only the network needs the
+// weights' shared memory, which leaves few warps on an SM, so the gather and the
+// Metropolis-Hastings step, most of the instructions, run on their own with many (a class of
+// 64^3 x 256: one kernel 510 us, the three 173 us).
 // Training: maximum likelihood of the A-sites given the boundary on configurations the plain
 // sweep produced (any temperature of the context's ladder), Adam, straight-through BF16
 // rounding (train.cuh).
@@ -45,9 +49,12 @@ constexpr int OFF_W1 = 0, OFF_B1 = OFF_W1 + NH * NI, OFF_W2 = OFF_B1 + NH, OFF_B
 constexpr int IMG_W1 = 0, IMG_W2 = 32768, IMG_W3 = 65536, IMG_B1 = 73728, IMG_B2 = IMG_B1 + 512,
               IMG_B3 = IMG_B2 + 512, IMG_BYTES = IMG_B3 + 128;
 // Shared memory of the patch kernel (from a 1024-byte aligned base).
-constexpr int SM_A = 73728, SM_BIAS = SM_A + 32768, SM_PATCH = SM_BIAS + 1152,
-              SM_BAR = SM_PATCH + 128 * 28, SM_BYTES = SM_BAR + 16;
-constexpr int kThreads = 128;
+constexpr int kGroups = 4, SM_A = 73728, SM_BIAS = SM_A + kGroups * 32768, SM_BAR = SM_BIAS + 1152,
+              SM_BYTES = SM_BAR + 8 * kGroups + 16;
+// Patches of one pass: bounds the logits' memory (128 MB).  Smaller passes, whose logits would
+// stay in L2, lose more at their ends: 2^18 and 2^17 made a 64^3 x 256 sweep 8 and 19% slower.
+constexpr long long kPassPatches = 1LL << 20;
+constexpr int kThreads = 128;  // rows of a tile = threads of a group
 
 // ------------------------------------------------------------------ patch geometry ----
 // Local sites 0..31 = A-sites, 32..63 = B-sites, packed (a | b << 2 | c << 4); boundary
@@ -142,25 +149,23 @@ __device__ __forceinline__ uint32_t thr_of_logit(float z) {
 struct PatchParams {
     const uint8_t *img;           // packed weights + biases (IMG_BYTES)
     int *err;
-    // lattice mode
+    // lattice mode: patches of class cls of replicas r0 .. (n of them, replica-major)
     uint8_t *spins;
     int L1, L2, L3, H;
     long long half;               // sites per colour per replica
-    int P1, P2, P3, cls;
-    long long Pc;                 // patches of one class per replica
-    int R;
+    int P1, P2, P3, cls, r0, n;
+    FastDiv fPc, fhalf1, fP2;     // patches of a class per replica, P1 / 2, P2
     const uint32_t *stream_id, *lstep;
     const int32_t *slot_of_rep;
     const float *k4, *betaJf;     // per slot
-    const uint32_t *TB;           // per slot x 7
-    const float *LBup, *LBdn;     // per slot x 7
-    uint32_t seed;
+    const uint4 *HB;              // per slot x 7: heat-bath threshold, log probabilities up, down
+    RoundKeys K;                  // of the context's seed
     unsigned long long *acc;      // per replica: accepted patches
-    float *dump;                  // optional [R][Pc][32] logits of this class
+    uint32_t *bits;               // [5][n]: boundary (3 words), A-sites, B-sites of a patch
+    float *dump;                  // optional [n][32]: the pass's logits, kept
     // forward mode
-    const __nv_bfloat16 *X;       // [B][128]
-    int B;
-    float *Z;                     // [B][32]
+    const __nv_bfloat16 *X;       // [n][128]
+    float *Z;                     // logits: [n][32] (forward mode), [8][n] of four (lattice mode)
 };
 
 __device__ __forceinline__ int wrap(int x, int L) { return x >= L ? x - L : (x < 0 ? x + L : x); }
@@ -174,216 +179,267 @@ __device__ __forceinline__ long long site_addr(const PatchParams &P, int o0, int
     return (long long)((x + y + z) & 1) * P.half + ((long long)z * P.L2 + y) * P.H + (x >> 1);
 }
 
-// Per tile of 128 patches:
-//   1. thread p decodes patch p (replica, origin, reflection) into shared memory;
-//   2. each warp gathers its 32 patches cooperatively: lane l loads sites l, l+32, .., l+128
-//      of the list [96 boundary | 32 A | 32 B] and five ballots give the patch's bit masks;
-//   3. thread p writes its network input row (boundary spins, 4 beta J) into the A tile;
-//   4. three tcgen05 layers, TMEM lane p = patch p;
-//   5. thread p's Metropolis-Hastings step from the masks and its 32 logits.
-template <int MODE>  // 0: lattice patches + Metropolis-Hastings, 1: network forward on X
-__global__ void __launch_bounds__(kThreads, 2) patch_kernel(PatchParams P) {
+// Patch w of a pass: replica, number, sweep counter, origin and reflection.
+struct Patch {
+    int r, o0, o1, o2, par;
+    uint32_t pidx, t, stream;
+};
+__device__ __forceinline__ Patch decode(const PatchParams &P, int w) {
+    Patch D;
+    const int rr = (int)fdiv((uint32_t)w, P.fPc);
+    const int q = w - rr * (int)P.fPc.d;
+    D.r = P.r0 + rr;
+    const int row = (int)fdiv((uint32_t)q, P.fhalf1);
+    const int tt = q - row * (int)P.fhalf1.d;
+    const int pk = (int)fdiv((uint32_t)row, P.fP2), pj = row - pk * P.P2;
+    const int pi = 2 * tt + ((P.cls + pj + pk) & 1);
+    D.pidx = (uint32_t)(pi + P.P1 * (pj + P.P2 * pk));
+    D.t = P.lstep[D.r];
+    D.stream = P.stream_id[D.r];
+    const U4 ow = draw_rk(0xFFFFFFFFu, D.t, D.stream, kLearn | (0xFFu << 8), P.K);
+    const int ox = (int)(ow.x & 3u), oy = (int)((ow.x >> 2) & 3u), oz = (int)((ow.x >> 4) & 3u);
+    D.par = (ox + oy + oz) & 1;
+    D.o0 = 4 * pi + ox;
+    D.o1 = 4 * pj + oy;
+    D.o2 = 4 * pk + oz;
+    return D;
+}
+
+// The spins of every patch of a pass as bits, one thread per patch.  The sites a = -1, 1, 3 (the
+// odd ones) of a patch row are three neighbouring bytes of one colour's array, and so are a = 0,
+// 2, 4: one or two aligned words and a byte permute (which also undoes the reflection) bring them,
+// and shifted additions collect the same a of eight rows in a byte.  Lanes are neighbouring
+// patches of a lattice row, four bytes apart.  (64^3 x 256, per class: a warp gathering its
+// patches one after another, five sites per lane, 240 us; a byte load per site 45 us; this
+// 34 us.)
+struct RowWords {
+    int w0, w1;     // byte offsets of the words in a row
+    uint32_t sel;   // the three bytes, in order of a
+    bool two;       // they reach into the second word
+};
+__device__ __forceinline__ RowWords row_words(int x, int H, bool reversed) {
+    RowWords W;
+    const int h = x >> 1, s = h & 3;
+    W.w0 = h & ~3;
+    W.w1 = W.w0 + 4 < H ? W.w0 + 4 : 0;
+    W.two = s > 1;
+    W.sel = reversed ? (uint32_t)((s + 2) | ((s + 1) << 4) | (s << 8)) : (uint32_t)(s | ((s + 1) << 4) | ((s + 2) << 8));
+    return W;
+}
+__device__ __forceinline__ uint32_t row_bytes(const uint8_t *row, const RowWords &W) {
+    const uint32_t lo = *reinterpret_cast<const uint32_t *>(row + W.w0);
+    uint32_t hi = 0;
+    if (W.two) hi = *reinterpret_cast<const uint32_t *>(row + W.w1);
+    return __byte_perm(lo, hi, W.sel) & 0x00FFFFFFu;
+}
+// 16 bits to the even positions.
+__host__ __device__ __forceinline__ uint32_t spread(uint32_t x) {
+    x = (x | (x << 8)) & 0x00FF00FFu;
+    x = (x | (x << 4)) & 0x0F0F0F0Fu;
+    x = (x | (x << 2)) & 0x33333333u;
+    return (x | (x << 1)) & 0x55555555u;
+}
+// Byte i of eight faces' rows (rows 0-3 of the low face, 4-7 of the high one): to bits 4 u.
+__host__ __device__ __forceinline__ uint32_t face_bits(uint32_t acc, int i) {
+    uint32_t x = (acc >> (8 * i)) & 0xFFu;
+    x = (x & 15u) | ((x & 0xF0u) << 12);
+    return (x | (x << 3) | (x << 6) | (x << 9)) & 0x11111111u;
+}
+// Bits of a 16-row class word from the a = 0, 2 (even) and a = 1, 3 (odd) columns over the rows;
+// the class has the even columns in the rows of `even_rows`.
+__host__ __device__ __forceinline__ uint32_t class_bits(uint32_t a0, uint32_t a2, uint32_t a1, uint32_t a3,
+                                                        uint32_t even_rows) {
+    const uint32_t odd_rows = ~even_rows & 0xFFFFu;
+    return spread((a0 & even_rows) | (a1 & odd_rows)) | (spread((a2 & even_rows) | (a3 & odd_rows)) << 1);
+}
+constexpr uint32_t kEvenRows = 0xA5A5u;  // bit b + 4 c set where b + c is even
+
+__global__ void __launch_bounds__(256) gather_kernel(const PatchParams P) {
+    const int w = blockIdx.x * 256 + threadIdx.x;
+    if (w >= P.n) return;
+    const Patch D = decode(P, w);
+    const uint8_t *sp = P.spins + (long long)D.r * 2 * P.half;
+    const bool rev = D.par != 0;
+    const int x0 = wrap(D.o0 - 1, P.L1), x1 = wrap(D.o0, P.L1);
+    const RowWords odd = row_words(rev ? x1 : x0, P.H, rev), even = row_words(rev ? x0 : x1, P.H, rev);
+    int yo[6];
+    long long zo[6];
+#pragma unroll
+    for (int a = 0; a < 6; ++a) {
+        yo[a] = wrap(D.o1 + a - 1, P.L2) * P.H;
+        zo[a] = (long long)wrap(D.o2 + a - 1, P.L3) * P.L2 * P.H;
+    }
+    uint32_t io[2] = {0, 0}, ie[2] = {0, 0};        // inner rows 0-7, 8-15: odd and even a
+    uint32_t fo[2] = {0, 0}, fe[2] = {0, 0};        // y and z faces' rows
+#pragma unroll
+    for (int c = -1; c <= 4; ++c) {
+#pragma unroll
+        for (int b = -1; b <= 4; ++b) {
+            const bool yin = b >= 0 && b < 4, zin = c >= 0 && c < 4;
+            if (!yin && !zin) continue;
+            const uint8_t *row = sp + zo[c + 1] + yo[b + 1];
+            const uint32_t vo = row_bytes(row + (((1 + b + c) & 1) ? P.half : 0), odd);
+            const uint32_t ve = row_bytes(row + (((b + c) & 1) ? P.half : 0), even);
+            if (yin && zin) {
+                const int k = b + 4 * c;
+                io[k >> 3] += vo << (k & 7);
+                ie[k >> 3] += ve << (k & 7);
+            } else {
+                const int f = yin ? 1 : 0, k = yin ? b + (c < 0 ? 0 : 4) : c + (b < 0 ? 0 : 4);
+                fo[f] += vo << k;
+                fe[f] += ve << k;
+            }
+        }
+    }
+    // odd bytes: a = -1, 1, 3; even bytes: a = 0, 2, 4
+    const uint32_t am = __byte_perm(io[0], io[1], 0x40) & 0xFFFFu, a1 = __byte_perm(io[0], io[1], 0x51) & 0xFFFFu,
+                   a3 = __byte_perm(io[0], io[1], 0x62) & 0xFFFFu, a0 = __byte_perm(ie[0], ie[1], 0x40) & 0xFFFFu,
+                   a2 = __byte_perm(ie[0], ie[1], 0x51) & 0xFFFFu, a4 = __byte_perm(ie[0], ie[1], 0x62) & 0xFFFFu;
+    uint32_t word[5];
+    word[0] = am | (a4 << 16);
+#pragma unroll
+    for (int f = 0; f < 2; ++f)
+        word[1 + f] = face_bits(fe[f], 0) | (face_bits(fo[f], 1) << 1) | (face_bits(fe[f], 1) << 2) |
+                      (face_bits(fo[f], 2) << 3);
+    word[3] = class_bits(a0, a2, a1, a3, kEvenRows);
+    word[4] = class_bits(a0, a2, a1, a3, ~kEvenRows & 0xFFFFu);
+#pragma unroll
+    for (int k = 0; k < 5; ++k) P.bits[(size_t)k * P.n + w] = word[k];
+}
+
+// All threads of group g agree (barrier 1 + g; 0 is __syncthreads).
+__device__ __forceinline__ void group_sync(int g) {
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(kThreads) : "memory");
+}
+__device__ __forceinline__ bool group_and(int g, bool v) {
+    int r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.and.pred q, %2, %3, p;\n\t"
+                 "selp.s32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"((int)v), "r"(1 + g), "n"(kThreads) : "memory");
+    return r != 0;
+}
+
+// The network on tiles of 128 rows: thread p of a group writes its input row (lattice mode:
+// boundary spins from the gathered bits, 4 beta J) into the group's A tile, then three tcgen05
+// layers, TMEM lane p = row p; logits to Z.  A layer is a chain (tile in shared memory, MMA,
+// TMEM to registers and back), so the time is latency: four groups share one copy of the weights
+// and keep 16 warps on the SM (two CTAs with a copy each keep 8; 524288 patches: 90 -> 71 us),
+// and a group loads its next 32 columns from TMEM while it works on these (-> 65 us).
+template <int MODE>  // 0: lattice patches, 1: network forward on X
+__global__ void __launch_bounds__(kGroups * kThreads, 1) patch_kernel(const PatchParams P) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     float *bias = reinterpret_cast<float *>(base + SM_BIAS);  // b1[128], b2[128], b3[32]
-    uint32_t *s_org = reinterpret_cast<uint32_t *>(base + SM_PATCH);  // origin | par << 30
-    int32_t *s_rep = reinterpret_cast<int32_t *>(s_org + 128);       // replica, -1 = none
-    uint32_t *s_bits = reinterpret_cast<uint32_t *>(s_rep + 128);    // [128][5]
     uint64_t *bar = reinterpret_cast<uint64_t *>(base + SM_BAR);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base + SM_BAR + 8);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base + SM_BAR + 8 * kGroups);
+    const int group = threadIdx.x >> 7, tid = threadIdx.x & 127, warp = tid >> 5;
+    bar += group;
 
     // weights and biases into shared memory (plain 16-byte copies; the image is pre-swizzled)
     {
         const uint4 *src = reinterpret_cast<const uint4 *>(P.img);
         uint4 *dw = reinterpret_cast<uint4 *>(base);
-        constexpr int nw = IMG_B1 / 16;  // 4608 = 36 x 128
-        for (int i0 = 0; i0 < nw; i0 += 8 * kThreads) {
-            uint4 v[8];
+        constexpr int nw = IMG_B1 / 16, nt = kGroups * kThreads;  // 4608 = 9 x 512
+        uint4 v[nw / nt];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int i = i0 + u * kThreads + tid;
-                if (i < nw) v[u] = __ldg(src + i);
-            }
+        for (int u = 0; u < nw / nt; ++u) v[u] = __ldg(src + u * nt + threadIdx.x);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int i = i0 + u * kThreads + tid;
-                if (i < nw) dw[i] = v[u];
-            }
-        }
+        for (int u = 0; u < nw / nt; ++u) dw[u * nt + threadIdx.x] = v[u];
         uint4 *db = reinterpret_cast<uint4 *>(base + SM_BIAS);
-        for (int i = tid; i < (IMG_BYTES - IMG_B1) / 16; i += kThreads) db[i] = src[nw + i];
+        for (int i = threadIdx.x; i < (IMG_BYTES - IMG_B1) / 16; i += nt) db[i] = src[nw + i];
     }
-    if (tid == 0) {
+    if (tid == 0) {  // a barrier per group
         tc::mbar_init(tc::smem_u32(bar), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(tc::smem_u32(tmem_slot)));
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(tc::smem_u32(tmem_slot)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     tc::fence_proxy_async();
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = *tmem_slot + 128u * (uint32_t)group;
     const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-    const uint32_t sA = tc::smem_u32(base + SM_A);
+    const uint32_t sA = tc::smem_u32(base + SM_A + group * 32768);
     const uint32_t sW1 = tc::smem_u32(base + IMG_W1), sW2 = tc::smem_u32(base + IMG_W2),
                    sW3 = tc::smem_u32(base + IMG_W3);
-    uint8_t *arow = base + SM_A;
+    uint8_t *arow = base + SM_A + group * 32768;
     uint32_t phase = 0;
     bool ok = true;
 
-    // this lane's five sites of every patch: canonical (a, b, c) + 1, packed 4 bits each
-    uint32_t my_site[5];
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-        const int i = lane + 32 * c;
-        if (i < 96) {
-            my_site[c] = c_bnd[i];
-        } else {
-            const uint8_t e = c_site[i - 96];
-            my_site[c] = (uint32_t)(((e & 3) + 1) | ((((e >> 2) & 3) + 1) << 4) | (((e >> 4) + 1) << 8));
-        }
-    }
-
-    const long long total = MODE == 0 ? (long long)P.R * P.Pc : (long long)P.B;
-    const long long ntiles = (total + kThreads - 1) / kThreads;
-    for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        const long long w = tile * kThreads + tid;
-        const bool valid = w < total;
-        int r = 0;
-        long long q = 0;
-        uint32_t pidx = 0, t = 0, stream = 0;
-        uint32_t bnd0 = 0, bnd1 = 0, bnd2 = 0, ao = 0, bo = 0;
+    const int ntiles = (P.n + kThreads - 1) / kThreads;
+    for (int tile = blockIdx.x + group * gridDim.x; tile < ntiles && ok; tile += kGroups * gridDim.x) {
+        const int w = tile * kThreads + tid;
+        const bool valid = w < P.n;
+        // ------------------------------------------------------------- input row ---------
+        uint32_t bw[4] = {0u, 0u, 0u, 0u};  // boundary bits; the last word stays zero
         float k4 = 0.f;
-        int o0 = 0, o1 = 0, o2 = 0, par = 0;
-        if (MODE == 0) {
-            // ------------------------------------------------------- 1. decode --------
-            if (valid) {
-                r = (int)(w / P.Pc);
-                q = w - (long long)r * P.Pc;
-                const int half1 = P.P1 >> 1;
-                const int tt = (int)(q % half1);
-                const long long row = q / half1;
-                const int pj = (int)(row % P.P2), pk = (int)(row / P.P2);
-                const int pi = 2 * tt + ((P.cls + pj + pk) & 1);
-                pidx = (uint32_t)(pi + P.P1 * (pj + P.P2 * pk));
-                t = P.lstep[r];
-                stream = P.stream_id[r];
-                const U4 ow = draw(0xFFFFFFFFu, t, stream, kLearn | (0xFFu << 8), P.seed);
-                const int ox = (int)(ow.x & 3u), oy = (int)((ow.x >> 2) & 3u), oz = (int)((ow.x >> 4) & 3u);
-                par = (ox + oy + oz) & 1;
-                o0 = 4 * pi + ox;
-                o1 = 4 * pj + oy;
-                o2 = 4 * pk + oz;
-                k4 = P.k4[P.slot_of_rep[r]];
-            }
-            s_org[tid] = (uint32_t)o0 | ((uint32_t)o1 << 10) | ((uint32_t)o2 << 20) | ((uint32_t)par << 30);
-            s_rep[tid] = valid ? r : -1;
-            __syncthreads();
-            // ------------------------------------------------------- 2. gather --------
-#pragma unroll 4
-            for (int j = 0; j < 32; ++j) {
-                const int pp = warp * 32 + j;
-                const int rr = s_rep[pp];
-                if (rr < 0) continue;  // warp-uniform
-                const uint32_t og = s_org[pp];
-                const int g0 = (int)(og & 1023u), g1 = (int)((og >> 10) & 1023u), g2 = (int)((og >> 20) & 1023u);
-                const int gp = (int)(og >> 30);
-                const uint8_t *sp = P.spins + (long long)rr * 2 * P.half;
-                uint32_t v[5];
+        if (MODE == 0 && valid) {
 #pragma unroll
-                for (int c = 0; c < 5; ++c) {
-                    const uint32_t e = my_site[c];
-                    v[c] = sp[site_addr(P, g0, g1, g2, gp, (int)(e & 15u) - 1, (int)((e >> 4) & 15u) - 1,
-                                        (int)(e >> 8) - 1)];
-                }
-#pragma unroll
-                for (int c = 0; c < 5; ++c) {
-                    const uint32_t m = __ballot_sync(0xffffffffu, v[c] != 0);
-                    if (lane == c) s_bits[pp * 5 + c] = m;
-                }
-            }
-            __syncthreads();
-            if (valid) {
-                bnd0 = s_bits[tid * 5 + 0];
-                bnd1 = s_bits[tid * 5 + 1];
-                bnd2 = s_bits[tid * 5 + 2];
-                ao = s_bits[tid * 5 + 3];
-                bo = s_bits[tid * 5 + 4];
-            }
+            for (int k = 0; k < 3; ++k) bw[k] = P.bits[(size_t)k * P.n + w];
+            k4 = P.k4[P.slot_of_rep[P.r0 + (int)fdiv((uint32_t)w, P.fPc)]];
         }
-        // ------------------------------------------------------------- 3. input row ------
-#pragma unroll 1
+#pragma unroll
         for (int ch = 0; ch < 16; ++ch) {
-            uint32_t pk4[4];
+            uint32_t pk4[4] = {0u, 0u, 0u, 0u};
             if (MODE == 1) {
                 if (valid) {
                     const uint4 v = reinterpret_cast<const uint4 *>(P.X + (size_t)w * NI)[ch];
                     pk4[0] = v.x; pk4[1] = v.y; pk4[2] = v.z; pk4[3] = v.w;
-                } else {
-                    pk4[0] = pk4[1] = pk4[2] = pk4[3] = 0u;
                 }
-            } else {
+            } else if (valid) {
+                if (ch < 12) {  // BF16 1.0 or -1.0 (sign bit from the complement of the spin)
+                    const uint32_t nb = ~(bw[ch >> 2] >> (8 * (ch & 3)));
 #pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    float v0 = 0.f, v1 = 0.f;
-                    const int i0 = ch * 8 + 2 * h, i1 = i0 + 1;
-                    if (valid) {
-                        if (i0 < 96) {
-                            const uint32_t wd = i0 < 32 ? bnd0 : (i0 < 64 ? bnd1 : bnd2);
-                            v0 = ((wd >> (i0 & 31)) & 1u) ? 1.0f : -1.0f;
-                            v1 = ((wd >> (i1 & 31)) & 1u) ? 1.0f : -1.0f;
-                        } else if (i0 == 96) {
-                            v0 = k4;
-                        }
-                    }
-                    const __nv_bfloat162 bv = __floats2bfloat162_rn(v0, v1);
-                    pk4[h] = *reinterpret_cast<const uint32_t *>(&bv);
+                    for (int h = 0; h < 4; ++h)
+                        pk4[h] = 0x3F803F80u | ((nb << (15 - 2 * h)) & 0x8000u) | ((nb << (30 - 2 * h)) & 0x80000000u);
+                } else if (ch == 12) {
+                    const __nv_bfloat162 bv = __floats2bfloat162_rn(k4, 0.f);
+                    pk4[0] = *reinterpret_cast<const uint32_t *>(&bv);
                 }
             }
             const int k = ch * 8;
             uint8_t *dst = arow + (k >> 6) * 16384 + tc::swz(tid, k & 63);
             *reinterpret_cast<uint4 *>(dst) = make_uint4(pk4[0], pk4[1], pk4[2], pk4[3]);
         }
-        // --------------------------------------------------------------- 4. layers -------
+        // ---------------------------------------------------------------- layers -------
         float z[32];
 #pragma unroll 1
         for (int layer = 0; layer < 3 && ok; ++layer) {
             tc::fence_proxy_async();
             tc::fence_before();
-            __syncthreads();
+            group_sync(group);
             if (tid == 0) {
                 tc::fence_after();
                 const int n = layer == 2 ? NO : NH;
                 const uint32_t idesc = tc::make_idesc(128, n);
                 const uint32_t sw = layer == 0 ? sW1 : (layer == 1 ? sW2 : sW3);
                 const uint32_t wtile = (uint32_t)n * 128u;  // bytes of one 64-column tile of W
-                const uint32_t dcol = layer == 1 ? 128u : 0u;
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk) {
                     const uint32_t ao_ = (uint32_t)(kk >> 2) * 16384u + (uint32_t)(kk & 3) * 32u;
                     const uint32_t bo_ = (uint32_t)(kk >> 2) * wtile + (uint32_t)(kk & 3) * 32u;
-                    tc::umma(tmem + dcol, tc::make_desc(sA + ao_), tc::make_desc(sw + bo_), idesc, kk > 0 ? 1u : 0u);
+                    tc::umma(tmem, tc::make_desc(sA + ao_), tc::make_desc(sw + bo_), idesc, kk > 0 ? 1u : 0u);
                 }
                 tc::umma_commit(tc::smem_u32(bar));
             }
             const bool got = tc::mbar_wait(tc::smem_u32(bar), phase, P.err, 1);
             phase ^= 1u;
-            ok = __syncthreads_and(got ? 1 : 0) != 0;
+            ok = group_and(group, got);
             if (!ok) break;
             tc::fence_after();
             if (layer < 2) {
                 // bias, ReLU, BF16, back into the A tile as the next layer's input
-                const uint32_t dcol = layer == 1 ? 128u : 0u;
                 const float *bl = bias + layer * 128;
-#pragma unroll 1
+                uint32_t v2[2][32];  // the next 32 columns come while these are worked on
+                tc::tmem_ld32(lane_base, v2[0]);
+#pragma unroll
                 for (int cc = 0; cc < 4; ++cc) {
-                    uint32_t v[32];
-                    tc::tmem_ld32(lane_base + dcol + 32u * cc, v);
-                    tc::tmem_wait_ld();
+                    uint32_t(&v)[32] = v2[cc & 1];
+                    tc::tmem_wait_ld(v);
+                    if (cc < 3) tc::tmem_ld32(lane_base + 32u * (cc + 1), v2[(cc + 1) & 1]);
 #pragma unroll
                     for (int g = 0; g < 4; ++g) {
                         uint32_t pk4[4];
@@ -411,97 +467,192 @@ __global__ void __launch_bounds__(kThreads, 2) patch_kernel(PatchParams P) {
         if (!ok) break;
         tc::fence_before();  // TMEM reads done before the next tile's MMAs (barrier at its layer 0)
         if (!valid) continue;
-        if (MODE == 1) {
-            float *zo = P.Z + (size_t)w * NO;
+        float4 *zo = reinterpret_cast<float4 *>(P.Z) + (MODE == 0 ? (size_t)w : (size_t)w * 8);
+        const size_t zs = MODE == 0 ? (size_t)P.n : 1;
 #pragma unroll
-            for (int k = 0; k < 32; ++k) zo[k] = z[k];
-            continue;
-        }
-        if (P.dump) {
-            float *zo = P.dump + ((size_t)r * P.Pc + q) * NO;
+        for (int k = 0; k < 8; ++k) zo[k * zs] = make_float4(z[4 * k], z[4 * k + 1], z[4 * k + 2], z[4 * k + 3]);
+        if (MODE == 0 && P.dump) {
+            float4 *dp = reinterpret_cast<float4 *>(P.dump + (size_t)w * NO);
 #pragma unroll
-            for (int k = 0; k < 32; ++k) zo[k] = z[k];
-        }
-        // ---------------------------------------------- 5. Metropolis-Hastings step ----
-        // d = log q(new) - log q(old): A-sites that changed add +-z_k (log-odds), then the
-        // B-sites' heat-bath log probabilities (tables); log alpha = (0 - d) - beta J dB.
-        const int slot = P.slot_of_rep[r];
-        const uint32_t *TB = P.TB + 7 * slot;
-        const float *LBup = P.LBup + 7 * slot, *LBdn = P.LBdn + 7 * slot;
-        uint32_t an = 0, bn = 0;
-        float d = 0.0f;
-        U4 rw{0, 0, 0, 0};
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-            if ((k & 3) == 0) rw = draw(pidx, t, stream, kLearn | ((uint32_t)(k >> 2) << 16), P.seed);
-            const uint32_t u = (k & 3) == 0 ? rw.x : (k & 3) == 1 ? rw.y : (k & 3) == 2 ? rw.z : rw.w;
-            const bool up = u < thr_of_logit(z[k]);
-            an |= (up ? 1u : 0u) << k;
-            if (up != (((ao >> k) & 1u) != 0)) d += up ? z[k] : -z[k];
-        }
-        int bond_n = 0, bond_o = 0;
-#pragma unroll
-        for (int m = 0; m < 32; ++m) {
-            if ((m & 3) == 0) rw = draw(pidx, t, stream, kLearn | ((uint32_t)(8 + (m >> 2)) << 16), P.seed);
-            const uint32_t u = (m & 3) == 0 ? rw.x : (m & 3) == 1 ? rw.y : (m & 3) == 2 ? rw.z : rw.w;
-            // up-neighbour counts (the heat-bath table index (n + 6) / 2)
-            int qn = 0, qo = 0;
-#pragma unroll
-            for (int qq = 0; qq < 6; ++qq) {
-                const int cd = geo_bn(m, qq);
-                if (cd >= 0) {
-                    qn += (int)((an >> cd) & 1u);
-                    qo += (int)((ao >> cd) & 1u);
-                } else {
-                    const int bi = -cd - 1;
-                    const uint32_t wd = bi < 32 ? bnd0 : (bi < 64 ? bnd1 : bnd2);
-                    const int sb = (int)((wd >> (bi & 31)) & 1u);
-                    qn += sb;
-                    qo += sb;
-                }
-            }
-            const int nn = 2 * qn - 6, no = 2 * qo - 6;
-            const bool up = u < TB[qn];
-            bn |= (up ? 1u : 0u) << m;
-            const bool upo = ((bo >> m) & 1u) != 0;
-            const float lbn = up ? LBup[qn] : LBdn[qn];
-            const float lbo = upo ? LBup[qo] : LBdn[qo];
-            d += lbn - lbo;
-            bond_n += (up ? 1 : -1) * nn;
-            bond_o += (upo ? 1 : -1) * no;
-        }
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-            int sb = 0;
-#pragma unroll
-            for (int qq = 0; qq < 6; ++qq) {
-                const int bi = geo_ab(k, qq);
-                if (bi < 0) continue;
-                const uint32_t wd = bi < 32 ? bnd0 : (bi < 64 ? bnd1 : bnd2);
-                sb += ((wd >> (bi & 31)) & 1u) ? 1 : -1;
-            }
-            bond_n += (((an >> k) & 1u) ? 1 : -1) * sb;
-            bond_o += (((ao >> k) & 1u) ? 1 : -1) * sb;
-        }
-        rw = draw(pidx, t, stream, kLearn | (16u << 16), P.seed);
-        const float la = (0.0f - d) - P.betaJf[slot] * (float)(bond_n - bond_o);
-        bool acc = la >= 0.0f;
-        if (!acc) acc = u01(rw.x) < expf_neg(la);
-        if (acc) {
-            uint8_t *sp = P.spins + (long long)r * 2 * P.half;
-            for (int k = 0; k < 32; ++k) {
-                const uint8_t e = c_site[k], f = c_site[32 + k];
-                sp[site_addr(P, o0, o1, o2, par, e & 3, (e >> 2) & 3, e >> 4)] = (uint8_t)((an >> k) & 1u);
-                sp[site_addr(P, o0, o1, o2, par, f & 3, (f >> 2) & 3, f >> 4)] = (uint8_t)((bn >> k) & 1u);
-            }
-            atomicAdd(P.acc + r, 1ull);
+            for (int k = 0; k < 8; ++k) dp[k] = make_float4(z[4 * k], z[4 * k + 1], z[4 * k + 2], z[4 * k + 3]);
         }
     }
     tc::fence_before();
     __syncthreads();
-    if (warp == 0) {
+    if (threadIdx.x < 32) {
         tc::fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+    }
+}
+
+// ------------------------------------------------------ Metropolis-Hastings by bit masks ----
+// The sites of a parity class of a patch are the bits 2 (b + 4 c) + (a >> 1) of a word, and with
+// p = (b + c) & 1 a row holds the A-sites a = p, p + 2 and the B-sites a = 1 - p, 3 - p.  So the
+// neighbours of all 32 sites of a class in one direction are a word: in x the other class's word
+// (rows of one parity) or that word moved by one bit (the others), in y moved by a row (2 bits),
+// in z by a plane (8 bits), with the boundary's faces where the patch ends.
+constexpr uint32_t rows_with(int parity) {  // bits of the rows with (b + c) & 1 == parity
+    uint32_t m = 0;
+    for (int row = 0; row < 16; ++row)
+        if ((((row & 3) + (row >> 2)) & 1) == parity) m |= 3u << (2 * row);
+    return m;
+}
+constexpr uint32_t kOdd = rows_with(1), kEven = rows_with(0), kBit0 = 0x55555555u, kBit1 = 0xAAAAAAAAu;
+constexpr uint32_t kY0 = 0x03030303u, kY3 = 0xC0C0C0C0u, kZ0 = 0x000000FFu, kZ3 = 0xFF000000u;
+
+// A y or z face (bits a + 4 u, u = c or b) to the sites of class cl (0 A, 1 B): of the four bits
+// of row u the two with a & 1 == (u + edge + cl) & 1 (edge: the face's b or c, 0 or 3), at bits
+// 2 u + (a >> 1) of the result.
+__device__ __forceinline__ uint32_t pick(uint32_t face, int odd_first) {
+    // bits a = 0, 2 (even) or 1, 3 (odd) of each nibble, alternating over the nibbles
+    const uint32_t even = face & 0x5555u, odd = (face >> 1) & 0x5555u;
+    uint32_t x = odd_first ? (odd & 0x0F0Fu) | (even & 0xF0F0u) : (even & 0x0F0Fu) | (odd & 0xF0F0u);
+    // x: nibble u holds the two bits at 0 and 2; bring them to 0 and 1, nibbles to pairs
+    x = (x | (x >> 1)) & 0x3333u;
+    x = (x | (x >> 2)) & 0x0F0Fu;
+    return (x | (x >> 4)) & 0x00FFu;
+}
+// The eight pairs of bits of `pairs` (2 bits per row u) to the y faces: rows b = 0 (at = 0) or 3.
+__device__ __forceinline__ uint32_t to_y(uint32_t pairs, int at) {
+    const uint32_t x = (pairs | (pairs << 12)) & 0x000F000Fu;   // u = 0, 1 | u = 2, 3
+    return ((x | (x << 6)) & 0x03030303u) << at;                // one pair per plane
+}
+
+// Boundary neighbours of one class's sites per direction, where there are any (mask m).
+struct Faces {
+    uint32_t w[6];
+};
+template <int CL>
+__device__ __forceinline__ Faces class_faces(uint32_t f0, uint32_t f1, uint32_t f2) {
+    // x: bnd bits 0-15 face a = -1 (row order), 16-31 face a = 4; the site next to a = -1 is bit
+    // 0 of its row where the class has a = 0 there (A: even rows, B: odd rows), the one next to
+    // a = 4 bit 1 where it has a = 3 (A: odd rows, B: even rows)
+    Faces F;
+    F.w[0] = spread(f0 & 0xFFFFu) & (CL ? kOdd : kEven);
+    F.w[1] = (spread(f0 >> 16) << 1) & (CL ? kEven : kOdd);
+    // y faces b = 0, 3: plane c, bits a + 4 c; class CL has a & 1 == (b + c + CL) & 1
+    F.w[2] = to_y(pick(f1 & 0xFFFFu, CL), 0);
+    F.w[3] = to_y(pick(f1 >> 16, CL ^ 1), 6);
+    // z faces c = 0, 3: row b, bits a + 4 b
+    F.w[4] = pick(f2 & 0xFFFFu, CL);
+    F.w[5] = pick(f2 >> 16, CL ^ 1) << 24;
+    return F;
+}
+__host__ __device__ constexpr uint32_t face_mask(int cl, int q) {
+    return q == 0 ? kBit0 & (cl ? kOdd : kEven) : q == 1 ? kBit1 & (cl ? kEven : kOdd)
+         : q == 2 ? kY0 : q == 3 ? kY3 : q == 4 ? kZ0 : kZ3;
+}
+// Up neighbours of the 32 B-sites as three bit planes, from the A-sites and the faces.
+struct Planes {
+    uint32_t n0, n1, n2;
+};
+__device__ __forceinline__ Planes b_neighbours(uint32_t A, const Faces &F) {
+    const uint32_t q0 = (A & kEven) | ((A << 1) & kBit1 & kOdd) | F.w[0];
+    const uint32_t q1 = (A & kOdd) | ((A >> 1) & kBit0 & kEven) | F.w[1];
+    const uint32_t q2 = ((A << 2) & ~kY0) | F.w[2], q3 = ((A >> 2) & ~kY3) | F.w[3];
+    const uint32_t q4 = (A << 8) | F.w[4], q5 = (A >> 8) | F.w[5];
+    const uint32_t s0 = q0 ^ q1 ^ q2, c0 = (q0 & q1) | (q2 & (q0 ^ q1));
+    const uint32_t s1 = q3 ^ q4 ^ q5, c1 = (q3 & q4) | (q5 & (q3 ^ q4));
+    const uint32_t k = s0 & s1;
+    return Planes{s0 ^ s1, c0 ^ c1 ^ k, (c0 & c1) | (k & (c0 ^ c1))};
+}
+// Sum over the B-sites of s (2 n - 6), s = +-1 from the bits of S.
+__device__ __forceinline__ int bond_sum(uint32_t S, const Planes &n) {
+    const int up = __popc(n.n0 & S) + 2 * __popc(n.n1 & S) + 4 * __popc(n.n2 & S);
+    const int all = __popc(n.n0) + 2 * __popc(n.n1) + 4 * __popc(n.n2);
+    return 2 * (2 * up - all) - 6 * (2 * __popc(S) - 32);
+}
+// Sum over the A-sites' boundary bonds of s_i s_j.
+__device__ __forceinline__ int edge_sum(uint32_t A, const Faces &F) {
+    int same = 0;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) same += __popc(~(A ^ F.w[q]) & face_mask(0, q));
+    return 2 * same - 48;  // 48 boundary bonds
+}
+
+// 17 Philox blocks, 32 sigmoids and 64 table rows per patch: instruction issue bounds it (524288
+// patches 73 us; with a loop over six neighbours per site, the loops unrolled and each thread
+// writing its own accepted patch 115 us).
+// One thread per patch: proposal from the logits, heat bath of the B-sites, acceptance.
+// d = log q(new) - log q(old): A-sites that changed add +-z_k (log-odds), then the B-sites'
+// heat-bath log probabilities (tables); log alpha = (0 - d) - beta J dB.
+__global__ void __launch_bounds__(128, 8) mh_kernel(const PatchParams P) {
+    if (*P.err) return;  // a network pass that gave up leaves the state as it was
+    const bool valid = blockIdx.x * 128 + threadIdx.x < P.n;
+    const int w = valid ? blockIdx.x * 128 + threadIdx.x : P.n - 1;
+    const Patch D = decode(P, w);
+    const uint32_t f0 = P.bits[w], f1 = P.bits[(size_t)P.n + w], f2 = P.bits[2 * (size_t)P.n + w];
+    const uint32_t ao = P.bits[3 * (size_t)P.n + w], bo = P.bits[4 * (size_t)P.n + w];
+    const int slot = P.slot_of_rep[D.r];
+    const uint4 *HB = P.HB + 7 * slot;
+    const float4 *z4 = reinterpret_cast<const float4 *>(P.Z) + w;
+    uint32_t an = 0, bn = 0;
+    float d = 0.0f;
+    // loops of four sites stay rolled: unrolled, the kernel waits on its own instructions
+    float4 z = z4[0];
+#pragma unroll 1
+    for (int k4 = 0; k4 < 8; ++k4) {
+        const float4 zn = k4 < 7 ? z4[(size_t)(k4 + 1) * P.n] : z;
+        const U4 rw = draw_rk(D.pidx, D.t, D.stream, kLearn | ((uint32_t)k4 << 16), P.K);
+        const float zs[4] = {z.x, z.y, z.z, z.w};
+        const uint32_t us[4] = {rw.x, rw.y, rw.z, rw.w};
+        const uint32_t old = ao >> (4 * k4);
+        uint32_t nib = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const bool up = us[j] < thr_of_logit(zs[j]);
+            nib |= (up ? 1u : 0u) << j;
+            if (up != (((old >> j) & 1u) != 0)) d += up ? zs[j] : -zs[j];
+        }
+        an |= nib << (4 * k4);
+        z = zn;
+    }
+    const Faces FB = class_faces<1>(f0, f1, f2);
+    const Planes nn = b_neighbours(an, FB), no = b_neighbours(ao, FB);
+    Planes sn = nn, so = no;
+#pragma unroll 1
+    for (int m4 = 0; m4 < 8; ++m4) {
+        const U4 rw = draw_rk(D.pidx, D.t, D.stream, kLearn | ((uint32_t)(8 + m4) << 16), P.K);
+        const uint32_t us[4] = {rw.x, rw.y, rw.z, rw.w};
+        const uint32_t old = bo >> (4 * m4);
+        uint32_t nib = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t qn = ((sn.n0 >> j) & 1u) | (((sn.n1 >> j) & 1u) << 1) | (((sn.n2 >> j) & 1u) << 2);
+            const uint32_t qo = ((so.n0 >> j) & 1u) | (((so.n1 >> j) & 1u) << 1) | (((so.n2 >> j) & 1u) << 2);
+            const uint4 hn = HB[qn], ho = HB[qo];
+            const bool up = us[j] < hn.x;
+            nib |= (up ? 1u : 0u) << j;
+            d += __uint_as_float(up ? hn.y : hn.z) - __uint_as_float(((old >> j) & 1u) ? ho.y : ho.z);
+        }
+        bn |= nib << (4 * m4);
+        sn.n0 >>= 4; sn.n1 >>= 4; sn.n2 >>= 4;
+        so.n0 >>= 4; so.n1 >>= 4; so.n2 >>= 4;
+    }
+    const Faces FA = class_faces<0>(f0, f1, f2);
+    const int bond_n = bond_sum(bn, nn) + edge_sum(an, FA), bond_o = bond_sum(bo, no) + edge_sum(ao, FA);
+    const U4 ra = draw_rk(D.pidx, D.t, D.stream, kLearn | (16u << 16), P.K);
+    const float la = (0.0f - d) - P.betaJf[slot] * (float)(bond_n - bond_o);
+    bool acc = la >= 0.0f;
+    if (!acc) acc = u01(ra.x) < expf_neg(la);
+    acc = acc && valid;
+    if (acc) atomicAdd(P.acc + D.r, 1ull);
+    // An accepted patch is written by its warp, two sites per lane (by its own thread it costs
+    // the warp the longest lane's number of changed sites).
+    const int lane = threadIdx.x & 31;
+    const uint32_t e0 = c_site[lane], e1 = c_site[32 + lane];
+    for (uint32_t m = __ballot_sync(0xffffffffu, acc); m; m &= m - 1) {
+        const int src = __ffs((int)m) - 1;
+        const uint32_t ca = __shfl_sync(0xffffffffu, an ^ ao, src), cb = __shfl_sync(0xffffffffu, bn ^ bo, src);
+        const uint32_t va = __shfl_sync(0xffffffffu, an, src), vb = __shfl_sync(0xffffffffu, bn, src);
+        const int o0 = __shfl_sync(0xffffffffu, D.o0, src), o1 = __shfl_sync(0xffffffffu, D.o1, src);
+        const int o2 = __shfl_sync(0xffffffffu, D.o2, src);
+        uint8_t *sp = P.spins + (long long)__shfl_sync(0xffffffffu, D.r, src) * 2 * P.half;
+        const int par = (o0 + o1 + o2) & 1;
+        if ((ca >> lane) & 1u)
+            sp[site_addr(P, o0, o1, o2, par, e0 & 3, (e0 >> 2) & 3, e0 >> 4)] = (uint8_t)((va >> lane) & 1u);
+        if ((cb >> lane) & 1u)
+            sp[site_addr(P, o0, o1, o2, par, e1 & 3, (e1 >> 2) & 3, e1 >> 4)] = (uint8_t)((vb >> lane) & 1u);
     }
 }
 
@@ -605,10 +756,13 @@ struct ether_learn {
     TrainBuffers tb;               // training scratch
     uint32_t *wp = nullptr;        // packed weights of the training kernels
     double *loss = nullptr;
-    // sweeps
+    // sweeps: a pass of up to `rows` patches
+    long long rows = 0;
+    uint32_t *bits = nullptr;
+    float *Zp = nullptr;
     uint32_t *lstep = nullptr;
-    float *k4 = nullptr, *betaJf = nullptr, *LBup = nullptr, *LBdn = nullptr;
-    uint32_t *TB = nullptr;
+    float *k4 = nullptr, *betaJf = nullptr;
+    uint4 *HB = nullptr;
     unsigned long long *acc = nullptr;
     float *dump = nullptr;
     bool dump_on = false;
@@ -663,8 +817,8 @@ int refresh_tables(ether_learn &l) {
     const Ctx &c = l.ctx->c;
     if (l.tables_for == c.beta_slots) return ETHER_OK;
     const int S = c.n_slots;
-    std::vector<float> k4(S), bj(S), lu(7 * S), ld(7 * S);
-    std::vector<uint32_t> tb(7 * S);
+    std::vector<float> k4(S), bj(S);
+    std::vector<uint4> hb(7 * S);
     for (int s = 0; s < S; ++s) {
         const double betaJ = c.beta_slots[s] * l.J;
         k4[s] = bf16_host((float)(4.0 * betaJ));
@@ -674,24 +828,23 @@ int refresh_tables(ether_learn &l) {
             const double pu = 1.0 / (1.0 + std::exp(2.0 * betaJ * nsum));
             double t = std::floor(pu * 4294967296.0 + 0.5);
             t = std::min(std::max(t, 1.0), 4294967295.0);
-            tb[7 * s + qi] = (uint32_t)t;
-            lu[7 * s + qi] = (float)std::log(t / 4294967296.0);
-            ld[7 * s + qi] = (float)std::log((4294967296.0 - t) / 4294967296.0);
+            const float up = (float)std::log(t / 4294967296.0);
+            const float dn = (float)std::log((4294967296.0 - t) / 4294967296.0);
+            uint4 &h = hb[7 * s + qi];
+            h = make_uint4((uint32_t)t, 0u, 0u, 0u);
+            std::memcpy(&h.y, &up, 4);
+            std::memcpy(&h.z, &dn, 4);
         }
     }
-    cudaFree(l.k4); cudaFree(l.betaJf); cudaFree(l.TB); cudaFree(l.LBup); cudaFree(l.LBdn);
-    l.k4 = l.betaJf = l.LBup = l.LBdn = nullptr;
-    l.TB = nullptr;
+    cudaFree(l.k4); cudaFree(l.betaJf); cudaFree(l.HB);
+    l.k4 = l.betaJf = nullptr;
+    l.HB = nullptr;
     LCUDA(cudaMalloc((void **)&l.k4, S * sizeof(float)));
     LCUDA(cudaMalloc((void **)&l.betaJf, S * sizeof(float)));
-    LCUDA(cudaMalloc((void **)&l.TB, 7 * S * sizeof(uint32_t)));
-    LCUDA(cudaMalloc((void **)&l.LBup, 7 * S * sizeof(float)));
-    LCUDA(cudaMalloc((void **)&l.LBdn, 7 * S * sizeof(float)));
+    LCUDA(cudaMalloc((void **)&l.HB, 7 * S * sizeof(uint4)));
     LCUDA(cudaMemcpy(l.k4, k4.data(), S * sizeof(float), cudaMemcpyHostToDevice));
     LCUDA(cudaMemcpy(l.betaJf, bj.data(), S * sizeof(float), cudaMemcpyHostToDevice));
-    LCUDA(cudaMemcpy(l.TB, tb.data(), 7 * S * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    LCUDA(cudaMemcpy(l.LBup, lu.data(), 7 * S * sizeof(float), cudaMemcpyHostToDevice));
-    LCUDA(cudaMemcpy(l.LBdn, ld.data(), 7 * S * sizeof(float), cudaMemcpyHostToDevice));
+    LCUDA(cudaMemcpy(l.HB, hb.data(), 7 * S * sizeof(uint4), cudaMemcpyHostToDevice));
     l.tables_for = c.beta_slots;
     return ETHER_OK;
 }
@@ -726,6 +879,7 @@ int read_err(ether_learn &l) {
     return ETHER_OK;
 }
 
+// One class of a learned sweep, in passes of whole replicas.
 int launch_patches(ether_learn &l, int cls, float *dump) {
     Ctx &c = l.ctx->c;
     PatchParams P;
@@ -737,19 +891,28 @@ int launch_patches(ether_learn &l, int cls, float *dump) {
     P.half = l.half;
     P.P1 = l.P[0]; P.P2 = l.P[1]; P.P3 = l.P[2];
     P.cls = cls;
-    P.Pc = l.Pc;
-    P.R = l.R;
+    P.fPc = make_fastdiv((uint32_t)l.Pc);
+    P.fhalf1 = make_fastdiv((uint32_t)(l.P[0] / 2));
+    P.fP2 = make_fastdiv((uint32_t)l.P[1]);
     P.stream_id = c.stream_id;
     P.lstep = l.lstep;
     P.slot_of_rep = c.slot_of_rep;
-    P.k4 = l.k4; P.betaJf = l.betaJf; P.TB = l.TB; P.LBup = l.LBup; P.LBdn = l.LBdn;
-    P.seed = c.seed;
+    P.k4 = l.k4; P.betaJf = l.betaJf; P.HB = l.HB;
+    P.K = round_keys(c.seed);
     P.acc = l.acc;
-    P.dump = dump;
-    const long long tiles = ((long long)l.R * l.Pc + kThreads - 1) / kThreads;
-    const int grid = (int)std::max<long long>(1, std::min<long long>(tiles, 2LL * l.sm_count));
-    patch_kernel<0><<<grid, kThreads, SM_BYTES + 1024, c.stream>>>(P);
-    l.launches++;
+    P.bits = l.bits;
+    P.Z = l.Zp;
+    const int per = (int)std::max<long long>(1, std::min<long long>(l.R, l.rows / l.Pc));
+    for (int r0 = 0; r0 < l.R; r0 += per) {
+        P.r0 = r0;
+        P.n = std::min(per, l.R - r0) * (int)l.Pc;
+        P.dump = dump ? dump + (size_t)r0 * l.Pc * NO : nullptr;
+        const int tiles = (P.n + kThreads - 1) / kThreads;
+        gather_kernel<<<(P.n + 255) / 256, 256, 0, c.stream>>>(P);
+        patch_kernel<0><<<std::min(tiles, l.sm_count), kGroups * kThreads, SM_BYTES + 1024, c.stream>>>(P);
+        mh_kernel<<<(P.n + 127) / 128, 128, 0, c.stream>>>(P);
+        l.launches += 3;
+    }
     LCUDA(cudaGetLastError());
     return ETHER_OK;
 }
@@ -810,6 +973,9 @@ extern "C" int ether_learn_create(ether_ctx *h, const ether_learn_desc *d, ether
     if (e == cudaSuccess) e = cudaMalloc((void **)&l->wp, Net::WORDS * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc((void **)&l->X, (size_t)l->cap * NI * sizeof(__nv_bfloat16));
     if (e == cudaSuccess) e = cudaMalloc((void **)&l->Y, (size_t)l->cap * sizeof(uint32_t));
+    l->rows = std::max<long long>(l->Pc, std::min<long long>((long long)l->R * l->Pc, kPassPatches));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&l->bits, 5 * (size_t)l->rows * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&l->Zp, (size_t)l->rows * NO * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&l->loss, sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc((void **)&l->lstep, l->R * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc((void **)&l->acc, l->R * sizeof(unsigned long long));
@@ -853,8 +1019,8 @@ extern "C" int ether_learn_destroy(ether_learn *l) {
     }
     if (l->ctx) cudaStreamSynchronize(l->ctx->c.stream);
     l->tb.release();
-    void *ptrs[] = {l->p, l->pq, l->g, l->m, l->v, l->img, l->X, l->Y, l->wp, l->loss, l->lstep, l->k4, l->betaJf, l->TB,
-                    l->LBup, l->LBdn, l->acc, l->dump, l->err};
+    void *ptrs[] = {l->p, l->pq, l->g, l->m, l->v, l->img, l->X, l->Y, l->wp, l->loss, l->bits, l->Zp, l->lstep, l->k4, l->betaJf, l->HB,
+                    l->acc, l->dump, l->err};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (l->e0) cudaEventDestroy(l->e0);
@@ -1090,10 +1256,10 @@ extern "C" int ether_learn_forward(ether_learn *l, const float *x, int32_t B, fl
         P.img = l->img;
         P.err = l->err;
         P.X = dX;
-        P.B = B;
+        P.n = B;
         P.Z = dZ;
         const int tiles = (B + kThreads - 1) / kThreads;
-        patch_kernel<1><<<std::min(tiles, 2 * l->sm_count), kThreads, SM_BYTES + 1024, st>>>(P);
+        patch_kernel<1><<<std::min(tiles, l->sm_count), kGroups * kThreads, SM_BYTES + 1024, st>>>(P);
         l->launches++;
         e = cudaGetLastError();
     }
