@@ -82,10 +82,10 @@ __host__ __device__ __forceinline__ float rcp_f(float x) {
 }
 
 // A von Mises-Fisher distribution on the unit sphere, vMF(m): kappa = |m|, rk = 1 / kappa,
-// log density at x = c + (m . x - kappa) with c = log(kappa / (1 - e^{-2 kappa})) - log 2 pi;
+// om = 1 - e^{-2 kappa}, log density at x = c + (m . x - kappa) with c = log(kappa / (1 - e^{-2 kappa})) - log 2 pi;
 // the uniform distribution (log density -log 4 pi) for kappa < kKappaMin.
 struct Vmf {
-    float mx, my, mz, kappa, rk, c;
+    float mx, my, mz, kappa, rk, om, c;
     bool uni;
 };
 __host__ __device__ __forceinline__ Vmf vmf_prep(float mx, float my, float mz) {
@@ -96,7 +96,8 @@ __host__ __device__ __forceinline__ Vmf vmf_prep(float mx, float my, float mz) {
     V.kappa = sqrtf(dot3(mx, my, mz, mx, my, mz));
     V.uni = V.kappa < kKappaMin;
     V.rk = V.uni ? 0.0f : rcp_f(V.kappa);
-    V.c = V.uni ? -kLog4Pi : logf_own(V.kappa * rcp_f(vmf_oneminus(V.kappa))) - kLog2Pi;
+    V.om = vmf_oneminus(V.kappa);
+    V.c = V.uni ? -kLog4Pi : logf_own(V.kappa * rcp_f(V.om)) - kLog2Pi;
     return V;
 }
 __host__ __device__ __forceinline__ float vmf_logpdf(const Vmf &V, float x, float y, float z) {
@@ -114,7 +115,7 @@ __host__ __device__ __forceinline__ void vmf_sample(const Vmf &V, float u, float
         ux = V.mx * V.rk;
         uy = V.my * V.rk;
         uz = V.mz * V.rk;
-        om = -log1m_own((1.0f - u) * vmf_oneminus(V.kappa)) * V.rk;
+        om = -log1m_own((1.0f - u) * V.om) * V.rk;
     }
     om = fminf(fmaxf(om, 0.0f), 2.0f);
     const float w = 1.0f - om;
@@ -146,6 +147,7 @@ struct XPatchParams {
     long long half;      // sites per colour per replica
     int P1, P2, P3, cls;
     long long Pc;        // patches of one class per replica
+    FastDiv fPc, fhalf1, fP2;  // Pc, P1 / 2, P2
     int r0, nrep;        // replicas of this pass
     const uint32_t *stream_id, *lstep;
     const int32_t *slot_of_rep;
@@ -173,28 +175,57 @@ __device__ __forceinline__ long long xsite(const XPatchParams &P, int o0, int o1
 struct XPatch {
     int r, o0, o1, o2, par, q;
     uint32_t pidx, t, stream;
+    float u;  // the acceptance's uniform
 };
+// By a whole warp: lane 31 draws the acceptance's block while the others draw the offset's.
 __device__ __forceinline__ XPatch xdecode(const XPatchParams &P, int w) {
     XPatch D;
-    const int Pc = (int)P.Pc;
-    const int rr = w / Pc;
+    const int rr = (int)fdiv((uint32_t)w, P.fPc);
     D.r = P.r0 + rr;
-    D.q = w - rr * Pc;
-    const int half1 = P.P1 >> 1;
-    const int row = D.q / half1;
-    const int tt = D.q - row * half1;
-    const int pk = row / P.P2, pj = row - pk * P.P2;
+    D.q = w - rr * (int)P.fPc.d;
+    const int row = (int)fdiv((uint32_t)D.q, P.fhalf1);
+    const int tt = D.q - row * (int)P.fhalf1.d;
+    const int pk = (int)fdiv((uint32_t)row, P.fP2), pj = row - pk * P.P2;
     const int pi = 2 * tt + ((P.cls + pj + pk) & 1);
     D.pidx = (uint32_t)(pi + P.P1 * (pj + P.P2 * pk));
     D.t = P.lstep[D.r];
     D.stream = P.stream_id[D.r];
-    const U4 ow = draw_rk(0xFFFFFFFFu, D.t, D.stream, kLearn | (0xFFu << 8), P.K);
-    const int ox = (int)(ow.x & 3u), oy = (int)((ow.x >> 2) & 3u), oz = (int)((ow.x >> 4) & 3u);
+    const bool last = (threadIdx.x & 31) == 31;
+    const U4 d = draw_rk(last ? D.pidx : 0xFFFFFFFFu, D.t, D.stream, last ? kLearn | (16u << 16) : kLearn | (0xFFu << 8), P.K);
+    const uint32_t ow = __shfl_sync(0xffffffffu, d.x, 0);
+    D.u = u01(__shfl_sync(0xffffffffu, d.x, 31));
+    const int ox = (int)(ow & 3u), oy = (int)((ow >> 2) & 3u), oz = (int)((ow >> 4) & 3u);
     D.par = (ox + oy + oz) & 1;
     D.o0 = 4 * pi + ox;
     D.o1 = 4 * pj + oy;
     D.o2 = 4 * pk + oz;
     return D;
+}
+
+// Storage offsets of a lane's five sites: boundary sites lane, lane + 32, lane + 64 (the x, y and
+// z faces) and the A- and B-site numbered lane.  A site's colour is its canonical (a + b + c) & 1,
+// and the five share coordinates, so a patch costs eleven wraps instead of one per coordinate of
+// every neighbour.  A replica holds fewer than 2^31 sites.
+struct LaneSites {
+    int off[5];
+};
+__device__ __forceinline__ int xwrap3(int x, int L) { return (int)__vimin3_u32((uint32_t)x, (uint32_t)(x + L), (uint32_t)(x - L)); }
+__device__ __forceinline__ LaneSites lane_sites(const XPatchParams &P, int o0, int o1, int o2, int par, int lane) {
+    const int u = lane & 3, v = (lane >> 2) & 3, e = (lane & 16) ? 4 : -1;
+    const int row = lane >> 1, b = row & 3, c = row >> 2, aa = geo_a_a(lane), ab = geo_b_a(lane);
+    const int xb = o0 + (par ? 3 : 0), xs = par ? -1 : 1, plane = P.L2 * P.H, half = (int)P.half;
+    const int xe = xwrap3(xb + xs * e, P.L1) >> 1, xu = xwrap3(xb + xs * u, P.L1) >> 1;
+    const int ye = xwrap3(o1 + e, P.L2) * P.H, yu = xwrap3(o1 + u, P.L2) * P.H, yv = xwrap3(o1 + v, P.L2) * P.H;
+    const int ze = xwrap3(o2 + e, P.L3) * plane, zv = xwrap3(o2 + v, P.L3) * plane;
+    const int yz = xwrap3(o1 + b, P.L2) * P.H + xwrap3(o2 + c, P.L3) * plane;
+    const int ce = ((e + u + v) & 1) ? half : 0;
+    LaneSites S;
+    S.off[0] = xe + yu + zv + ce;
+    S.off[1] = xu + ye + zv + ce;
+    S.off[2] = xu + yv + ze + ce;
+    S.off[3] = (xwrap3(xb + xs * aa, P.L1) >> 1) + yz;
+    S.off[4] = (xwrap3(xb + xs * ab, P.L1) >> 1) + yz + half;
+    return S;
 }
 
 __device__ __forceinline__ float xbf16r(float f) { return __bfloat162float(__float2bfloat16_rn(f)); }
@@ -206,13 +237,16 @@ __device__ __forceinline__ void xput(__nv_bfloat16 *p, float v) { *p = __float2b
 template <typename T>
 __device__ __forceinline__ void xinput_row(const XPatchParams &P, const float4 *sp, int o0, int o1, int o2, int par,
                                            float beta, T *row, int lane) {
-    for (int i = lane; i < 96; i += 32) {
-        int a, b, c;
-        geo_bnd(i, a, b, c);
-        const float4 S = sp[xsite(P, o0, o1, o2, par, a, b, c)];
-        xput(row + 3 * i, xbf16r(S.x));
-        xput(row + 3 * i + 1, xbf16r(S.y));
-        xput(row + 3 * i + 2, xbf16r(S.z));
+    const LaneSites A = lane_sites(P, o0, o1, o2, par, lane);
+    float4 S[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) S[j] = sp[A.off[j]];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        T *p = row + 3 * (lane + 32 * j);
+        xput(p, xbf16r(S[j].x));
+        xput(p + 1, xbf16r(S[j].y));
+        xput(p + 2, xbf16r(S[j].z));
     }
     if (lane < XNI - 288) {
         const float v = lane == 0 ? beta * P.jx : lane == 1 ? beta * P.jy : lane == 2 ? beta * P.jz : 0.0f;
@@ -268,42 +302,73 @@ __global__ void to_bf16_kernel(const float *__restrict__ q, __nv_bfloat16 *__res
 
 // The Metropolis-Hastings step of the patches of one pass (one warp per patch; lane k owns
 // A-site k and B-site k).  Z: the pass's network outputs (bias b3 added here); dump: optional
-// [R][Pc][96] parameters m of this class.
+// [R][Pc][96] parameters m of this class.  The patch's boundary and A-sites lie in shared memory
+// at addresses that do not change from patch to patch; the new A-sites take the old ones' place
+// once the old sums are made.  Instruction issue bounds it: 1170 per patch, of which three vMF
+// densities and two samples are most (131072 patches: 2050 per patch and 325 us with the storage
+// address of every neighbour worked out and shuffled A-sites, 175 us so).
 __global__ void __launch_bounds__(256, 4) xpatch_kernel(XPatchParams P, const float *__restrict__ Z,
                                                      const float *__restrict__ b3, float *__restrict__ dump,
                                                      unsigned long long *__restrict__ acc) {
+    __shared__ float4 s_sites[8][129];  // per warp: 96 boundary sites, 32 A-sites, zero
     const int k = threadIdx.x & 31;
+    float4 *ss = s_sites[threadIdx.x >> 5];
+    int nb[6], bnd[3] = {128, 128, 128};  // the B-site's neighbours, the A-site's boundary neighbours
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        const int cd = geo_bn(k, q);
+        nb[q] = cd >= 0 ? 96 + cd : -(cd + 1);
+    }
+    {
+        int n = 0;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            const int bi = geo_ab(k, q);
+            if (bi < 0) continue;
+            if (n == 0) bnd[0] = bi;
+            if (n == 1) bnd[1] = bi;
+            if (n == 2) bnd[2] = bi;
+            ++n;
+        }
+    }
+    if (k == 0) ss[128] = make_float4(0.f, 0.f, 0.f, 0.f);
     const int nwarps = (int)gridDim.x * (int)(blockDim.x >> 5);
     const int total = P.nrep * (int)P.Pc;
     for (int w = (int)blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5); w < total; w += nwarps) {
         const XPatch D = xdecode(P, w);
         float4 *sp = P.spins4 + (long long)D.r * 2 * P.half;
-        const float beta = P.beta_slot_f[P.slot_of_rep[D.r]];
-        const float nbeta = -beta;
-        // ---- A-site k: vMF(m_k) proposal; its bonds to the boundary
-        const int rowk = k >> 1;
-        const long long ia = xsite(P, D.o0, D.o1, D.o2, D.par, geo_a_a(k), rowk & 3, rowk >> 2);
-        const float4 xo = sp[ia];
+        const LaneSites A = lane_sites(P, D.o0, D.o1, D.o2, D.par, k);
+        const float4 xo = sp[A.off[3]], yo = sp[A.off[4]];
+        const float4 f0 = sp[A.off[0]], f1 = sp[A.off[1]], f2 = sp[A.off[2]];
         const float *zr = Z + (size_t)w * XNO + 3 * k;
         const float mx = zr[0] + b3[3 * k], my = zr[1] + b3[3 * k + 1], mz = zr[2] + b3[3 * k + 2];
+        const float nbeta = -P.beta_slot_f[P.slot_of_rep[D.r]];
         if (dump) {
             float *dr = dump + ((size_t)D.r * P.Pc + D.q) * XNO + 3 * k;
             dr[0] = mx;
             dr[1] = my;
             dr[2] = mz;
         }
-        float bx = 0.0f, by = 0.0f, bz = 0.0f;
+        __syncwarp();  // the previous patch's reads
+        ss[k] = f0;
+        ss[32 + k] = f1;
+        ss[64 + k] = f2;
+        ss[96 + k] = xo;
+        __syncwarp();
+        // ---- old neighbours of the B-site; the A-site's bonds to the boundary (at most three;
+        // the zero stands for the others)
+        float gox = 0.0f, goy = 0.0f, goz = 0.0f, bx = 0.0f, by = 0.0f, bz = 0.0f;
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
-            const int bi = geo_ab(k, q);
-            if (bi < 0) continue;
-            int a, b, c;
-            geo_bnd(bi, a, b, c);
-            const float4 S = sp[xsite(P, D.o0, D.o1, D.o2, D.par, a, b, c)];
-            bx += S.x;
-            by += S.y;
-            bz += S.z;
+            const float4 S = ss[nb[q]];
+            gox += S.x; goy += S.y; goz += S.z;
         }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const float4 S = ss[bnd[q]];
+            bx += S.x; by += S.y; bz += S.z;
+        }
+        // ---- A-site k: vMF(m_k) proposal
         const float hx = P.jx * bx, hy = P.jy * by, hz = P.jz * bz;
         const U4 rw = draw_rk(D.pidx, D.t, D.stream, kLearn | ((uint32_t)(32 + k) << 16), P.K);
         const Vmf VA = vmf_prep(mx, my, mz);
@@ -312,28 +377,14 @@ __global__ void __launch_bounds__(256, 4) xpatch_kernel(XPatchParams P, const fl
         const float sa_new = nbeta * dot3(nx, ny, nz, hx, hy, hz) - vmf_logpdf(VA, nx, ny, nz);
         const float sa_old = nbeta * dot3(xo.x, xo.y, xo.z, hx, hy, hz) - vmf_logpdf(VA, xo.x, xo.y, xo.z);
         // ---- B-site k: heat bath vMF(-beta J o (sum of its six neighbours)), new and old
-        const int rowm = k >> 1;
-        const long long ib = xsite(P, D.o0, D.o1, D.o2, D.par, geo_b_a(k), rowm & 3, rowm >> 2);
-        const float4 yo = sp[ib];
-        float gnx = 0.0f, gny = 0.0f, gnz = 0.0f, gox = 0.0f, goy = 0.0f, goz = 0.0f;
+        __syncwarp();
+        ss[96 + k] = make_float4(nx, ny, nz, 0.f);
+        __syncwarp();
+        float gnx = 0.0f, gny = 0.0f, gnz = 0.0f;
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
-            const int cd = geo_bn(k, q);
-            const int src = cd >= 0 ? cd : k;
-            float snx = __shfl_sync(0xffffffffu, nx, src), sny = __shfl_sync(0xffffffffu, ny, src),
-                  snz = __shfl_sync(0xffffffffu, nz, src);
-            float sox = __shfl_sync(0xffffffffu, xo.x, src), soy = __shfl_sync(0xffffffffu, xo.y, src),
-                  soz = __shfl_sync(0xffffffffu, xo.z, src);
-            if (cd < 0) {
-                int a, b, c;
-                geo_bnd(-cd - 1, a, b, c);
-                const float4 S = sp[xsite(P, D.o0, D.o1, D.o2, D.par, a, b, c)];
-                snx = sox = S.x;
-                sny = soy = S.y;
-                snz = soz = S.z;
-            }
-            gnx += snx; gny += sny; gnz += snz;
-            gox += sox; goy += soy; goz += soz;
+            const float4 S = ss[nb[q]];
+            gnx += S.x; gny += S.y; gnz += S.z;
         }
         const float mbnx = nbeta * (P.jx * gnx), mbny = nbeta * (P.jy * gny), mbnz = nbeta * (P.jz * gnz);
         const float mbox = nbeta * (P.jx * gox), mboy = nbeta * (P.jy * goy), mboz = nbeta * (P.jz * goz);
@@ -346,11 +397,10 @@ __global__ void __launch_bounds__(256, 4) xpatch_kernel(XPatchParams P, const fl
         float la = (sa_new + sb_new) - (sa_old + sb_old);
 #pragma unroll
         for (int o = 16; o >= 1; o >>= 1) la += __shfl_xor_sync(0xffffffffu, la, o);
-        const U4 ra = draw_rk(D.pidx, D.t, D.stream, kLearn | (16u << 16), P.K);
-        const bool accept = la >= 0.0f || u01(ra.x) < expf_neg(la);
+        const bool accept = la >= 0.0f || D.u < expf_neg(la);
         if (accept) {
-            sp[ia] = make_float4(nx, ny, nz, xo.w);
-            sp[ib] = make_float4(ynx, yny, ynz, yo.w);
+            sp[A.off[3]] = make_float4(nx, ny, nz, xo.w);
+            sp[A.off[4]] = make_float4(ynx, yny, ynz, yo.w);
             if (k == 0) atomicAdd(acc + D.r, 1ull);
         }
     }
@@ -359,17 +409,19 @@ __global__ void __launch_bounds__(256, 4) xpatch_kernel(XPatchParams P, const fl
 // ------------------------------------------------------------ inference network ----
 // xmlp_kernel: Z = W3 . h2, h2 = bf16(relu(W2 . h1 + b2)), h1 = bf16(relu(W1 . x + b1)) for
 // 128-row tiles of X (M x 304, BF16) on the fifth-generation tensor cores.  A persistent CTA of
-// four warps keeps the three weight matrices in shared memory (the image packed by
+// eight warps keeps the three weight matrices in shared memory (the image packed by
 // xpack_kernel: BF16, K-major, 128-byte swizzle, W1's K zero-padded to 320) and per tile:
 //   * thread 0 loads the X tile with five TMA copies (64 columns each; the columns past 304
 //     and the rows past M read as zeros), then issues each layer's tcgen05.mma chain (K = 16
 //     per instruction, FP32 accumulators in tensor memory: layer 1 in columns 0-127, layer 2
 //     in 128-255, layer 3 in 0-95) and commits it to an mbarrier;
-//   * thread p owns row p = TMEM lane p: after layers 1 and 2 it reads its 128 accumulators
-//     (tcgen05.ld), adds the BF16 bias, applies ReLU, rounds to BF16 and writes the next
+//   * threads p and p + 128 own row p = TMEM lane p, half of the columns each: after layers 1 and
+//     2 they read their accumulators (tcgen05.ld), add the BF16 bias, applies ReLU, rounds to BF16 and writes the next
 //     layer's A operand over the X tile; after layer 3 it writes its 96 outputs to Z;
 //   * once layer 3 has read its operand, the next tile's X copies start, under the last
 //     epilogue.
+// The weights come by one bulk copy.  131072 rows, cold: 45 us (four warps that copied the weights
+// themselves and owned whole rows: 55 us); the chain of the three layers of a tile bounds it.
 // Every wait is bounded (2 s of %globaltimer): on expiry the kernel records an error code,
 // stops, waits (bounded) for the copies and MMAs it started, and frees its tensor memory.
 constexpr int XKT1 = 5;  // 64-column K-tiles of layer 1
@@ -404,25 +456,23 @@ __device__ __forceinline__ void xtma_load(uint32_t dst, const CUtensorMap *map, 
         ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar) : "memory");
 }
 
-__global__ void __launch_bounds__(128, 1)
+constexpr int kXmlpThreads = 256;
+__global__ void __launch_bounds__(kXmlpThreads, 1)
 xmlp_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict__ img, float *__restrict__ Z, int M,
             int *__restrict__ err) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t *bar_x = reinterpret_cast<uint64_t *>(base + XSM_BAR);  // the X tile has landed
     uint64_t *bar_m = bar_x + 1;                                     // a layer's MMAs are done
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_m + 1);
-    const int tid = threadIdx.x, warp = tid >> 5;
+    uint64_t *bar_w = bar_m + 1;                                     // the weights have landed
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_w + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, row = tid & 127, part = tid >> 7;
     const int ntiles = (M + 127) / 128;
 
-    {  // weights and biases into shared memory (plain 16-byte copies of the swizzled image)
-        const uint4 *src = reinterpret_cast<const uint4 *>(img);
-        uint4 *dst = reinterpret_cast<uint4 *>(base);
-        for (int i = tid; i < XIMG_BYTES / 16; i += 128) dst[i] = __ldg(src + i);
-    }
     if (tid == 0) {
         tc::mbar_init(tc::smem_u32(bar_x), 1);
         tc::mbar_init(tc::smem_u32(bar_m), 1);
+        tc::mbar_init(tc::smem_u32(bar_w), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -434,7 +484,7 @@ xmlp_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict_
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t sA = tc::smem_u32(base + XSM_A);
     const uint32_t sW1 = tc::smem_u32(base + XIMG_W1), sW2 = tc::smem_u32(base + XIMG_W2),
                    sW3 = tc::smem_u32(base + XIMG_W3);
@@ -459,13 +509,16 @@ xmlp_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict_
         }
         tc::umma_commit(tc::smem_u32(bar_m));
     };
-    // this thread's 128 accumulators at dcol -> bf16(relu(acc + b)) -> A tiles 0, 1 of row tid
+    // this thread's 64 accumulators at dcol -> bf16(relu(acc + b)) -> A tile `part` of its row
     auto hidden = [&](uint32_t dcol, const float *b) {
-#pragma unroll 1
-        for (int cc = 0; cc < 4; ++cc) {
-            uint32_t v[32];
-            tc::tmem_ld32(lane_base + dcol + 32u * cc, v);
-            tc::tmem_wait_ld();
+        uint32_t v2[2][32];
+        tc::tmem_ld32(lane_base + dcol + 64u * part, v2[0]);
+#pragma unroll
+        for (int c2 = 0; c2 < 2; ++c2) {
+            const int cc = 2 * part + c2;
+            uint32_t(&v)[32] = v2[c2];
+            tc::tmem_wait_ld(v);
+            if (c2 == 0) tc::tmem_ld32(lane_base + dcol + 64u * part + 32u, v2[1]);
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
                 uint32_t pk4[4];
@@ -478,7 +531,7 @@ xmlp_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict_
                     pk4[h] = *reinterpret_cast<const uint32_t *>(&bv);
                 }
                 const int k = 32 * cc + 8 * g;
-                *reinterpret_cast<uint4 *>(arow + (k >> 6) * 16384 + tc::swz(tid, k & 63)) =
+                *reinterpret_cast<uint4 *>(arow + (k >> 6) * 16384 + tc::swz(row, k & 63)) =
                     make_uint4(pk4[0], pk4[1], pk4[2], pk4[3]);
             }
         }
@@ -496,10 +549,19 @@ xmlp_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict_
         tc::fence_after();
         return all;
     };
-    if (tid == 0 && (int)blockIdx.x < ntiles) {
-        load_x(blockIdx.x);
-        x_pending = true;
+    if (tid == 0) {
+        tc::mbar_arrive_tx(tc::smem_u32(bar_w), (uint32_t)XIMG_BYTES);
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         tc::smem_u32(base)),
+                     "l"(img), "r"(XIMG_BYTES), "r"(tc::smem_u32(bar_w))
+                     : "memory");
+        if ((int)blockIdx.x < ntiles) {
+            load_x(blockIdx.x);
+            x_pending = true;
+        }
     }
+    const bool w_got = tc::mbar_wait(tc::smem_u32(bar_w), 0, err, 7);
+    ok = __syncthreads_and(w_got ? 1 : 0) != 0;
     for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
         // ---- layer 1 on the X tile, once every thread has read the previous tile's layer-3
         // accumulators (the barrier) and the copies have landed
@@ -544,14 +606,13 @@ xmlp_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict_
             x_pending = true;
         }
         // tcgen05.ld is warp-collective: every lane reads, lanes past M store nothing
-        const int row = tile * 128 + tid;
-        float4 *z4 = reinterpret_cast<float4 *>(Z + (size_t)(row < M ? row : 0) * XNO);
-#pragma unroll 1
-        for (int cc = 0; cc < 3; ++cc) {
+        const int zrow = tile * 128 + row;
+        float4 *z4 = reinterpret_cast<float4 *>(Z + (size_t)(zrow < M ? zrow : 0) * XNO);
+        for (int cc = part ? 2 : 0; cc < (part ? 3 : 2); ++cc) {
             uint32_t v[32];
             tc::tmem_ld32(lane_base + 32u * cc, v);
-            tc::tmem_wait_ld();
-            if (row < M) {
+            tc::tmem_wait_ld(v);
+            if (zrow < M) {
 #pragma unroll
                 for (int g = 0; g < 8; ++g)
                     z4[8 * cc + g] = make_float4(__uint_as_float(v[4 * g]), __uint_as_float(v[4 * g + 1]),
@@ -562,6 +623,7 @@ xmlp_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict_
     }
     // after a failed wait: the copies and MMAs already started still write this block's
     // shared and tensor memory; wait for them (bounded) before freeing and exiting
+    if (tid == 0 && !w_got) tc::mbar_wait(tc::smem_u32(bar_w), 0, err, 8);
     if (tid == 0 && x_pending) tc::mbar_wait(tc::smem_u32(bar_x), ph_x, err, 5);
     bool drained = true;
     if (tid == 0 && m_pending) drained = tc::mbar_wait(tc::smem_u32(bar_m), ph_m, err, 6);
@@ -635,6 +697,9 @@ XPatchParams patch_params(const XyzLearn &x, int cls, int r0, int nrep) {
     P.P1 = x.P[0]; P.P2 = x.P[1]; P.P3 = x.P[2];
     P.cls = cls;
     P.Pc = x.Pc;
+    P.fPc = make_fastdiv((uint32_t)x.Pc);
+    P.fhalf1 = make_fastdiv((uint32_t)(x.P[0] / 2));
+    P.fP2 = make_fastdiv((uint32_t)x.P[1]);
     P.r0 = r0;
     P.nrep = nrep;
     P.stream_id = c.stream_id;
@@ -687,7 +752,7 @@ int infer_rows(XyzLearn &x, cudaStream_t st, int M, const __nv_bfloat16 *Xh, flo
         return xfail(ETHER_ERR_CUDA, "learned proposal: cuTensorMapEncodeTiled failed");
     XCUDA(cudaFuncSetAttribute(xmlp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, XSM_BYTES));
     const int ntiles = (M + 127) / 128;
-    xmlp_kernel<<<std::min(ntiles, x.sm_count), 128, XSM_BYTES, st>>>(map, x.ximg, Z, M, x.err);
+    xmlp_kernel<<<std::min(ntiles, x.sm_count), kXmlpThreads, XSM_BYTES, st>>>(map, x.ximg, Z, M, x.err);
     x.launches++;
     XCUDA(cudaGetLastError());
     return ETHER_OK;

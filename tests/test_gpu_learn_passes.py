@@ -6,6 +6,7 @@ import pytest
 import ether_gb300 as eg
 from oracle import pyoracle as po
 from tests.helpers import beta_of
+from tests import test_gpu_learn_xyz as xyz
 from tests.test_gpu_learn import FM, KTC, random_params, storage_spins
 
 pytestmark = pytest.mark.gpu
@@ -40,3 +41,9 @@ def test_passes_and_remainders_replay(L, R, look):
         np.testing.assert_array_equal(sp, storage_spins(lat, sw, r))
         assert a == int(acc[r])
     lr.close()
+
+
+# the Heisenberg learner's patches: every wrap of every axis, three different extents
+@pytest.mark.parametrize("L", [(16, 24, 8), (24, 8, 16)])
+def test_heisenberg_patches_replay(L):
+    xyz.test_learned_sweep_replays_bit_exact(L)
