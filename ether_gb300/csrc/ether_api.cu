@@ -208,7 +208,7 @@ void free_ctx(Ctx &c) {
                     c.beta_slot_f, c.slot_of_rep, c.rep_of_slot, c.thr, c.stream_id,
                     c.step, c.ovrr_step, c.fresh_call, c.acc_count, c.E, c.M, c.sums,
                     c.partials, c.pt_accepts, c.swap_dev, c.copy_from, c.spiral_ptr,
-                    c.spiral_nbr, c.acc_before, c.acc_ratio, c.spiral_part, c.spiral_sums,
+                    c.spiral_nbr, c.acc_before, c.acc_ratio, c.obs_done, c.spiral_part, c.spiral_sums,
                     c.acc_slot, c.acc_mark, c.t.sia_cls, c.t.sia_ax, c.t.mweight_f, c.t.storage};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -574,7 +574,7 @@ extern "C" int ether_create(const ether_desc *d, ether_ctx **out) {
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         const size_t room = optin > 1024 ? (size_t)optin - 1024 : 0;  // leave the static shared memory
         c.resident = !(c.flags & ETHER_FLAG_NO_RESIDENT) && ising_resident_possible(c, room) &&
-                     (long)c.R * c.N <= (16L << 20) && 2 * c.R >= c.sm_count;
+                     (long)c.R * c.N <= (16L << 20) && (ising_resident_in_registers(c) || 2 * c.R >= c.sm_count);
         if (c.resident) CUDA_TRY(prepare_ising_resident(c));
     }
     TRY(dev_alloc(c, &c.partials, (size_t)c.R * c.partial_blocks * 5));
@@ -582,6 +582,7 @@ extern "C" int ether_create(const ether_desc *d, ether_ctx **out) {
     TRY(dev_alloc(c, &c.swap_dev, 1));
     TRY(dev_alloc(c, &c.acc_before, c.R));
     TRY(dev_alloc(c, &c.acc_ratio, c.R));
+    TRY(dev_alloc(c, &c.obs_done, c.R));
     TRY(dev_alloc(c, &c.acc_slot, c.R));
     TRY(dev_alloc(c, &c.acc_mark, c.R));
     CUDA_TRY(cudaMallocHost((void **)&c.acc_host, sizeof(double) * c.R));
@@ -593,6 +594,7 @@ extern "C" int ether_create(const ether_desc *d, ether_ctx **out) {
     CUDA_TRY(cudaMemset(c.step, 0, sizeof(uint32_t) * c.R));
     CUDA_TRY(cudaMemset(c.ovrr_step, 0, sizeof(uint32_t) * c.R));
     CUDA_TRY(cudaMemset(c.fresh_call, 0, sizeof(uint32_t) * c.R));
+    CUDA_TRY(cudaMemset(c.obs_done, 0, sizeof(uint32_t) * c.R));
     CUDA_TRY(cudaMemset(c.acc_count, 0, sizeof(unsigned long long) * c.R));
     CUDA_TRY(cudaMemset(c.acc_slot, 0, sizeof(unsigned long long) * c.R));
     CUDA_TRY(cudaMemset(c.acc_mark, 0, sizeof(unsigned long long) * c.R));
@@ -1185,6 +1187,18 @@ extern "C" int ether_metropolis(ether_ctx *h, int32_t nsweeps, double *accept) {
     Ctx &c = h->c;
     if (nsweeps < 0) return fail(ETHER_ERR_ARG, "negative sweep count");
     if (!c.beta_set) return fail(ETHER_ERR_STATE, "beta not set (ether_set_beta / ether_set_ladder)");
+    const bool resident = c.resident && c.ising_code == 0;  // a variant that was asked for names a phase kernel
+    if (resident && nsweeps >= 1 && nsweeps <= 256) {
+        // one launch, which writes the acceptance into pinned host memory
+        ResidentEvents ev;
+        ev.ratio = accept ? c.acc_host : nullptr;
+        CUDA_TRY(launch_ising_resident(c, nsweeps, ev));
+        if (accept) {
+            CUDA_TRY(cudaStreamSynchronize(c.stream));
+            std::memcpy(accept, c.acc_host, sizeof(double) * c.R);
+        }
+        return ETHER_OK;
+    }
     if (accept && nsweeps == 1 && !(c.flags & ETHER_FLAG_NO_GRAPHS)) {
         // the reference's per-MCS call (Metropolis, then its acceptance): snapshot, sweep,
         // ratios and the copy to pinned memory captured once per kernel variant and replayed
@@ -1225,9 +1239,11 @@ extern "C" int ether_metropolis(ether_ctx *h, int32_t nsweeps, double *accept) {
         const int rc = ensure_parts(c);
         if (rc) return rc;
     }
-    if (nsweeps > 1 && c.gen_resident) {
-        for (int k = 0; k < nsweeps; k += 256)  // bounded launches
-            CUDA_TRY(launch_general_resident(c, std::min(256, nsweeps - k)));
+    if (resident || (nsweeps > 1 && c.gen_resident)) {
+        for (int k = 0; k < nsweeps; k += 256) {  // bounded launches
+            const int m = std::min(256, nsweeps - k);
+            CUDA_TRY(resident ? launch_ising_resident(c, m) : launch_general_resident(c, m));
+        }
     } else if (nsweeps > 1 && c.n_parts > 1) {  // general lattices: replica parts side by side, same bits
         const int rc = sweeps_in_parts(c, nsweeps);
         if (rc) return rc;
@@ -1267,7 +1283,7 @@ extern "C" int ether_overrelaxation(ether_ctx *h, double ovrr_para) {
 extern "C" int ether_tot_energy(ether_ctx *h, double *E) {
     if (!h) return fail(ETHER_ERR_ARG, "null context");
     Ctx &c = h->c;
-    CUDA_TRY(launch_energy_mag(c, true));
+    CUDA_TRY(launch_energy_mag(c, false));
     if (E) {
         CUDA_TRY(cudaMemcpyAsync(E, c.E, sizeof(double) * c.R, cudaMemcpyDeviceToHost, c.stream));
         CUDA_TRY(cudaStreamSynchronize(c.stream));
@@ -1291,8 +1307,7 @@ extern "C" int ether_observable(ether_ctx *h, int32_t step, int32_t tmcs_eq, int
     if (coa <= 0) return fail(ETHER_ERR_ARG, "coa must be positive");
     Ctx &c = h->c;
     if (step > tmcs_eq && step % coa == 0) {
-        CUDA_TRY(launch_energy_mag(c, true));
-        CUDA_TRY(launch_measure(c));
+        CUDA_TRY(launch_energy_mag(c, true /* measure */));
     }
     return ETHER_OK;
 }
@@ -1369,7 +1384,7 @@ extern "C" int ether_parallel_tempering(ether_ctx *h, int32_t swap_count, int32_
     Ctx &c = h->c;
     if (!c.beta_set) return fail(ETHER_ERR_STATE, "beta not set");
     if (swap_count < 0) return fail(ETHER_ERR_ARG, "negative swap_count");
-    CUDA_TRY(launch_energy_mag(c, true));
+    CUDA_TRY(launch_energy_mag(c, false));
     CUDA_TRY(launch_pt(c, swap_count));
     if (accepted) {
         CUDA_TRY(cudaMemcpyAsync(accepted, c.pt_accepts, sizeof(int32_t), cudaMemcpyDeviceToHost, c.stream));
@@ -1420,12 +1435,11 @@ int mcs_before_sweep(Ctx &c, const ether_schedule *sch, int gates) {
 
 int mcs_after_sweep(Ctx &c, int gates) {
     if (gates & 2) {
-        CUDA_TRY(launch_energy_mag(c, true));
+        CUDA_TRY(launch_energy_mag(c, false));
         CUDA_TRY(launch_pt(c, -1));  // the swap counter lives on the device
     }
     if (gates & 4) {
-        CUDA_TRY(launch_energy_mag(c, true));
-        CUDA_TRY(launch_measure(c));
+        CUDA_TRY(launch_energy_mag(c, true /* measure */));
         if (c.spiral_ptr) CUDA_TRY(launch_spiral_measure(c));  // src/observable.f90:41
     }
     return ETHER_OK;
@@ -1484,6 +1498,20 @@ static int issue_steps(Ctx &c, const ether_schedule *sch, const int8_t *sig, int
         for (int k = 0; k < n; ++k) {
             int rc = issue_step(c, sch, sig[k]);
             if (rc) return rc;
+        }
+        return ETHER_OK;
+    }
+    if (c.resident && !c.spiral_ptr && ising_resident_measures(c)) {
+        // the launch measures too: runs end only where PT lets replicas meet (n <= 256)
+        for (int k = 0, j; k < n; k = j) {
+            ResidentEvents ev;
+            for (j = k; j < n;) {
+                if (sig[j] & 4) ev.measure[(j - k) >> 5] |= 1u << ((j - k) & 31);
+                if (sig[j++] & 2) break;
+            }
+            ev.energy = (sig[j - 1] & 2) ? 1 : 0;
+            CUDA_TRY(launch_ising_resident(c, j - k, ev));
+            if (ev.energy) CUDA_TRY(launch_pt(c, -1));
         }
         return ETHER_OK;
     }

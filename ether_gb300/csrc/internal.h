@@ -126,6 +126,7 @@ struct Ctx {
     bool resident = false;       // ether_mcs runs runs of sweeps with ising_sc_resident
     unsigned long long *acc_before = nullptr;  // R: acceptance counts at the start of a call
     double *acc_ratio = nullptr;               // R: device acceptance ratios of a call
+    uint32_t *obs_done = nullptr;              // R: finished blocks of an energy reduction (zero between launches)
     double *acc_host = nullptr;                // R: pinned host copy
     void *stage = nullptr;                     // pinned staging of ether_{set,get}_spins_batch
     bool ion_direct = false;                   // the device reads / writes the host records in place
@@ -227,8 +228,8 @@ struct ObsTable {
     int M = 0, eblocks = 0, rtotal = 0, ptotal = 0;
 };
 ObsMember obs_member(const Ctx &c);
-// The per-member sequences of launch_energy_mag, launch_pt(c, -1) (true-swap mode) and
-// launch_measure for every member of the table, one launch per kernel on stream st.
+// The per-member sequences of launch_energy_mag and launch_pt(c, -1) (true-swap mode)
+// for every member of the table, one launch per kernel on stream st.
 cudaError_t launch_batch_energy(const ObsTable &t, cudaStream_t st);
 cudaError_t launch_batch_pt(const ObsTable &t, cudaStream_t st);
 cudaError_t launch_batch_measure(const ObsTable &t, cudaStream_t st);
@@ -237,7 +238,17 @@ cudaError_t launch_batch_measure(const ObsTable &t, cudaStream_t st);
 cudaError_t launch_ising_sweep(Ctx &c, int colour);
 bool ising_resident_possible(const Ctx &c, size_t smem_max);
 cudaError_t prepare_ising_resident(const Ctx &c);
-cudaError_t launch_ising_resident(Ctx &c, int nsweeps);
+// What a resident launch does besides its sweeps: the call's acceptance into ratio[R]; a
+// measurement after each sweep whose bit is set; the energies after the last sweep.
+struct ResidentEvents {
+    double *ratio = nullptr;
+    uint32_t measure[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    int energy = 0;
+};
+cudaError_t launch_ising_resident(Ctx &c, int nsweeps, const ResidentEvents &ev = ResidentEvents());
+bool ising_resident_measures(const Ctx &c);  // may the launch measure?
+bool ising_counts(const Ctx &c);             // Ising sums by integer counts
+bool ising_resident_in_registers(const Ctx &c);
 // k_resident.cu
 void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &row_ptr, const std::vector<int32_t> &nbr,
                            const std::vector<uint16_t> &jidx, const std::vector<int32_t> &wstride,
@@ -257,8 +268,7 @@ cudaError_t launch_broadcast(Ctx &c, void *base, size_t bytes_per_replica);
 // replicas r0 .. r0+n-1 from (to_device) or into the ion(0:8, N, n) records at ion, on c.stream
 bool ion_direct_possible(int dev);
 cudaError_t launch_ion_copy(Ctx &c, int r0, int n, double *ion, bool to_device);
-cudaError_t launch_energy_mag(Ctx &c, bool want_energy);
-cudaError_t launch_measure(Ctx &c);
+cudaError_t launch_energy_mag(Ctx &c, bool measure);
 // Row t of the |M| (and E) series; with t_dev the row is read from device memory and
 // advanced afterwards (for captured graphs).
 cudaError_t launch_record(Ctx &c, int t, bool want_e, double *mser, double *eser, int32_t *t_dev = nullptr);

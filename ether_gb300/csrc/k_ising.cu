@@ -1,6 +1,7 @@
 // k_ising.cu -- per-context launches of the Ising colour phase (bodies in sweep_ising.cuh).
 #include <algorithm>
 
+#include "measure.cuh"
 #include "sweep_ising.cuh"
 
 namespace ether {
@@ -186,87 +187,285 @@ static int blocks_for(const Ctx &c, long work, int bs) {
     return (int)need;
 }
 
-// Resident form for small simple-cubic lattices: one block per replica holds both colour
+// Resident forms for small simple-cubic lattices: one block per replica holds both colour
 // arrays in shared memory and runs nsweeps whole sweeps (colour 0, colour 1, counter + 1)
 // between two visits to global memory.  The draws, thresholds and vector update are the
-// phase kernels' (ising_sc_vectors), so every decision is the same; the sweep counter is
-// advanced here instead of by advance_kernel.
-template <int W>
-__global__ void __launch_bounds__(256)
-ising_sc_resident(uint8_t *__restrict__ spins, int L1, int L2, int L3, FastDiv fH, FastDiv fL2,
-                  const uint32_t *__restrict__ thr, int table_entries,
-                  const int32_t *__restrict__ slot_of_rep, const uint32_t *__restrict__ stream_id,
-                  uint32_t *__restrict__ step, uint32_t seed, const RoundKeys K, int nsweeps,
-                  unsigned long long *__restrict__ acc_count) {
+// phase kernels', so every decision is the same; the sweep counter is advanced here instead of
+// by advance_kernel.
+struct ResidentIsing {
+    uint8_t *spins;
+    int L1, L2, L3;
+    FastDiv fH, fL2;
+    const uint32_t *thr;
+    int table_entries;
+    const int32_t *slot_of_rep;
+    const uint32_t *stream_id;
+    uint32_t *step;
+    uint32_t seed;
+    RoundKeys K;
+    int nsweeps;
+    unsigned long long *acc_count;
+    double invN;
+    ResidentEvents ev;
+    // measurements
+    int N, R, nblk, n_slots, zeeman;
+    double juni, mw_abs;
+    const double *zeed;
+    double *E, *M, *sums;
+};
+constexpr int kMeasureBlocks = 32;  // partial sums a measuring launch can keep
+
+__device__ __forceinline__ void resident_load(const ResidentIsing &P, uint8_t *s_sp, uint32_t *s_tab, unsigned *s_acc) {
+    const int r = blockIdx.x, n16 = (P.L1 * P.L2 * P.L3) >> 4;  // W | H and the even extents: whole
+    const uint4 *g = reinterpret_cast<const uint4 *>(P.spins) + (size_t)r * n16;
+    for (int i = threadIdx.x; i < n16; i += blockDim.x) reinterpret_cast<uint4 *>(s_sp)[i] = g[i];
+    fill_sc_table(P.thr + (size_t)P.slot_of_rep[r] * P.table_entries, s_tab, threadIdx.x, blockDim.x);
+    if (threadIdx.x == 0) *s_acc = 0;
+    __syncthreads();
+}
+__device__ __forceinline__ void resident_store(const ResidentIsing &P, const uint8_t *s_sp, unsigned *s_acc,
+                                               unsigned flips, uint32_t t0) {
+    const int r = blockIdx.x, n16 = (P.L1 * P.L2 * P.L3) >> 4;
+    uint4 *g = reinterpret_cast<uint4 *>(P.spins) + (size_t)r * n16;
+    for (int i = threadIdx.x; i < n16; i += blockDim.x) g[i] = reinterpret_cast<const uint4 *>(s_sp)[i];
+    flips = __reduce_add_sync(0xffffffffu, flips);
+    if ((threadIdx.x & 31) == 0) atomicAdd(s_acc, flips);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        P.step[r] = t0 + (uint32_t)P.nsweeps;
+        P.acc_count[r] += *s_acc;
+        if (P.ev.ratio) P.ev.ratio[r] = (double)*s_acc * P.invN;
+    }
+}
+
+// The energy and the magnetisation of the replica from the counts of its energy blocks, in the
+// division and the order of energy_mag_kernel and its finish (whose tree over 128 slots is this
+// one over the first 32: the others hold zeros), by the first warp; measure: into the sums too.
+__device__ __forceinline__ void resident_measure(const ResidentIsing &P, int (*cnt)[2], bool measure) {
+    const int r = blockIdx.x, lane = threadIdx.x;
+    double q[3] = {0.0, 0.0, 0.0};  // total energy, exchange energy, M_z
+    if (lane < P.nblk) {
+        const int t0 = cnt[lane][0], t1 = cnt[lane][1];
+        cnt[lane][0] = cnt[lane][1] = 0;
+        const double e_ex = P.juni * (double)t0;
+        q[0] = P.zeeman ? e_ex + P.zeed[2] * (double)t1 : e_ex;
+        q[1] = e_ex;
+        q[2] = P.mw_abs * (double)t1;
+    }
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) q[j] += __shfl_down_sync(0xffffffffu, q[j], w);
+    if (lane == 0) {
+        P.E[r] = q[0];
+        P.E[P.R + r] = q[1];
+        P.M[3 * r] = P.M[3 * r + 1] = 0.0;
+        P.M[3 * r + 2] = q[2];
+        if (measure) measure_one(P.E, P.M, P.N, P.n_slots, P.slot_of_rep, P.sums, r);
+    }
+}
+
+// NV vectors of each colour per thread, kept in registers; shared memory serves the neighbours.
+// A half-sweep is a chain: barrier, neighbour loads, table, decision, store, barrier.  The
+// addresses are worked out once, the vector opposite is the thread's own of the other colour,
+// and the next half-sweep's random numbers are drawn before the barrier that ends this one.
+// Measurements (counts of colour 0's bonds, as sc_ising_counts) stay in the launch too, so a run
+// ends only where replicas meet.
+// (16^3, 190 replicas, per sweep: 1.8 us with the addresses and draws inside the
+// chain, 0.90 so; by launches per colour 11.4.  One replica: 0.59 and 11.4.)
+template <int W, int NV, bool MEASURE>
+__global__ void __launch_bounds__(1024) ising_sc_resident(const ResidentIsing P) {
     extern __shared__ __align__(16) uint8_t s_sp[];  // colour 0 array, then colour 1
     __shared__ uint32_t s_tab[kScTabWords];
-    const int r = blockIdx.x;
-    const int H = L1 >> 1;
-    const int half = H * L2 * L3;
-    const int nvec = half / W;
-    uint4 *g = reinterpret_cast<uint4 *>(spins + (size_t)r * 2 * half);
-    uint4 *sv = reinterpret_cast<uint4 *>(s_sp);
-    const int n16 = (2 * half) >> 4;  // 2 half is a multiple of 16 (W | H)
-    for (int i = threadIdx.x; i < n16; i += blockDim.x) sv[i] = g[i];
-    fill_sc_table(thr + (size_t)slot_of_rep[r] * table_entries, s_tab, threadIdx.x, blockDim.x);
-    const uint32_t stream = stream_id[r];
-    const uint32_t t0 = step[r];
-    __syncthreads();
+    __shared__ unsigned s_acc;
+    __shared__ int s_cnt[kMeasureBlocks][2];
+    for (int i = threadIdx.x; i < 2 * kMeasureBlocks; i += blockDim.x) (&s_cnt[0][0])[i] = 0;
+    constexpr int G = W == 16 ? 2 : 1;  // random-number groups of a vector
+    const int H = P.L1 >> 1, L2 = P.L2, L3 = P.L3, half = H * L2 * L3, nvec = half / W;
+    const uint32_t stream = P.stream_id[blockIdx.x], t0 = P.step[blockIdx.x];
+    int rho[NV], oa[NV], ob[NV], oc[NV], od[NV], e0[NV], e1[NV];
+    bool odd[NV], live[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int v = threadIdx.x + j * blockDim.x;
+        live[j] = v < nvec;
+        rho[j] = live[j] ? v * W : 0;
+        const int row = (int)fdiv((uint32_t)rho[j], P.fH), xh = rho[j] - row * H;
+        const int z = (int)fdiv((uint32_t)row, P.fL2), y = row - z * L2;
+        odd[j] = (y + z) & 1;
+        oa[j] = (z * L2 + (y == 0 ? L2 - 1 : y - 1)) * H + xh;
+        ob[j] = (z * L2 + (y == L2 - 1 ? 0 : y + 1)) * H + xh;
+        oc[j] = ((z == 0 ? L3 - 1 : z - 1) * L2 + y) * H + xh;
+        od[j] = ((z == L3 - 1 ? 0 : z + 1) * L2 + y) * H + xh;
+        const int before = row * H + (xh == 0 ? H - 1 : xh - 1), after = row * H + (xh + W == H ? 0 : xh + W);
+        e0[j] = odd[j] ? after : before;  // colour 0: parity y + z
+        e1[j] = odd[j] ? before : after;
+    }
+    U4 rnd[NV][G];
+    auto draws = [&](uint32_t t, uint32_t c3) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+#pragma unroll
+            for (int g = 0; g < G; ++g) rnd[j][g] = draw_rk((uint32_t)((rho[j] >> 3) + g), t, stream, c3, P.K);
+    };
+    draws(t0, kMetro);
+    resident_load(P, s_sp, s_tab, &s_acc);
+    Vec<W> me[2][NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        me[0][j] = ldv<W>(s_sp + rho[j]);
+        me[1][j] = ldv<W>(s_sp + half + rho[j]);
+    }
+    const ScTab tab = sc_tab(s_tab);
     unsigned flips = 0;
-    for (int k = 0; k < nsweeps; ++k) {
+    uint32_t cnt = 0;
+    for (int k = 0; k < P.nsweeps; ++k) {
+        const uint32_t t = t0 + (uint32_t)k;
+#pragma unroll
+        for (int colour = 0; colour < 2; ++colour) {
+            uint8_t *own = s_sp + colour * half;
+            const uint8_t *opp = s_sp + (colour ^ 1) * half;
+            const uint32_t c3 = kMetro | ((uint32_t)colour << 8);
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                if (!live[j]) continue;
+                const Vec<W> &o0 = me[colour ^ 1][j];
+                const Vec<W> a = ldv<W>(opp + oa[j]), b = ldv<W>(opp + ob[j]), c = ldv<W>(opp + oc[j]),
+                             d = ldv<W>(opp + od[j]);
+                const uint32_t edge = opp[colour ? e1[j] : e0[j]];
+                const int par = (odd[j] ? 1 : 0) ^ colour;
+                Vec<W> n;
+#pragma unroll
+                for (int q = 0; q < W / 4; ++q)
+                    n.w[q] = o0.w[q] + sc_side<W>(o0, edge, par, q) + a.w[q] + b.w[q] + c.w[q] + d.w[q];
+                me[colour][j] = ising_sc_decide_by<W>(me[colour][j], n, rho[j], tab, t, stream, c3, P.seed,
+                                                      [&](int g) { return rnd[j][g]; }, cnt);
+                stv<W>(own + rho[j], me[colour][j]);
+            }
+            draws(colour ? t + 1u : t, colour ? kMetro : kMetro | (1u << 8));
+            __syncthreads();
+        }
+        // a byte counts at most NV W / 4 <= 8 flips per half-sweep
+        if ((k & 7) == 7 || k + 1 == P.nsweeps) {
+            flips += byte_sum(flip_bytes(cnt));
+            cnt = 0;
+        }
+        const bool measure = (P.ev.measure[(k >> 5) & 7] >> (k & 31)) & 1u;
+        if (MEASURE && (measure || (P.ev.energy && k + 1 == P.nsweeps))) {
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                int sn = 0, ssn = 0, ss = 0, so = 0;
+                if (live[j]) {
+                    const uint8_t *opp = s_sp + half;
+                    const Vec<W> &o0 = me[1][j];
+                    const Vec<W> a = ldv<W>(opp + oa[j]), b = ldv<W>(opp + ob[j]), c = ldv<W>(opp + oc[j]),
+                                 d = ldv<W>(opp + od[j]);
+                    const uint32_t edge = opp[e0[j]];
+#pragma unroll
+                    for (int q = 0; q < W / 4; ++q) {
+                        const uint32_t n = o0.w[q] + sc_side<W>(o0, edge, odd[j] ? 1 : 0, q) + a.w[q] + b.w[q] + c.w[q] + d.w[q];
+                        sn = (int)__dp4a(n, 0x01010101u, (uint32_t)sn);
+                        ssn = (int)__dp4a(n, me[0][j].w[q], (uint32_t)ssn);
+                        ss = (int)__dp4a(me[0][j].w[q], 0x01010101u, (uint32_t)ss);
+                        so = (int)__dp4a(o0.w[q], 0x01010101u, (uint32_t)so);
+                    }
+                }
+                const int same = live[j] ? 6 * W - sn + 2 * ssn - 6 * ss : 3 * W;
+                const int bonds = __reduce_add_sync(0xffffffffu, 2 * (2 * same - 6 * W));
+                const int spins = __reduce_add_sync(0xffffffffu, live[j] ? 2 * (ss + so) - 2 * W : 0);
+                if ((threadIdx.x & 31) == 0) {
+                    const int blk = ((threadIdx.x + j * blockDim.x) >> 8) % P.nblk;
+                    atomicAdd(&s_cnt[blk][0], bonds);
+                    atomicAdd(&s_cnt[blk][1], spins);
+                }
+            }
+            __syncthreads();  // the next counts come two barriers later
+            if (threadIdx.x < 32) resident_measure(P, s_cnt, measure);
+        }
+    }
+    resident_store(P, s_sp, &s_acc, flips, t0);
+}
+
+// More vectors than a block's threads can keep: a loop over them.
+template <int W>
+__global__ void __launch_bounds__(256) ising_sc_resident_loop(const ResidentIsing P) {
+    extern __shared__ __align__(16) uint8_t s_sp[];
+    __shared__ uint32_t s_tab[kScTabWords];
+    __shared__ unsigned s_acc;
+    const int H = P.L1 >> 1, half = H * P.L2 * P.L3, nvec = half / W;
+    const uint32_t stream = P.stream_id[blockIdx.x], t0 = P.step[blockIdx.x];
+    resident_load(P, s_sp, s_tab, &s_acc);
+    unsigned flips = 0;
+    for (int k = 0; k < P.nsweeps; ++k) {
         const uint32_t t = t0 + (uint32_t)k;
         for (int colour = 0; colour < 2; ++colour) {
             const IsingSc A{s_sp + (size_t)colour * half, s_sp + (size_t)(colour ^ 1) * half,
-                            L1, L2, L3, H, fH, fL2, (uint32_t)colour};
+                            P.L1, P.L2, P.L3, H, P.fH, P.fL2, (uint32_t)colour};
             uint32_t cnt = 0;
             for (int v = threadIdx.x; v < nvec; v += blockDim.x)
                 cnt += ising_sc_vectors<W, 1>(A, v, 0, nvec, sc_tab(s_tab), t, stream, kMetro | ((uint32_t)colour << 8),
-                                              seed, K);
+                                              P.seed, P.K);
             flips += byte_sum(cnt);  // each byte <= (W / 4) * ceil(nvec / blockDim) per colour
             __syncthreads();
         }
     }
-    for (int i = threadIdx.x; i < n16; i += blockDim.x) g[i] = sv[i];
-    if (threadIdx.x == 0) step[r] = t0 + (uint32_t)nsweeps;
-    warp_add_count(acc_count + r, flips);
+    resident_store(P, s_sp, &s_acc, flips, t0);
 }
+
+static long resident_vectors(const Ctx &c, int W) { return (long)c.L[0] * c.L[1] * c.L[2] / 2 / W; }
 
 bool ising_resident_possible(const Ctx &c, size_t smem_max) {
     if (!c.fast || c.model != ETHER_MODEL_ISING || c.vec_bytes == 0) return false;
     const size_t bytes = (size_t)c.L[0] * c.L[1] * c.L[2];  // both colours
     // (W/4) ceil(nvec/256) flips per byte of a vector count must stay below 256
-    const size_t nvec = bytes / 2 / (size_t)c.vec_bytes;
-    return bytes <= smem_max && (c.vec_bytes / 4) * ((nvec + 255) / 256) < 256;
+    return bytes <= smem_max && (c.vec_bytes / 4) * ((resident_vectors(c, c.vec_bytes) + 255) / 256) < 256;
+}
+bool ising_resident_in_registers(const Ctx &c) { return resident_vectors(c, c.vec_bytes) <= 2048; }
+
+// Vectors in registers up to two per thread of the largest block.
+using ResidentKernel = void (*)(ResidentIsing);
+template <int W, bool MEASURE>
+static ResidentKernel resident_kernel(long nvec) {
+    return nvec <= 1024 ? ising_sc_resident<W, 1, MEASURE> : nvec <= 2048 ? ising_sc_resident<W, 2, MEASURE> : ising_sc_resident_loop<W>;
+}
+template <bool MEASURE>
+static ResidentKernel resident_kernel(const Ctx &c, int W) {
+    const long n = resident_vectors(c, W);
+    return W == 16 ? resident_kernel<16, MEASURE>(n) : W == 8 ? resident_kernel<8, MEASURE>(n) : resident_kernel<4, MEASURE>(n);
 }
 
-// Opts the resident kernel into the shared memory a replica needs (once, at creation: not
-// during a stream capture).
+// Opts the kernels of every vector width into the shared memory a replica needs (once, at
+// creation: not during a stream capture); never below what another context asked for.
 cudaError_t prepare_ising_resident(const Ctx &c) {
     const int smem = c.L[0] * c.L[1] * c.L[2];
-    return c.vec_bytes == 16  ? cudaFuncSetAttribute(ising_sc_resident<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
-           : c.vec_bytes == 8 ? cudaFuncSetAttribute(ising_sc_resident<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
-                              : cudaFuncSetAttribute(ising_sc_resident<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    for (int k = 0; k < 6; ++k) {
+        const ResidentKernel kern = k & 1 ? resident_kernel<true>(c, 4 << (k >> 1)) : resident_kernel<false>(c, 4 << (k >> 1));
+        cudaFuncAttributes fa;
+        cudaError_t e = cudaFuncGetAttributes(&fa, kern);
+        if (e == cudaSuccess && smem > fa.maxDynamicSharedSizeBytes)
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
-cudaError_t launch_ising_resident(Ctx &c, int nsweeps) {
-    const int smem = c.L[0] * c.L[1] * c.L[2];
-    const int bs = 256;
-    if (c.vec_bytes == 16) {
-        ising_sc_resident<16><<<c.R, bs, smem, c.stream>>>(
-            c.spins, c.L[0], c.L[1], c.L[2], make_fastdiv((uint32_t)(c.L[0] / 2)), make_fastdiv((uint32_t)c.L[1]),
-            c.thr, c.table_entries, c.slot_of_rep, c.stream_id, c.step, c.seed, round_keys(c.seed), nsweeps,
-            c.acc_count);
-    } else if (c.vec_bytes == 8) {
-        ising_sc_resident<8><<<c.R, bs, smem, c.stream>>>(
-            c.spins, c.L[0], c.L[1], c.L[2], make_fastdiv((uint32_t)(c.L[0] / 2)), make_fastdiv((uint32_t)c.L[1]),
-            c.thr, c.table_entries, c.slot_of_rep, c.stream_id, c.step, c.seed, round_keys(c.seed), nsweeps,
-            c.acc_count);
-    } else {
-        ising_sc_resident<4><<<c.R, bs, smem, c.stream>>>(
-            c.spins, c.L[0], c.L[1], c.L[2], make_fastdiv((uint32_t)(c.L[0] / 2)), make_fastdiv((uint32_t)c.L[1]),
-            c.thr, c.table_entries, c.slot_of_rep, c.stream_id, c.step, c.seed, round_keys(c.seed), nsweeps,
-            c.acc_count);
-    }
+bool ising_resident_measures(const Ctx &c) {
+    return ising_resident_in_registers(c) && ising_counts(c) && c.mw_pos && c.partial_blocks <= kMeasureBlocks;
+}
+
+cudaError_t launch_ising_resident(Ctx &c, int nsweeps, const ResidentEvents &ev) {
+    const long nvec = resident_vectors(c, c.vec_bytes);
+    const int nv = nvec <= 1024 ? 1 : 2;
+    const int bs = nvec > 2048 ? 256 : (int)(((nvec + nv - 1) / nv + 31) / 32 * 32);
+    const ResidentIsing P{c.spins, c.L[0], c.L[1], c.L[2], make_fastdiv((uint32_t)(c.L[0] / 2)),
+                          make_fastdiv((uint32_t)c.L[1]), c.thr, c.table_entries, c.slot_of_rep, c.stream_id, c.step,
+                          c.seed, round_keys(c.seed), nsweeps, c.acc_count, 1.0 / (double)c.N, ev,
+                          c.N, c.R, c.partial_blocks, c.n_slots, c.zeeman ? 1 : 0, c.ising_juni, c.mw_abs, c.t.zeed,
+                          c.E, c.M, c.sums};
+    bool measures = ev.energy != 0;
+    for (uint32_t m : ev.measure) measures = measures || m != 0;
+    const ResidentKernel kern = measures ? resident_kernel<true>(c, c.vec_bytes) : resident_kernel<false>(c, c.vec_bytes);
+    kern<<<c.R, bs, c.L[0] * c.L[1] * c.L[2], c.stream>>>(P);
     c.launches++;
     return cudaGetLastError();
 }

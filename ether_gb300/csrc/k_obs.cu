@@ -15,6 +15,7 @@
 // significant bits, summed over the warp and the block the same way and turned into FP64 once
 // per block.
 #include "internal.h"
+#include "measure.cuh"
 #include "rng_math.cuh"
 #include "sweep_ising.cuh"
 #include "sweep_xyz.cuh"
@@ -333,19 +334,17 @@ __device__ __forceinline__ void energy_block(const ObsMember &a, int r, int b) {
     }
 }
 
-__global__ void __launch_bounds__(kRedBs) energy_mag_kernel(const ObsMember a) {
-    energy_block(a, blockIdx.y, blockIdx.x);
-}
-
-// Replica r: sums the partials in index order (a block of 128 threads).
+// Replica r: sums the partials in index order (by the first 128 threads of a block).  __ldcg:
+// another block of the same launch may have written them.
 __device__ __forceinline__ void finish_block(const double *__restrict__ partials, int nblk, int R, int r,
                                              double *__restrict__ E, double *__restrict__ M) {
     __shared__ double sm[kNq][128];
-    for (int j = 0; j < kNq; ++j) {
-        double v = 0.0;
-        for (int b = threadIdx.x; b < nblk; b += blockDim.x) v += partials[((size_t)r * nblk + b) * kNq + j];
-        sm[j][threadIdx.x] = v;
-    }
+    if (threadIdx.x < 128)
+        for (int j = 0; j < kNq; ++j) {
+            double v = 0.0;
+            for (int b = threadIdx.x; b < nblk; b += 128) v += __ldcg(&partials[((size_t)r * nblk + b) * kNq + j]);
+            sm[j][threadIdx.x] = v;
+        }
     __syncthreads();
     for (int w = 64; w > 0; w >>= 1) {
         if ((int)threadIdx.x < w)
@@ -361,35 +360,28 @@ __device__ __forceinline__ void finish_block(const double *__restrict__ partials
     }
 }
 
-// One block per replica.
-__global__ void finish_energy_kernel(const double *__restrict__ partials, int nblk, int R,
-                                     double *__restrict__ E, double *__restrict__ M) {
-    finish_block(partials, nblk, R, blockIdx.x, E, M);
-}
-
-// get_eng('eng') / get_mag('mag') of replica r, into its (group, slot) accumulator.
-__device__ __forceinline__ void measure_one(const double *__restrict__ E, const double *__restrict__ M,
-                                            int N, int n_slots, const int32_t *__restrict__ slot_of_rep,
-                                            double *__restrict__ sums, int r) {
-    const int idx = (r / n_slots) * n_slots + slot_of_rep[r];
-    const double e = E[r] / (2.0 * N);
-    const double mx = M[3 * r], my = M[3 * r + 1], mz = M[3 * r + 2];
-    const double m = sqrt(mx * mx + my * my + mz * mz) / N;
-    double *a = sums + (size_t)idx * 7;
-    a[0] += 1.0;
-    a[1] += e;
-    a[2] += e * e;
-    a[3] += (e * e) * (e * e);
-    a[4] += m;
-    a[5] += m * m;
-    a[6] += (m * m) * (m * m);
-}
-
-__global__ void measure_kernel(const double *__restrict__ E, const double *__restrict__ M, int N,
-                               int R, int n_slots, const int32_t *__restrict__ slot_of_rep,
-                               double *__restrict__ sums) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < R) measure_one(E, M, N, n_slots, slot_of_rep, sums, r);
+// One block per (replica, energy block); the block of a replica that ends last sums the
+// replica's partials and, with `measure`, adds them to the accumulators.  done[r] counts the
+// blocks that have written theirs and is zero again when the launch ends.  (As launches of their
+// own, the sum and the measurement are two gaps of about 2 us after a reduction that itself
+// takes 3 us at 16^3 x 190.)
+__global__ void __launch_bounds__(kRedBs) energy_mag_kernel(const ObsMember a, uint32_t *__restrict__ done, int measure) {
+    const int r = blockIdx.y;
+    energy_block(a, r, blockIdx.x);
+    __shared__ int s_last;
+    if (threadIdx.x < 32) {  // the partials' writers are in the first warp
+        __threadfence();
+        __syncwarp();
+        if (threadIdx.x == 0) s_last = atomicAdd(done + r, 1u) == gridDim.x - 1u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    finish_block(a.partials, a.nblk, a.R, r, a.E, a.M);
+    if (threadIdx.x == 0) {
+        done[r] = 0u;
+        if (measure) measure_one(a.E, a.M, a.N, a.n_slots, a.slot_of_rep, a.sums, r);
+    }
 }
 
 // parallel_tempering: pair tid = (group, pair) of one ladder set.  Exponent in FP64.
@@ -466,6 +458,10 @@ int energy_blocks(const Ctx &c) {
     return (int)(need < 1 ? 1 : need);
 }
 
+bool ising_counts(const Ctx &c) {
+    return c.model == 0 && c.juni_set && c.mw_abs > 0.0 && (!c.zeeman || c.nsp == 1);
+}
+
 ObsMember obs_member(const Ctx &c) {
     ObsMember a{};
     a.spins = c.spins;
@@ -490,7 +486,7 @@ ObsMember obs_member(const Ctx &c) {
     a.juni = c.ising_juni;
     a.mw_abs = c.mw_abs;
     a.nsp = c.nsp;
-    a.count_form = (c.model == 0 && c.juni_set && c.mw_abs > 0.0 && (!c.zeeman || c.nsp == 1)) ? 1 : 0;
+    a.count_form = ising_counts(c) ? 1 : 0;
     a.sc_xyz = (c.fast && c.model == 1) ? 1 : 0;
     a.sc_ising = (c.fast && c.model == 0 && a.count_form) ? 1 : 0;
     a.mw_pos = (c.mw_pos && c.mw_abs > 0.0) ? 1 : 0;
@@ -526,12 +522,10 @@ ObsMember obs_member(const Ctx &c) {
     return a;
 }
 
-cudaError_t launch_energy_mag(Ctx &c, bool) {
-    const int nblk = c.partial_blocks;
-    dim3 grid(nblk, c.R);
-    energy_mag_kernel<<<grid, kRedBs, 0, c.stream>>>(obs_member(c));
-    finish_energy_kernel<<<c.R, 128, 0, c.stream>>>(c.partials, nblk, c.R, c.E, c.M);
-    c.launches += 2;
+cudaError_t launch_energy_mag(Ctx &c, bool measure) {
+    dim3 grid(c.partial_blocks, c.R);
+    energy_mag_kernel<<<grid, kRedBs, 0, c.stream>>>(obs_member(c), c.obs_done, measure ? 1 : 0);
+    c.launches++;
     return cudaGetLastError();
 }
 
@@ -639,7 +633,7 @@ __global__ void record_bump_kernel(int32_t *__restrict__ t_dev) {
 
 cudaError_t launch_record(Ctx &c, int t, bool want_e, double *mser, double *eser, int32_t *t_dev) {
     if (want_e) {
-        cudaError_t e = launch_energy_mag(c, true);
+        cudaError_t e = launch_energy_mag(c, false);
         if (e != cudaSuccess) return e;
         record_kernel<<<(c.R + 127) / 128, 128, 0, c.stream>>>(c.partials, c.partial_blocks, c.R, 0,
                                                                 c.M, c.E, mser, eser, t, t_dev);
@@ -655,13 +649,6 @@ cudaError_t launch_record(Ctx &c, int t, bool want_e, double *mser, double *eser
         record_bump_kernel<<<1, 32, 0, c.stream>>>(t_dev);
         c.launches++;
     }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_measure(Ctx &c) {
-    measure_kernel<<<(c.R + 127) / 128, 128, 0, c.stream>>>(c.E, c.M, c.N, c.R, c.n_slots,
-                                                            c.slot_of_rep, c.sums);
-    c.launches++;
     return cudaGetLastError();
 }
 

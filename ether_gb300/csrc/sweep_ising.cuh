@@ -210,10 +210,11 @@ __device__ __forceinline__ uint32_t sign_bytes(uint32_t a, uint32_t b) {
 // Bound: ALU and FMA-heavy pipes.  Against one site at a time (a threshold load, an extracted
 // half, two compares and a predicated OR per site: 22.7 instructions per update) this takes
 // about half the instructions; 64^3 x 1024 replicas: see ising_sc_kernel.
-template <int W>
-__device__ __forceinline__ Vec<W> ising_sc_decide(const Vec<W> &me, const Vec<W> &n, int rho0, const ScTab &tab,
-                                                  uint32_t t, uint32_t stream, uint32_t c3, uint32_t seed,
-                                                  const RoundKeys &K, uint32_t &cnt) {
+// block(g) is the draw of the vector's group g (first block); ising_sc_decide makes it in place.
+template <int W, class Block>
+__device__ __forceinline__ Vec<W> ising_sc_decide_by(const Vec<W> &me, const Vec<W> &n, int rho0, const ScTab &tab,
+                                                     uint32_t t, uint32_t stream, uint32_t c3, uint32_t seed,
+                                                     const Block &block, uint32_t &cnt) {
     constexpr int NW = W / 4;
     Vec<W> out;
     uint32_t E[NW];
@@ -224,7 +225,7 @@ __device__ __forceinline__ Vec<W> ising_sc_decide(const Vec<W> &me, const Vec<W>
     for (int q = 0; q < NW; ++q) {
         // word q's half of its group's block: q & 1, or for W = 4 the vector's own half
         const int odd = W == 4 ? (rho0 >> 2) & 1 : q & 1;
-        if (W == 4 || (q & 1) == 0) rh = draw_rk((uint32_t)((rho0 >> 3) + (q >> 1)), t, stream, c3, K);
+        if (W == 4 || (q & 1) == 0) rh = block(q >> 1);
         // byte offsets 56 e0 + 4 e1 of the pairs (0, 1) and (2, 3) by one byte dot product each
         E[q] = me.w[q] * 7u + n.w[q];
         const uint32_t t01 = *reinterpret_cast<const uint32_t *>(pair + __dp4a(E[q], 0x00000438u, 0u));
@@ -255,6 +256,14 @@ __device__ __forceinline__ Vec<W> ising_sc_decide(const Vec<W> &me, const Vec<W>
         }
     }
     return out;
+}
+template <int W>
+__device__ __forceinline__ Vec<W> ising_sc_decide(const Vec<W> &me, const Vec<W> &n, int rho0, const ScTab &tab,
+                                                  uint32_t t, uint32_t stream, uint32_t c3, uint32_t seed,
+                                                  const RoundKeys &K, uint32_t &cnt) {
+    return ising_sc_decide_by<W>(
+        me, n, rho0, tab, t, stream, c3, seed,
+        [&](int g) { return draw_rk((uint32_t)((rho0 >> 3) + g), t, stream, c3, K); }, cnt);
 }
 
 // Bytewise flip counts from ising_sc_decide's sum: that sum is 255 times the counts' word
