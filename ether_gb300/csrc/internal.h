@@ -69,7 +69,9 @@ struct DevTables {
     int32_t *ell_ws = nullptr;    // Ising: stride of the threshold-table index
     uint16_t *ell_deg = nullptr;  // N: neighbours of a storage index
     int2 *ell_desc = nullptr;     // per colour: (offset of its ELL block, entries per rank)
+    int4 *ell_class = nullptr;    // per colour: (first storage index, sites, offset, entries per rank)
     uint4 *res_ent = nullptr;     // the lists packed for the resident sweep (k_resident.cu), or null
+    int32_t *res_order = nullptr; // its order of the storage indices
     float4 *J4 = nullptr;         // nJ: (Jxx, Jyy, Jzz, 0) in FP32
     uint8_t *sia_cls = nullptr;   // N: local-axis anisotropy class of a storage index
     float4 *sia_ax = nullptr;     // classes: (a_x, a_y, a_z, D) in FP32
@@ -186,9 +188,12 @@ struct ObsMember {
     const uint8_t *spins;
     const float4 *spins4;
     int N, model, zeeman, sia;
-    const int32_t *row_ptr, *nbr;
+    const int32_t *row_ptr, *nbr;      // CSR: the Ising FP64 form
     const uint16_t *jidx;
-    const float *J;
+    const int4 *ell_class;             // ELL blocks: the others
+    const int32_t *ell_nbr;
+    const uint16_t *ell_j, *ell_deg;
+    const float4 *J4;
     const double *Jd;
     const uint8_t *species;
     const float *zee;
@@ -204,7 +209,7 @@ struct ObsMember {
     FastDiv sc_fH, sc_fL2;
     float sc_jx, sc_jy, sc_jz;
     float mw_abs_f;          // mw_abs in FP32 (exact when mweight_f is set)
-    int sc_pad2, sc_pad3;
+    int n_j, sc_pad3;        // couplings
     double juni, mw_abs;     // Ising counting form: the one bond coupling, the one |weight|
     int count_form, nsp;     // count_form: Ising sums by integer counts (juni, mw_abs, one species)
     double *partials;
@@ -252,7 +257,7 @@ bool ising_resident_in_registers(const Ctx &c);
 // k_resident.cu
 void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &row_ptr, const std::vector<int32_t> &nbr,
                            const std::vector<uint16_t> &jidx, const std::vector<int32_t> &wstride,
-                           std::vector<uint4> &ent);
+                           std::vector<uint4> &ent, std::vector<int32_t> &order);
 cudaError_t prepare_general_resident(const Ctx &c);
 cudaError_t launch_general_resident(Ctx &c, int nsweeps);
 bool ising_staged_shape(const Ctx &c, int vectors_per_step);

@@ -186,14 +186,36 @@ __device__ __forceinline__ void block_sum_mixed(const double (&q)[Q], const DS (
 
 // Partial sums of block b (of a.nblk) of replica r into a.partials[(r * nblk + b) * kNq ..]:
 // the whole block calls it.
+// General XYZ lattices read their neighbours from the coalesced ELL lists and the couplings from
+// shared memory (pyrochlore 12^3 x 64, 18 neighbours: 95 us with the CSR rows and the couplings in
+// global memory, 80 us so; L1 wavefronts of the scattered spins bound it).
+// FORM: Ising, XYZ on the simple-cubic lattice, XYZ on any other (the three differ in registers).
+constexpr int kObsCouplings = 64;  // couplings kept in shared memory
+enum { kObsIsing = 0, kObsCubic = 1, kObsGeneral = 2 };
+__host__ __device__ inline int obs_form(const ObsMember &a) {
+    return a.model == 0 ? kObsIsing : a.sc_xyz ? kObsCubic : kObsGeneral;
+}
+template <int FORM>
 __device__ __forceinline__ void energy_block(const ObsMember &a, int r, int b) {
     const int N = a.N;
     const int stride = a.nblk * blockDim.x;
     double q[kNq] = {0, 0, 0, 0, 0};
     int ci[3] = {0, 0, 0};
     DS qd[kNq];
+    __shared__ float s_j[FORM == kObsGeneral ? kObsCouplings : 1][3];
+    if constexpr (FORM == kObsGeneral) {
+        for (int q = threadIdx.x; q < min(a.n_j, kObsCouplings); q += blockDim.x) {
+            s_j[q][0] = a.J4[q].x;
+            s_j[q][1] = a.J4[q].y;
+            s_j[q][2] = a.J4[q].z;
+        }
+        __syncthreads();
+    }
     int form = kFormDouble;
-    if (a.model == 0 && a.count_form) {
+    int colour = 0;  // general lattices: the class of the thread's site, found as it goes up
+    int4 cls = make_int4(0, 0, 0, 0);
+    if constexpr (FORM != kObsCubic) cls = a.ell_class[0];
+    if (FORM == kObsIsing && a.count_form) {
         // E_ex = J sum s_i s_j, the field term z sum s_i, M = |w| sum sign(w_i) s_i
         const uint8_t *sp = a.spins + (size_t)r * N;
         int cb = 0, cz = 0, cm = 0;
@@ -208,10 +230,16 @@ __device__ __forceinline__ void energy_block(const ObsMember &a, int r, int b) {
         for (int s = b * blockDim.x + threadIdx.x; s < N; s += stride) {
             const uint8_t own = sp[s];
             if (a.sc_ising) {
-                const int colour = s >= half ? 1 : 0;
-                cb += sc_ising_bonds(sp + (size_t)(colour ^ 1) * half, a, H, colour, s - colour * half, own);
+                const int par = s >= half ? 1 : 0;
+                cb += sc_ising_bonds(sp + (size_t)(par ^ 1) * half, a, H, par, s - par * half, own);
             } else {
-                for (int k = a.row_ptr[s]; k < a.row_ptr[s + 1]; ++k) cb += (sp[a.nbr[k]] == own) ? 1 : -1;
+                while (s >= cls.x + cls.y) cls = a.ell_class[++colour];
+                const int32_t *nb = a.ell_nbr + cls.z + (s - cls.x);
+                const int deg = a.ell_deg[s];
+                int same = 0;
+#pragma unroll 6
+                for (int k = 0; k < cls.w; ++k) same += (k < deg && sp[nb[k * cls.y]] == own) ? 1 : 0;
+                cb += 2 * same - deg;
             }
             cz += own ? 1 : -1;
             const bool wneg = a.mw_pos ? false : __double_as_longlong(a.mweight[s]) < 0;
@@ -222,7 +250,7 @@ __device__ __forceinline__ void energy_block(const ObsMember &a, int r, int b) {
         ci[1] = __reduce_add_sync(0xffffffffu, cz);
         ci[2] = __reduce_add_sync(0xffffffffu, cm);
         form = kFormCount;
-    } else if (a.model == 0) {
+    } else if (FORM == kObsIsing) {
         const uint8_t *sp = a.spins + (size_t)r * N;
         for (int s = b * blockDim.x + threadIdx.x; s < N; s += stride) {
             const uint8_t own = sp[s];
@@ -244,27 +272,42 @@ __device__ __forceinline__ void energy_block(const ObsMember &a, int r, int b) {
         for (int s = b * blockDim.x + threadIdx.x; s < N; s += stride) {
             const float4 S = sp[s];
             float hx = 0.f, hy = 0.f, hz = 0.f;
-            if (a.sc_xyz) {
+            if constexpr (FORM == kObsCubic) {
                 // simple cubic: storage index s = colour * half + rank; the six neighbours in
                 // closed form from the other colour's array, summed in the CSR's order
-                const int colour = s >= half ? 1 : 0, rho = s - colour * half;
+                const int par = s >= half ? 1 : 0, rho = s - par * half;
                 const int row = (int)fdiv((uint32_t)rho, a.sc_fH);
                 const int xh = rho - row * H;
                 const int z = (int)fdiv((uint32_t)row, a.sc_fL2), y = row - z * a.sc_L2;
-                const int p = (y + z + colour) & 1;
-                const Acc3 h = sc_field(sp + (size_t)(colour ^ 1) * half + rho, a.sc_L2, a.sc_L3, H, xh, y, z, p,
+                const int p = (y + z + par) & 1;
+                const Acc3 h = sc_field(sp + (size_t)(par ^ 1) * half + rho, a.sc_L2, a.sc_L3, H, xh, y, z, p,
                                         a.sc_jx, a.sc_jy, a.sc_jz);
                 hx = h.x;
                 hy = h.y;
                 hz = h.z;
             } else {
-                for (int k = a.row_ptr[s]; k < a.row_ptr[s + 1]; ++k) {
-                    float4 Sj = sp[a.nbr[k]];
-                    const float *Jp = a.J + 3 * a.jidx[k];
-                    hx = fmaf(Jp[0], Sj.x, hx);
-                    hy = fmaf(Jp[1], Sj.y, hy);
-                    hz = fmaf(Jp[2], Sj.z, hz);
+                while (s >= cls.x + cls.y) cls = a.ell_class[++colour];
+                // ell_field's sum, with the couplings from shared memory where they fit
+                const int32_t *nb = a.ell_nbr + cls.z + (s - cls.x);
+                const uint16_t *ej = a.ell_j + cls.z + (s - cls.x);
+                const int deg = a.ell_deg[s];
+                Acc3 h{0.f, 0.f, 0.f};
+                if (a.n_j <= kObsCouplings) {
+#pragma unroll 6
+                    for (int k = 0; k < cls.w; ++k, nb += cls.y, ej += cls.y) {
+                        const float4 Sj = sp[*nb];
+                        const float *Jq = s_j[*ej];
+                        if (k < deg) fma3(h, Jq[0], Jq[1], Jq[2], Sj);
+                    }
+                } else {
+                    for (int k = 0; k < deg; ++k, nb += cls.y, ej += cls.y) {
+                        const float4 Jv = a.J4[*ej];
+                        fma3(h, Jv.x, Jv.y, Jv.z, sp[*nb]);
+                    }
                 }
+                hx = h.x;
+                hy = h.y;
+                hz = h.z;
             }
             float e = S.x * hx;
             e = fmaf(S.y, hy, e);
@@ -365,9 +408,10 @@ __device__ __forceinline__ void finish_block(const double *__restrict__ partials
 // blocks that have written theirs and is zero again when the launch ends.  (As launches of their
 // own, the sum and the measurement are two gaps of about 2 us after a reduction that itself
 // takes 3 us at 16^3 x 190.)
-__global__ void __launch_bounds__(kRedBs) energy_mag_kernel(const ObsMember a, uint32_t *__restrict__ done, int measure) {
+template <int FORM>
+__global__ void __launch_bounds__(kRedBs, 4) energy_mag_kernel(const ObsMember a, uint32_t *__restrict__ done, int measure) {
     const int r = blockIdx.y;
-    energy_block(a, r, blockIdx.x);
+    energy_block<FORM>(a, r, blockIdx.x);
     __shared__ int s_last;
     if (threadIdx.x < 32) {  // the partials' writers are in the first warp
         __threadfence();
@@ -473,7 +517,12 @@ ObsMember obs_member(const Ctx &c) {
     a.row_ptr = c.t.row_ptr;
     a.nbr = c.t.nbr;
     a.jidx = c.t.jidx;
-    a.J = c.t.J;
+    a.ell_class = c.t.ell_class;
+    a.ell_nbr = c.t.ell_nbr;
+    a.ell_j = c.t.ell_j;
+    a.ell_deg = c.t.ell_deg;
+    a.J4 = c.t.J4;
+    a.n_j = (int)(c.h_Jf.size() / 3);
     a.Jd = c.t.Jd;
     a.species = c.t.species;
     a.zee = c.t.zee;
@@ -490,7 +539,7 @@ ObsMember obs_member(const Ctx &c) {
     a.sc_xyz = (c.fast && c.model == 1) ? 1 : 0;
     a.sc_ising = (c.fast && c.model == 0 && a.count_form) ? 1 : 0;
     a.mw_pos = (c.mw_pos && c.mw_abs > 0.0) ? 1 : 0;
-    a.sc_pad2 = a.sc_pad3 = 0;
+    a.sc_pad3 = 0;
     a.sc_L1 = c.L[0];
     a.sc_L2 = c.L[1];
     a.sc_L3 = c.L[2];
@@ -524,7 +573,11 @@ ObsMember obs_member(const Ctx &c) {
 
 cudaError_t launch_energy_mag(Ctx &c, bool measure) {
     dim3 grid(c.partial_blocks, c.R);
-    energy_mag_kernel<<<grid, kRedBs, 0, c.stream>>>(obs_member(c), c.obs_done, measure ? 1 : 0);
+    const ObsMember a = obs_member(c);
+    const int form = obs_form(a);
+    auto k = form == kObsIsing ? energy_mag_kernel<kObsIsing> : form == kObsCubic ? energy_mag_kernel<kObsCubic>
+                                                                                   : energy_mag_kernel<kObsGeneral>;
+    k<<<grid, kRedBs, 0, c.stream>>>(a, c.obs_done, measure ? 1 : 0);
     c.launches++;
     return cudaGetLastError();
 }
@@ -746,7 +799,10 @@ batch_energy_kernel(const ObsMember *__restrict__ mem, const int32_t *__restrict
     }
     __syncthreads();
     const int local = blockIdx.x - eoff[m];
-    energy_block(a, local / a.nblk, local % a.nblk);
+    const int r = local / a.nblk, b = local % a.nblk, form = obs_form(a);
+    if (form == kObsIsing) energy_block<kObsIsing>(a, r, b);
+    else if (form == kObsCubic) energy_block<kObsCubic>(a, r, b);
+    else energy_block<kObsGeneral>(a, r, b);
 }
 
 // One block of 128 per (member, replica).

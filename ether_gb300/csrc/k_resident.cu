@@ -20,6 +20,12 @@
 // site's real neighbours stays the reference's, so one species is required (the coupling then
 // depends on the shell alone).
 //
+// A warp reads the same slot of 32 sites at once; the 16-byte spins of eight lanes cost one
+// wavefront where they lie side by side.  On a lattice with a basis the sites of a rank range mix
+// the basis, and their neighbours lie scattered; so a block takes and keeps the sites of a colour
+// basis by basis (res_arrange: pyrochlore 12^3, 18 slots, 153 -> 100 wavefronts a warp, a third
+// fewer warps with a neighbour in the other block; a sweep of 64 replicas 80 -> 64 us).
+//
 // A cluster divides every colour class evenly by rank; ranks follow the site numbers, so a
 // block's share is a slab of the lattice and only the slab's faces read the other blocks'
 // shared memory.
@@ -27,6 +33,7 @@
 #include <cmath>
 #include <cstring>
 #include <type_traits>
+#include <utility>
 
 #include "sweep_ising.cuh"
 #include "sweep_xyz.cuh"
@@ -202,7 +209,8 @@ __device__ __forceinline__ Acc3 res_field(const uint4 (&e)[NQ], int slots, const
 template <int OPT, int CS, int NQ>
 __global__ void __launch_bounds__(kResThreads, 1)
 xyz_resident_general(float4 *__restrict__ spins4, int N, const __grid_constant__ ResShape C,
-                     const uint4 *__restrict__ ent, const __grid_constant__ ResCouplings J, XyzParams P,
+                     const uint4 *__restrict__ ent, const int32_t *__restrict__ order,
+                     const __grid_constant__ ResCouplings J, XyzParams P,
                      const float *__restrict__ beta_slot_f, const int32_t *__restrict__ slot_of_rep,
                      const uint32_t *__restrict__ stream_id, uint32_t *__restrict__ step, const RoundKeys K,
                      int nsweeps, unsigned long long *__restrict__ acc_count) {
@@ -229,20 +237,29 @@ xyz_resident_general(float4 *__restrict__ spins4, int N, const __grid_constant__
     for (int col = 0, loc = 1; col < C.ncol; ++col) {
         int a, b;
         share(col, a, b);
-        for (int rho = a + (int)threadIdx.x; rho < b; rho += blockDim.x) s_sp[loc + rho - a] = g[C.off[col] + rho];
+        for (int i = a + (int)threadIdx.x; i < b; i += blockDim.x) s_sp[loc + i - a] = g[order[C.off[col] + i]];
         loc += b - a;
     }
-    uint4 e[NQ];  // the next site's entries and draws
+    // the next site's entries and rank come while this one is decided, and the first of the next
+    // phase, with its draws, before the barrier
+    uint4 e[NQ];
     U4 b0, b1;
-    auto fetch = [&](int col, int rho, uint32_t t) {
+    int rho = 0;
+    auto fetch = [&](int col, int i) {
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) e[q] = ent[(size_t)q * N + C.off[col] + rho];
+        for (int q = 0; q < NQ; ++q) e[q] = ent[(size_t)q * N + C.off[col] + i];
+        rho = order[C.off[col] + i] - C.off[col];
+    };
+    auto draws = [&](int col, uint32_t t) {
         site_draws<OPT>(P, (uint32_t)rho, t, kMetro | ((uint32_t)col << 8), K, stream, b0, b1);
     };
     {
         int a, b;
         share(0, a, b);
-        if (a + (int)threadIdx.x < b) fetch(0, a + (int)threadIdx.x, t0);
+        if (a + (int)threadIdx.x < b) {
+            fetch(0, a + (int)threadIdx.x);
+            draws(0, t0);
+        }
     }
     if constexpr (CS > 1) cluster_barrier();
     else __syncthreads();
@@ -252,8 +269,8 @@ xyz_resident_general(float4 *__restrict__ spins4, int N, const __grid_constant__
         for (int col = 0, loc = 1; col < C.ncol; ++col) {
             int a, b;
             share(col, a, b);
-            for (int rho = a + (int)threadIdx.x; rho < b; rho += blockDim.x) {
-                if (rho != a + (int)threadIdx.x) fetch(col, rho, t);
+            for (int i = a + (int)threadIdx.x; i < b; i += blockDim.x) {
+                if (i != a + (int)threadIdx.x) draws(col, t);
                 bool local = true;
                 if constexpr (CS > 1) {  // own block's number in the block bits of every entry
                     const uint32_t mine2 = (blk << kResIdxBits) | (blk << (16 + kResIdxBits));
@@ -266,10 +283,12 @@ xyz_resident_general(float4 *__restrict__ spins4, int N, const __grid_constant__
                 }
                 const Acc3 h = local ? res_field<CS, NQ, true>(e, C.slots, J, base, first, delta)
                                      : res_field<CS, NQ, false>(e, C.slots, J, base, first, delta);
-                float4 *mine = s_sp + loc + rho - a;
+                const int site = rho;
+                if (i + (int)blockDim.x < b) fetch(col, i + (int)blockDim.x);
+                float4 *mine = s_sp + loc + i - a;
                 const float4 S = *mine;
                 float4 nv;
-                if (metro_decide<OPT>(P, C.off[col] + rho, S, b0, b1, h.x, h.y, h.z, beta_f, (uint32_t)rho, t,
+                if (metro_decide<OPT>(P, C.off[col] + site, S, b0, b1, h.x, h.y, h.z, beta_f, (uint32_t)site, t,
                                       kMetro | ((uint32_t)col << 8), K, stream, nv)) {
                     *mine = nv;
                     ++acc;
@@ -280,7 +299,10 @@ xyz_resident_general(float4 *__restrict__ spins4, int N, const __grid_constant__
             const int nc = col + 1 < C.ncol ? col + 1 : 0;
             if (nc || k + 1 < nsweeps) {
                 share(nc, a, b);
-                if (a + (int)threadIdx.x < b) fetch(nc, a + (int)threadIdx.x, nc ? t : t + 1);
+                if (a + (int)threadIdx.x < b) {
+                    fetch(nc, a + (int)threadIdx.x);
+                    draws(nc, nc ? t : t + 1);
+                }
             }
             if constexpr (CS > 1) cluster_barrier();
             else __syncthreads();
@@ -289,7 +311,7 @@ xyz_resident_general(float4 *__restrict__ spins4, int N, const __grid_constant__
     for (int col = 0, loc = 1; col < C.ncol; ++col) {
         int a, b;
         share(col, a, b);
-        for (int rho = a + (int)threadIdx.x; rho < b; rho += blockDim.x) g[C.off[col] + rho] = s_sp[loc + rho - a];
+        for (int i = a + (int)threadIdx.x; i < b; i += blockDim.x) g[order[C.off[col] + i]] = s_sp[loc + i - a];
         loc += b - a;
     }
     if (blk == 0 && threadIdx.x == 0) step[r] = t0 + (uint32_t)nsweeps;
@@ -346,12 +368,48 @@ static const void *res_kernel(const Ctx &c, int cs) {
                                 : pick(std::integral_constant<int, kXyzGeneral>{});
 }
 
+// Orders every block's share of every colour by (site number modulo period, site number) into
+// `order` (entry col_off + i: the storage index in place i) and returns the shared-memory wavefronts
+// of a sample of its neighbour loads: eight lanes read 16-byte spins from eight banks' width.
+static long res_arrange(const Ctx &c, int cs, int period, const std::vector<int32_t> &row_ptr,
+                        const std::vector<int32_t> &nbr, std::vector<int32_t> &order, std::vector<int32_t> &pos) {
+    std::vector<int> used(cs, 1), start(period);
+    for (int col = 0; col < c.ncol; ++col)
+        for (int k = 0; k < cs; ++k) {
+            int a, b;
+            res_range(c, cs, col, k, a, b);
+            int32_t *o = order.data() + c.col_off[col];
+            // ranks follow the site numbers: one bucket per remainder
+            std::fill(start.begin(), start.end(), 0);
+            for (int i = a; i < b; ++i) ++start[c.site_of_storage[c.col_off[col] + i] % period];
+            for (int m = 0, n = a; m < period; ++m) n += std::exchange(start[m], n);
+            for (int i = a; i < b; ++i) o[start[c.site_of_storage[c.col_off[col] + i] % period]++] = c.col_off[col] + i;
+            for (int i = a; i < b; ++i) pos[o[i]] = used[k] + i - a;
+            used[k] += b - a;
+        }
+    const int step = 8 * std::max(1, c.N / 4096);  // about 512 groups of eight lanes
+    long cost = 0;
+    for (int i = 0; i + 8 <= c.N; i += step)
+        for (int m = 0; m < c.res_slots; ++m) {
+            int hits[8] = {0, 0, 0, 0, 0, 0, 0, 0}, most = 0, p[8];
+            for (int j = 0; j < 8; ++j) {
+                const int s = order[i + j];
+                p[j] = row_ptr[s] + m < row_ptr[s + 1] ? pos[nbr[row_ptr[s] + m]] : 0;
+                bool seen = false;
+                for (int q = 0; q < j; ++q) seen = seen || p[q] == p[j];
+                if (!seen) most = std::max(most, ++hits[p[j] & 7]);
+            }
+            cost += most;
+        }
+    return cost;
+}
+
 // Sets up a context's resident sweep from its neighbour lists (CSR in storage order; shell of an
 // entry = its coupling index, one species): cluster size, slots and packed entries.  smem_max:
 // the opt-in shared memory of a block.  Leaves c.gen_resident 0 where it does not apply.
 void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &row_ptr, const std::vector<int32_t> &nbr,
                            const std::vector<uint16_t> &jidx, const std::vector<int32_t> &wstride,
-                           std::vector<uint4> &ent) {
+                           std::vector<uint4> &ent, std::vector<int32_t> &order) {
     c.gen_resident = 0;
     const bool ising = c.model == ETHER_MODEL_ISING;
     if (c.fast || c.nsp != 1 || c.nsh < 1 || c.nsh > (ising ? 4 : 8)) return;
@@ -407,6 +465,22 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
         if (here > there) cs = 0;
     }
     if (!cs) return;
+    // the order in which a block takes a colour's sites and keeps them: sites that are equal modulo
+    // a period (a basis of the unit cell) side by side, with the period whose sampled loads have the
+    // fewest bank conflicts (none: sites in rank order)
+    order.resize(c.N);
+    for (int s = 0; s < c.N; ++s) order[s] = s;
+    if (!ising) {
+        long best = -1;
+        std::vector<int32_t> trial(c.N), pos(c.N);
+        for (int period : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32}) {
+            const long cost = res_arrange(c, cs, period, row_ptr, nbr, trial, pos);
+            if (best < 0 || cost < best) {
+                best = cost;
+                order = trial;
+            }
+        }
+    }
     // where a storage index lives: XYZ, 1 + its place in the owning block's array | block << 14
     std::vector<uint16_t> where(c.N);
     std::vector<int> used(cs, ising ? 0 : 1);
@@ -414,8 +488,8 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
         for (int k = 0; k < cs; ++k) {
             int a, b;
             res_range(c, cs, col, k, a, b);
-            for (int rho = a; rho < b; ++rho)
-                where[c.col_off[col] + rho] = (uint16_t)((used[k] + rho - a) | (cs > 1 ? k << kResIdxBits : 0));
+            for (int i = a; i < b; ++i)
+                where[order[c.col_off[col] + i]] = (uint16_t)((used[k] + i - a) | (cs > 1 ? k << kResIdxBits : 0));
             used[k] += b - a;
         }
     std::vector<uint16_t> e16((size_t)c.res_q * c.N * 8, ising ? (uint16_t)c.N : (uint16_t)0);
@@ -423,18 +497,18 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
         for (int blk = 0; blk < cs; ++blk) {
             int a, b;
             res_range(c, cs, col, blk, a, b);
-            for (int rho = a; rho < b; ++rho) {
-                const int s = c.col_off[col] + rho;
+            for (int i = a; i < b; ++i) {
+                const int s = order[c.col_off[col] + i], e = c.col_off[col] + i;
                 // the zero spin of the block that updates the site
                 const uint16_t zero = ising ? (uint16_t)c.N : (uint16_t)(cs > 1 ? blk << kResIdxBits : 0);
-                for (int m = 0; m < 8 * c.res_q; ++m) e16[((size_t)(m >> 3) * c.N + s) * 8 + (m & 7)] = zero;
+                for (int m = 0; m < 8 * c.res_q; ++m) e16[((size_t)(m >> 3) * c.N + e) * 8 + (m & 7)] = zero;
                 int sh = -1, m = 0;
                 for (int k = row_ptr[s]; k < row_ptr[s + 1]; ++k) {
                     if (jidx[k] != sh) {
                         sh = jidx[k];
                         m = sh ? c.res_shell_end[sh - 1] : 0;
                     }
-                    e16[((size_t)(m >> 3) * c.N + s) * 8 + (m & 7)] = where[nbr[k]];
+                    e16[((size_t)(m >> 3) * c.N + e) * 8 + (m & 7)] = where[nbr[k]];
                     ++m;
                 }
             }
@@ -498,7 +572,7 @@ cudaError_t launch_general_resident(Ctx &c, int nsweeps) {
         J.y[m] = c.h_Jf[3 * sh + 1];
         J.z[m] = c.h_Jf[3 * sh + 2];
     }
-    void *args[] = {&c.spins4, &c.N, &C, &c.t.res_ent, &J, &P, &c.beta_slot_f, &c.slot_of_rep, &c.stream_id,
+    void *args[] = {&c.spins4, &c.N, &C, &c.t.res_ent, &c.t.res_order, &J, &P, &c.beta_slot_f, &c.slot_of_rep, &c.stream_id,
                     &c.step, &K, &nsweeps, &c.acc_count};
     return cudaLaunchKernelExC(&cfg, res_kernel(c, cs), args);
 }
