@@ -30,15 +30,20 @@ xyz_ell_kernel(float4 *__restrict__ spins4, int N, int col_off, int n_c, uint32_
     warp_add_count_x(acc_count + r, acc);
 }
 
-// Simple cubic, a thread per column and chunk of ZC planes (xyz_sc_column).  64 registers, four
-// blocks per SM.  Bound: issue (65%) and the latency of the neighbour loads between ALU and
-// FMA-heavy phases (53% each); 285 instructions per update, 400 when every site looked up its
-// six neighbours and its indices itself.  Updates/ns at T_c, before and now: 64^3 x 64 66 and
-// 83.8 (0.60 of the measured copy rate at 48 bytes per update), 32^3 x 290 58 and 74.8.
-// Measured and not kept: three blocks per SM without the register cap (81.2), five with spills
-// (54), the neighbour offsets' cases in a branch before the loads (75.9; 60.3 on 32^3).
-template <int OPT>
-__global__ void __launch_bounds__(256, 4)
+// Simple cubic, a thread per column and chunk of ZC planes.  POOL > 0: Marsaglia proposals whose
+// second blocks a warp draws together (xyz_sc_columns); 0: each site's draws in place (angle
+// proposals, which need one block only, single planes, and arrays of 4 GB and more).  Bound: issue
+// (65%; IMAD.WIDE occupies the dispatch port longer) and the neighbour loads behind it: 275
+// instructions per update, 1.3 Philox blocks among them (292 and 2.3 in place; 400 when every site
+// looked up its six neighbours and its indices itself).  Updates/ns at T_c, every site on its own,
+// by columns, and pooled: 64^3 x 64 66, 83.8 and 92.7 (0.66 of the measured copy rate at 48 bytes
+// per update), 32^3 x 290 58, 74.8 and 82.9.
+// Measured and not kept: 256 threads (four blocks: 87.1 and 77.5); nine and ten blocks (90.7 and
+// 87.0: less L1 for the neighbours); 8 planes a pool in 24 KB a block (81.9); the next site's
+// loads one site ahead, in registers (83.6) or as prefetches (91.2).
+constexpr int kColThreads = 128, kColBlocks = 8;
+template <int OPT, bool NEAR, int POOL>
+__global__ void __launch_bounds__(kColThreads, kColBlocks)
 xyz_col_kernel(float4 *__restrict__ spins4, int L1, int L2, int L3, FastDiv fH, FastDiv fP, int ZC, int items,
                uint32_t colour, float jx, float jy, float jz, XyzParams P, const float *__restrict__ beta_slot_f,
                const int32_t *__restrict__ slot_of_rep, const uint32_t *__restrict__ stream_id,
@@ -52,8 +57,14 @@ xyz_col_kernel(float4 *__restrict__ spins4, int L1, int L2, int L3, FastDiv fH, 
     const float beta_f = beta_slot_f[slot_of_rep[r]];
     const uint32_t k1 = stream_id[r], t = step[r];
     unsigned acc = 0;
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i < items) {
+    const int i = blockIdx.x * kColThreads + threadIdx.x;
+    if constexpr (POOL > 0) {
+        __shared__ ScPool<POOL> pool[kColThreads / 32];
+        const int u = min(i, items - 1), chunk = (int)fdiv((uint32_t)u, fP), col = u - chunk * (int)fP.d;
+        const int nz = i < items ? min(ZC, L3 - chunk * ZC) : 0;
+        acc = xyz_sc_columns<OPT, NEAR, POOL>(A, P, col, chunk * ZC, nz, ZC, beta_f, t, kMetro | (colour << 8), K, k1,
+                                        pool[threadIdx.x >> 5]);
+    } else if (i < items) {
         const int chunk = (int)fdiv((uint32_t)i, fP), col = i - chunk * (int)fP.d;
         acc = xyz_sc_column<OPT>(A, P, col, chunk * ZC, min(chunk * ZC + ZC, L3), beta_f, t, kMetro | (colour << 8), K,
                                  k1);
@@ -214,9 +225,9 @@ XyzParams xyz_params(const Ctx &c) {
     return P;
 }
 
-// Planes per thread: the most of 8, 4, 2 that still gives six blocks per SM (64^3 x 64: 83.8
-// updates/ns with 8, 80.5 with 4, 73.3 with 2; 48^3 x 32, where 8 leaves 864 blocks: 65.5 and
-// 66.9; 16^3 x 512, where it leaves 512: 51.5 and 56.7).  Variants 12 and 13 halve and double it.
+// Planes per thread: the most of 8, 4, 2 that still gives six blocks of 256 per SM (64^3 x 64: 92.7
+// updates/ns with 8, 90.0 with 4, 91.1 with 16; 48^3 x 32, where 8 leaves 864 blocks: 68.3, 71.8
+// with 4, 61.6 with 2; 16^3 x 512: 56.7 with 2, 52.1 with 1).  Variants 12 and 13 halve and double it.
 static int xyz_planes(const Ctx &c) {
     const long plane = (long)(c.L[0] / 2) * c.L[1];
     int zc = 1;
@@ -231,11 +242,14 @@ template <int OPT>
 static void launch_xyz_col(Ctx &c, int colour, const XyzParams &P, const RoundKeys &K) {
     const int half = c.N / 2, plane = c.L[0] / 2 * c.L[1], ZC = xyz_planes(c);
     const int items = plane * ((c.L[2] + ZC - 1) / ZC);
-    dim3 grid((items + 255) / 256, c.R);
+    dim3 grid((items + kColThreads - 1) / kColThreads, c.R);
     XyzParams Pc = P;  // the kernel indexes sites by rank in the colour array
     if (Pc.sia_cls) Pc.sia_cls += (size_t)colour * half;
     // single shell, single species: J(1,1,1,:)
-    xyz_col_kernel<OPT><<<grid, 256, 0, c.stream>>>(
+    auto k = xyz_col_kernel<OPT, false, 0>;  // rejected pairs in place
+    if (!P.angle && half < (1 << 28))
+        k = ZC >= 4 ? xyz_col_kernel<OPT, true, 4> : ZC >= 2 ? xyz_col_kernel<OPT, true, 2> : k;
+    k<<<grid, kColThreads, 0, c.stream>>>(
         c.spins4, c.L[0], c.L[1], c.L[2], make_fastdiv((uint32_t)(c.L[0] / 2)), make_fastdiv((uint32_t)plane), ZC, items,
         (uint32_t)colour, c.h_Jf[0], c.h_Jf[1], c.h_Jf[2], Pc, c.beta_slot_f, c.slot_of_rep, c.stream_id, c.step, K,
         c.acc_count);

@@ -219,6 +219,22 @@ constexpr int kMarsagliaMaxPairs = 64;
 // rejected (probability ~1e-43): no proposal.
 struct Spin4 { float x, y, z, w; };
 
+// Pairs 3 and later, from block 2 on.
+ETHER_HD bool marsaglia_tail(uint32_t c0, uint32_t t, uint32_t stream, uint32_t tag, const RoundKeys &K,
+                             float *v1, float *v2, float *s) {
+    bool ok = false;
+    for (int blk = 2; blk <= kMarsagliaMaxPairs / 2 && !ok; ++blk) {
+        const U4 o = draw_rk(c0, t, stream, tag | ((uint32_t)blk << 16), K);
+        float w1 = upm1(o.x), w2 = upm1(o.y), q = w1 * w1 + w2 * w2;
+        if (q < 1.0f) {
+            *v1 = w1; *v2 = w2; *s = q; ok = true;
+        } else if (2 * blk != kMarsagliaMaxPairs) {
+            w1 = upm1(o.z); w2 = upm1(o.w); q = w1 * w1 + w2 * w2;
+            if (q < 1.0f) { *v1 = w1; *v2 = w2; *s = q; ok = true; }
+        }
+    }
+    return ok;
+}
 ETHER_HD bool marsaglia(uint32_t c0, uint32_t t, uint32_t stream, uint32_t tag, const RoundKeys &K,
                         const U4 &b0, const U4 &b1, float *v1o, float *v2o, float *so) {
     const float a0 = upm1(b0.y), a1 = upm1(b0.z);
@@ -230,20 +246,14 @@ ETHER_HD bool marsaglia(uint32_t c0, uint32_t t, uint32_t stream, uint32_t tag, 
     float v2 = k0 ? a1 : (k1 ? c1a : d1);
     float s = k0 ? s0 : (k1 ? s1 : s2);
     bool ok = k0 || k1 || k2;
-    if (!ok) {
-        for (int blk = 2; blk <= kMarsagliaMaxPairs / 2 && !ok; ++blk) {
-            const U4 o = draw_rk(c0, t, stream, tag | ((uint32_t)blk << 16), K);
-            float w1 = upm1(o.x), w2 = upm1(o.y), q = w1 * w1 + w2 * w2;
-            if (q < 1.0f) {
-                v1 = w1; v2 = w2; s = q; ok = true;
-            } else if (2 * blk != kMarsagliaMaxPairs) {
-                w1 = upm1(o.z); w2 = upm1(o.w); q = w1 * w1 + w2 * w2;
-                if (q < 1.0f) { v1 = w1; v2 = w2; s = q; ok = true; }
-            }
-        }
-    }
+    if (!ok) ok = marsaglia_tail(c0, t, stream, tag, K, &v1, &v2, &s);
     *v1o = v1; *v2o = v2; *so = s;
     return ok;
+}
+// The spin of an accepted pair.
+ETHER_HD Spin4 marsaglia_spin(float v1, float v2, float s) {
+    const float tq = sqrtf(1.0f - s);
+    return Spin4{(2.0f * v1) * tq, (2.0f * v2) * tq, 1.0f - 2.0f * s, 0.0f};
 }
 
 // b0, b1: blocks 0 and 1 of the site's draw (block 1 is used by Marsaglia only).
@@ -254,11 +264,8 @@ ETHER_HD bool propose(bool angle, float dphi, const Spin4 &S, uint32_t c0, uint3
     if (!angle) {
         float v1, v2, s;
         if (!marsaglia(c0, t, stream, tag, K, b0, b1, &v1, &v2, &s)) return false;
-        float tq = sqrtf(1.0f - s);
-        nx = (2.0f * v1) * tq;
-        ny = (2.0f * v2) * tq;
-        nz = 1.0f - 2.0f * s;
-        nphi = 0.0f;
+        *out = marsaglia_spin(v1, v2, s);
+        return true;
     } else {
         nz = upm1(b0.y);
         nphi = S.w + dphi * upm1(b0.z);

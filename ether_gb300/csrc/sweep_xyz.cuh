@@ -76,6 +76,17 @@ __device__ __forceinline__ float delta_e(const XyzParams &P, int s, const float4
     return e;
 }
 
+// Is the proposal n for a site in state S accepted?
+template <int OPT>
+__device__ __forceinline__ bool metro_accept(const XyzParams &P, int s, const float4 &S, const Spin4 &n, float eta,
+                                             float hx, float hy, float hz, float beta_f, float4 &out) {
+    const float e = delta_e<OPT>(P, s, S, n, hx, hy, hz);
+    // exp evaluated on every lane (no divergent short-circuit); e <= 0 accepts regardless
+    const float p = expf_neg(-(beta_f * fmaxf(e, 0.0f)));
+    out = make_float4(n.x, n.y, n.z, n.w);
+    return (e <= 0.0f) || (eta < p);
+}
+
 // The Metropolis decision of one site from its state S, the exchange field h and blocks 0
 // and 1 of its draw (block 1 only for Marsaglia proposals): returns whether the proposal is
 // accepted and, if so, the new state in out.
@@ -89,11 +100,7 @@ __device__ __forceinline__ bool metro_decide(const XyzParams &P, int s, const fl
     Spin4 n;
     const Spin4 So{S.x, S.y, S.z, S.w};
     if (!propose(angle, P.dphi, So, rho, t, stream, c3, K, b0, b1, &n)) return false;
-    const float e = delta_e<OPT>(P, s, S, n, hx, hy, hz);
-    // exp evaluated on every lane (no divergent short-circuit); e <= 0 accepts regardless
-    const float p = expf_neg(-(beta_f * fmaxf(e, 0.0f)));
-    out = make_float4(n.x, n.y, n.z, n.w);
-    return (e <= 0.0f) || (eta < p);
+    return metro_accept<OPT>(P, s, S, n, eta, hx, hy, hz, beta_f, out);
 }
 
 template <int OPT>
@@ -249,35 +256,43 @@ struct XyzSc {
     uint32_t colour;
     float jx, jy, jz;
 };
-// The sites (col, z), z0 <= z < z1, of one column (col = y H + xh) up the z axis.  Of a site's
-// neighbours two are known from the site below it -- its z - 1 neighbour was that site's x
+// One column (col = y H + xh) of a simple-cubic replica, its sites taken up the z axis.  Of a
+// site's neighbours two are known from the site below it -- its z - 1 neighbour was that site's x
 // neighbour at offset 0, and its own one at offset 0 was that site's z + 1 neighbour -- and
 // the column fixes all indices but z: four neighbour loads a site instead of six, and a fifth
-// fewer instructions.  The random numbers are drawn while the loads are in flight.
-template <int OPT>
-__device__ __forceinline__ unsigned xyz_sc_column(const XyzSc &A, const XyzParams &P, int col, int z0, int z1,
-                                                  float beta_f, uint32_t t, uint32_t c3, const RoundKeys &K,
-                                                  uint32_t stream) {
-    const int H = A.H, L2 = A.L2, L3 = A.L3, plane = L2 * H;
-    const int y = (int)fdiv((uint32_t)col, A.fH), xh = col - y * H;
-    const int d0 = xh == 0 ? H - 1 : -1, d1 = xh == H - 1 ? 1 - H : 1;
-    const bool y0 = y == 0, y1 = y == L2 - 1;
-    const int dym = y0 ? plane - H : -H, dyp = y1 ? H - plane : H;
-    int rho = z0 * plane + col;
-    int p = (y + z0 + (int)A.colour) & 1;
-    const float4 *o = A.opp + rho;
-    float4 *w = A.own + rho;
-    float4 zm = o[z0 == 0 ? (L3 - 1) * plane : -plane], x0 = o[0];
-    unsigned acc = 0;
-#pragma unroll 1
-    for (int z = z0; z < z1; ++z) {
-        const int d = p ? d1 : d0;
-        const float4 ym = o[dym], yp = o[dyp], xd = o[d], zp = o[z == L3 - 1 ? plane - L3 * plane : plane];
-        const float4 S = *w;
-        U4 b0, b1;
-        site_draws<OPT>(P, (uint32_t)rho, t, c3, K, stream, b0, b1);
-        // increasing site number; at a face the wrapped neighbour changes side
+// fewer instructions.  NEAR: arrays below 4 GB, byte offsets of 32 bits beside their addresses.
+template <bool NEAR>
+struct ScColumn {
+    const XyzSc &A;
+    const int H, L2, L3, plane, y, xh, d0, d1, dym, dyp;
+    const bool y0, y1;
+    int z, rho, p;
+    float4 zm, x0;            // carried up
+    float4 ym, yp, xd, zp, S;  // loaded for the present site
+
+    __device__ __forceinline__ const float4 *at(const float4 *base, int i) const {
+        if constexpr (NEAR) return reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(base) + (uint32_t)i * 16u);
+        else return base + i;
+    }
+    __device__ __forceinline__ ScColumn(const XyzSc &A_, int col, int z0)
+        : A(A_), H(A_.H), L2(A_.L2), L3(A_.L3), plane(A_.L2 * A_.H), y((int)fdiv((uint32_t)col, A_.fH)),
+          xh(col - y * A_.H), d0(xh == 0 ? H - 1 : -1), d1(xh == H - 1 ? 1 - H : 1),
+          dym(y == 0 ? plane - H : -H), dyp(y == L2 - 1 ? H - plane : H), y0(y == 0), y1(y == L2 - 1), z(z0),
+          rho(z0 * plane + col), p((y + z0 + (int)A_.colour) & 1) {
+        zm = *at(A.opp, rho + (z0 == 0 ? (L3 - 1) * plane : -plane));
+        x0 = *at(A.opp, rho);
+    }
+    __device__ __forceinline__ void load() {
+        ym = *at(A.opp, rho + dym);
+        yp = *at(A.opp, rho + dyp);
+        xd = *at(A.opp, rho + (p ? d1 : d0));
+        zp = *at(A.opp, rho + (z == L3 - 1 ? plane - L3 * plane : plane));
+        S = *at(A.own, rho);
+    }
+    // increasing site number; at a face the wrapped neighbour changes side
+    __device__ __forceinline__ Acc3 field() const {
         Acc3 h{0.f, 0.f, 0.f};
+        const int d = p ? d1 : d0;
         const float4 xa = d < 0 ? xd : x0, xb = d < 0 ? x0 : xd;
         if (!y0 && !y1 && z != 0 && z != L3 - 1) {
             fma3(h, A.jx, A.jy, A.jz, zm);
@@ -298,17 +313,102 @@ __device__ __forceinline__ unsigned xyz_sc_column(const XyzSc &A, const XyzParam
             if (z != L3 - 1) fma3(h, A.jx, A.jy, A.jz, zp);
             if (z == 0) fma3(h, A.jx, A.jy, A.jz, zm);
         }
-        float4 nv;
-        if (metro_decide<OPT>(P, rho, S, b0, b1, h.x, h.y, h.z, beta_f, (uint32_t)rho, t, c3, K, stream, nv)) {
-            *w = nv;
-            ++acc;
-        }
+        return h;
+    }
+    __device__ __forceinline__ float4 *site() const { return const_cast<float4 *>(at(A.own, rho)); }
+    __device__ __forceinline__ void up() {
         zm = x0;
         x0 = zp;
-        o += plane;
-        w += plane;
         rho += plane;
+        ++z;
         p ^= 1;
+    }
+};
+
+// The sites z0 <= z < z1 of a column, each with its own draws, made while its loads are in flight.
+template <int OPT>
+__device__ __forceinline__ unsigned xyz_sc_column(const XyzSc &A, const XyzParams &P, int col, int z0, int z1,
+                                                  float beta_f, uint32_t t, uint32_t c3, const RoundKeys &K,
+                                                  uint32_t stream) {
+    ScColumn<false> C(A, col, z0);
+    unsigned acc = 0;
+#pragma unroll 1
+    while (C.z < z1) {
+        C.load();
+        U4 b0, b1;
+        site_draws<OPT>(P, (uint32_t)C.rho, t, c3, K, stream, b0, b1);
+        const Acc3 h = C.field();
+        float4 nv;
+        if (metro_decide<OPT>(P, C.rho, C.S, b0, b1, h.x, h.y, h.z, beta_f, (uint32_t)C.rho, t, c3, K, stream, nv)) {
+            *C.site() = nv;
+            ++acc;
+        }
+        C.up();
+    }
+    return acc;
+}
+
+// The same for a warp's 32 columns of one replica, nz <= planes sites each (lanes without work:
+// nz = 0), Marsaglia proposals only.  21% of the sites need pairs beyond their first block, so
+// almost every warp would draw a second block for all its sites; here the sites of POOL planes
+// that need one are queued and drawn for 32 at a time (1.3 blocks a site instead of 2.3).
+template <int POOL>
+struct ScPool {                     // of a warp, in shared memory
+    float4 prop[POOL][32];          // v1 (of a rejected pair: the rank), v2, s, eta
+    uint8_t queue[POOL * 32];       // places in prop
+};
+template <int OPT, bool NEAR, int POOL>
+__device__ __forceinline__ unsigned xyz_sc_columns(const XyzSc &A, const XyzParams &P, int col, int z0, int nz, int planes,
+                                                   float beta_f, uint32_t t, uint32_t c3, const RoundKeys &K,
+                                                   uint32_t stream, ScPool<POOL> &pool) {
+    const int lane = threadIdx.x & 31;
+    ScColumn<NEAR> C(A, col, z0);
+    unsigned acc = 0;
+#pragma unroll 1
+    for (int zb = 0; zb < planes; zb += POOL) {
+        int queued = 0;
+#pragma unroll 1
+        for (int j = 0; j < POOL; ++j) {
+            const uint32_t rho = (uint32_t)(C.rho + j * C.plane);
+            const U4 b = draw_rk(rho, t, stream, c3, K);
+            const float v1 = upm1(b.y), v2 = upm1(b.z), s = v1 * v1 + v2 * v2;
+            const bool more = !(s < 1.0f) && zb + j < nz;
+            pool.prop[j][lane] = make_float4(more ? __uint_as_float(rho) : v1, v2, s, u01(b.x));
+            const uint32_t m = __ballot_sync(0xffffffffu, more);
+            if (more) pool.queue[queued + __popc(m & ((1u << lane) - 1u))] = (uint8_t)(j * 32 + lane);
+            queued += __popc(m);
+        }
+        __syncwarp();
+        for (int q = lane; q < queued; q += 32) {
+            float4 *const w = &pool.prop[0][0] + pool.queue[q];
+            const uint32_t rho = __float_as_uint(w->x);
+            const U4 b = draw_rk(rho, t, stream, c3 | (1u << 16), K);
+            float v1 = upm1(b.x), v2 = upm1(b.y), s = v1 * v1 + v2 * v2;
+            if (!(s < 1.0f)) {
+                v1 = upm1(b.z);
+                v2 = upm1(b.w);
+                s = v1 * v1 + v2 * v2;
+                // with no pair accepted this one stays, and there is no proposal
+                if (!(s < 1.0f)) marsaglia_tail(rho, t, stream, c3, K, &v1, &v2, &s);
+            }
+            w->x = v1;
+            w->y = v2;
+            w->z = s;
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int j = 0; j < POOL && zb + j < nz; ++j) {
+            C.load();
+            const float4 v = pool.prop[j][lane];
+            const Acc3 h = C.field();
+            float4 nv;
+            if (v.z < 1.0f && metro_accept<OPT>(P, C.rho, C.S, marsaglia_spin(v.x, v.y, v.z), v.w, h.x, h.y, h.z, beta_f, nv)) {
+                *C.site() = nv;
+                ++acc;
+            }
+            C.up();
+        }
+        __syncwarp();
     }
     return acc;
 }
