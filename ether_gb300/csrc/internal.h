@@ -129,7 +129,7 @@ struct Ctx {
     unsigned long long *acc_before = nullptr;  // R: acceptance counts at the start of a call
     double *acc_ratio = nullptr;               // R: device acceptance ratios of a call
     uint32_t *obs_done = nullptr;              // R: finished blocks of an energy reduction (zero between launches)
-    double *acc_host = nullptr;                // R: pinned host copy
+    double *acc_host = nullptr;                // 3 R: pinned host copy of a call's results
     void *stage = nullptr;                     // pinned staging of ether_{set,get}_spins_batch
     bool ion_direct = false;                   // the device reads / writes the host records in place
     // ether_{set,get}_spins_batch where ion_direct: measured rates (replicas per second) of the
@@ -273,7 +273,7 @@ cudaError_t launch_broadcast(Ctx &c, void *base, size_t bytes_per_replica);
 // replicas r0 .. r0+n-1 from (to_device) or into the ion(0:8, N, n) records at ion, on c.stream
 bool ion_direct_possible(int dev);
 cudaError_t launch_ion_copy(Ctx &c, int r0, int n, double *ion, bool to_device);
-cudaError_t launch_energy_mag(Ctx &c, bool measure);
+cudaError_t launch_energy_mag(Ctx &c, bool measure, double *host_e = nullptr, double *host_m = nullptr);
 // Row t of the |M| (and E) series; with t_dev the row is read from device memory and
 // advanced afterwards (for captured graphs).
 cudaError_t launch_record(Ctx &c, int t, bool want_e, double *mser, double *eser, int32_t *t_dev = nullptr);

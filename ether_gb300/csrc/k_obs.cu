@@ -405,11 +405,13 @@ __device__ __forceinline__ void finish_block(const double *__restrict__ partials
 
 // One block per (replica, energy block); the block of a replica that ends last sums the
 // replica's partials and, with `measure`, adds them to the accumulators.  done[r] counts the
-// blocks that have written theirs and is zero again when the launch ends.  (As launches of their
+// blocks that have written theirs and is zero again when the launch ends.  host_e, host_m: pinned
+// host memory that takes the energies or magnetisations as well, or null.  (As launches of their
 // own, the sum and the measurement are two gaps of about 2 us after a reduction that itself
 // takes 3 us at 16^3 x 190.)
 template <int FORM>
-__global__ void __launch_bounds__(kRedBs, 4) energy_mag_kernel(const ObsMember a, uint32_t *__restrict__ done, int measure) {
+__global__ void __launch_bounds__(kRedBs, 4) energy_mag_kernel(const ObsMember a, uint32_t *__restrict__ done, int measure,
+                                                                double *host_e, double *host_m) {
     const int r = blockIdx.y;
     energy_block<FORM>(a, r, blockIdx.x);
     __shared__ int s_last;
@@ -425,6 +427,9 @@ __global__ void __launch_bounds__(kRedBs, 4) energy_mag_kernel(const ObsMember a
     if (threadIdx.x == 0) {
         done[r] = 0u;
         if (measure) measure_one(a.E, a.M, a.N, a.n_slots, a.slot_of_rep, a.sums, r);
+        if (host_e) host_e[r] = a.E[r];
+        if (host_m)
+            for (int j = 0; j < 3; ++j) host_m[3 * r + j] = a.M[3 * r + j];
     }
 }
 
@@ -571,13 +576,13 @@ ObsMember obs_member(const Ctx &c) {
     return a;
 }
 
-cudaError_t launch_energy_mag(Ctx &c, bool measure) {
+cudaError_t launch_energy_mag(Ctx &c, bool measure, double *host_e, double *host_m) {
     dim3 grid(c.partial_blocks, c.R);
     const ObsMember a = obs_member(c);
     const int form = obs_form(a);
     auto k = form == kObsIsing ? energy_mag_kernel<kObsIsing> : form == kObsCubic ? energy_mag_kernel<kObsCubic>
                                                                                    : energy_mag_kernel<kObsGeneral>;
-    k<<<grid, kRedBs, 0, c.stream>>>(a, c.obs_done, measure ? 1 : 0);
+    k<<<grid, kRedBs, 0, c.stream>>>(a, c.obs_done, measure ? 1 : 0, host_e, host_m);
     c.launches++;
     return cudaGetLastError();
 }
