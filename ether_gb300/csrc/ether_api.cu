@@ -544,7 +544,7 @@ extern "C" int ether_create(const ether_desc *d, ether_ctx **out) {
             cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
             std::vector<uint4> ent;
             std::vector<int32_t> order;
-            plan_general_resident(c, optin, row_ptr, nbr, jidx, wstr, ent, order);
+            plan_general_resident(c, std::max(0, optin - 256), row_ptr, nbr, jidx, wstr, ent, order);
             if (c.gen_resident) {
                 TRY(dev_upload(c, &c.t.res_ent, ent));
                 TRY(dev_upload(c, &c.t.res_order, order));
@@ -1129,6 +1129,9 @@ extern "C" int ether_fresh_spins(ether_ctx *h) {
     return ETHER_OK;
 }
 
+// Does the context's resident sweep of k_resident.cu run?
+static bool general_resident(const Ctx &c) { return c.gen_resident && !(c.fast && c.variant_asked); }
+
 static int sweep_once(Ctx &c) {
     for (int col = 0; col < c.ncol; ++col) {
         if (c.model == ETHER_MODEL_ISING) CUDA_TRY(launch_ising_sweep(c, col));
@@ -1138,7 +1141,20 @@ static int sweep_once(Ctx &c) {
     return ETHER_OK;
 }
 
-int ether::plain_sweep(Ctx &c) { return sweep_once(c); }
+// n sweeps: in the launches of a resident kernel (of at most 256 sweeps each) or phase by phase.
+int ether::plain_sweeps(Ctx &c, int n) {
+    const bool resident = c.resident && !c.variant_asked;
+    if (!resident && !general_resident(c)) {
+        int rc = ETHER_OK;
+        for (int k = 0; k < n && rc == ETHER_OK; ++k) rc = sweep_once(c);
+        return rc;
+    }
+    for (int k = 0; k < n; k += 256) {
+        const int m = std::min(256, n - k);
+        CUDA_TRY(resident ? launch_ising_resident(c, m) : launch_general_resident(c, m));
+    }
+    return ETHER_OK;
+}
 
 // How many replica parts ether_mcs splits this context's sweeps into (general lattices:
 // their colour phases are small, dependent, latency-bound launches): 1 (no split), 2 or 4.
@@ -1193,12 +1209,17 @@ extern "C" int ether_metropolis(ether_ctx *h, int32_t nsweeps, double *accept) {
     Ctx &c = h->c;
     if (nsweeps < 0) return fail(ETHER_ERR_ARG, "negative sweep count");
     if (!c.beta_set) return fail(ETHER_ERR_STATE, "beta not set (ether_set_beta / ether_set_ladder)");
-    const bool resident = c.resident && c.ising_code == 0;  // a variant that was asked for names a phase kernel
-    if (resident && nsweeps >= 1 && nsweeps <= 256) {
+    const bool resident = c.resident && !c.variant_asked, general = general_resident(c);
+    if ((resident || (general && (c.gen_resident == 1 || !accept))) && nsweeps >= 1 && nsweeps <= 256) {
         // one launch, which writes the acceptance into pinned host memory
-        ResidentEvents ev;
-        ev.ratio = accept ? c.acc_host : nullptr;
-        CUDA_TRY(launch_ising_resident(c, nsweeps, ev));
+        double *ratio = accept ? c.acc_host : nullptr;
+        if (resident) {
+            ResidentEvents ev;
+            ev.ratio = ratio;
+            CUDA_TRY(launch_ising_resident(c, nsweeps, ev));
+        } else {
+            CUDA_TRY(launch_general_resident(c, nsweeps, ratio));
+        }
         if (accept) {
             CUDA_TRY(cudaStreamSynchronize(c.stream));
             std::memcpy(accept, c.acc_host, sizeof(double) * c.R);
@@ -1245,11 +1266,9 @@ extern "C" int ether_metropolis(ether_ctx *h, int32_t nsweeps, double *accept) {
         const int rc = ensure_parts(c);
         if (rc) return rc;
     }
-    if (resident || (nsweeps > 1 && c.gen_resident)) {
-        for (int k = 0; k < nsweeps; k += 256) {  // bounded launches
-            const int m = std::min(256, nsweeps - k);
-            CUDA_TRY(resident ? launch_ising_resident(c, m) : launch_general_resident(c, m));
-        }
+    if (resident || general) {
+        const int rc = plain_sweeps(c, nsweeps);
+        if (rc) return rc;
     } else if (nsweeps > 1 && c.n_parts > 1) {  // general lattices: replica parts side by side, same bits
         const int rc = sweeps_in_parts(c, nsweeps);
         if (rc) return rc;
@@ -1507,7 +1526,7 @@ static int issue_steps(Ctx &c, const ether_schedule *sch, const int8_t *sig, int
         }
         return ETHER_OK;
     }
-    if (!c.resident && !c.gen_resident) {
+    if (!c.resident && !general_resident(c)) {
         for (int k = 0; k < n; ++k) {
             int rc = issue_step(c, sch, sig[k]);
             if (rc) return rc;
@@ -1570,7 +1589,7 @@ extern "C" int ether_mcs(ether_ctx *h, const ether_schedule *sch, int32_t step0,
     int chunk = mcs_chunk(period);
     // resident contexts: the longest multiple of the period up to 256 steps, so that the
     // eventless stretches (equilibration) run as few long resident launches
-    if ((c.resident || c.gen_resident) && period <= 256) chunk = (int)(256 / period * period);
+    if ((c.resident || general_resident(c)) && period <= 256) chunk = (int)(256 / period * period);
     const bool use_graphs = !(c.flags & ETHER_FLAG_NO_GRAPHS);
     int step = step0 + 1;
     const int last = step0 + nsteps;
@@ -1827,6 +1846,7 @@ extern "C" int ether_autotune(ether_ctx *h, int32_t *variant, float *best_ms) {
     if (best_ms) *best_ms = 0.f;
     if (!c.fast) return ETHER_OK;
     if (!c.beta_set) return fail(ETHER_ERR_STATE, "beta not set");
+    c.variant_asked = false;
     if (c.model == ETHER_MODEL_XYZ) return autotune_xyz(c, variant, best_ms);
     const std::vector<long> key = {c.model, c.L[0], c.L[1], c.L[2], c.R};
     {
@@ -1892,6 +1912,7 @@ extern "C" int ether_set_variant(ether_ctx *h, int32_t variant) {
     Ctx &c = h->c;
     if (!c.fast) return ETHER_OK;
     if (!apply_variant(c, variant)) return fail(ETHER_ERR_ARG, "variant not available for this lattice");
+    c.variant_asked = true;
     return ETHER_OK;
 }
 
@@ -1931,7 +1952,7 @@ extern "C" int ether_record_series(ether_ctx *h, int32_t nsweeps, int32_t stride
         cudaError_t e = cudaMemsetAsync(t_dev, 0, sizeof(int32_t), c.stream);
         if (e == cudaSuccess) e = cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            for (int k = 0; k < stride && rc == ETHER_OK; ++k) rc = sweep_once(c);
+            rc = plain_sweeps(c, stride);
             if (rc == ETHER_OK) e = launch_record(c, 0, E != nullptr, mser, eser, t_dev);
             const cudaError_t ee = cudaStreamEndCapture(c.stream, &g);
             if (e == cudaSuccess) e = ee;
@@ -1941,15 +1962,15 @@ extern "C" int ether_record_series(ether_ctx *h, int32_t nsweeps, int32_t stride
         for (int i = 0; i < nrec && rc == ETHER_OK && e == cudaSuccess; ++i) e = cudaGraphLaunch(ex, c.stream);
         if (rc == ETHER_OK && e != cudaSuccess) rc = fail(ETHER_ERR_CUDA, std::string("series graph: ") + cudaGetErrorString(e));
         // the sweeps after the last recorded row
-        for (int k = nrec * stride + 1; k <= nsweeps && rc == ETHER_OK; ++k) rc = sweep_once(c);
+        if (rc == ETHER_OK) rc = plain_sweeps(c, nsweeps - nrec * stride);
     } else {
-        for (int k = 1; k <= nsweeps && rc == ETHER_OK; ++k) {
-            rc = sweep_once(c);
-            if (rc == ETHER_OK && k % stride == 0 && t < nrec) {
-                cudaError_t e = launch_record(c, t++, E != nullptr, mser, eser);
-                if (e != cudaSuccess) rc = fail(ETHER_ERR_CUDA, std::string("record: ") + cudaGetErrorString(e));
-            }
+        for (; t < nrec && rc == ETHER_OK; ++t) {
+            rc = plain_sweeps(c, stride);
+            if (rc != ETHER_OK) break;
+            cudaError_t e = launch_record(c, t, E != nullptr, mser, eser);
+            if (e != cudaSuccess) rc = fail(ETHER_ERR_CUDA, std::string("record: ") + cudaGetErrorString(e));
         }
+        if (rc == ETHER_OK) rc = plain_sweeps(c, nsweeps - nrec * stride);
     }
     if (rc == ETHER_OK) {
         cudaError_t e = cudaMemcpyAsync(absM, mser, bytes, cudaMemcpyDeviceToHost, c.stream);

@@ -122,6 +122,7 @@ struct Ctx {
     uint32_t *thr = nullptr;     // n_slots * table_entries: flip iff u32 <= thr
     int ising_vpt = 1;           // vectors per thread of the simple-cubic Ising kernel
     int ising_code = 0;          // the variant that was asked for (0: the default choice)
+    bool variant_asked = false;  // by ether_set_variant: it names a phase kernel
     int xyz_variant = 11;        // simple-cubic XYZ kernel: planes per thread (xyz_planes, k_xyz.cu)
     int gen_resident = 0;        // general lattices: blocks per replica of the resident sweep, 0 none
     int res_q = 0, res_slots = 0, res_shell_end[8] = {0}, res_stride[8] = {0};  // its entries
@@ -259,7 +260,8 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
                            const std::vector<uint16_t> &jidx, const std::vector<int32_t> &wstride,
                            std::vector<uint4> &ent, std::vector<int32_t> &order);
 cudaError_t prepare_general_resident(const Ctx &c);
-cudaError_t launch_general_resident(Ctx &c, int nsweeps);
+// ratio: with gen_resident 1, takes the launch's acceptance per replica
+cudaError_t launch_general_resident(Ctx &c, int nsweeps, double *ratio = nullptr);
 bool ising_staged_shape(const Ctx &c, int vectors_per_step);
 int ising_default_vpt(const Ctx &c);
 cudaError_t launch_xyz_sweep(Ctx &c, int colour);
@@ -281,7 +283,7 @@ cudaError_t launch_pt(Ctx &c, int set_swap_count);
 cudaError_t launch_acc_bin(Ctx &c);
 cudaError_t launch_spiral_measure(Ctx &c);
 int energy_blocks(const Ctx &c);
-int plain_sweep(Ctx &c);  // one Metropolis sweep of every replica (ETHER_OK or an error code)
+int plain_sweeps(Ctx &c, int n);  // n Metropolis sweeps of every replica (ETHER_OK or an error code)
 int ctx_variant(const Ctx &c);  // the context's kernel variant code (ether_set_variant's numbering)
 void *tma_encode_tiled_fn();    // cuTensorMapEncodeTiled (PFN_cuTensorMapEncodeTiled_v12000), or null
 

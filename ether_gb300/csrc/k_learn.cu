@@ -1116,11 +1116,9 @@ extern "C" int ether_learn_batch_sweep(ether_learn *const *learns, int32_t n, in
     // work in order, the contexts run side by side
     for (int s = 0; s < nsweeps; ++s)
         for (int k = 0; k < n; ++k) {
-            for (int p = 0; p < plain_per_sweep; ++p) {
-                const int rc = plain_sweep(learns[k]->ctx->c);
-                if (rc) return rc;
-            }
-            const int rc = ether_learn_sweep(learns[k], 1);
+            int rc = plain_sweeps(learns[k]->ctx->c, plain_per_sweep);
+            if (rc) return rc;
+            rc = ether_learn_sweep(learns[k], 1);
             if (rc) return rc;
         }
     return ETHER_OK;
@@ -1142,7 +1140,7 @@ extern "C" int ether_learn_record_series(ether_learn *l, int32_t nsteps, int32_t
     double *mser = nullptr;
     LCUDA(cudaMalloc((void **)&mser, bytes));
     for (int t = 0; t < nsteps && rc == ETHER_OK; ++t) {
-        for (int k = 0; k < plain_per_step && rc == ETHER_OK; ++k) rc = plain_sweep(c);
+        rc = plain_sweeps(c, plain_per_step);
         for (int k = 0; k < learned_per_step && rc == ETHER_OK; ++k) {
             for (int cls = 0; cls < 2 && rc == ETHER_OK; ++cls) rc = launch_patches(*l, cls, nullptr);
             if (rc == ETHER_OK) {

@@ -981,7 +981,7 @@ int xyz_record_series(XyzLearn *x, int nsteps, int plain_per_step, int learned_p
     XCUDA(cudaMalloc((void **)&mser, bytes));
     int rc = ETHER_OK;
     for (int t = 0; t < nsteps && rc == ETHER_OK; ++t) {
-        for (int k = 0; k < plain_per_step && rc == ETHER_OK; ++k) rc = plain_sweep(c);
+        rc = plain_sweeps(c, plain_per_step);
         for (int k = 0; k < learned_per_step && rc == ETHER_OK; ++k) rc = learned_sweep(*x, nullptr);
         if (rc == ETHER_OK && (t + 1) % stride == 0 && (t + 1) / stride <= nrec) {
             const cudaError_t e = launch_record(c, (t + 1) / stride - 1, false, mser, nullptr);

@@ -496,10 +496,13 @@ __global__ void pt_copy_kernel(uint8_t *__restrict__ spins, float4 *__restrict__
 // Blocks per replica of the reductions: no more than four blocks per SM over all replicas
 // (the context's own launch fills the GPU once, each thread running through many sites), and
 // at least eight sites per thread, so that the per-warp and per-block sums stay a small part
-// of a thread's work also for the many small contexts of a batch.  The same number serves the
-// context's own launches and the batched ones, so the two sum in the same order.
+// of a thread's work also for the many small contexts of a batch; on general lattices, where a
+// site is a chain of two gathers, at least two (21 x 18 x 15 x 64: 22 -> 15 us, cold).  The
+// same number serves the context's own launches and the batched ones, so the two sum in the same
+// order.
 int energy_blocks(const Ctx &c) {
-    long need = (c.N + kRedBs * 8 - 1) / (kRedBs * 8);
+    const int least = c.fast ? 8 : 2;
+    long need = (c.N + kRedBs * least - 1) / (kRedBs * least);
     long cap = (long)c.sm_count * 4 / (c.R > 0 ? c.R : 1);
     if (cap < 1) cap = 1;
     if (need > cap) need = cap;

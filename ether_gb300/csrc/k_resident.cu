@@ -57,6 +57,20 @@ struct ResCouplings {
 // ------------------------------------------------------------------------ Ising ----
 // One block per replica; a thread takes two neighbouring ranks (one Philox block serves both).
 // s_sp[N] is the zero spin.  Threshold-table index = sum over shells of stride * up-spins.
+// The block's accepted moves into the replica's counter and, for a whole replica, their share of its
+// sites into *ratio.
+__device__ __forceinline__ void res_accepts(unsigned long long *count, unsigned acc, double invN, double *ratio) {
+    __shared__ unsigned s_acc[32];
+    acc = __reduce_add_sync(0xffffffffu, acc);
+    if ((threadIdx.x & 31) == 0) s_acc[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) acc += s_acc[w];
+        atomicAdd(count, (unsigned long long)acc);
+        if (ratio) *ratio = (double)acc * invN;
+    }
+}
+
 template <int NQ>
 __global__ void __launch_bounds__(kResThreads, 1)
 ising_resident_general(uint8_t *__restrict__ spins, int N, const __grid_constant__ ResShape C, int4 stride4,
@@ -64,7 +78,7 @@ ising_resident_general(uint8_t *__restrict__ spins, int N, const __grid_constant
                        const int32_t *__restrict__ type_base, const int32_t *__restrict__ type_half, int n_types,
                        const uint32_t *__restrict__ thr, int table_entries, const int32_t *__restrict__ slot_of_rep,
                        const uint32_t *__restrict__ stream_id, uint32_t *__restrict__ step, const RoundKeys K,
-                       int nsweeps, unsigned long long *__restrict__ acc_count) {
+                       int nsweeps, unsigned long long *__restrict__ acc_count, double invN, double *ratio) {
     extern __shared__ __align__(16) uint8_t s_raw[];
     uint32_t *s_tb = reinterpret_cast<uint32_t *>(s_raw);         // table_entries thresholds
     int2 *s_ty = reinterpret_cast<int2 *>(s_tb + ((table_entries + 1) & ~1));  // per type: base, half
@@ -144,7 +158,7 @@ ising_resident_general(uint8_t *__restrict__ spins, int N, const __grid_constant
     }
     for (int i = threadIdx.x; i < N; i += blockDim.x) g[i] = s_sp[i];
     if (threadIdx.x == 0) step[r] = t0 + (uint32_t)nsweeps;
-    warp_add_count(acc_count + r, acc);
+    res_accepts(acc_count + r, acc, invN, ratio ? ratio + r : nullptr);
 }
 
 // -------------------------------------------------------------------------- XYZ ----
@@ -213,7 +227,7 @@ xyz_resident_general(float4 *__restrict__ spins4, int N, const __grid_constant__
                      const __grid_constant__ ResCouplings J, XyzParams P,
                      const float *__restrict__ beta_slot_f, const int32_t *__restrict__ slot_of_rep,
                      const uint32_t *__restrict__ stream_id, uint32_t *__restrict__ step, const RoundKeys K,
-                     int nsweeps, unsigned long long *__restrict__ acc_count) {
+                     int nsweeps, unsigned long long *__restrict__ acc_count, double invN, double *ratio) {
     extern __shared__ __align__(16) float4 s_sp[];
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(s_sp);
     const int r = blockIdx.x / CS;
@@ -315,7 +329,7 @@ xyz_resident_general(float4 *__restrict__ spins4, int N, const __grid_constant__
         loc += b - a;
     }
     if (blk == 0 && threadIdx.x == 0) step[r] = t0 + (uint32_t)nsweeps;
-    warp_add_count_x(acc_count + r, acc);
+    res_accepts(acc_count + r, acc, invN, CS == 1 && ratio ? ratio + r : nullptr);
 }
 
 // ------------------------------------------------------------------------ host side ----
@@ -412,7 +426,7 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
                            std::vector<uint4> &ent, std::vector<int32_t> &order) {
     c.gen_resident = 0;
     const bool ising = c.model == ETHER_MODEL_ISING;
-    if (c.fast || c.nsp != 1 || c.nsh < 1 || c.nsh > (ising ? 4 : 8)) return;
+    if ((c.fast && ising) || c.nsp != 1 || c.nsh < 1 || c.nsh > (ising ? 4 : 8)) return;
     std::vector<int> slots(c.nsh, 0), count(c.nsh);
     std::vector<int> stride(c.nsh, 0);
     for (int s = 0; s < c.N; ++s) {
@@ -456,11 +470,11 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
     }
     // Against the phase kernels: a replica's sweep here takes its sites' time in turn, theirs the
     // whole context's work over the GPU but at least a launch's latency per colour.  Measured per
-    // site: here 1.9 ns (Ising), 1.6 + 0.145 per slot (XYZ; 1.3 times that in a cluster); there,
+    // site: here 1.9 ns (Ising), 1.0 + 0.1425 per slot (XYZ; 1.3 times that in a cluster); there,
     // over all replicas, 0.037 ns (Ising), 0.004 per slot - 0.008 (XYZ), and 3 us (4 us) a colour.
     if (cs) {
         const double waves = std::ceil((double)c.R * cs / c.sm_count), share = (double)c.N / cs, all = (double)c.N * c.R;
-        const double here = waves * share * (ising ? 1.9e-3 : (1.6e-3 + 0.145e-3 * total) * (cs > 1 ? 1.3 : 1.0));
+        const double here = waves * share * (ising ? 1.9e-3 : (1.0e-3 + 0.1425e-3 * total) * (cs > 1 ? 1.3 : 1.0));
         const double there = std::max(c.ncol * (ising ? 3.0 : 4.0), all * (ising ? 0.037e-3 : std::max(0.008e-3, 0.004e-3 * total - 0.008e-3)));
         if (here > there) cs = 0;
     }
@@ -530,7 +544,7 @@ cudaError_t prepare_general_resident(const Ctx &c) {
                ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, want) : cudaSuccess;
 }
 
-cudaError_t launch_general_resident(Ctx &c, int nsweeps) {
+cudaError_t launch_general_resident(Ctx &c, int nsweeps, double *ratio) {
     if (nsweeps < 1) return cudaSuccess;
     const int cs = c.gen_resident;
     const bool ising = c.model == ETHER_MODEL_ISING;
@@ -558,10 +572,11 @@ cudaError_t launch_general_resident(Ctx &c, int nsweeps) {
     cfg.attrs = at;
     cfg.numAttrs = cs > 1 ? 1 : 0;
     c.launches++;
+    double invN = 1.0 / (double)c.N;
     if (ising) {
         void *args[] = {&c.spins, &c.N, &C, &stride4, &c.t.res_ent, &c.t.itype, &c.t.type_base, &c.t.type_half,
                         &c.n_types, &c.thr, &c.table_entries, &c.slot_of_rep, &c.stream_id, &c.step, &K, &nsweeps,
-                        &c.acc_count};
+                        &c.acc_count, &invN, &ratio};
         return cudaLaunchKernelExC(&cfg, res_kernel(c, cs), args);
     }
     XyzParams P = xyz_params(c);
@@ -573,7 +588,7 @@ cudaError_t launch_general_resident(Ctx &c, int nsweeps) {
         J.z[m] = c.h_Jf[3 * sh + 2];
     }
     void *args[] = {&c.spins4, &c.N, &C, &c.t.res_ent, &c.t.res_order, &J, &P, &c.beta_slot_f, &c.slot_of_rep, &c.stream_id,
-                    &c.step, &K, &nsweeps, &c.acc_count};
+                    &c.step, &K, &nsweeps, &c.acc_count, &invN, &ratio};
     return cudaLaunchKernelExC(&cfg, res_kernel(c, cs), args);
 }
 
