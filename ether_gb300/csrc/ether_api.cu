@@ -1132,23 +1132,25 @@ extern "C" int ether_fresh_spins(ether_ctx *h) {
 // Does the context's resident sweep of k_resident.cu run?
 static bool general_resident(const Ctx &c) { return c.gen_resident && !(c.fast && c.variant_asked); }
 
-static int sweep_once(Ctx &c) {
-    for (int col = 0; col < c.ncol; ++col) {
-        if (c.model == ETHER_MODEL_ISING) CUDA_TRY(launch_ising_sweep(c, col));
-        else CUDA_TRY(launch_xyz_sweep(c, col));
+// n sweeps phase by phase; the counters are advanced once, after the last (a launch less per sweep).
+static int sweeps_by_phase(Ctx &c, int n) {
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < n && e == cudaSuccess; ++k) {
+        c.ahead = (uint32_t)k;
+        for (int col = 0; col < c.ncol && e == cudaSuccess; ++col)
+            e = c.model == ETHER_MODEL_ISING ? launch_ising_sweep(c, col) : launch_xyz_sweep(c, col);
     }
-    CUDA_TRY(launch_advance(c, c.step));
+    c.ahead = 0;
+    CUDA_TRY(e);
+    if (n > 0) CUDA_TRY(launch_advance(c, c.step, n));
     return ETHER_OK;
 }
+static int sweep_once(Ctx &c) { return sweeps_by_phase(c, 1); }
 
 // n sweeps: in the launches of a resident kernel (of at most 256 sweeps each) or phase by phase.
 int ether::plain_sweeps(Ctx &c, int n) {
     const bool resident = c.resident && !c.variant_asked;
-    if (!resident && !general_resident(c)) {
-        int rc = ETHER_OK;
-        for (int k = 0; k < n && rc == ETHER_OK; ++k) rc = sweep_once(c);
-        return rc;
-    }
+    if (!resident && !general_resident(c)) return sweeps_by_phase(c, n);
     for (int k = 0; k < n; k += 256) {
         const int m = std::min(256, n - k);
         CUDA_TRY(resident ? launch_ising_resident(c, m) : launch_general_resident(c, m));
@@ -1176,7 +1178,7 @@ static int sweeps_in_parts(Ctx &c, int m) {
         c.stream = p ? c.aux[p - 1] : own;
         c.rw0 = (int)((long)c.R * p / P);
         c.rwn = (int)((long)c.R * (p + 1) / P) - c.rw0;
-        for (int k = 0; k < m && !rc; ++k) rc = sweep_once(c);
+        rc = sweeps_by_phase(c, m);
     }
     c.stream = own;
     c.rw0 = c.rwn = 0;
@@ -1273,10 +1275,8 @@ extern "C" int ether_metropolis(ether_ctx *h, int32_t nsweeps, double *accept) {
         const int rc = sweeps_in_parts(c, nsweeps);
         if (rc) return rc;
     } else {
-        for (int k = 0; k < nsweeps; ++k) {
-            int rc = sweep_once(c);
-            if (rc) return rc;
-        }
+        const int rc = sweeps_by_phase(c, nsweeps);
+        if (rc) return rc;
     }
     if (accept) {
         CUDA_TRY(launch_accept_ratio(c, c.acc_ratio));
@@ -1496,16 +1496,6 @@ int mcs_chunk(long period) {
 
 }  // namespace ether
 
-// One MCS of src/ether.f90:163-201 given its gates: OVRR (:163-169), Metropolis (:172),
-// total energy + PT when PT runs (:177, :189-198), observable on measurement steps (:201).
-static int issue_step(Ctx &c, const ether_schedule *sch, int gates) {
-    int rc = mcs_before_sweep(c, sch, gates);
-    if (rc) return rc;
-    rc = sweep_once(c);
-    if (rc) return rc;
-    return mcs_after_sweep(c, gates);
-}
-
 static int variant_of(const Ctx &c);
 
 // Steps sig[0 .. n): with a resident context the sweeps that no OVRR, PT or measurement
@@ -1527,9 +1517,16 @@ static int issue_steps(Ctx &c, const ether_schedule *sch, const int8_t *sig, int
         return ETHER_OK;
     }
     if (!c.resident && !general_resident(c)) {
-        for (int k = 0; k < n; ++k) {
-            int rc = issue_step(c, sch, sig[k]);
+        for (int k = 0; k < n;) {
+            int rc = mcs_before_sweep(c, sch, sig[k]);
             if (rc) return rc;
+            int j = k + 1;
+            while (j < n && !(sig[j - 1] & 6) && !(sig[j] & 1)) ++j;
+            rc = sweeps_by_phase(c, j - k);
+            if (rc) return rc;
+            rc = mcs_after_sweep(c, sig[j - 1]);
+            if (rc) return rc;
+            k = j;
         }
         return ETHER_OK;
     }

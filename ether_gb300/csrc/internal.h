@@ -169,6 +169,8 @@ struct Ctx {
     int32_t *swap_dev = nullptr;    // 1: PT swap counter
     int32_t *copy_from = nullptr;   // R (reference-copy PT mode)
     std::map<std::string, cudaGraphExec_t> graphs;  // ether_mcs chunks by gate pattern
+    // sweeps issued since the counters were advanced: the phase kernels add it to a replica's counter
+    uint32_t ahead = 0;
     // replica window of the general-lattice sweep launchers and launch_advance: replicas
     // rw0 .. rw0 + rwn - 1 (rwn 0: all); ether_mcs runs parts of a general lattice's replicas
     // on c.stream and the aux streams side by side between its PT and measurement steps
@@ -268,7 +270,7 @@ cudaError_t launch_xyz_sweep(Ctx &c, int colour);
 bool xyz_variant_valid(int variant);
 cudaError_t launch_overrelax(Ctx &c, int colour, int pass, float part);
 cudaError_t launch_fresh(Ctx &c);
-cudaError_t launch_advance(Ctx &c, uint32_t *counter);
+cudaError_t launch_advance(Ctx &c, uint32_t *counter, int by = 1);
 cudaError_t launch_accept_ratio(Ctx &c, double *out);
 cudaError_t launch_broadcast(Ctx &c, void *base, size_t bytes_per_replica);
 // k_ion.cu: whether device dev addresses pageable host memory through the host's page tables;

@@ -19,12 +19,12 @@ ising_ell_kernel(uint8_t *__restrict__ spins, int N, int col_off, int n_c, uint3
                  const int32_t *__restrict__ type_base, const int32_t *__restrict__ type_half,
                  const uint32_t *__restrict__ thr, int table_entries,
                  const int32_t *__restrict__ slot_of_rep, const uint32_t *__restrict__ stream_id,
-                 const uint32_t *__restrict__ step, uint32_t seed,
+                 const uint32_t *__restrict__ step, uint32_t ahead, uint32_t seed,
                  unsigned long long *__restrict__ acc_count) {
     const int r = blockIdx.y;
     uint8_t *sp = spins + (size_t)r * N;
     const uint32_t *tb = thr + (size_t)slot_of_rep[r] * table_entries;
-    const uint32_t stream = stream_id[r], t = step[r];
+    const uint32_t stream = stream_id[r], t = step[r] + ahead;
     const uint32_t c3 = kMetro | (colour << 8);
     const int ng = (n_c + 7) >> 3;
     unsigned acc = 0;
@@ -88,12 +88,12 @@ ising_ell_site_kernel(uint8_t *__restrict__ spins, int N, int col_off, int n_c, 
                       const int32_t *__restrict__ type_base, const int32_t *__restrict__ type_half,
                       const uint32_t *__restrict__ thr, int table_entries,
                       const int32_t *__restrict__ slot_of_rep, const uint32_t *__restrict__ stream_id,
-                      const uint32_t *__restrict__ step, uint32_t seed,
+                      const uint32_t *__restrict__ step, uint32_t ahead, uint32_t seed,
                       unsigned long long *__restrict__ acc_count) {
     const int r = blockIdx.y;
     uint8_t *sp = spins + (size_t)r * N;
     const uint32_t *tb = thr + (size_t)slot_of_rep[r] * table_entries;
-    const uint32_t stream = stream_id[r], t = step[r];
+    const uint32_t stream = stream_id[r], t = step[r] + ahead;
     const uint32_t c3 = kMetro | (colour << 8);
     unsigned acc = 0;
     const IsingEll A{sp, col_off, n_c, width, ell, ews, deg, itype, type_base, type_half, tb};
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256, MINB)
 ising_sc_kernel(uint8_t *__restrict__ spins, int L1, int L2, int L3, FastDiv fH, FastDiv fL2,
                 uint32_t colour, const uint32_t *__restrict__ thr, int table_entries,
                 const int32_t *__restrict__ slot_of_rep, const uint32_t *__restrict__ stream_id,
-                const uint32_t *__restrict__ step, uint32_t seed, const RoundKeys K,
+                const uint32_t *__restrict__ step, uint32_t ahead, uint32_t seed, const RoundKeys K,
                 unsigned long long *__restrict__ acc_count) {
     const int r = blockIdx.y;
     const int H = L1 >> 1;
@@ -126,7 +126,7 @@ ising_sc_kernel(uint8_t *__restrict__ spins, int L1, int L2, int L3, FastDiv fH,
                     spins + (size_t)r * 2 * half + (size_t)(colour ^ 1u) * half,
                     L1, L2, L3, H, fH, fL2, colour};
     const uint32_t c3 = kMetro | (colour << 8);
-    const uint32_t t = step[r], stream = stream_id[r];
+    const uint32_t t = step[r] + ahead, stream = stream_id[r];
     uint32_t cnt = 0;
     if constexpr (VPT == 1) {
         fill_sc_table(thr + (size_t)slot_of_rep[r] * table_entries, s_tab, threadIdx.x, 256);
@@ -175,7 +175,7 @@ static void launch_sc(Ctx &c, int colour) {
     ising_sc_kernel<W, VPT, MINB><<<grid, bs, 0, c.stream>>>(
         c.spins, c.L[0], c.L[1], c.L[2], make_fastdiv((uint32_t)(c.L[0] / 2)),
         make_fastdiv((uint32_t)c.L[1]), (uint32_t)colour, c.thr, c.table_entries, c.slot_of_rep,
-        c.stream_id, c.step, c.seed, round_keys(c.seed), c.acc_count);
+        c.stream_id, c.step, c.ahead, c.seed, round_keys(c.seed), c.acc_count);
 }
 
 static int blocks_for(const Ctx &c, long work, int bs) {
@@ -522,13 +522,13 @@ cudaError_t launch_ising_sweep(Ctx &c, int colour) {
             k<<<grid, bs, 0, c.stream>>>(
                 spins, c.N, c.col_off[colour], n_c, (uint32_t)colour, ell, ews, c.t.ell_deg,
                 c.ell_width[colour], c.t.itype, c.t.type_base, c.t.type_half, c.thr, c.table_entries,
-                c.slot_of_rep + r0, c.stream_id + r0, c.step + r0, c.seed, c.acc_count + r0);
+                c.slot_of_rep + r0, c.stream_id + r0, c.step + r0, c.ahead, c.seed, c.acc_count + r0);
         } else {
             dim3 grid(blocks_for(c, (n_c + 7) / 8, bs), nr);
             ising_ell_kernel<<<grid, bs, 0, c.stream>>>(
                 spins, c.N, c.col_off[colour], n_c, (uint32_t)colour, ell, ews, c.t.ell_deg,
                 c.ell_width[colour], c.t.itype, c.t.type_base, c.t.type_half, c.thr, c.table_entries,
-                c.slot_of_rep + r0, c.stream_id + r0, c.step + r0, c.seed, c.acc_count + r0);
+                c.slot_of_rep + r0, c.stream_id + r0, c.step + r0, c.ahead, c.seed, c.acc_count + r0);
         }
     }
     c.launches++;

@@ -16,12 +16,12 @@ xyz_ell_kernel(float4 *__restrict__ spins4, int N, int col_off, int n_c, uint32_
                const int32_t *__restrict__ ell, const uint16_t *__restrict__ ej,
                const uint16_t *__restrict__ deg, int width, const float4 *__restrict__ J4, XyzParams P,
                const float *__restrict__ beta_slot_f, const int32_t *__restrict__ slot_of_rep,
-               const uint32_t *__restrict__ stream_id, const uint32_t *__restrict__ step,
+               const uint32_t *__restrict__ stream_id, const uint32_t *__restrict__ step, uint32_t ahead,
                const RoundKeys K, unsigned long long *__restrict__ acc_count) {
     const int r = blockIdx.y;
     float4 *sp = spins4 + (size_t)r * N;
     const float beta_f = beta_slot_f[slot_of_rep[r]];
-    const uint32_t k1 = stream_id[r], t = step[r];
+    const uint32_t k1 = stream_id[r], t = step[r] + ahead;
     const uint32_t c3 = kMetro | (colour << 8);
     unsigned acc = 0;
     for (int rho = blockIdx.x * blockDim.x + threadIdx.x; rho < n_c; rho += gridDim.x * blockDim.x) {
@@ -47,7 +47,8 @@ __global__ void __launch_bounds__(kColThreads, kColBlocks)
 xyz_col_kernel(float4 *__restrict__ spins4, int L1, int L2, int L3, FastDiv fH, FastDiv fP, int ZC, int items,
                uint32_t colour, float jx, float jy, float jz, XyzParams P, const float *__restrict__ beta_slot_f,
                const int32_t *__restrict__ slot_of_rep, const uint32_t *__restrict__ stream_id,
-               const uint32_t *__restrict__ step, const RoundKeys K, unsigned long long *__restrict__ acc_count) {
+               const uint32_t *__restrict__ step, uint32_t ahead, const RoundKeys K,
+               unsigned long long *__restrict__ acc_count) {
     const int r = blockIdx.y;
     const int H = L1 >> 1;
     const int half = H * L2 * L3;
@@ -55,7 +56,7 @@ xyz_col_kernel(float4 *__restrict__ spins4, int L1, int L2, int L3, FastDiv fH, 
     const XyzSc A{base + (size_t)colour * half, base + (size_t)(colour ^ 1u) * half, L1, L2, L3, H,
                   fH, fP, colour, jx, jy, jz};
     const float beta_f = beta_slot_f[slot_of_rep[r]];
-    const uint32_t k1 = stream_id[r], t = step[r];
+    const uint32_t k1 = stream_id[r], t = step[r] + ahead;
     unsigned acc = 0;
     const int i = blockIdx.x * kColThreads + threadIdx.x;
     if constexpr (POOL > 0) {
@@ -195,9 +196,9 @@ __global__ void fresh_kernel(uint8_t *__restrict__ spins, float4 *__restrict__ s
     }
 }
 
-__global__ void advance_kernel(uint32_t *__restrict__ counter, int R) {
+__global__ void advance_kernel(uint32_t *__restrict__ counter, int R, uint32_t by) {
     int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < R) counter[r] += 1u;
+    if (r < R) counter[r] += by;
 }
 
 static int blocks_for_x(const Ctx &c, long work, int bs) {
@@ -251,7 +252,7 @@ static void launch_xyz_col(Ctx &c, int colour, const XyzParams &P, const RoundKe
         k = ZC >= 4 ? xyz_col_kernel<OPT, true, 4> : ZC >= 2 ? xyz_col_kernel<OPT, true, 2> : k;
     k<<<grid, kColThreads, 0, c.stream>>>(
         c.spins4, c.L[0], c.L[1], c.L[2], make_fastdiv((uint32_t)(c.L[0] / 2)), make_fastdiv((uint32_t)plane), ZC, items,
-        (uint32_t)colour, c.h_Jf[0], c.h_Jf[1], c.h_Jf[2], Pc, c.beta_slot_f, c.slot_of_rep, c.stream_id, c.step, K,
+        (uint32_t)colour, c.h_Jf[0], c.h_Jf[1], c.h_Jf[2], Pc, c.beta_slot_f, c.slot_of_rep, c.stream_id, c.step, c.ahead, K,
         c.acc_count);
 }
 
@@ -291,7 +292,7 @@ cudaError_t launch_xyz_sweep(Ctx &c, int colour) {
                                : ell_kernel_for<kXyzGeneral>(c.ell_width[colour]);
         k<<<grid, bs, 0, c.stream>>>(c.spins4 + (size_t)r0 * c.N, c.N, c.col_off[colour], n_c, (uint32_t)colour, ell,
                                      ej, c.t.ell_deg, c.ell_width[colour], c.t.J4, P, c.beta_slot_f,
-                                     c.slot_of_rep + r0, c.stream_id + r0, c.step + r0, K, c.acc_count + r0);
+                                     c.slot_of_rep + r0, c.stream_id + r0, c.step + r0, c.ahead, K, c.acc_count + r0);
     }
     c.launches++;
     return cudaGetLastError();
@@ -368,9 +369,9 @@ cudaError_t launch_accept_ratio(Ctx &c, double *out) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_advance(Ctx &c, uint32_t *counter) {
+cudaError_t launch_advance(Ctx &c, uint32_t *counter, int by) {
     const int r0 = c.rw0, nr = c.rwn ? c.rwn : c.R;
-    advance_kernel<<<(nr + 255) / 256, 256, 0, c.stream>>>(counter + r0, nr);
+    advance_kernel<<<(nr + 255) / 256, 256, 0, c.stream>>>(counter + r0, nr, (uint32_t)by);
     c.launches++;
     return cudaGetLastError();
 }
