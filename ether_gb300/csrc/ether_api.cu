@@ -1212,7 +1212,7 @@ extern "C" int ether_metropolis(ether_ctx *h, int32_t nsweeps, double *accept) {
     if (nsweeps < 0) return fail(ETHER_ERR_ARG, "negative sweep count");
     if (!c.beta_set) return fail(ETHER_ERR_STATE, "beta not set (ether_set_beta / ether_set_ladder)");
     const bool resident = c.resident && !c.variant_asked, general = general_resident(c);
-    if ((resident || (general && (c.gen_resident == 1 || !accept))) && nsweeps >= 1 && nsweeps <= 256) {
+    if ((resident || general) && nsweeps >= 1 && nsweeps <= 256) {
         // one launch, which writes the acceptance into pinned host memory
         double *ratio = accept ? c.acc_host : nullptr;
         if (resident) {

@@ -262,7 +262,7 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
                            const std::vector<uint16_t> &jidx, const std::vector<int32_t> &wstride,
                            std::vector<uint4> &ent, std::vector<int32_t> &order);
 cudaError_t prepare_general_resident(const Ctx &c);
-// ratio: with gen_resident 1, takes the launch's acceptance per replica
+// ratio: takes the launch's acceptance per replica, or null
 cudaError_t launch_general_resident(Ctx &c, int nsweeps, double *ratio = nullptr);
 bool ising_staged_shape(const Ctx &c, int vectors_per_step);
 int ising_default_vpt(const Ctx &c);

@@ -1,7 +1,7 @@
 // k_resident.cu -- general lattices whose replicas fit in shared memory: whole runs of Metropolis
 // sweeps (src/Metropolis.f90:34-68) without a launch per colour phase.
 //
-// A cluster of 1, 2 or 4 thread blocks (Ising: one block) holds a replica's spins in shared
+// A cluster of 1, 2 or 4 thread blocks (Ising: 1 or 2, which both hold all spins) holds a replica's spins in shared
 // memory and runs nsweeps sweeps with a cluster (block) barrier between colour phases; the spins
 // are read from and written to global memory once per run.  Each site's arithmetic, draws and
 // neighbour order are the phase kernels' (sweep_ising.cuh, sweep_xyz.cuh), so the results are
@@ -57,21 +57,38 @@ struct ResCouplings {
 // ------------------------------------------------------------------------ Ising ----
 // One block per replica; a thread takes two neighbouring ranks (one Philox block serves both).
 // s_sp[N] is the zero spin.  Threshold-table index = sum over shells of stride * up-spins.
-// The block's accepted moves into the replica's counter and, for a whole replica, their share of its
-// sites into *ratio.
-__device__ __forceinline__ void res_accepts(unsigned long long *count, unsigned acc, double invN, double *ratio) {
-    __shared__ unsigned s_acc[32];
+__device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();  // .aligned: the warp arrives as one
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The block's accepted moves into the replica's counter and, where ratio is given, the whole
+// replica's share of its sites into *ratio (the cluster's first block adds up).
+template <int CS>
+__device__ __forceinline__ void res_accepts(unsigned long long *count, unsigned acc, double invN, double *ratio, int blk) {
+    __shared__ unsigned s_acc[32], s_part[4];
     acc = __reduce_add_sync(0xffffffffu, acc);
     if ((threadIdx.x & 31) == 0) s_acc[threadIdx.x >> 5] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int w = 1; w < (int)(blockDim.x >> 5); ++w) acc += s_acc[w];
         atomicAdd(count, (unsigned long long)acc);
-        if (ratio) *ratio = (double)acc * invN;
     }
+    if (!ratio) return;
+    if constexpr (CS > 1) {
+        if (threadIdx.x == 0) {
+            uint32_t to;
+            asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(to) : "r"((uint32_t)__cvta_generic_to_shared(s_part + blk)));
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(to), "r"(acc) : "memory");
+        }
+        cluster_barrier();
+        if (blk == 0 && threadIdx.x == 0)
+            for (int k = 1; k < CS; ++k) acc += *(volatile unsigned *)(s_part + k);
+    }
+    if (blk == 0 && threadIdx.x == 0) *ratio = (double)acc * invN;
 }
 
-template <int NQ>
+template <int NQ, int CS>
 __global__ void __launch_bounds__(kResThreads, 1)
 ising_resident_general(uint8_t *__restrict__ spins, int N, const __grid_constant__ ResShape C, int4 stride4,
                        const uint4 *__restrict__ ent, const uint16_t *__restrict__ itype,
@@ -83,14 +100,29 @@ ising_resident_general(uint8_t *__restrict__ spins, int N, const __grid_constant
     uint32_t *s_tb = reinterpret_cast<uint32_t *>(s_raw);         // table_entries thresholds
     int2 *s_ty = reinterpret_cast<int2 *>(s_tb + ((table_entries + 1) & ~1));  // per type: base, half
     uint8_t *s_sp = reinterpret_cast<uint8_t *>(s_ty + n_types);
-    const int r = blockIdx.x;
+    const int r = blockIdx.x / CS;
+    const int blk = CS > 1 ? (int)(blockIdx.x % CS) : 0;
+    // the other block's spins, in the cluster window
+    uint32_t other = 0;
+    if constexpr (CS == 2)
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(other) : "r"((uint32_t)__cvta_generic_to_shared(s_sp)), "r"(blk ^ 1));
+    auto barrier = [] {
+        if constexpr (CS > 1) cluster_barrier();
+        else __syncthreads();
+    };
+    // this block's pairs of a colour of n sites
+    auto share = [&](int n, int &a, int &b) {
+        const int pairs = (n + 1) / 2;
+        a = pairs * blk / CS;
+        b = pairs * (blk + 1) / CS;
+    };
     uint8_t *g = spins + (size_t)r * N;
     const uint32_t *tb = thr + (size_t)slot_of_rep[r] * table_entries;
     const uint32_t stream = stream_id[r], t0 = step[r];
     for (int i = threadIdx.x; i < table_entries; i += blockDim.x) s_tb[i] = tb[i];
     for (int i = threadIdx.x; i < n_types; i += blockDim.x) s_ty[i] = make_int2(type_base[i], type_half[i]);
     for (int i = threadIdx.x; i <= N; i += blockDim.x) s_sp[i] = i < N ? g[i] : (uint8_t)0;
-    __syncthreads();
+    barrier();
     unsigned acc = 0;
     struct Next {  // a pair of sites: what does not depend on the spins
         uint4 e[2][NQ];
@@ -108,13 +140,16 @@ ising_resident_general(uint8_t *__restrict__ spins, int N, const __grid_constant
         }
         nx.hi = draw_rk((uint32_t)rho >> 3, t, stream, kMetro | ((uint32_t)col << 8), K);
     };
-    if ((int)threadIdx.x < (C.off[1] + 1) / 2) fetch(0, threadIdx.x, t0);
+    int a, b;
+    share(C.off[1], a, b);
+    if (a + (int)threadIdx.x < b) fetch(0, a + (int)threadIdx.x, t0);
     for (int k = 0; k < nsweeps; ++k) {
         const uint32_t t = t0 + (uint32_t)k;
         for (int col = 0; col < C.ncol; ++col) {
-            const int off = C.off[col], n = C.off[col + 1] - off, pairs = (n + 1) / 2;
-            for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-                if (p != (int)threadIdx.x) fetch(col, p, t);
+            const int off = C.off[col], n = C.off[col + 1] - off;
+            share(n, a, b);
+            for (int p = a + (int)threadIdx.x; p < b; p += blockDim.x) {
+                if (p != a + (int)threadIdx.x) fetch(col, p, t);
                 const int rho = 2 * p;
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
@@ -145,27 +180,25 @@ ising_resident_general(uint8_t *__restrict__ spins, int N, const __grid_constant
                     }
                     if (flip) {
                         s_sp[s] = (uint8_t)(own ^ 1);
+                        if constexpr (CS == 2)
+                            asm volatile("st.shared::cluster.u8 [%0], %1;" ::"r"(other + (uint32_t)s), "r"(own ^ 1) : "memory");
                         ++acc;
                     }
                 }
             }
             // the first pair of the next phase
             const int nc = col + 1 < C.ncol ? col + 1 : 0;
-            if ((nc || k + 1 < nsweeps) && (int)threadIdx.x < (C.off[nc + 1] - C.off[nc] + 1) / 2)
-                fetch(nc, threadIdx.x, nc ? t : t + 1);
-            __syncthreads();
+            share(C.off[nc + 1] - C.off[nc], a, b);
+            if ((nc || k + 1 < nsweeps) && a + (int)threadIdx.x < b) fetch(nc, a + (int)threadIdx.x, nc ? t : t + 1);
+            barrier();
         }
     }
-    for (int i = threadIdx.x; i < N; i += blockDim.x) g[i] = s_sp[i];
-    if (threadIdx.x == 0) step[r] = t0 + (uint32_t)nsweeps;
-    res_accepts(acc_count + r, acc, invN, ratio ? ratio + r : nullptr);
+    for (int i = blk * (int)blockDim.x + (int)threadIdx.x; i < N; i += CS * blockDim.x) g[i] = s_sp[i];
+    if (blk == 0 && threadIdx.x == 0) step[r] = t0 + (uint32_t)nsweeps;
+    res_accepts<CS>(acc_count + r, acc, invN, ratio ? ratio + r : nullptr, (int)blk);
 }
 
 // -------------------------------------------------------------------------- XYZ ----
-__device__ __forceinline__ void cluster_barrier() {
-    __syncwarp();  // .aligned: the warp arrives as one
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // The spin of a 16-bit entry: index i in block blk of the cluster.  base: this block's array in
 // the shared window; first, delta: the first block's in the cluster window, the distance to the
 // second's.
@@ -329,7 +362,7 @@ xyz_resident_general(float4 *__restrict__ spins4, int N, const __grid_constant__
         loc += b - a;
     }
     if (blk == 0 && threadIdx.x == 0) step[r] = t0 + (uint32_t)nsweeps;
-    res_accepts(acc_count + r, acc, invN, CS == 1 && ratio ? ratio + r : nullptr);
+    res_accepts<CS>(acc_count + r, acc, invN, ratio ? ratio + r : nullptr, (int)blk);
 }
 
 // ------------------------------------------------------------------------ host side ----
@@ -366,8 +399,10 @@ static size_t res_smem(const Ctx &c, int cs) {
 static const void *res_kernel(const Ctx &c, int cs) {
     const int q = c.res_q;
     if (c.model == ETHER_MODEL_ISING)
-        return q == 1 ? (const void *)ising_resident_general<1> : q == 2 ? (const void *)ising_resident_general<2>
-             : q == 3 ? (const void *)ising_resident_general<3> : (const void *)ising_resident_general<4>;
+        return cs == 1 ? (q == 1 ? (const void *)ising_resident_general<1, 1> : q == 2 ? (const void *)ising_resident_general<2, 1>
+                          : q == 3 ? (const void *)ising_resident_general<3, 1> : (const void *)ising_resident_general<4, 1>)
+                       : (q == 1 ? (const void *)ising_resident_general<1, 2> : q == 2 ? (const void *)ising_resident_general<2, 2>
+                          : q == 3 ? (const void *)ising_resident_general<3, 2> : (const void *)ising_resident_general<4, 2>);
     auto pick = [&](auto opt) -> const void * {
         constexpr int O = decltype(opt)::value;
         auto qs = [&](auto csv) -> const void * {
@@ -457,6 +492,10 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
     int cs = 0;
     if (ising) {
         if (c.N < 65535 && res_smem(c, 1) <= smem_max) cs = 1;
+        // two blocks, which both hold all spins, while all replicas still run at once and a colour is
+        // more than a round of pairs (per sweep: 30 x 34 x 38 x 60 31 us with one block, 18 with two;
+        // 23 x 21 x 19 16.6 and 9.0; 21 x 18 x 15 8.4 and 8.0; 14^3 3.4 and 3.8)
+        if (cs && 2L * c.R * 10 <= 9L * c.sm_count && res_share(c, 1, true) >= 2048) cs = 2;
     } else {
         // the smallest cluster that holds a replica; then larger ones while all replicas still run
         // at once (nine tenths of the SMs: clusters need neighbouring ones) and a block keeps 512
@@ -474,7 +513,7 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
     // over all replicas, 0.037 ns (Ising), 0.004 per slot - 0.008 (XYZ), and 3 us (4 us) a colour.
     if (cs) {
         const double waves = std::ceil((double)c.R * cs / c.sm_count), share = (double)c.N / cs, all = (double)c.N * c.R;
-        const double here = waves * share * (ising ? 1.9e-3 : (1.0e-3 + 0.1425e-3 * total) * (cs > 1 ? 1.3 : 1.0));
+        const double here = waves * share * (ising ? (cs > 1 ? 2.6e-3 : 1.9e-3) : (1.0e-3 + 0.1425e-3 * total) * (cs > 1 ? 1.3 : 1.0));
         const double there = std::max(c.ncol * (ising ? 3.0 : 4.0), all * (ising ? 0.037e-3 : std::max(0.008e-3, 0.004e-3 * total - 0.008e-3)));
         if (here > there) cs = 0;
     }
@@ -503,7 +542,8 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
             int a, b;
             res_range(c, cs, col, k, a, b);
             for (int i = a; i < b; ++i)
-                where[order[c.col_off[col] + i]] = (uint16_t)((used[k] + i - a) | (cs > 1 ? k << kResIdxBits : 0));
+                where[order[c.col_off[col] + i]] =
+                    ising ? (uint16_t)(c.col_off[col] + i) : (uint16_t)((used[k] + i - a) | (cs > 1 ? k << kResIdxBits : 0));
             used[k] += b - a;
         }
     std::vector<uint16_t> e16((size_t)c.res_q * c.N * 8, ising ? (uint16_t)c.N : (uint16_t)0);
@@ -557,7 +597,7 @@ cudaError_t launch_general_resident(Ctx &c, int nsweeps, double *ratio) {
     int4 stride4 = make_int4(c.res_stride[0], c.res_stride[1], c.res_stride[2], c.res_stride[3]);
     RoundKeys K = round_keys(c.seed);
     // full rounds of at most 1024 threads over the largest class (Ising: pairs of sites)
-    const int work = ising ? (res_share(c, 1, true) + 1) / 2 : res_share(c, cs, true);
+    const int work = ising ? ((res_share(c, 1, true) + 1) / 2 + cs - 1) / cs : res_share(c, cs, true);
     const int rounds = std::max(1, (work + kResThreads - 1) / kResThreads);
     const int threads = std::max(64, ((work + rounds - 1) / rounds + 31) / 32 * 32);
     cudaLaunchConfig_t cfg = {};
