@@ -935,7 +935,7 @@ def main():
                      "unit": "GB/s", "frac": res["achieved_gbs"] / hbm_peak,
                      "peak_source": peak_src, "traffic": traffic,
                      "kernel": ("ising_sc_kernel (one colour phase)" if model == 0
-                                else "xyz_sc_kernel (one colour phase)"),
+                                else "xyz_col_kernel (one colour phase)"),
                      "bytes_per_update": res["bytes_per_update"], "phase_ms": res["phase_ms"],
                      "autotuned_variant": res["variant"]},
         "e2e": {"value": res["e2e"], "unit": "spin updates/ns",
