@@ -45,9 +45,9 @@ constexpr int kResMaxQ = 4;      // 16-byte words of entries per site: at most 3
 constexpr int kResIdxBits = 14;  // clusters: index in the owning block's array, block above it
 
 struct ResShape {
-    int ncol, slots, nsh;        // slots: of all shells together
+    int ncol, slots;             // slots: of all shells together
     int off[kMaxColours + 1];    // first storage index of a colour
-    int shell_end[8];            // slot at which a shell's slots end
+    int stride[8 * kResMaxQ];    // Ising: stride of a slot's shell in the threshold table
 };
 // XYZ: the coupling of each slot, a kernel parameter so that every fmaf takes it as a constant.
 struct ResCouplings {
@@ -90,7 +90,7 @@ __device__ __forceinline__ void res_accepts(unsigned long long *count, unsigned 
 
 template <int NQ, int CS>
 __global__ void __launch_bounds__(kResThreads, 1)
-ising_resident_general(uint8_t *__restrict__ spins, int N, const __grid_constant__ ResShape C, int4 stride4,
+ising_resident_general(uint8_t *__restrict__ spins, int N, const __grid_constant__ ResShape C,
                        const uint4 *__restrict__ ent, const uint16_t *__restrict__ itype,
                        const int32_t *__restrict__ type_base, const int32_t *__restrict__ type_half, int n_types,
                        const uint32_t *__restrict__ thr, int table_entries, const int32_t *__restrict__ slot_of_rep,
@@ -155,18 +155,18 @@ ising_resident_general(uint8_t *__restrict__ spins, int N, const __grid_constant
                 for (int j = 0; j < 2; ++j) {
                     const int s = off + rho + j;
                     if (rho + j >= n) break;
-                    int idx = 0, sum = 0, sh = 0;
-                    // up-spins per shell; the shells' ends are uniform
+                    // table index: every up spin adds its shell's stride, a constant operand per slot
+                    // (a sum per shell with its ends tested took ten instructions a slot: pyrochlore
+                    // 6^3 cells, Ising, 17.6 us a sweep; 10.6 so; 21 x 18 x 15 8.0 and 6.5)
+                    int idx = 0;
 #pragma unroll
-                    for (int m = 0; m < 8 * NQ; ++m) {
-                        if (m >= C.slots) break;
-                        const uint4 &q = nx.e[j][m >> 3];
-                        const uint32_t w = (m & 6) == 0 ? q.x : (m & 6) == 2 ? q.y : (m & 6) == 4 ? q.z : q.w;
-                        sum += s_sp[(m & 1) ? w >> 16 : w & 0xFFFFu];
-                        if (m + 1 == C.shell_end[sh]) {
-                            idx += sum * (sh == 0 ? stride4.x : sh == 1 ? stride4.y : sh == 2 ? stride4.z : stride4.w);
-                            sum = 0;
-                            ++sh;
+                    for (int e = 0; e < NQ; ++e) {
+                        if (8 * e >= C.slots) break;  // uniform; also keeps the loads of a word together
+                        const uint4 &q = nx.e[j][e];
+#pragma unroll
+                        for (int m = 0; m < 8; ++m) {
+                            const uint32_t w = (m & 6) == 0 ? q.x : (m & 6) == 2 ? q.y : (m & 6) == 4 ? q.z : q.w;
+                            idx += (int)s_sp[(m & 1) ? w >> 16 : w & 0xFFFFu] * C.stride[8 * e + m];
                         }
                     }
                     const int own = s_sp[s];
@@ -461,6 +461,7 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
                            std::vector<uint4> &ent, std::vector<int32_t> &order) {
     c.gen_resident = 0;
     const bool ising = c.model == ETHER_MODEL_ISING;
+    if (c.N >= 65535) return;  // 16-bit entries; four blocks' shared memory holds fewer XYZ spins still
     if ((c.fast && ising) || c.nsp != 1 || c.nsh < 1 || c.nsh > (ising ? 4 : 8)) return;
     std::vector<int> slots(c.nsh, 0), count(c.nsh);
     std::vector<int> stride(c.nsh, 0);
@@ -493,8 +494,9 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
     if (ising) {
         if (c.N < 65535 && res_smem(c, 1) <= smem_max) cs = 1;
         // two blocks, which both hold all spins, while all replicas still run at once and a colour is
-        // more than a round of pairs (per sweep: 30 x 34 x 38 x 60 31 us with one block, 18 with two;
-        // 23 x 21 x 19 16.6 and 9.0; 21 x 18 x 15 8.4 and 8.0; 14^3 3.4 and 3.8)
+        // more than a round of pairs (per sweep, before the slots' constant strides: 30 x 34 x 38 x 60
+        // 31 us with one block, 18 with two; 23 x 21 x 19 16.6 and 9.0; 21 x 18 x 15 8.4 and 8.0; 14^3
+        // 3.4 and 3.8)
         if (cs && 2L * c.R * 10 <= 9L * c.sm_count && res_share(c, 1, true) >= 2048) cs = 2;
     } else {
         // the smallest cluster that holds a replica; then larger ones while all replicas still run
@@ -509,11 +511,12 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
     }
     // Against the phase kernels: a replica's sweep here takes its sites' time in turn, theirs the
     // whole context's work over the GPU but at least a launch's latency per colour.  Measured per
-    // site: here 1.9 ns (Ising), 1.0 + 0.1425 per slot (XYZ; 1.3 times that in a cluster); there,
+    // site: here 0.3 ns + 0.07 per slot, and 1 us a colour (Ising), 1.0 + 0.1425 per slot (XYZ; 1.3 times that in a cluster); there,
     // over all replicas, 0.037 ns (Ising), 0.004 per slot - 0.008 (XYZ), and 3 us (4 us) a colour.
     if (cs) {
         const double waves = std::ceil((double)c.R * cs / c.sm_count), share = (double)c.N / cs, all = (double)c.N * c.R;
-        const double here = waves * share * (ising ? (cs > 1 ? 2.6e-3 : 1.9e-3) : (1.0e-3 + 0.1425e-3 * total) * (cs > 1 ? 1.3 : 1.0));
+        const double here = ising ? 1.0 * c.ncol + waves * share * (0.3e-3 + 0.07e-3 * total)
+                                  : waves * share * (1.0e-3 + 0.1425e-3 * total) * (cs > 1 ? 1.3 : 1.0);
         const double there = std::max(c.ncol * (ising ? 3.0 : 4.0), all * (ising ? 0.037e-3 : std::max(0.008e-3, 0.004e-3 * total - 0.008e-3)));
         if (here > there) cs = 0;
     }
@@ -591,10 +594,11 @@ cudaError_t launch_general_resident(Ctx &c, int nsweeps, double *ratio) {
     ResShape C;
     C.ncol = c.ncol;
     C.slots = c.res_slots;
-    C.nsh = c.nsh;
     for (int col = 0; col <= c.ncol; ++col) C.off[col] = col < c.ncol ? c.col_off[col] : c.N;
-    for (int sh = 0; sh < 8; ++sh) C.shell_end[sh] = sh < c.nsh ? c.res_shell_end[sh] : -1;
-    int4 stride4 = make_int4(c.res_stride[0], c.res_stride[1], c.res_stride[2], c.res_stride[3]);
+    for (int m = 0, sh = 0; m < 8 * kResMaxQ; ++m) {
+        if (m < c.res_slots && m >= c.res_shell_end[sh]) ++sh;
+        C.stride[m] = m < c.res_slots ? c.res_stride[sh] : 0;
+    }
     RoundKeys K = round_keys(c.seed);
     // full rounds of at most 1024 threads over the largest class (Ising: pairs of sites)
     const int work = ising ? ((res_share(c, 1, true) + 1) / 2 + cs - 1) / cs : res_share(c, cs, true);
@@ -614,7 +618,7 @@ cudaError_t launch_general_resident(Ctx &c, int nsweeps, double *ratio) {
     c.launches++;
     double invN = 1.0 / (double)c.N;
     if (ising) {
-        void *args[] = {&c.spins, &c.N, &C, &stride4, &c.t.res_ent, &c.t.itype, &c.t.type_base, &c.t.type_half,
+        void *args[] = {&c.spins, &c.N, &C, &c.t.res_ent, &c.t.itype, &c.t.type_base, &c.t.type_half,
                         &c.n_types, &c.thr, &c.table_entries, &c.slot_of_rep, &c.stream_id, &c.step, &K, &nsweeps,
                         &c.acc_count, &invN, &ratio};
         return cudaLaunchKernelExC(&cfg, res_kernel(c, cs), args);
