@@ -255,8 +255,10 @@ __host__ __device__ __forceinline__ uint32_t class_bits(uint32_t a0, uint32_t a2
 constexpr uint32_t kEvenRows = 0xA5A5u;  // bit b + 4 c set where b + c is even
 
 __global__ void __launch_bounds__(256) gather_kernel(const PatchParams P) {
+    after_release();
     const int w = blockIdx.x * 256 + threadIdx.x;
     if (w >= P.n) return;
+    after_wait();
     const Patch D = decode(P, w);
     const uint8_t *sp = P.spins + (long long)D.r * 2 * P.half;
     const bool rev = D.par != 0;
@@ -334,6 +336,7 @@ __global__ void __launch_bounds__(kGroups * kThreads, 1) patch_kernel(const Patc
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base + SM_BAR + 8 * kGroups);
     const int group = threadIdx.x >> 7, tid = threadIdx.x & 127, warp = tid >> 5;
     bar += group;
+    after_release();
 
     // weights and biases into shared memory (plain 16-byte copies; the image is pre-swizzled)
     {
@@ -369,6 +372,7 @@ __global__ void __launch_bounds__(kGroups * kThreads, 1) patch_kernel(const Patc
     uint32_t phase = 0;
     bool ok = true;
 
+    after_wait();  // the gathered bits
     const int ntiles = (P.n + kThreads - 1) / kThreads;
     for (int tile = blockIdx.x + group * gridDim.x; tile < ntiles && ok; tile += kGroups * gridDim.x) {
         const int w = tile * kThreads + tid;
@@ -577,6 +581,8 @@ __device__ __forceinline__ int edge_sum(uint32_t A, const Faces &F) {
 // d = log q(new) - log q(old): A-sites that changed add +-z_k (log-odds), then the B-sites'
 // heat-bath log probabilities (tables); log alpha = (0 - d) - beta J dB.
 __global__ void __launch_bounds__(128, 8) mh_kernel(const PatchParams P) {
+    after_release();
+    after_wait();
     if (*P.err) return;  // a network pass that gave up leaves the state as it was
     const bool valid = blockIdx.x * 128 + threadIdx.x < P.n;
     const int w = valid ? blockIdx.x * 128 + threadIdx.x : P.n - 1;
@@ -908,9 +914,9 @@ int launch_patches(ether_learn &l, int cls, float *dump) {
         P.n = std::min(per, l.R - r0) * (int)l.Pc;
         P.dump = dump ? dump + (size_t)r0 * l.Pc * NO : nullptr;
         const int tiles = (P.n + kThreads - 1) / kThreads;
-        gather_kernel<<<(P.n + 255) / 256, 256, 0, c.stream>>>(P);
-        patch_kernel<0><<<std::min(tiles, l.sm_count), kGroups * kThreads, SM_BYTES + 1024, c.stream>>>(P);
-        mh_kernel<<<(P.n + 127) / 128, 128, 0, c.stream>>>(P);
+        LCUDA(launch_after(gather_kernel, (P.n + 255) / 256, 256, 0, c.stream, true, P));
+        LCUDA(launch_after(patch_kernel<0>, std::min(tiles, l.sm_count), kGroups * kThreads, SM_BYTES + 1024, c.stream, true, P));
+        LCUDA(launch_after(mh_kernel, (P.n + 127) / 128, 128, 0, c.stream, true, P));
         l.launches += 3;
     }
     LCUDA(cudaGetLastError());

@@ -256,6 +256,7 @@ __device__ __forceinline__ void xinput_row(const XPatchParams &P, const float4 *
 
 // Network inputs of the patches of one pass (one warp per patch).
 __global__ void __launch_bounds__(256) xinputs_kernel(XPatchParams P, __nv_bfloat16 *__restrict__ X) {
+    after_wait();
     const int lane = threadIdx.x & 31;
     const int nwarps = (int)gridDim.x * (int)(blockDim.x >> 5);
     const int total = P.nrep * (int)P.Pc;
@@ -265,6 +266,7 @@ __global__ void __launch_bounds__(256) xinputs_kernel(XPatchParams P, __nv_bfloa
         const float beta = P.beta_slot_f[P.slot_of_rep[D.r]];
         xinput_row(P, sp, D.o0, D.o1, D.o2, D.par, beta, X + (size_t)w * XNI, lane);
     }
+    after_release();  // not before: the network's shared memory would take this kernel's L1
 }
 
 // Training samples (one warp each): per replica a random offset and patch, its input row
@@ -331,6 +333,7 @@ __global__ void __launch_bounds__(256, 4) xpatch_kernel(XPatchParams P, const fl
             ++n;
         }
     }
+    after_wait();
     if (k == 0) ss[128] = make_float4(0.f, 0.f, 0.f, 0.f);
     const int nwarps = (int)gridDim.x * (int)(blockDim.x >> 5);
     const int total = P.nrep * (int)P.Pc;
@@ -404,6 +407,7 @@ __global__ void __launch_bounds__(256, 4) xpatch_kernel(XPatchParams P, const fl
             if (k == 0) atomicAdd(acc + D.r, 1ull);
         }
     }
+    after_release();
 }
 
 // ------------------------------------------------------------ inference network ----
@@ -555,11 +559,14 @@ xmlp_kernel(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict_
                          tc::smem_u32(base)),
                      "l"(img), "r"(XIMG_BYTES), "r"(tc::smem_u32(bar_w))
                      : "memory");
+        after_release();
+        after_wait();  // the inputs
         if ((int)blockIdx.x < ntiles) {
             load_x(blockIdx.x);
             x_pending = true;
         }
     }
+    after_wait();
     const bool w_got = tc::mbar_wait(tc::smem_u32(bar_w), 0, err, 7);
     ok = __syncthreads_and(w_got ? 1 : 0) != 0;
     for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
@@ -712,6 +719,7 @@ XPatchParams patch_params(const XyzLearn &x, int cls, int r0, int nrep) {
     return P;
 }
 
+bool close_pass(const XyzLearn &x, long long patches) { return patches <= 64LL * x.sm_count; }
 int warp_grid(const XyzLearn &x, long long warps) {
     return (int)std::max<long long>(1, std::min<long long>((warps + 7) / 8, 8LL * x.sm_count));
 }
@@ -752,7 +760,7 @@ int infer_rows(XyzLearn &x, cudaStream_t st, int M, const __nv_bfloat16 *Xh, flo
         return xfail(ETHER_ERR_CUDA, "learned proposal: cuTensorMapEncodeTiled failed");
     XCUDA(cudaFuncSetAttribute(xmlp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, XSM_BYTES));
     const int ntiles = (M + 127) / 128;
-    xmlp_kernel<<<std::min(ntiles, x.sm_count), kXmlpThreads, XSM_BYTES, st>>>(map, x.ximg, Z, M, x.err);
+    XCUDA(launch_after(xmlp_kernel, std::min(ntiles, x.sm_count), kXmlpThreads, XSM_BYTES, st, close_pass(x, M), map, x.ximg, Z, M, x.err));
     x.launches++;
     XCUDA(cudaGetLastError());
     return ETHER_OK;
@@ -774,6 +782,9 @@ int xread_err(XyzLearn &x) {
 
 // One class of a learned sweep, in passes of whole replicas: network inputs, the network, the
 // Metropolis-Hastings step.
+// Passes of one patch a warp at most launch their kernels closely (16 x 8 x 40 x 35: 84 -> 69 us a
+// step).  Larger ones do not: an SM that never empties keeps the network's division between shared
+// memory and L1, and the gathers then run with hardly any L1 (64^3 x 64: 8.2 -> 9.9 ms per ten steps).
 int class_pass(XyzLearn &x, int cls, float *dump) {
     Ctx &c = x.ctx->c;
     cudaStream_t st = c.stream;
@@ -782,10 +793,10 @@ int class_pass(XyzLearn &x, int cls, float *dump) {
         const int nrep = std::min(per, x.R - r0);
         const XPatchParams P = patch_params(x, cls, r0, nrep);
         const long long M = (long long)nrep * x.Pc;
-        xinputs_kernel<<<warp_grid(x, M), 256, 0, st>>>(P, x.Xh);
+        XCUDA(launch_after(xinputs_kernel, warp_grid(x, M), 256, 0, st, close_pass(x, M), P, x.Xh));
         int rc = infer_rows(x, st, (int)M, x.Xh, x.Zi);
         if (rc) return rc;
-        xpatch_kernel<<<warp_grid(x, M), 256, 0, st>>>(P, x.Zi, x.pq + XOFF_B3, dump, x.acc);
+        XCUDA(launch_after(xpatch_kernel, warp_grid(x, M), 256, 0, st, close_pass(x, M), P, x.Zi, x.pq + XOFF_B3, dump, x.acc));
         x.launches += 2;
         XCUDA(cudaGetLastError());
     }

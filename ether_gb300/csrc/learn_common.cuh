@@ -53,6 +53,27 @@ __host__ __device__ inline void geo_bnd(int i, int &a, int &b, int &c) {
 
 __global__ void advance_lstep_kernel(uint32_t *c, int R);
 
+// The kernels of a class follow one another closely: each lets the next one start while it runs
+// (after_release), and reads what the one before it wrote only when that has ended
+// (after_wait).  What lies before the wait -- a network's weights, a patch's position -- overlaps,
+// and so does the launch.  close = false: an ordinary launch.
+__device__ __forceinline__ void after_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void after_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, bool close, A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = close ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // ------------------------------------------------ the Heisenberg learner (k_learn_xyz.cu) ----
 struct XyzLearn;
 int xyz_create(ether_ctx *h, const ether_learn_desc *d, XyzLearn **out);
