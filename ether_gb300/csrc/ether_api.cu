@@ -588,7 +588,7 @@ extern "C" int ether_create(const ether_desc *d, ether_ctx **out) {
     TRY(dev_alloc(c, &c.swap_dev, 1));
     TRY(dev_alloc(c, &c.acc_before, c.R));
     TRY(dev_alloc(c, &c.acc_ratio, c.R));
-    TRY(dev_alloc(c, &c.obs_done, c.R));
+    TRY(dev_alloc(c, &c.obs_done, (size_t)c.R + 1));
     TRY(dev_alloc(c, &c.acc_slot, c.R));
     TRY(dev_alloc(c, &c.acc_mark, c.R));
     CUDA_TRY(cudaMallocHost((void **)&c.acc_host, sizeof(double) * 3 * c.R));
@@ -600,7 +600,7 @@ extern "C" int ether_create(const ether_desc *d, ether_ctx **out) {
     CUDA_TRY(cudaMemset(c.step, 0, sizeof(uint32_t) * c.R));
     CUDA_TRY(cudaMemset(c.ovrr_step, 0, sizeof(uint32_t) * c.R));
     CUDA_TRY(cudaMemset(c.fresh_call, 0, sizeof(uint32_t) * c.R));
-    CUDA_TRY(cudaMemset(c.obs_done, 0, sizeof(uint32_t) * c.R));
+    CUDA_TRY(cudaMemset(c.obs_done, 0, sizeof(uint32_t) * ((size_t)c.R + 1)));
     CUDA_TRY(cudaMemset(c.acc_count, 0, sizeof(unsigned long long) * c.R));
     CUDA_TRY(cudaMemset(c.acc_slot, 0, sizeof(unsigned long long) * c.R));
     CUDA_TRY(cudaMemset(c.acc_mark, 0, sizeof(unsigned long long) * c.R));

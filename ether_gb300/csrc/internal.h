@@ -129,7 +129,7 @@ struct Ctx {
     bool resident = false;       // ether_mcs runs runs of sweeps with ising_sc_resident
     unsigned long long *acc_before = nullptr;  // R: acceptance counts at the start of a call
     double *acc_ratio = nullptr;               // R: device acceptance ratios of a call
-    uint32_t *obs_done = nullptr;              // R: finished blocks of an energy reduction (zero between launches)
+    uint32_t *obs_done = nullptr;              // R + 1: finished blocks of a reduction, recorded replicas (zero between launches)
     double *acc_host = nullptr;                // 3 R: pinned host copy of a call's results
     void *stage = nullptr;                     // pinned staging of ether_{set,get}_spins_batch
     bool ion_direct = false;                   // the device reads / writes the host records in place

@@ -403,6 +403,27 @@ __device__ __forceinline__ void finish_block(const double *__restrict__ partials
     }
 }
 
+// Row of a time series: |M| (and E) of every replica at row t, or at the row *t_dev (graph replays),
+// which the last replica to be written moves on.
+struct RecordRow {
+    double *m, *e;     // series, null: not recorded
+    int t;
+    int32_t *t_dev;
+};
+// By one thread, once the replica's M (and E) are summed; done: a counter of replicas.
+__device__ __forceinline__ void record_replica(const RecordRow &row, int R, int r, double mx, double my, double mz,
+                                               double e, uint32_t *done) {
+    const int t = row.t_dev ? *(volatile int32_t *)row.t_dev : row.t;
+    row.m[(size_t)t * R + r] = sqrt(mx * mx + my * my + mz * mz);
+    if (row.e) row.e[(size_t)t * R + r] = e;
+    if (!row.t_dev) return;
+    __threadfence();
+    if (atomicAdd(done, 1u) == (uint32_t)R - 1u) {
+        *done = 0u;
+        *row.t_dev = t + 1;
+    }
+}
+
 // One block per (replica, energy block); the block of a replica that ends last sums the
 // replica's partials and, with `measure`, adds them to the accumulators.  done[r] counts the
 // blocks that have written theirs and is zero again when the launch ends.  host_e, host_m: pinned
@@ -411,7 +432,7 @@ __device__ __forceinline__ void finish_block(const double *__restrict__ partials
 // takes 3 us at 16^3 x 190.)
 template <int FORM>
 __global__ void __launch_bounds__(kRedBs, 4) energy_mag_kernel(const ObsMember a, uint32_t *__restrict__ done, int measure,
-                                                                double *host_e, double *host_m) {
+                                                                double *host_e, double *host_m, const RecordRow row) {
     const int r = blockIdx.y;
     energy_block<FORM>(a, r, blockIdx.x);
     __shared__ int s_last;
@@ -430,6 +451,7 @@ __global__ void __launch_bounds__(kRedBs, 4) energy_mag_kernel(const ObsMember a
         if (host_e) host_e[r] = a.E[r];
         if (host_m)
             for (int j = 0; j < 3; ++j) host_m[3 * r + j] = a.M[3 * r + j];
+        if (row.m) record_replica(row, a.R, r, a.M[3 * r], a.M[3 * r + 1], a.M[3 * r + 2], a.E[r], done + a.R);
     }
 }
 
@@ -579,22 +601,24 @@ ObsMember obs_member(const Ctx &c) {
     return a;
 }
 
-cudaError_t launch_energy_mag(Ctx &c, bool measure, double *host_e, double *host_m) {
+static cudaError_t launch_energy(Ctx &c, bool measure, double *host_e, double *host_m, const RecordRow &row) {
     dim3 grid(c.partial_blocks, c.R);
     const ObsMember a = obs_member(c);
     const int form = obs_form(a);
     auto k = form == kObsIsing ? energy_mag_kernel<kObsIsing> : form == kObsCubic ? energy_mag_kernel<kObsCubic>
                                                                                    : energy_mag_kernel<kObsGeneral>;
-    k<<<grid, kRedBs, 0, c.stream>>>(a, c.obs_done, measure ? 1 : 0, host_e, host_m);
+    k<<<grid, kRedBs, 0, c.stream>>>(a, c.obs_done, measure ? 1 : 0, host_e, host_m, row);
     c.launches++;
     return cudaGetLastError();
+}
+cudaError_t launch_energy_mag(Ctx &c, bool measure, double *host_e, double *host_m) {
+    return launch_energy(c, measure, host_e, host_m, RecordRow{nullptr, nullptr, 0, nullptr});
 }
 
 // Magnetisation only (src/get_tot_magnetisation.f90:32-40), no neighbour reads: per-block
 // partial sums of w_s S_s into partials[(r*nblk + b)*kNq + 2..4], summed per thread and
 // warp as energy_block sums them (so the two give the same M).
-__global__ void __launch_bounds__(kRedBs) mag_kernel(const ObsMember a) {
-    const int r = blockIdx.y;
+__device__ __forceinline__ void mag_block(const ObsMember &a, int r) {
     const int N = a.N;
     const int stride = gridDim.x * blockDim.x;
     double q[3] = {0, 0, 0};
@@ -663,53 +687,38 @@ __global__ void __launch_bounds__(kRedBs) mag_kernel(const ObsMember a) {
     }
     block_sum_mixed<3>(q, qd, form == kFormDS ? 3 : 0, out);
 }
-
-// One row t of the time series: |M| (and E) of every replica.  from_partials: M is summed
-// here from mag_kernel's partials (in block order); otherwise M and E come from the last
-// energy / magnetisation reduction.
-__global__ void record_kernel(const double *__restrict__ partials, int nblk, int R,
-                              int from_partials, double *__restrict__ M,
-                              const double *__restrict__ E, double *__restrict__ mser,
-                              double *__restrict__ eser, int t_arg, const int32_t *__restrict__ t_dev) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= R) return;
-    const int t = t_dev ? *t_dev : t_arg;  // t_dev: the row from device memory (graph replays)
-    double m[3];
-    if (from_partials) {
-        m[0] = m[1] = m[2] = 0.0;
-        for (int b = 0; b < nblk; ++b)
-            for (int j = 0; j < 3; ++j) m[j] += partials[((size_t)r * nblk + b) * kNq + 2 + j];
-        for (int j = 0; j < 3; ++j) M[3 * r + j] = m[j];
-    } else {
-        for (int j = 0; j < 3; ++j) m[j] = M[3 * r + j];
+// The block of a replica that ends last sums its partials in block order and records the row.
+__global__ void __launch_bounds__(kRedBs) mag_kernel(const ObsMember a, uint32_t *__restrict__ done, const RecordRow row) {
+    const int r = blockIdx.y;
+    mag_block(a, r);
+    __shared__ int s_last;
+    __shared__ double s_m[3];
+    if (threadIdx.x < 32) {  // the partials' writers are in the first warp
+        __threadfence();
+        __syncwarp();
+        if (threadIdx.x == 0) s_last = atomicAdd(done + r, 1u) == gridDim.x - 1u;
     }
-    mser[(size_t)t * R + r] = sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
-    if (eser) eser[(size_t)t * R + r] = E[r];
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x < 3) {
+        double v = 0.0;
+        for (int b = 0; b < (int)gridDim.x; ++b) v += __ldcg(&a.partials[((size_t)r * gridDim.x + b) * kNq + 2 + threadIdx.x]);
+        a.M[3 * r + threadIdx.x] = s_m[threadIdx.x] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        done[r] = 0u;
+        record_replica(row, a.R, r, s_m[0], s_m[1], s_m[2], 0.0, done + a.R);
+    }
 }
 
-// The next row of a series whose row index lives in device memory.
-__global__ void record_bump_kernel(int32_t *__restrict__ t_dev) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *t_dev += 1;
-}
-
+// One row of the time series, in the reduction's own launch.
 cudaError_t launch_record(Ctx &c, int t, bool want_e, double *mser, double *eser, int32_t *t_dev) {
-    if (want_e) {
-        cudaError_t e = launch_energy_mag(c, false);
-        if (e != cudaSuccess) return e;
-        record_kernel<<<(c.R + 127) / 128, 128, 0, c.stream>>>(c.partials, c.partial_blocks, c.R, 0,
-                                                                c.M, c.E, mser, eser, t, t_dev);
-        c.launches++;
-    } else {
-        dim3 grid(c.partial_blocks, c.R);
-        mag_kernel<<<grid, kRedBs, 0, c.stream>>>(obs_member(c));
-        record_kernel<<<(c.R + 127) / 128, 128, 0, c.stream>>>(c.partials, c.partial_blocks, c.R, 1,
-                                                                c.M, c.E, mser, nullptr, t, t_dev);
-        c.launches += 2;
-    }
-    if (t_dev) {
-        record_bump_kernel<<<1, 32, 0, c.stream>>>(t_dev);
-        c.launches++;
-    }
+    const RecordRow row{mser, want_e ? eser : nullptr, t, t_dev};
+    if (want_e) return launch_energy(c, false, nullptr, nullptr, row);
+    mag_kernel<<<dim3(c.partial_blocks, c.R), kRedBs, 0, c.stream>>>(obs_member(c), c.obs_done, row);
+    c.launches++;
     return cudaGetLastError();
 }
 
