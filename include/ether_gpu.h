@@ -61,9 +61,9 @@ enum {
                                           instead of exchanging the two                     */
     ETHER_FLAG_NO_GRAPHS = 1 << 3,        /* ether_mcs launches kernels one by one instead of
                                           replaying captured CUDA graphs                    */
-    ETHER_FLAG_NO_RESIDENT = 1 << 4,      /* ether_mcs never runs a small simple-cubic Ising
-                                          lattice's sweeps in the shared-memory resident
-                                          kernel (same results, one launch per phase)        */
+    ETHER_FLAG_NO_RESIDENT = 1 << 4,      /* no call runs a small lattice's sweeps in the
+                                          shared-memory resident kernels (same results, one
+                                          launch per phase)                                  */
     ETHER_FLAG_STAGED_SPINS = 1 << 5      /* ether_{set,get}_spins_batch convert on the host's
                                           cores through pinned staging even where the device
                                           could read and write the ion records in place
@@ -266,7 +266,8 @@ int ether_end_sweep(ether_ctx *ctx);
  * 5015, 5021, 5022 run as 5011.  best_ms = one colour phase.  Either
  * output may be NULL. */
 int ether_autotune(ether_ctx *ctx, int32_t *variant, float *best_ms);
-/* Force a kernel variant (same encoding as ether_autotune). */
+/* Force a kernel variant (same encoding as ether_autotune); single calls then run its phase
+ * kernels even where a small lattice's sweeps would stay in shared memory. */
 int ether_set_variant(ether_ctx *ctx, int32_t variant);
 
 /* structure_factor (utility/Structure_Factor/structure_factor.f90:99-183) of every replica's
