@@ -1147,9 +1147,16 @@ static int sweeps_by_phase(Ctx &c, int n) {
 }
 static int sweep_once(Ctx &c) { return sweeps_by_phase(c, 1); }
 
+// Do n sweeps of a simple-cubic Ising context run in shared memory?  Short runs of many sites do
+// not: loading and storing them costs more than the two phases (a sweep and its recorded row,
+// 16 x 52 x 16 x 722: 38 us in shared memory, 33 by phases; 16^3 x 1024 26 and 27).
+static bool ising_resident_runs(const Ctx &c, int n) {
+    return c.resident && !c.variant_asked && (n >= 4 || (long)c.R * c.N <= (4L << 20) + (1L << 18));
+}
+
 // n sweeps: in the launches of a resident kernel (of at most 256 sweeps each) or phase by phase.
 int ether::plain_sweeps(Ctx &c, int n) {
-    const bool resident = c.resident && !c.variant_asked;
+    const bool resident = ising_resident_runs(c, n);
     if (!resident && !general_resident(c)) return sweeps_by_phase(c, n);
     for (int k = 0; k < n; k += 256) {
         const int m = std::min(256, n - k);
@@ -1211,7 +1218,7 @@ extern "C" int ether_metropolis(ether_ctx *h, int32_t nsweeps, double *accept) {
     Ctx &c = h->c;
     if (nsweeps < 0) return fail(ETHER_ERR_ARG, "negative sweep count");
     if (!c.beta_set) return fail(ETHER_ERR_STATE, "beta not set (ether_set_beta / ether_set_ladder)");
-    const bool resident = c.resident && !c.variant_asked, general = general_resident(c);
+    const bool resident = ising_resident_runs(c, nsweeps), general = general_resident(c);
     if ((resident || general) && nsweeps >= 1 && nsweeps <= 256) {
         // one launch, which writes the acceptance into pinned host memory
         double *ratio = accept ? c.acc_host : nullptr;

@@ -436,7 +436,7 @@ static long res_arrange(const Ctx &c, int cs, int period, const std::vector<int3
             for (int i = a; i < b; ++i) pos[o[i]] = used[k] + i - a;
             used[k] += b - a;
         }
-    const int step = 8 * std::max(1, c.N / 4096);  // about 512 groups of eight lanes
+    const int step = 8 * std::max(1, c.N / 1024);  // about 128 groups of eight lanes
     long cost = 0;
     for (int i = 0; i + 8 <= c.N; i += step)
         for (int m = 0; m < c.res_slots; ++m) {
