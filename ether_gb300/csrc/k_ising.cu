@@ -2,6 +2,7 @@
 #include <algorithm>
 
 #include "measure.cuh"
+#include "shared_limit.h"
 #include "sweep_ising.cuh"
 
 namespace ether {
@@ -434,16 +435,12 @@ static ResidentKernel resident_kernel(const Ctx &c, int W) {
     return W == 16 ? resident_kernel<16, MEASURE>(n) : W == 8 ? resident_kernel<8, MEASURE>(n) : resident_kernel<4, MEASURE>(n);
 }
 
-// Opts the kernels of every vector width into the shared memory a replica needs (once, at
-// creation: not during a stream capture); never below what another context asked for.
+// Opts the kernels of every vector width into shared memory (once, at creation: not during a
+// stream capture).
 cudaError_t prepare_ising_resident(const Ctx &c) {
-    const int smem = c.L[0] * c.L[1] * c.L[2];
     for (int k = 0; k < 6; ++k) {
         const ResidentKernel kern = k & 1 ? resident_kernel<true>(c, 4 << (k >> 1)) : resident_kernel<false>(c, 4 << (k >> 1));
-        cudaFuncAttributes fa;
-        cudaError_t e = cudaFuncGetAttributes(&fa, kern);
-        if (e == cudaSuccess && smem > fa.maxDynamicSharedSizeBytes)
-            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const cudaError_t e = allow_shared((const void *)kern);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

@@ -35,6 +35,7 @@
 #include <type_traits>
 #include <utility>
 
+#include "shared_limit.h"
 #include "sweep_ising.cuh"
 #include "sweep_xyz.cuh"
 
@@ -577,15 +578,7 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
 }
 
 // Opts the context's kernel into its shared memory (once, at creation: not during a capture).
-cudaError_t prepare_general_resident(const Ctx &c) {
-    const void *k = res_kernel(c, c.gen_resident);
-    cudaFuncAttributes fa;
-    cudaError_t e = cudaFuncGetAttributes(&fa, k);
-    if (e != cudaSuccess) return e;
-    const int want = (int)res_smem(c, c.gen_resident);  // never lower what another context asked for
-    return want > fa.maxDynamicSharedSizeBytes
-               ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, want) : cudaSuccess;
-}
+cudaError_t prepare_general_resident(const Ctx &c) { return allow_shared(res_kernel(c, c.gen_resident)); }
 
 cudaError_t launch_general_resident(Ctx &c, int nsweeps, double *ratio) {
     if (nsweeps < 1) return cudaSuccess;

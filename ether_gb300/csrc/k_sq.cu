@@ -42,6 +42,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "shared_limit.h"
 #include "tc_util.cuh"
 
 namespace ether {
@@ -464,7 +465,7 @@ int structure_factor_launch(Ctx &c, const double *frac /*3N, storage order*/, co
         const int stage_bytes = 2 * Smem::a_bytes + (ising ? 1 : 2) * BN * kBK * 2;
         const int smem = 1024 + kStages * stage_bytes + 64;
         auto kern = ising ? sq_kernel<true> : sq_kernel<false>;
-        SQ_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        SQ_TRY(allow_shared((const void *)kern));
         const int tiles = (int)(Q / 64);
         cudaEvent_t ev0, ev1;
         SQ_TRY(cudaEventCreate(&ev0));
