@@ -255,10 +255,10 @@ __host__ __device__ __forceinline__ uint32_t class_bits(uint32_t a0, uint32_t a2
 constexpr uint32_t kEvenRows = 0xA5A5u;  // bit b + 4 c set where b + c is even
 
 __global__ void __launch_bounds__(256) gather_kernel(const PatchParams P) {
-    after_release();
     const int w = blockIdx.x * 256 + threadIdx.x;
     if (w >= P.n) return;
     after_wait();
+    after_release();  // not before the wait: patch_kernel reads the weights before its own
     const Patch D = decode(P, w);
     const uint8_t *sp = P.spins + (long long)D.r * 2 * P.half;
     const bool rev = D.par != 0;

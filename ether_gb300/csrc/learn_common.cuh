@@ -56,7 +56,9 @@ __global__ void advance_lstep_kernel(uint32_t *c, int R);
 // The kernels of a class follow one another closely: each lets the next one start while it runs
 // (after_release), and reads what the one before it wrote only when that has ended
 // (after_wait).  What lies before the wait -- a network's weights, a patch's position -- overlaps,
-// and so does the launch.  close = false: an ordinary launch.
+// and so does the launch.  Only the wait makes an earlier kernel's writes visible, so a class's
+// first kernel, which may follow the one that packed the weights, releases the network's kernel
+// after its own wait.  close = false: an ordinary launch.
 __device__ __forceinline__ void after_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void after_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class... P, class... A>
