@@ -1129,7 +1129,9 @@ extern "C" int ether_fresh_spins(ether_ctx *h) {
     return ETHER_OK;
 }
 
-// Does the context's resident sweep of k_resident.cu run?
+// Does the context's resident sweep of k_resident.cu run in a single call?  (A variant that was
+// named is a phase kernel's.  ether_mcs asks neither this nor ising_resident_runs: its route, and so
+// its graphs, depend on the context alone.)
 static bool general_resident(const Ctx &c) { return c.gen_resident && !(c.fast && c.variant_asked); }
 
 // n sweeps phase by phase; the counters are advanced once, after the last (a launch less per sweep).
@@ -1523,7 +1525,7 @@ static int issue_steps(Ctx &c, const ether_schedule *sch, const int8_t *sig, int
         }
         return ETHER_OK;
     }
-    if (!c.resident && !general_resident(c)) {
+    if (!c.resident && !c.gen_resident) {
         for (int k = 0; k < n;) {
             int rc = mcs_before_sweep(c, sch, sig[k]);
             if (rc) return rc;
@@ -1593,7 +1595,7 @@ extern "C" int ether_mcs(ether_ctx *h, const ether_schedule *sch, int32_t step0,
     int chunk = mcs_chunk(period);
     // resident contexts: the longest multiple of the period up to 256 steps, so that the
     // eventless stretches (equilibration) run as few long resident launches
-    if ((c.resident || general_resident(c)) && period <= 256) chunk = (int)(256 / period * period);
+    if ((c.resident || c.gen_resident) && period <= 256) chunk = (int)(256 / period * period);
     const bool use_graphs = !(c.flags & ETHER_FLAG_NO_GRAPHS);
     int step = step0 + 1;
     const int last = step0 + nsteps;

@@ -267,7 +267,8 @@ int ether_end_sweep(ether_ctx *ctx);
  * output may be NULL. */
 int ether_autotune(ether_ctx *ctx, int32_t *variant, float *best_ms);
 /* Force a kernel variant (same encoding as ether_autotune); single calls then run its phase
- * kernels even where a small lattice's sweeps would stay in shared memory. */
+ * kernels even where a small lattice's sweeps would stay in shared memory.  ether_mcs keeps such
+ * a lattice in shared memory all the same (ETHER_FLAG_NO_RESIDENT: never). */
 int ether_set_variant(ether_ctx *ctx, int32_t variant);
 
 /* structure_factor (utility/Structure_Factor/structure_factor.f90:99-183) of every replica's
