@@ -963,12 +963,14 @@ static int spins_batch(Ctx &c, int32_t r0, int32_t n, double *ion, bool to_devic
     // a small call goes through the kernel alone: its threads and staging cost the shared form
     // about 1.2 ms whatever the size
     if (sizeof(double) * 9 * (size_t)c.N * n <= kKernelOnlyBytes) {
-        const cudaError_t e = launch_ion_copy(c, r0, n, ion, to_device);
-        const cudaError_t e2 = e == cudaSuccess ? cudaStreamSynchronize(c.stream) : e;
-        if (e2 != cudaSuccess) {
+        cudaError_t e = launch_ion_copy(c, r0, n, ion, to_device);
+        // also where a launch failed: those before it may still be moving the caller's records
+        const cudaError_t done = cudaStreamSynchronize(c.stream);
+        if (e == cudaSuccess) e = done;
+        if (e != cudaSuccess) {
             cudaGetLastError();
             return fail(ETHER_ERR_CUDA, std::string(to_device ? "ether_set_spins_batch: " : "ether_get_spins_batch: ") +
-                                            cudaGetErrorString(e2));
+                                            cudaGetErrorString(e));
         }
         c.ion_last_kernel[to_device ? 1 : 0] = n;
         return ETHER_OK;
