@@ -960,10 +960,19 @@ static int spins_batch(Ctx &c, int32_t r0, int32_t n, double *ion, bool to_devic
         return fail(ETHER_ERR_ARG, std::string(to_device ? "ether_set_spins_batch" : "ether_get_spins_batch") +
                                        ": ion is not host memory mapped for n replicas' records");
     const size_t per_rep = c.model == ETHER_MODEL_ISING ? (size_t)c.N : sizeof(float4) * c.N;
-    // a small call goes through the kernel alone: its threads and staging cost the shared form
-    // about 1.2 ms whatever the size
-    if (sizeof(double) * 9 * (size_t)c.N * n <= kKernelOnlyBytes) {
+    // a small call goes through the kernel alone: threads and staging cost the shared form about
+    // 1.2 ms whatever the size; unless this context has found its link slow (LinkChoice)
+    const size_t bytes = sizeof(double) * 9 * (size_t)c.N * n;
+    auto can_share = [&] { return n >= 2 && per_rep * (size_t)n <= kStageMax && host_threads() >= 2; };  // (20 us)
+    LinkChoice &link = c.ion_link[to_device ? 1 : 0];
+    if (bytes <= kKernelOnlyBytes && (link.kernel_alone(bytes) || !can_share())) {
+        const bool timed = link.time_it(bytes);
+        const auto t0 = std::chrono::steady_clock::now();
+        for (int k = 0; k < 2 && timed; ++k)
+            if (!c.ion_ev[k]) CUDA_TRY(cudaEventCreate(&c.ion_ev[k]));
+        if (timed) CUDA_TRY(cudaEventRecord(c.ion_ev[0], c.stream));
         cudaError_t e = launch_ion_copy(c, r0, n, ion, to_device);
+        if (timed && e == cudaSuccess) e = cudaEventRecord(c.ion_ev[1], c.stream);
         // also where a launch failed: those before it may still be moving the caller's records
         const cudaError_t done = cudaStreamSynchronize(c.stream);
         if (e == cudaSuccess) e = done;
@@ -972,10 +981,17 @@ static int spins_batch(Ctx &c, int32_t r0, int32_t n, double *ion, bool to_devic
             return fail(ETHER_ERR_CUDA, std::string(to_device ? "ether_set_spins_batch: " : "ether_get_spins_batch: ") +
                                             cudaGetErrorString(e));
         }
+        const double wall = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+        float ms = 0.f;
+        if (timed && cudaEventElapsedTime(&ms, c.ion_ev[0], c.ion_ev[1]) != cudaSuccess) {
+            cudaGetLastError();
+            ms = 0.f;
+        }
+        link.took(bytes, wall, ms);
         c.ion_last_kernel[to_device ? 1 : 0] = n;
         return ETHER_OK;
     }
-    if (n >= 2 && host_threads() >= 2 && per_rep * (size_t)n <= kStageMax) {
+    if (can_share()) {
         int nk = 0;
         const int rc = spins_shared(c, r0, n, ion, to_device, &nk);
         if (rc == ETHER_OK) c.ion_last_kernel[to_device ? 1 : 0] = nk;

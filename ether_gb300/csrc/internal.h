@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../include/ether_gpu.h"
+#include "link_choice.h"
 
 namespace ether {
 
@@ -137,6 +138,7 @@ struct Ctx {
     // in-place kernel and of the host's staged conversion, per direction (0 read-back, 1
     // upload), the replicas the kernel moved in the last call, and the kernel's timing events
     double ion_rate_k[2] = {0.0, 0.0}, ion_rate_h[2] = {0.0, 0.0};
+    LinkChoice ion_link[2];         // ... and of the link, for calls that the kernel alone may move
     int ion_last_kernel[2] = {0, 0};
     int ion_gets = 0;  // read-backs so far (the first three try the kernel, the cores, the kernel)
     cudaEvent_t ion_ev[2] = {nullptr, nullptr};
