@@ -203,7 +203,7 @@ int upload_ladder(Ctx &c) {
 void free_ctx(Ctx &c) {
     void *ptrs[] = {c.t.row_ptr, c.t.nbr, c.t.jidx, c.t.wstride, c.t.species, c.t.itype,
                     c.t.ell_nbr, c.t.ell_j, c.t.ell_deg, c.t.res_ent, c.t.res_order, c.t.J4, c.t.ell_ws, c.t.ell_desc, c.t.ell_class,
-                    c.t.type_base, c.t.type_half, c.t.J, c.t.Jd, c.t.zee, c.t.zeed, c.t.D,
+                    c.t.type_base, c.t.type_half, c.t.Jd, c.t.zee, c.t.zeed, c.t.D,
                     c.t.mweight, c.t.site_of_storage, c.spins, c.spins4, c.beta_slot,
                     c.beta_slot_f, c.slot_of_rep, c.rep_of_slot, c.thr, c.stream_id,
                     c.step, c.ovrr_step, c.fresh_call, c.acc_count, c.E, c.M, c.sums,
@@ -466,7 +466,6 @@ extern "C" int ether_create(const ether_desc *d, ether_ctx **out) {
     TRY(dev_upload(c, &c.t.itype, ity));
     TRY(dev_upload(c, &c.t.type_base, c.h_type_base));
     TRY(dev_upload(c, &c.t.type_half, c.h_type_half));
-    TRY(dev_upload(c, &c.t.J, c.h_Jf));
     TRY(dev_upload(c, &c.t.Jd, c.h_Jd));
     TRY(dev_upload(c, &c.t.zee, zee));
     TRY(dev_upload(c, &c.t.zeed, zeed));

@@ -54,7 +54,6 @@ struct DevTables {
     uint16_t *itype = nullptr;    // N (Ising table site type)
     int32_t *type_base = nullptr; // n_types: offset of a type's table inside one slot's table
     int32_t *type_half = nullptr; // n_types: entries per own-spin half
-    float *J = nullptr;           // nJ * 3 (FP32 couplings)
     double *Jd = nullptr;         // nJ * 3 (FP64 couplings, Ising energy)
     float *zee = nullptr;         // nsp * 3: -g mb s H
     double *zeed = nullptr;       // nsp * 3

@@ -43,13 +43,6 @@ __host__ __device__ constexpr int geo_ab(int k, int q) {
          : q == 4 ? (c == 0 ? 64 + a + 4 * b : -1)
                   : (c == 3 ? 80 + a + 4 * b : -1);
 }
-// Canonical coordinates of boundary site i (the inverse of the numbering above).
-__host__ __device__ inline void geo_bnd(int i, int &a, int &b, int &c) {
-    const int f = i >> 4, u = i & 3, v = (i >> 2) & 3, e = (f & 1) ? 4 : -1;
-    if (f < 2) { a = e; b = u; c = v; }
-    else if (f < 4) { a = u; b = e; c = v; }
-    else { a = u; b = v; c = e; }
-}
 
 __global__ void advance_lstep_kernel(uint32_t *c, int R);
 
