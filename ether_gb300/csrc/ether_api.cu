@@ -1166,9 +1166,13 @@ static int sweeps_by_phase(Ctx &c, int n) {
 }
 static int sweep_once(Ctx &c) { return sweeps_by_phase(c, 1); }
 
-// Do n sweeps of a simple-cubic Ising context run in shared memory?  Short runs of many sites do
-// not: loading and storing them costs more than the two phases (a sweep and its recorded row,
-// 16 x 52 x 16 x 722: 38 us in shared memory, 33 by phases; 16^3 x 1024 26 and 27).
+// Do n sweeps of a simple-cubic Ising context run in shared memory in a single call?  Short runs of
+// many sites do not: loading and storing them costs more than the two phases (a sweep and its
+// recorded row, 16 x 52 x 16 x 722: 38 us in shared memory, 33 by phases; 16^3 x 1024 26 and 27).
+// ether_mcs has no such rule: its launches make the energies of a swap too (a swap every step,
+// shared memory and phases: 16 x 52 x 16 x 722 33.1 and 36.8 us a step, 64 x 32 x 32 x 250 33.7 and
+// 32.6, 24^3 x 1000 54.2 and 53.8, 16^3 x 2048 25.1 and 49.5; every other step 19.7 and 25.6, 23.3
+// and 24.3, 34.9 and 40.5, 14.3 and 32.6).
 static bool ising_resident_runs(const Ctx &c, int n) {
     return c.resident && !c.variant_asked && (n >= 4 || (long)c.R * c.N <= (4L << 20) + (1L << 18));
 }

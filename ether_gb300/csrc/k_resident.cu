@@ -497,7 +497,8 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
         // two blocks, which both hold all spins, while all replicas still run at once and a colour is
         // more than a round of pairs (per sweep, before the slots' constant strides: 30 x 34 x 38 x 60
         // 31 us with one block, 18 with two; 23 x 21 x 19 16.6 and 9.0; 21 x 18 x 15 8.4 and 8.0; 14^3
-        // 3.4 and 3.8)
+        // 3.4 and 3.8; with them pyrochlore 12^3 39.8 and 27.7, 33 x 31 x 45 27.1 and 15.8, 29 x 27 x 25
+        // 13.4 and 10.7, 21 x 18 x 15 6.0 and 6.5)
         if (cs && 2L * c.R * 10 <= 9L * c.sm_count && res_share(c, 1, true) >= 2048) cs = 2;
     } else {
         // the smallest cluster that holds a replica; then larger ones while all replicas still run
@@ -514,6 +515,10 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
     // whole context's work over the GPU but at least a launch's latency per colour.  Measured per
     // site: here 0.3 ns + 0.07 per slot, and 1 us a colour (Ising), 1.0 + 0.1425 per slot (XYZ; 1.3 times that in a cluster); there,
     // over all replicas, 0.037 ns (Ising), 0.004 per slot - 0.008 (XYZ), and 3 us (4 us) a colour.
+    // The Ising terms are those of the kernel before its slots' constant strides; it takes 0.22 ns +
+    // 0.055 per slot and 0.9 us a colour now (152 replicas: 13^3 3.7 us, 29 x 27 x 25 13.4,
+    // pyrochlore 12^3 39.8), its phases 4.1 us a colour, so the line lies on the phases' side: a single
+    // pyrochlore 12^3 replica stays with them at 45 us where two blocks would take 28.
     if (cs) {
         const double waves = std::ceil((double)c.R * cs / c.sm_count), share = (double)c.N / cs, all = (double)c.N * c.R;
         const double here = ising ? 1.0 * c.ncol + waves * share * (0.3e-3 + 0.07e-3 * total)
