@@ -16,8 +16,10 @@
 // the tiles: Adam divides by the gradient's size, so after a few steps another order of the
 // batch sums moves the weights by 1e-3, through the BF16 roundings.  That rules a split of
 // the batch out (measured 12x against the 20 launches, with other weights).  As it stands a
-// step of 1024 rows of the XYZ network takes 53 us (580 before; train_rows 37 us and
-// train_wgrad 21 us with cold caches), latency of the chained sums and of the weights' loads.
+// step of 1024 rows of the XYZ network takes 53 us (580 before; train_rows 37-39 us and
+// train_wgrad 21-22 us with cold caches).  train_rows waits for its weights: of 12 warp cycles per
+// issue 7.7 are loads from the L2, each layer's begun when the layer before has ended (the chain of
+// 784 fmaf itself is about 2 us); train_wgrad has one warp a scheduler, short of parallel work.
 #pragma once
 #include <cuda_bf16.h>
 
