@@ -6,7 +6,7 @@
 namespace ether {
 
 // One direction of one context.  The kernel alone is the faster on a good link (16^3 x 190, 56 MB:
-// 0.24 ms up and 0.32 down, shared with the host's cores 1.36 and 1.53), but the link of some boxes
+// 0.24 ms up and 0.32 down, shared with the host's cores 1.36 and 1.53), but the link of some hosts
 // has been several times slower (27 GB/s of records), and then the cores are: 128 MB take about
 // 4.8 ms by the kernel and 2.5 shared (the estimate below).  A call whose wall time is above the
 // estimate -- its link may be slow, or it waited for sweeps -- has the next ones timed on the device
