@@ -464,6 +464,9 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
     const bool ising = c.model == ETHER_MODEL_ISING;
     if (c.N >= 65535) return;  // 16-bit entries; four blocks' shared memory holds fewer XYZ spins still
     if ((c.fast && ising) || c.nsp != 1 || c.nsh < 1 || c.nsh > (ising ? 4 : 8)) return;
+    if (!ising)  // a free slot adds its coupling times zero
+        for (float j : c.h_Jf)
+            if (!std::isfinite(j)) return;
     std::vector<int> slots(c.nsh, 0), count(c.nsh);
     std::vector<int> stride(c.nsh, 0);
     for (int s = 0; s < c.N; ++s) {
