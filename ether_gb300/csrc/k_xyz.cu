@@ -9,7 +9,11 @@ namespace ether {
 
 // ------------------------------------------------------------------ general lattice ----
 // One thread per rank of the colour class (xyz_ell_site); W: the class's ELL width at compile
-// time (0: at run time).
+// time (0: at run time).  Bound: latency of the neighbour loads.  With the counter from a read-only
+// load the compiler keeps all of a site's loads in flight (exchange only: 60 registers; 44 with a
+// plain load, and they wait in turns).  A sweep, plain and read-only: pyrochlore 12^3 x 1 38.0 and
+// 30.5 us, x 64 89.5 and 82.7; 20^3 fcc cells, 18 neighbours, x 1 73.8 and 59.0; bcc, 8, x 1 7.9 and
+// 6.3; 31 x 33 x 35 cubic x 64 37.8 both.  The run-time width loses by it (26 neighbours 127 and 132).
 template <int OPT, int W>
 __global__ void __launch_bounds__(256)
 xyz_ell_kernel(float4 *__restrict__ spins4, int N, int col_off, int n_c, uint32_t colour,
@@ -21,7 +25,7 @@ xyz_ell_kernel(float4 *__restrict__ spins4, int N, int col_off, int n_c, uint32_
     const int r = blockIdx.y;
     float4 *sp = spins4 + (size_t)r * N;
     const float beta_f = beta_slot_f[slot_of_rep[r]];
-    const uint32_t k1 = stream_id[r], t = step[r] + ahead;
+    const uint32_t k1 = stream_id[r], t = (W > 0 ? __ldg(step + r) : step[r]) + ahead;
     const uint32_t c3 = kMetro | (colour << 8);
     unsigned acc = 0;
     for (int rho = blockIdx.x * blockDim.x + threadIdx.x; rho < n_c; rho += gridDim.x * blockDim.x) {
