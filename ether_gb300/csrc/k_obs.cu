@@ -403,25 +403,56 @@ __device__ __forceinline__ void finish_block(const double *__restrict__ partials
     }
 }
 
+// The same where a replica has one block: its partials are the sums.  The whole block calls it, after
+// energy_block.  (An energy call, 8 x 4 x 4 x 60000: 632 us with the counter and the tree, 325 as two
+// launches, 187 so; 4^3 XYZ x 16384 205, 133, 82.)
+__device__ __forceinline__ void finish_alone(const double *__restrict__ partials, int R, int r, double *__restrict__ E,
+                                             double *__restrict__ M) {
+    __syncthreads();
+    const int j = threadIdx.x;
+    if (j < kNq) {
+        const double v = 0.0 + partials[(size_t)r * kNq + j];
+        if (j < 2) E[j * R + r] = v;
+        else M[3 * r + j - 2] = v;
+    }
+    __syncthreads();
+}
+
 // Row of a time series: |M| (and E) of every replica at row t, or at the row *t_dev (graph replays),
-// which the last replica to be written moves on.
+// which the last of `parts` parts to be written moves on.  Up to kRowReplicas replicas the reduction's
+// own launch writes it, a replica a part; more of them would wait for the parts' counter and for a
+// lone thread's root, and get a launch of their own, a block of replicas a part (a sweep and its row,
+// in one launch and so, 16^3 x 4000 51 and 46 us; 5^3 x 10000 74 and 60; in the other direction
+// 8 x 4 x 4 x 128 9.4 and 11.1).
 struct RecordRow {
     double *m, *e;     // series, null: not recorded
     int t;
     int32_t *t_dev;
 };
-// By one thread, once the replica's M (and E) are summed; done: a counter of replicas.
-__device__ __forceinline__ void record_replica(const RecordRow &row, int R, int r, double mx, double my, double mz,
-                                               double e, uint32_t *done) {
-    const int t = row.t_dev ? *(volatile int32_t *)row.t_dev : row.t;
+constexpr int kRowReplicas = 512;
+__device__ __forceinline__ int record_row(const RecordRow &row) {
+    return row.t_dev ? *(volatile int32_t *)row.t_dev : row.t;
+}
+__device__ __forceinline__ void record_replica(const RecordRow &row, int t, int R, int r, double mx, double my, double mz,
+                                               double e) {
     row.m[(size_t)t * R + r] = sqrt(mx * mx + my * my + mz * mz);
     if (row.e) row.e[(size_t)t * R + r] = e;
+}
+// By one thread of a part, once the part's replicas are written; done: a counter of parts.
+__device__ __forceinline__ void record_done(const RecordRow &row, int t, int parts, uint32_t *done) {
     if (!row.t_dev) return;
     __threadfence();
-    if (atomicAdd(done, 1u) == (uint32_t)R - 1u) {
+    if (atomicAdd(done, 1u) == (uint32_t)parts - 1u) {
         *done = 0u;
         *row.t_dev = t + 1;
     }
+}
+__global__ void __launch_bounds__(kRedBs) record_kernel(const double *__restrict__ E, const double *__restrict__ M, int R,
+                                                         const RecordRow row, uint32_t *__restrict__ done) {
+    const int r = blockIdx.x * kRedBs + threadIdx.x, t = record_row(row);
+    if (r < R) record_replica(row, t, R, r, M[3 * r], M[3 * r + 1], M[3 * r + 2], row.e ? E[r] : 0.0);
+    __syncthreads();
+    if (threadIdx.x == 0) record_done(row, t, gridDim.x, done);
 }
 
 // One block per (replica, energy block); the block of a replica that ends last sums the
@@ -435,23 +466,31 @@ __global__ void __launch_bounds__(kRedBs, 4) energy_mag_kernel(const ObsMember a
                                                                 double *host_e, double *host_m, const RecordRow row) {
     const int r = blockIdx.y;
     energy_block<FORM>(a, r, blockIdx.x);
-    __shared__ int s_last;
-    if (threadIdx.x < 32) {  // the partials' writers are in the first warp
+    if (gridDim.x == 1) {
+        finish_alone(a.partials, a.R, r, a.E, a.M);
+    } else {
+        __shared__ int s_last;
+        if (threadIdx.x < 32) {  // the partials' writers are in the first warp
+            __threadfence();
+            __syncwarp();
+            if (threadIdx.x == 0) s_last = atomicAdd(done + r, 1u) == gridDim.x - 1u;
+        }
+        __syncthreads();
+        if (!s_last) return;
         __threadfence();
-        __syncwarp();
-        if (threadIdx.x == 0) s_last = atomicAdd(done + r, 1u) == gridDim.x - 1u;
+        finish_block(a.partials, a.nblk, a.R, r, a.E, a.M);
+        if (threadIdx.x == 0) done[r] = 0u;
     }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    finish_block(a.partials, a.nblk, a.R, r, a.E, a.M);
     if (threadIdx.x == 0) {
-        done[r] = 0u;
         if (measure) measure_one(a.E, a.M, a.N, a.n_slots, a.slot_of_rep, a.sums, r);
         if (host_e) host_e[r] = a.E[r];
         if (host_m)
             for (int j = 0; j < 3; ++j) host_m[3 * r + j] = a.M[3 * r + j];
-        if (row.m) record_replica(row, a.R, r, a.M[3 * r], a.M[3 * r + 1], a.M[3 * r + 2], a.E[r], done + a.R);
+        if (row.m) {
+            const int t = record_row(row);
+            record_replica(row, t, a.R, r, a.M[3 * r], a.M[3 * r + 1], a.M[3 * r + 2], a.E[r]);
+            record_done(row, t, a.R, done + a.R);
+        }
     }
 }
 
@@ -616,15 +655,14 @@ cudaError_t launch_energy_mag(Ctx &c, bool measure, double *host_e, double *host
 }
 
 // Magnetisation only (src/get_tot_magnetisation.f90:32-40), no neighbour reads: per-block
-// partial sums of w_s S_s into partials[(r*nblk + b)*kNq + 2..4], summed per thread and
-// warp as energy_block sums them (so the two give the same M).
-__device__ __forceinline__ void mag_block(const ObsMember &a, int r) {
+// partial sums of w_s S_s into out[0..2], summed per thread and warp as energy_block sums them (so
+// the two give the same M).
+__device__ __forceinline__ void mag_block(const ObsMember &a, int r, double *out) {
     const int N = a.N;
     const int stride = gridDim.x * blockDim.x;
     double q[3] = {0, 0, 0};
     DS qd[3];
     int form = kFormDouble;
-    double *out = a.partials + ((size_t)r * gridDim.x + blockIdx.x) * kNq + 2;
     if (a.model == 0 && a.count_form) {
         const uint8_t *sp = a.spins + (size_t)r * N;
         int cm = 0;
@@ -687,37 +725,65 @@ __device__ __forceinline__ void mag_block(const ObsMember &a, int r) {
     }
     block_sum_mixed<3>(q, qd, form == kFormDS ? 3 : 0, out);
 }
-// The block of a replica that ends last sums its partials in block order and records the row.
+// The block of a replica that ends last sums its partials in block order and records the row; a
+// replica's only block keeps its sums in shared memory.
 __global__ void __launch_bounds__(kRedBs) mag_kernel(const ObsMember a, uint32_t *__restrict__ done, const RecordRow row) {
     const int r = blockIdx.y;
-    mag_block(a, r);
     __shared__ int s_last;
     __shared__ double s_m[3];
-    if (threadIdx.x < 32) {  // the partials' writers are in the first warp
+    const bool alone = gridDim.x == 1;
+    mag_block(a, r, alone ? s_m : a.partials + ((size_t)r * gridDim.x + blockIdx.x) * kNq + 2);
+    if (!alone) {
+        if (threadIdx.x < 32) {  // the partials' writers are in the first warp
+            __threadfence();
+            __syncwarp();
+            if (threadIdx.x == 0) s_last = atomicAdd(done + r, 1u) == gridDim.x - 1u;
+        }
+        __syncthreads();
+        if (!s_last) return;
         __threadfence();
-        __syncwarp();
-        if (threadIdx.x == 0) s_last = atomicAdd(done + r, 1u) == gridDim.x - 1u;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    if (threadIdx.x < 3) {
+        if (threadIdx.x == 0) done[r] = 0u;
+        // added in block order by three threads; many are fetched by all threads first (90 blocks,
+        // 33 x 31 x 45 x 1: a row 27.4 us so, 29.4 where the three fetch them)
+        constexpr int kStage = 64;
+        __shared__ double s_p[kStage][3];
         double v = 0.0;
-        for (int b = 0; b < (int)gridDim.x; ++b) v += __ldcg(&a.partials[((size_t)r * gridDim.x + b) * kNq + 2 + threadIdx.x]);
-        a.M[3 * r + threadIdx.x] = s_m[threadIdx.x] = v;
+        if (gridDim.x <= 32 && threadIdx.x < 3)
+            for (int b = 0; b < (int)gridDim.x; ++b) v += __ldcg(&a.partials[((size_t)r * gridDim.x + b) * kNq + 2 + threadIdx.x]);
+        for (int b0 = 0; b0 < (int)gridDim.x && gridDim.x > 32; b0 += kStage) {
+            const int nb = min(kStage, (int)gridDim.x - b0);
+            for (int i = threadIdx.x; i < 3 * nb; i += kRedBs)
+                s_p[i / 3][i % 3] = __ldcg(&a.partials[((size_t)r * gridDim.x + b0 + i / 3) * kNq + 2 + i % 3]);
+            __syncthreads();
+            if (threadIdx.x < 3)
+                for (int b = 0; b < nb; ++b) v += s_p[b][threadIdx.x];
+            __syncthreads();
+        }
+        if (threadIdx.x < 3) s_m[threadIdx.x] = v;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        done[r] = 0u;
-        record_replica(row, a.R, r, s_m[0], s_m[1], s_m[2], 0.0, done + a.R);
+    if (threadIdx.x < 3) a.M[3 * r + threadIdx.x] = 0.0 + s_m[threadIdx.x];
+    if (threadIdx.x == 0 && row.m) {
+        const int t = record_row(row);
+        record_replica(row, t, a.R, r, 0.0 + s_m[0], 0.0 + s_m[1], 0.0 + s_m[2], 0.0);
+        record_done(row, t, a.R, done + a.R);
     }
 }
 
-// One row of the time series, in the reduction's own launch.
+// One row of the time series.
 cudaError_t launch_record(Ctx &c, int t, bool want_e, double *mser, double *eser, int32_t *t_dev) {
-    const RecordRow row{mser, want_e ? eser : nullptr, t, t_dev};
-    if (want_e) return launch_energy(c, false, nullptr, nullptr, row);
-    mag_kernel<<<dim3(c.partial_blocks, c.R), kRedBs, 0, c.stream>>>(obs_member(c), c.obs_done, row);
+    const RecordRow row{mser, want_e ? eser : nullptr, t, t_dev}, none{nullptr, nullptr, 0, nullptr};
+    const bool own = c.R > kRowReplicas;
+    cudaError_t e = cudaSuccess;
+    if (want_e) {
+        e = launch_energy(c, false, nullptr, nullptr, own ? none : row);
+    } else {
+        mag_kernel<<<dim3(c.partial_blocks, c.R), kRedBs, 0, c.stream>>>(obs_member(c), c.obs_done, own ? none : row);
+        c.launches++;
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess || !own) return e;
+    record_kernel<<<(c.R + kRedBs - 1) / kRedBs, kRedBs, 0, c.stream>>>(c.E, c.M, c.R, row, c.obs_done + c.R);
     c.launches++;
     return cudaGetLastError();
 }
