@@ -1148,7 +1148,7 @@ extern "C" int ether_fresh_spins(ether_ctx *h) {
 
 // Does the context's resident sweep of k_resident.cu run in a single call?  (A variant that was
 // named is a phase kernel's.  ether_mcs asks neither this nor ising_resident_runs: its route, and so
-// its graphs, depend on the context alone.)
+// its graphs, depend on the context and the lengths of the runs alone.)
 static bool general_resident(const Ctx &c) { return c.gen_resident && !(c.fast && c.variant_asked); }
 
 // n sweeps phase by phase; the counters are advanced once, after the last (a launch less per sweep).
@@ -1174,13 +1174,22 @@ static int sweep_once(Ctx &c) { return sweeps_by_phase(c, 1); }
 // 32.6, 24^3 x 1000 54.2 and 53.8, 16^3 x 2048 25.1 and 49.5; every other step 19.7 and 25.6, 23.3
 // and 24.3, 34.9 and 40.5, 14.3 and 32.6).
 static bool ising_resident_runs(const Ctx &c, int n) {
-    return c.resident && !c.variant_asked && (n >= 4 || (long)c.R * c.N <= (4L << 20) + (1L << 18));
+    return c.resident && !c.variant_asked &&
+           (n >= 4 || ising_resident_tiny(c, n) || (long)c.R * c.N <= (4L << 20) + (1L << 18));
+}
+
+// Are n sweeps on a context's general resident sweep better off by phases?  Only where a graph
+// replays them.
+static bool phases_pay(const Ctx &c, int n) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return !general_resident_pays(c, n) && cudaStreamIsCapturing(c.stream, &st) == cudaSuccess &&
+           st == cudaStreamCaptureStatusActive;
 }
 
 // n sweeps: in the launches of a resident kernel (of at most 256 sweeps each) or phase by phase.
 int ether::plain_sweeps(Ctx &c, int n) {
     const bool resident = ising_resident_runs(c, n);
-    if (!resident && !general_resident(c)) return sweeps_by_phase(c, n);
+    if (!resident && (!general_resident(c) || phases_pay(c, n))) return sweeps_by_phase(c, n);
     for (int k = 0; k < n; k += 256) {
         const int m = std::min(256, n - k);
         CUDA_TRY(resident ? launch_ising_resident(c, m) : launch_general_resident(c, m));
@@ -1575,13 +1584,20 @@ static int issue_steps(Ctx &c, const ether_schedule *sch, const int8_t *sig, int
         return ETHER_OK;
     }
     // runs of sweeps that no OVRR, PT or measurement separates: one resident launch each
-    auto run = [&](int m) { return c.resident ? launch_ising_resident(c, m) : launch_general_resident(c, m); };
     for (int k = 0; k < n;) {
         int rc = mcs_before_sweep(c, sch, sig[k]);
         if (rc) return rc;
         int j = k + 1;
         while (j < n && !(sig[j - 1] & 6) && !(sig[j] & 1)) ++j;
-        CUDA_TRY(run(j - k));
+        const int m = j - k;
+        if (c.resident) {
+            CUDA_TRY(launch_ising_resident(c, m));
+        } else if ((c.fast || c.R < 16) && phases_pay(c, m)) {  // (more replicas would want them in parts)
+            rc = sweeps_by_phase(c, m);
+            if (rc) return rc;
+        } else {
+            CUDA_TRY(launch_general_resident(c, m));
+        }
         rc = mcs_after_sweep(c, sig[j - 1]);
         if (rc) return rc;
         k = j;

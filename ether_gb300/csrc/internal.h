@@ -258,11 +258,14 @@ cudaError_t launch_ising_resident(Ctx &c, int nsweeps, const ResidentEvents &ev 
 bool ising_resident_measures(const Ctx &c);  // may the launch measure?
 bool ising_counts(const Ctx &c);             // Ising sums by integer counts
 bool ising_resident_in_registers(const Ctx &c);
+bool ising_resident_tiny(const Ctx &c, int n);
 // k_resident.cu
 void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &row_ptr, const std::vector<int32_t> &nbr,
                            const std::vector<uint16_t> &jidx, const std::vector<int32_t> &wstride,
                            std::vector<uint4> &ent, std::vector<int32_t> &order);
 cudaError_t prepare_general_resident(const Ctx &c);
+// Do n sweeps take less time in shared memory than by phases where a graph replays the launches?
+bool general_resident_pays(const Ctx &c, int n);
 // ratio: takes the launch's acceptance per replica, or null
 cudaError_t launch_general_resident(Ctx &c, int nsweeps, double *ratio = nullptr);
 bool ising_staged_shape(const Ctx &c, int vectors_per_step);

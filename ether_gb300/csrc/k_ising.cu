@@ -421,6 +421,11 @@ bool ising_resident_possible(const Ctx &c, size_t smem_max) {
     // (W/4) ceil(nvec/256) flips per byte of a vector count must stay below 256
     return bytes <= smem_max && (c.vec_bytes / 4) * ((resident_vectors(c, c.vec_bytes) + 255) / 256) < 256;
 }
+// Replicas of so few vectors that a phase kernel's blocks mostly fill their table: n sweeps are better
+// off in shared memory (a sweep and |M|, shared memory and phases, us: 8^3 x 9000 54.7 and 69.7, x
+// 30000 151 and 197, 16 x 8 x 12 x 10000 66 and 87; 16^3 x 4000, 256 vectors, 50 and 50, two sweeps 58
+// and 76; 24 x 16 x 16 x 2500, 768, 75 and 51).
+bool ising_resident_tiny(const Ctx &c, int n) { return resident_vectors(c, c.vec_bytes) <= (n > 1 ? 256 : 128); }
 bool ising_resident_in_registers(const Ctx &c) { return resident_vectors(c, c.vec_bytes) <= 2048; }
 
 // Vectors in registers up to two per thread of the largest block.

@@ -585,6 +585,26 @@ void plan_general_resident(Ctx &c, size_t smem_max, const std::vector<int32_t> &
     c.gen_resident = cs;
 }
 
+// A graph replays launches 2.1 us apart and more (the calls that launch directly, 4.1), so there a short run
+// of a few large replicas is better off by phases: no load and store of all spins, no cluster
+// barriers.  Fitted to the rows of series (a sweep and |M|), shared memory and phases, us: Ising
+// 29 x 27 x 25 x 1 27.6 and 19.6 (four sweeps a row 58.3 and 46.9), 21 x 18 x 15 x 1 19.4 and 17.7 (two
+// sweeps 25.6 and 26.1), 9^3 x 1 13.1 and 15.6; XYZ 16^3 x 16 19.5 and 17.5 (four 31.3 and 32.2), 16^3 x
+// 64 21.6 and 19.7 (three 33.3 and 36.3), 20^3 x 1 19.4 and 15.4 (four 37.9 and 30.0), 8^3 x 1 11.3
+// and 12.2; pyrochlore 8^3 Ising x 8, 18 neighbours, 32.1 and 39.1.
+bool general_resident_pays(const Ctx &c, int n) {
+    const bool ising = c.model == ETHER_MODEL_ISING;
+    const int cs = c.gen_resident, slots = c.res_slots;
+    const double share = (double)c.N / cs, waves = std::ceil((double)c.R * cs / c.sm_count);
+    const double barrier = (ising ? 0.6 : 0.6 * 0.95) * (cs > 1 ? 2.0 : 1.0);
+    const double site = (ising ? 0.22e-3 + 0.055e-3 * slots : 0.35e-3 + 0.15e-3 * slots) * (!ising && cs > 1 ? 1.5 : 1.0);
+    const double once = ising ? 2.3 + 0.25e-3 * c.N : 0.5 + 1.2e-3 * share + (cs > 1 ? 1.0 : 0.0);
+    const double here = once + n * (barrier * c.ncol + waves * share * site);
+    const double launch = ising ? 1.6 + 0.083 * slots : c.fast ? 2.1 : 2.0 + 0.1 * slots, size = ising ? 0.04e-3 : c.fast ? 0.03e-3 : 0.26e-3;
+    const double rate = ising ? 0.011e-3 : c.fast ? 0.016e-3 : 0.026e-3;
+    return here <= n * (launch * c.ncol + size * c.N + rate * c.N * c.R);
+}
+
 // Opts the context's kernel into its shared memory (once, at creation: not during a capture).
 cudaError_t prepare_general_resident(const Ctx &c) { return allow_shared(res_kernel(c, c.gen_resident)); }
 
