@@ -916,7 +916,11 @@ int launch_patches(ether_learn &l, int cls, float *dump) {
         const int tiles = (P.n + kThreads - 1) / kThreads;
         LCUDA(launch_after(gather_kernel, (P.n + 255) / 256, 256, 0, c.stream, true, P));
         LCUDA(launch_after(patch_kernel<0>, std::min(tiles, l.sm_count), kGroups * kThreads, SM_BYTES + 1024, c.stream, true, P));
-        LCUDA(launch_after(mh_kernel, (P.n + 127) / 128, 128, 0, c.stream, true, P));
+        // mh_kernel follows closely only where an SM is free for each of its blocks: the network's
+        // blocks fill an SM's registers, so blocks that start beside them crowd on the few SMs left
+        // and stay there (a class of 32^3 x 64, 128 tiles: 37 us closely, 25 so; x 100 38 and 27;
+        // 64^3 x 32 45 and 36; 16^3 x 16, four tiles, 21 and 23)
+        LCUDA(launch_after(mh_kernel, (P.n + 127) / 128, 128, 0, c.stream, 2 * tiles <= l.sm_count, P));
         l.launches += 3;
     }
     LCUDA(cudaGetLastError());
