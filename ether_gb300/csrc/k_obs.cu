@@ -422,8 +422,8 @@ __device__ __forceinline__ void finish_alone(const double *__restrict__ partials
 // which the last of `parts` parts to be written moves on.  Up to kRowReplicas replicas the reduction's
 // own launch writes it, a replica a part; more of them would wait for the parts' counter and for a
 // lone thread's root, and get a launch of their own, a block of replicas a part (a sweep and its row,
-// in one launch and so, 16^3 x 4000 51 and 46 us; 5^3 x 10000 74 and 60; in the other direction
-// 8 x 4 x 4 x 128 9.4 and 11.1).
+// in one launch and so, 16^3 x 4000 51 and 46 us; 5^3 x 10000 74 and 60; the other way round
+// 8^3 XYZ x 64 11.0 and 13.1).
 struct RecordRow {
     double *m, *e;     // series, null: not recorded
     int t;
